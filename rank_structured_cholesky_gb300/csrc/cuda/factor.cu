@@ -688,11 +688,16 @@ void FactorEngine<T>::plan() {
     if (!nd.compressed || nd.m() == 0) continue;
     const int r = S.offRank[j], m = nd.m(), n = nd.n;
     rank[j] = r;
-    vOff[j] = curV; curV += (long long)m * r;
-    uOff[j] = curV; curV += (long long)n * r;
-    qOff[j] = curV; curV += (long long)r * r;
-    xOff[j] = curV; curV += (long long)m * r;
-    gmOff[j] = curV; curV += (long long)n * r + r;   // Householder QR scratch
+    auto take = [&](long long e) {   // 16-byte boundaries: the apply's bulk copies of V start on one
+      const long long at = curV;
+      curV = (curV + e + 3) & ~3LL;
+      return at;
+    };
+    vOff[j] = take((long long)m * r);
+    uOff[j] = take((long long)n * r);
+    qOff[j] = take((long long)r * r);
+    xOff[j] = take((long long)m * r);
+    gmOff[j] = take((long long)n * r + r);   // Householder QR scratch
   }
   // HODLR internal-node buffers, per internal node (rows x cols block, rank r):
   // V (rows*r) | Y/U (cols*r) | X (rows*r) | QR scratch (cols*r + r) |

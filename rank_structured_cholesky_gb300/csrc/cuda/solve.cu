@@ -1,4 +1,5 @@
 #include <algorithm>
+#include <climits>
 #include <mutex>
 #include <cstdlib>
 #include <type_traits>
@@ -12,629 +13,915 @@ namespace {
 
 using namespace solvedev;
 
-// out[k] = sum_{i < rows} M[i][k] v[i] (v == nullptr: v[i] = 1, and M was
-// written by other blocks of this launch, so its loads bypass L1) for k < r,
-// M row-major with leading dimension ld.  Eight warps split the rows, lanes
-// run along k (coalesced), and the eight warp partials are added in a fixed
-// order.  blockDim.x == 256; red: 8 x 256 shared; every thread must call it.
-template <class T>
-__device__ void rows_t_gemv(const T* __restrict__ M, int ld, int rows, int r, const T* v, T* out, T (*red)[256]) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int k0 = 0; k0 < r; k0 += 256) {
-    T acc[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) acc[c] = T(0);
-    for (int i = warp; i < rows; i += 8) {
-      const T vi = v ? v[i] : T(1);
-      const T* row = M + (size_t)i * ld + k0;
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        if (k0 + lane + 32 * c < r) acc[c] += (v ? row[lane + 32 * c] : __ldcg(row + lane + 32 * c)) * vi;
-    }
-#pragma unroll
-    for (int c = 0; c < 8; ++c) red[warp][lane + 32 * c] = acc[c];
-    __syncthreads();
-    if (k0 + (int)threadIdx.x < r) {
-      T s = T(0);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) s += red[q][threadIdx.x];
-      out[k0 + threadIdx.x] = s;
-    }
-    __syncthreads();
-  }
+// 16-byte vectors of the factor's type.
+template <class T> struct Vec16;
+template <> struct Vec16<float> {
+  using type = float4;
+  static constexpr int V = 4;
+};
+template <> struct Vec16<double> {
+  using type = double2;
+  static constexpr int V = 2;
+};
+__device__ __forceinline__ float vdot(float4 a, float4 b, float s) {
+  return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s))));
 }
-
-// f := L^{-1} f with the inverted 64 x 64 diagonal blocks of L (block b:
-// h_b x h_b row-major at D + 4096 b; only the last block can be smaller).
-// f (n) and t (64) in shared memory.  A warp per row: loads coalesced along
-// the row of L or D.
-template <class T>
-__device__ void trsv_dinv(const T* __restrict__ L, int ld, int n, const T* __restrict__ D, T* f, T* t) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  for (int i0 = 0; i0 < n; i0 += 64) {
-    const int h = min(64, n - i0);
-    for (int i = warp; i < h; i += nwarp) {
-      const T* row = L + (size_t)(i0 + i) * ld;
-      T s = T(0);
-      for (int j = lane; j < i0; j += 32) s += row[j] * f[j];
-      s = warp_sum(s);
-      if (lane == 0) t[i] = f[i0 + i] - s;
-    }
-    __syncthreads();
-    const T* Db = D + (size_t)i0 * 64;
-    for (int i = warp; i < h; i += nwarp) {
-      const T* row = Db + (size_t)i * h;
-      T s = T(0);
-      for (int j = lane; j <= i; j += 32) s += row[j] * t[j];
-      s = warp_sum(s);
-      if (lane == 0) f[i0 + i] = s;
-    }
-    __syncthreads();
-  }
+__device__ __forceinline__ double vdot(double2 a, double2 b, double s) { return fma(a.y, b.y, fma(a.x, b.x, s)); }
+__device__ __forceinline__ void vaxpy(float4& acc, float4 a, float x) {
+  acc.x = fmaf(a.x, x, acc.x);
+  acc.y = fmaf(a.y, x, acc.y);
+  acc.z = fmaf(a.z, x, acc.z);
+  acc.w = fmaf(a.w, x, acc.w);
 }
-
-// f := L^{-T} f with the same inverted diagonal blocks.  red: 4 x 64 shared.
-template <class T>
-__device__ void trsv_dinv_t(const T* __restrict__ L, int ld, int n, const T* __restrict__ D, T* f, T* t,
-                            T (*red)[64]) {
-  const int c = threadIdx.x & 63, grp = threadIdx.x >> 6, ngrp = blockDim.x >> 6;
-  if (n <= 0) return;
-  for (int i0 = ((n - 1) / 64) * 64; i0 >= 0; i0 -= 64) {
-    const int h = min(64, n - i0);
-    T s = T(0);
-    if (c < h)
-      for (int i = i0 + h + grp; i < n; i += ngrp) s += L[(size_t)i * ld + i0 + c] * f[i];
-    red[grp][c] = s;
-    __syncthreads();
-    if (threadIdx.x < h) {
-      T u = T(0);
-      for (int g = 0; g < ngrp; ++g) u += red[g][threadIdx.x];
-      t[threadIdx.x] = f[i0 + threadIdx.x] - u;
-    }
-    __syncthreads();
-    if (threadIdx.x < h) {
-      const T* Db = D + (size_t)i0 * 64;
-      T x = T(0);
-      for (int i = threadIdx.x; i < h; ++i) x += Db[(size_t)i * h + threadIdx.x] * t[i];
-      f[i0 + threadIdx.x] = x;
-    }
-    __syncthreads();
-  }
+__device__ __forceinline__ void vaxpy(double2& acc, double2 a, double x) {
+  acc.x = fma(a.x, x, acc.x);
+  acc.y = fma(a.y, x, acc.y);
 }
-
-// Small interior supernodes (n <= IW_N, m <= ICH: one chunk) take a warp
-// each, eight to a block, so the thousands of bottom-level supernodes do not
-// each pay a block's scheduling, ticket and barrier latencies.  (Widening
-// this to n <= 64, m <= 320 -- a warp per supernode of the next two levels --
-// measured slower on c2: 1.15 vs 0.92 ms per apply; to m <= 192, the same.)  The steps and
-// the waits are those of a chunk block below; the per-warp shared buffers
-// hold f (IW_N) and the update vector (ICH).
-constexpr int IW_N = 32;
-
-template <class T>
-__device__ void interior_forward_warp(const SNode<T>* __restrict__ nodes, int s, const int* __restrict__ rel,
-                                      const int* __restrict__ child, int* sync, int epoch, const T* w, T* yout, T* wu,
-                                      T* f, T* u) {
-  const int lane = threadIdx.x & 31;
-  int* err = sync;
-  const SNode<T>& nd = nodes[s];
-  const int n = nd.n, m = nd.m;
-  for (int c = nd.childBegin; c < nd.childEnd; ++c) {   // every child has stored its update vector
-    const SNode<T>& cn = nodes[child[c]];
-    if (!wait_geq(sync + cn.syncOff + 1, epoch * max(1, cn.nch), err)) break;
-  }
-  if (lane < n) f[lane] = w[nd.c0 + lane];
-  for (int a = lane; a < m; a += 32) u[a] = T(0);
-  __syncwarp();
-  for (int c = nd.childBegin; c < nd.childEnd; ++c) {   // children's update vectors, in child order
-    const SNode<T>& cn = nodes[child[c]];
-    const T* wuc = wu + cn.wuOff;
-    const int* rl = rel + cn.relOff;
-    for (int a = lane; a < cn.m; a += 32) {
-      const int t = rl[a];
-      const T v = __ldcg(wuc + a);
-      if (t < n) f[t] += v;
-      else u[t - n] += v;
-    }
-    __syncwarp();
-  }
-  // y = L11^{-1} f through the inverted diagonal block (n x n, row-major)
-  T y = T(0);
-  if (lane < n)
-    for (int j = 0; j <= lane; ++j) y += nd.Dinv[lane * n + j] * f[j];
-  __syncwarp();
-  if (lane < n) {
-    f[lane] = y;
-    yout[nd.c0 + lane] = y;
-  }
-  __syncwarp();
-  T* wud = wu + nd.wuOff;
-  for (int a = lane; a < m; a += 32) {   // u_a -= L21[a] . y
-    const T* row = nd.L + (size_t)(n + a) * nd.ld;
-    T acc = T(0);
-    for (int j = 0; j < n; ++j) acc += row[j] * f[j];
-    wud[a] = u[a] - acc;
-  }
-  __syncwarp();
-  if (lane == 0) {
-    __threadfence();
-    atomicAdd(sync + nd.syncOff + 1, 1);
-  }
+__device__ __forceinline__ void vadd(float4& a, float4 b) {
+  a.x += b.x;
+  a.y += b.y;
+  a.z += b.z;
+  a.w += b.w;
 }
-
-template <class T>
-__device__ void interior_backward_warp(const SNode<T>* __restrict__ nodes, int s, const int* __restrict__ rows,
-                                       int* sync, int epoch, const T* yin, T* w, T* f, T* xr) {
-  const int lane = threadIdx.x & 31;
-  int* err = sync;
-  const SNode<T>& nd = nodes[s];
-  const int n = nd.n, m = nd.m;
-  if (nd.parentI >= 0) wait_geq(sync + nodes[nd.parentI].syncOff + 2, epoch, err);   // ancestors solved
-  const int* rw = rows + nd.rowsOff;
-  for (int a = lane; a < m; a += 32) xr[a] = __ldcg(w + rw[a]);
-  __syncwarp();
-  T t = T(0);   // f_j = y_j - (L21^T x_R)_j, lanes over the columns
-  if (lane < n) {
-    for (int a = 0; a < m; ++a) t += nd.L[(size_t)(n + a) * nd.ld + lane] * xr[a];
-    f[lane] = yin[nd.c0 + lane] - t;
-  }
-  __syncwarp();
-  T x = T(0);   // x = L11^{-T} f: x_i = sum_{k >= i} D_ki f_k
-  if (lane < n) {
-    for (int k = lane; k < n; ++k) x += nd.Dinv[k * n + lane] * f[k];
-    w[nd.c0 + lane] = x;
-  }
-  __syncwarp();
-  if (lane == 0) {
-    __threadfence();
-    st_release(sync + nd.syncOff + 2, epoch);   // x of this supernode is final
-  }
+__device__ __forceinline__ void vadd(double2& a, double2 b) {
+  a.x += b.x;
+  a.y += b.y;
 }
-
-// Interior supernodes: all levels in one launch per direction.  A block takes
-// the next (supernode, 128-row chunk of its off-diagonal rows) from a ticket
-// counter, in level order, so it only waits on blocks that started before it:
-// forward, on the chunk blocks of the supernode's children (per-supernode
-// completion counters that grow by one per chunk); backward, on the solve of
-// its interior parent (a flag set to 1).  The apply's last kernel clears the
-// counters (clear_piece), so every apply starts from zeros with no host
-// state and the same launches replay unchanged inside a CUDA graph.  Every
-// chunk block assembles and solves the supernode's own n columns (n is
-// small); chunk 0 stores y.
-
-template <class T>
-__global__ void __launch_bounds__(256) interior_forward_chunks(const SNode<T>* __restrict__ nodes,
-                                                               const RowBlock* __restrict__ work,
-                                                               const int* __restrict__ rel,
-                                                               const int* __restrict__ child,
-                                                               int* __restrict__ sync, int epoch,
-                                                               const T* __restrict__ w, T* __restrict__ yout,
-                                                               T* __restrict__ wu, const int* __restrict__ small) {
-  pdl_enter();
-  extern __shared__ __align__(16) unsigned char smraw[];
-  T* f = reinterpret_cast<T*>(smraw);
-  __shared__ T tb[64];
-  __shared__ int sTicket;
-  int* err = sync;
-  if (threadIdx.x == 0) sTicket = atomicAdd(&sync[SYNC_TICK_F], 1);
-  __syncthreads();
-  if (sTicket >= (int)gridDim.x) {   // counters not reset: report, touch nothing
-    if (threadIdx.x == 0) atomicExch(err, 2);
-    return;
-  }
-  const RowBlock wk = work[sTicket];
-  if (wk.node < 0) {   // a group of small supernodes (node = -1 - group, b = count), a warp each
-    const int warp = threadIdx.x >> 5;
-    if (warp < wk.b)
-      interior_forward_warp<T>(nodes, small[8 * (-1 - wk.node) + warp], rel, child, sync, epoch, w, yout, wu,
-                               f + warp * (IW_N + ICH), f + warp * (IW_N + ICH) + IW_N);
-    launch_done(&sync[SYNC_TICK_F], &sync[SYNC_DONE_F]);
-    return;
-  }
-  const SNode<T>& nd = nodes[wk.node];
-  const int n = nd.n, a0 = wk.b * ICH, a1 = min(nd.m, a0 + ICH);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  T* wud = wu + nd.wuOff;
-  if (warp == 0)   // every chunk block of every child has stored its update rows
-    for (int c = nd.childBegin; c < nd.childEnd; ++c) {
-      const SNode<T>& cn = nodes[child[c]];
-      if (!wait_geq(sync + cn.syncOff + 1, epoch * max(1, cn.nch), err)) break;
-    }
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) f[i] = w[nd.c0 + i];
-  for (int a = a0 + threadIdx.x; a < a1; a += blockDim.x) wud[a] = T(0);
-  __syncthreads();
-  // children's update vectors, in child order
-  for (int c = nd.childBegin; c < nd.childEnd; ++c) {
-    const SNode<T>& cn = nodes[child[c]];
-    const T* wuc = wu + cn.wuOff;
-    const int* rl = rel + cn.relOff;
-    for (int a = threadIdx.x; a < cn.m; a += blockDim.x) {
-      const int t = rl[a];
-      if (t < n) f[t] += __ldcg(wuc + a);
-      else if (t - n >= a0 && t - n < a1) wud[t - n] += __ldcg(wuc + a);
-    }
-    __syncthreads();
-  }
-  trsv_dinv<T>(nd.L, nd.ld, n, nd.Dinv, f, tb);
-  // y goes to a separate vector: the other chunk blocks still read w
-  if (wk.b == 0)
-    for (int i = threadIdx.x; i < n; i += blockDim.x) yout[nd.c0 + i] = f[i];
-  // wud[a] -= L21[a] . y: a warp per 4 rows (loads coalesced along the rows)
-  for (int a = a0 + warp * 4; a < a1; a += 32) {
-    T s[4] = {T(0), T(0), T(0), T(0)};
-    const T* row = nd.L + (size_t)(n + a) * nd.ld;
-    for (int j = lane; j < n; j += 32) {
-      const T fj = f[j];
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (a + q < a1) s[q] += row[(size_t)q * nd.ld + j] * fj;
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const T v = warp_sum(s[q]);
-      if (lane == 0 && a + q < a1) wud[a + q] -= v;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {   // this chunk's rows of the update vector are final
-    __threadfence();
-    atomicAdd(sync + nd.syncOff + 1, 1);
-  }
-  launch_done(&sync[SYNC_TICK_F], &sync[SYNC_DONE_F]);
+__device__ __forceinline__ float4 vzero(float) { return make_float4(0.f, 0.f, 0.f, 0.f); }
+__device__ __forceinline__ double2 vzero(double) { return make_double2(0.0, 0.0); }
+__device__ __forceinline__ void vshfl_add(float4& v, int o) {
+  v.x += __shfl_xor_sync(FULL, v.x, o);
+  v.y += __shfl_xor_sync(FULL, v.y, o);
+  v.z += __shfl_xor_sync(FULL, v.z, o);
+  v.w += __shfl_xor_sync(FULL, v.w, o);
 }
-
-// Backward: each chunk block forms its part of L21^T x_R; the last chunk
-// block of the supernode to finish sums the parts in fixed order and solves
-// with L11^T.
-template <class T>
-__global__ void __launch_bounds__(256) interior_backward_chunks(const SNode<T>* __restrict__ nodes,
-                                                                const RowBlock* __restrict__ work,
-                                                                const int* __restrict__ rows,
-                                                                int* __restrict__ sync, int epoch,
-                                                                T* __restrict__ ipart, const T* __restrict__ yin,
-                                                                T* __restrict__ w, const int* __restrict__ small) {
-  pdl_enter();
-  extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ T tb[64];
-  __shared__ T red[8][256];
-  __shared__ int sLast, sTicket;
-  int* err = sync;
-  if (threadIdx.x == 0) sTicket = atomicAdd(&sync[SYNC_TICK_B], 1);
-  __syncthreads();
-  if (sTicket >= (int)gridDim.x) {   // counters not reset: report, touch nothing
-    if (threadIdx.x == 0) atomicExch(err, 2);
-    return;
-  }
-  const RowBlock wk = work[sTicket];
-  if (wk.node < 0) {   // a group of small supernodes, a warp each
-    const int warp = threadIdx.x >> 5;
-    T* fw = reinterpret_cast<T*>(smraw) + warp * (IW_N + ICH);
-    if (warp < wk.b)
-      interior_backward_warp<T>(nodes, small[8 * (-1 - wk.node) + warp], rows, sync, epoch, yin, w, fw, fw + IW_N);
-    launch_done(&sync[SYNC_TICK_B], &sync[SYNC_DONE_B]);
-    return;
-  }
-  const SNode<T>& nd = nodes[wk.node];
-  if (nd.parentI >= 0 && (threadIdx.x >> 5) == 0)   // the parent (and so every ancestor) is solved
-    wait_geq(sync + nodes[nd.parentI].syncOff + 2, epoch, err);
-  __syncthreads();
-  const int n = nd.n, a0 = wk.b * ICH, a1 = min(nd.m, a0 + ICH);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  T* f = reinterpret_cast<T*>(smraw);   // n values
-  T* xr = f + ((n + 1) & ~1);           // ICH values
-  const int nch = (nd.m + ICH - 1) / ICH;
-  if (nch > 0) {
-    const int* rw = rows + nd.rowsOff;
-    for (int a = a0 + threadIdx.x; a < a1; a += blockDim.x) xr[a - a0] = __ldcg(w + rw[a]);
-    __syncthreads();
-    // part[j] = sum_{a in chunk} L21[a][j] x_a: warp w takes rows w, w+8, ...
-    // (lanes along the row), then the 8 warp partials are summed in order
-    const T* L21 = nd.L + (size_t)(n + a0) * nd.ld;
-    for (int jt = 0; jt < n; jt += 256) {
-      T acc[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) acc[q] = T(0);
-      for (int a = warp; a < a1 - a0; a += 8) {
-        const T x = xr[a];
-        const T* row = L21 + (size_t)a * nd.ld + jt;
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (jt + lane + 32 * q < n) acc[q] += row[lane + 32 * q] * x;
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) red[warp][lane + 32 * q] = acc[q];
-      __syncthreads();
-      const int j = jt + threadIdx.x;
-      if (threadIdx.x < 256 && j < n) {
-        T s = T(0);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) s += red[q][threadIdx.x];
-        ipart[nd.zpOff + (size_t)wk.b * n + j] = s;
-      }
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      __threadfence();
-      sLast = (atomicAdd(sync + nd.syncOff, 1) == nch - 1);
-      __threadfence();
-    }
-    __syncthreads();
-    if (!sLast) {
-      launch_done(&sync[SYNC_TICK_B], &sync[SYNC_DONE_B]);
-      return;
-    }
-  }
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    T t = T(0);
-    for (int c = 0; c < nch; ++c) t += __ldcg(ipart + nd.zpOff + (size_t)c * n + i);
-    f[i] = yin[nd.c0 + i] - t;
-  }
-  __syncthreads();
-  trsv_dinv_t<T>(nd.L, nd.ld, n, nd.Dinv, f, tb, reinterpret_cast<T(*)[64]>(&red[0][0]));
-  for (int i = threadIdx.x; i < n; i += blockDim.x) w[nd.c0 + i] = f[i];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    if (nch > 0) sync[nd.syncOff] = 0;
-    st_release(sync + nd.syncOff + 2, epoch);   // x of this supernode is final
-  }
-  launch_done(&sync[SYNC_TICK_B], &sync[SYNC_DONE_B]);
+__device__ __forceinline__ void vshfl_add(double2& v, int o) {
+  v.x += __shfl_xor_sync(FULL, v.x, o);
+  v.y += __shfl_xor_sync(FULL, v.y, o);
 }
 
 // ---------------------------------------------------------------------------
-// Compressed supernodes.  X = L11^{-1} is formed once per factorisation, so
-// the triangular solves are GEMVs: every 64-row (or 64-column) block of a
-// supernode is an independent thread block.
+// The apply engine: one persistent launch runs a whole preconditioner
+// application as a list of work items (ApplyItem) in a topological order.
+//
+// Roles: a CTA is one producer warp and two groups of four consumer warps.  The
+// producer takes the next item from a ticket counter and bulk-copies
+// (cp.async.bulk, completion on an mbarrier) its descriptor and its piece of
+// the factor into one of three shared-memory stages, running ahead of the
+// consumers: the factor does not depend on the right-hand side, so its bytes
+// arrive while earlier items still wait or compute.  The groups take the items
+// in turn: a group waits (bounded) until the counters the item names have
+// reached their targets, gathers the vector entries, forms the products from
+// shared memory, stores, and one thread releases the item's own counter.  An
+// item is about 3 us of dependent steps whatever its bytes, so what counts is
+// the bytes being worked on at once: six groups an SM.
+//
+// Every item waits only on items earlier in the list (checked when the list is
+// built) and a group works its tickets in order, so the smallest unfinished
+// ticket can always proceed, whatever else shares the GPU.  The next kernel
+// (clear_counters / convert_out_kernel) zeroes ticket and counters, so the
+// launch needs no host state and replays inside a CUDA graph.
+//
+// Bound: a chain of hand-overs (release, poll, gather, product: ~3 us each, one
+// or two a tree level and direction), then the factor's bytes.  The triangles X
+// and the products with S lie off that chain and fill its gaps.  Measured, one
+// application (before: a triangular solve per supernode on the chain, two
+// ticketed launches for the interior and eight launches per compressed level):
+// 3D 64^3 FP32 0.914 -> 0.376 ms (591 MB, 0.087 ms at the copy rate), 3D 96^3
+// FP32 2.23 -> 1.18 ms, 2D 193 x 187 FP64 0.632 -> 0.149 ms, 2D 40 x 37 FP64
+// 0.159 -> 0.066 ms.  Two groups of four warps against one of eight (half the
+// items in work at once): 3D 64^3 0.400 against 0.494 ms.
 
-// The pieces of a compressed level, as device functions of one thread block
-// (a warp per row where rows are independent).  Data another block wrote is
-// read through L2 (ld.global.cg).
+constexpr int ST_DATA = 16384, ST_DESC = 4096, ST_BYTES = ST_DATA + ST_DESC;
+constexpr int NSTAGE = 3;
+constexpr int NGRP = 2, GT = 128, GW = GT / 32;   // consumer groups of a CTA, threads and warps of one
+constexpr int IW_N = 32, IW_M = 128;     // members of a group item: n <= IW_N, m <= IW_M
+constexpr int GRP = 8;                   // most members of a group
+constexpr int GH = 10;                   // header words of a member
+constexpr int SHALLOW = 1;               // phases of up to this many items a group (in all CTAs) draw tickets singly
+constexpr int ROWS8 = 8 * GW;            // most rows of W or V in an item (eight a warp)
 
-// w[c0 + i] += the fixed-order contribution list of row i (one warp).
-template <class T>
-__device__ void cgather_row(const SNode<T>& nd, int i, const long long* __restrict__ cstart,
-                            const long long* __restrict__ ent, const T* wu, T* w) {
-  const int lane = threadIdx.x & 31;
-  const long long* cs = cstart + nd.cOff;
-  T acc = T(0);
-  for (long long e = cs[i] + lane; e < cs[i + 1]; e += 32) acc += __ldcg(wu + ent[e]);
-  acc = warp_sum(acc);
-  if (lane == 0) w[nd.c0 + i] = __ldcg(w + nd.c0 + i) + acc;
+enum ItemKind : int { IT_FGRP = 0, IT_FWD, IT_CF, IT_CU, IT_Y, IT_XT, IT_CS, IT_CX, IT_BGRP, IT_BWD, IT_CR, IT_BR, IT_END };
+
+// tile of X of the Y = X f items (rows x columns) and of the t = X^T y items
+constexpr int Y_ROWS = 16, T_COLS = 64;
+template <class T> constexpr int Y_COLS = ST_DATA / Y_ROWS / (int)sizeof(T);
+template <class T> constexpr int T_ROWS = ST_DATA / T_COLS / (int)sizeof(T);
+
+// barrier of the caller's consumer group (bar.sync wants whole warps)
+__device__ __forceinline__ void cbar() {
+  __syncwarp();
+  asm volatile("bar.sync %0, 128;" ::"r"(1 + (int)(threadIdx.x / GT)) : "memory");
 }
 
-// Partial products of y = X f and x = X^T g over 64 x 256 tiles of X (tiles
-// entirely above the diagonal are not listed): a level's tiles are spread
-// over all SMs, each thread keeping 64 independent loads in flight.
-//   P[i][jb] = sum_{j in column block jb} X[i][j] f_j    (forward)
-//   Q[j][ib] = sum_{i in row block ib} X[i][j] g_i       (backward)
-template <class T>
-__device__ void cytile(const SNode<T>& nd, const XTile& tl, const T* w, T* part) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = nd.n;
-  const int i0 = tl.ib * SOLVE_RB + warp * 8, j0 = tl.jb * XT_COLS;
-  T fj[8];
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    const int j = j0 + lane + 32 * c;
-    fj[c] = (j < n) ? __ldcg(w + nd.c0 + j) : T(0);
-  }
-  T acc[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    acc[q] = T(0);
-    const int i = i0 + q;
-    if (i < n) {
-      const T* xr = nd.X + (size_t)i * n;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const int j = j0 + lane + 32 * c;
-        if (j < n) acc[q] += xr[j] * fj[c];
+__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(unsigned bar, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(unsigned bar, int bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_test(unsigned bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Warp-wide wait for a phase: lane 0 polls, for at most about four seconds;
+// false when it gave up.
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
+  int ok = 1;
+  if ((threadIdx.x & 31) == 0 && !mbar_test(bar, parity)) {
+    unsigned long long t0, t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    for (int it = 1; !mbar_test(bar, parity); ++it) {
+      if (it > 64) __nanosleep(20);
+      if ((it & 255) == 0) {
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+        if (t - t0 > 4000000000ull) {
+          ok = 0;
+          break;
+        }
       }
     }
   }
+  ok = __shfl_sync(FULL, ok, 0);
+  __syncwarp();   // what lane 0 has seen complete, the others may read
+  return ok != 0;
+}
+// global -> shared, 16-byte aligned addresses and size, completion on bar
+__device__ __forceinline__ void bulk_copy(void* dst, const void* src, int bytes, unsigned bar) {
+  asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+
+// Warp-wide bounded wait until every listed counter has reached its target
+// (pairs of counter index and target).
+__device__ __forceinline__ void wait_list(const int* pairs, int count, const int* sync, int* err) {
+  const int lane = threadIdx.x & 31;
+  for (int c0 = 0; c0 < count; c0 += 32) {
+    const bool have = c0 + lane < count;
+    const int idx = have ? pairs[2 * (c0 + lane)] : 0, target = have ? pairs[2 * (c0 + lane) + 1] : 0;
+    for (int it = 0;; ++it) {
+      const bool ok = !have || ld_acquire(sync + idx) >= target;
+      if (__all_sync(FULL, ok)) break;
+      if (it >= SPIN_LIMIT) {
+        if (lane == 0) atomicExch(err, 1);
+        return;
+      }
+      if ((it & 63) == 63 && __any_sync(FULL, ld_volatile(err) != 0)) return;
+      if (it) __nanosleep(20);
+    }
+  }
+}
+
+// v[i] + the pull list [b[i], e[i]) of wu entries, in order, for N targets at
+// once: the loads of a round (two entries a target) are all in flight together.
+template <class T, int N>
+__device__ __forceinline__ void pull_sums(T (&v)[N], const int* const (&ent)[N], int (&b)[N], const int (&e)[N],
+                                          const T* wu) {
+  bool more = true;
+  while (more) {
+    T x[N], y[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      x[i] = b[i] < e[i] ? __ldcg(wu + ent[i][b[i]]) : T(0);
+      y[i] = b[i] + 1 < e[i] ? __ldcg(wu + ent[i][b[i] + 1]) : T(0);
+    }
+    more = false;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      v[i] = (v[i] + x[i]) + y[i];
+      b[i] += 2;
+      more = more || b[i] < e[i];
+    }
+  }
+}
+
+// zs[k] = the sum of `parts` partial rows (row stride rp, 16-byte aligned) over
+// the columns [k0, k0 + GT vectors), in a fixed order: groups of threads take
+// every ng-th row, the groups are added in order.
+template <class T>
+__device__ __forceinline__ void sum_parts(const T* __restrict__ part, int rp, int k0, int parts, T* zs, T* redT) {
+  using Vt = typename Vec16<T>::type;
+  constexpr int V = Vec16<T>::V;
+  Vt* red = reinterpret_cast<Vt*>(redT);
+  const int tid = threadIdx.x % GT;
+  const int nv = min(GT, (rp - k0) / V);
+  int ng = GT / nv;
+  if (ng > parts) ng = parts;
+  const int g = tid / nv, c = tid - g * nv;
+  const Vt* p = reinterpret_cast<const Vt*>(part + k0) + c;
+  const size_t stride = rp / V;
+  if (g < ng) {
+    Vt a0 = vzero(T(0));
+    for (int i = g; i < parts; i += 8 * ng) {
+      Vt v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = i + q * ng < parts ? __ldcg(p + (size_t)(i + q * ng) * stride) : vzero(T(0));
+#pragma unroll
+      for (int q = 0; q < 8; ++q) vadd(a0, v[q]);
+    }
+    red[g * nv + c] = a0;
+  }
+  cbar();
+  for (int k = tid; k < nv * V; k += GT) {
+    T s = T(0);
+    for (int q = 0; q < ng; ++q) s += redT[q * nv * V + k];
+    zs[k] = s;
+  }
+  cbar();
+}
+
+// out[k] = sum_{i < h} M[i][k] v[i], k < r (and zeros up to whole sectors), M in
+// shared or global memory (row stride r): 2^g-wide column groups, rows split over the remaining threads and
+// the parts added in a fixed order.
+template <class T>
+__device__ __forceinline__ void cols_gemv(const T* M, int r, int h, const T* v, T* out, T* red) {
+  const int tid = threadIdx.x % GT;
+  int wd = 32;
+  while (wd < r && wd < GT) wd <<= 1;
+  const int ng = GT / wd, g = tid / wd, c = tid & (wd - 1);
+  for (int k0 = 0; k0 < r; k0 += wd) {
+    T s = T(0);
+    if (k0 + c < r) {
+#pragma unroll 8
+      for (int i = g; i < h; i += ng) s += M[(size_t)i * r + k0 + c] * v[i];
+    }
+    if (ng == 1) {
+      if (k0 + c < ((r + 7) & ~7)) out[k0 + c] = s;
+    } else {
+      red[tid] = s;
+      cbar();
+      if (tid < wd && k0 + tid < ((r + 7) & ~7)) {
+        T z = T(0);
+        for (int q = 0; q < ng; ++q) z += red[q * wd + tid];
+        out[k0 + tid] = z;
+      }
+      cbar();
+    }
+  }
+}
+
+template <class T>
+struct ApplyArgs {
+  const ApplyItem* items;
+  int nItems;
+  const int* blob;
+  int* sync;        // [0] error word, [1] ticket, then the counters
+  T* w;             // permuted vector, in place
+  T* t;             // S f of the interior columns
+  T* wu;            // update vectors
+  T* zp;            // partials of z = W^T f
+  T* sp;            // partials of s = V^T x_R
+  T* yp;            // partials of X f
+  T* xp;            // partials of X^T y
+  T* ip;            // partials of G^T x_R
+  int work;         // elements of a group's work area in shared memory
+};
+
+// A group of small interior supernodes, forward: u = (children's rows) - G f
+// and t = S f; a warp a member, or several when there are fewer members.  FP32:
+// lanes along the rows, partial sums by shuffles.  FP64 adds run at 1/64 of the
+// FP32 rate, so there a lane forms a whole row (the odd row stride in 16-byte
+// units keeps that free of bank conflicts).
+template <class T>
+__device__ __forceinline__ void item_fgrp(const ApplyArgs<T>& A, const int* hdr0, const int* d, int cnt, const T* data,
+                                          T* wk) {
+  using Vt = typename Vec16<T>::type;
+  constexpr int V = Vec16<T>::V;
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % GW;
+  const int wpn = cnt <= 1 ? GW : cnt <= GW / 2 ? GW / (GW / 2) : 1;
+  T* f = wk + warp * (IW_N + IW_M);
+  T* ub = f + IW_N;
+  const int part = warp % wpn;
+  for (int q = warp / wpn; q < cnt; q += GW / wpn) {
+    const int* h = hdr0 + GH * q;
+    const int n = h[0], m = h[1], c0 = h[2], nv = h[7] / V;
+    const Vt* G = reinterpret_cast<const Vt*>(data + h[4]);
+    const Vt* S = reinterpret_cast<const Vt*>(data + h[5]);
+    const int* ps = h[6] ? d + h[6] : nullptr;
+    const int* ent = ps + n + m + 1;
+    const int mp = ((m + wpn - 1) / wpn + 7) & ~7, aLo = part * mp, aHi = min(m, aLo + mp);
+    T* u = A.wu + h[3];
+    T* t = A.t + h[8];
+    __syncwarp();
+    T v[1 + IW_M / 32];   // the lane's column, then its rows
+    int b[1 + IW_M / 32], e[1 + IW_M / 32];
+    v[0] = lane < n ? __ldcg(A.w + c0 + lane) : T(0);
+    b[0] = ps && lane < n ? ps[lane] : 0;
+    e[0] = ps && lane < n ? ps[lane + 1] : 0;
+#pragma unroll
+    for (int i = 1; i <= IW_M / 32; ++i) {
+      const int a = aLo + lane + 32 * (i - 1);
+      const bool in = ps && a < aHi;
+      v[i] = T(0);
+      b[i] = in ? ps[n + a] : 0;
+      e[i] = in ? ps[n + a + 1] : 0;
+    }
+    if (ps) {
+      const int* const lists[1 + IW_M / 32] = {ent, ent, ent, ent, ent};
+      pull_sums(v, lists, b, e, A.wu);
+    }
+#pragma unroll
+    for (int i = 1; i <= IW_M / 32; ++i)
+      if (aLo + lane + 32 * (i - 1) < aHi) ub[aLo + lane + 32 * (i - 1)] = v[i];
+    f[lane] = v[0];
+    __syncwarp();
+    if constexpr (sizeof(T) == 8) {
+      const int rows = max(0, aHi - aLo), sp = ((n + wpn - 1) / wpn + 7) & ~7, sLo = part * sp, sRows = max(0, min(n, sLo + sp) - sLo);
+      const Vt* fs = reinterpret_cast<const Vt*>(f);
+      const int nq = (n + V - 1) / V;
+      for (int i = lane; i < rows + sRows; i += 32) {   // rows of G, then of S
+        const Vt* row = i < rows ? G + (aLo + i) * nv : S + (sLo + i - rows) * nv;
+        T v0 = T(0), v1 = T(0);
+        int c = 0;
+        for (; c + 1 < nq; c += 2) {
+          v0 = vdot(row[c], fs[c], v0);
+          v1 = vdot(row[c + 1], fs[c + 1], v1);
+        }
+        if (c < nq) v0 = vdot(row[c], fs[c], v0);
+        if (i < rows) u[aLo + i] = ub[aLo + i] - (v0 + v1);
+        else t[sLo + i - rows] = v0 + v1;
+      }
+    } else {
+      const int lg = nv <= 4 ? 2 : 3;   // lanes per row: 2^lg
+      const int c = lane & ((1 << lg) - 1), g = lane >> lg, rpl = 32 >> lg;
+      const Vt fc = c < nv ? reinterpret_cast<const Vt*>(f)[c] : vzero(T(0));
+#pragma unroll 4
+      for (int a0 = aLo; a0 < aHi; a0 += rpl) {
+        const int a = a0 + g;
+        T v = (a < aHi && c < nv) ? vdot(G[a * nv + c], fc, T(0)) : T(0);
+        for (int o = 1; o < (1 << lg); o <<= 1) v += __shfl_xor_sync(FULL, v, o);
+        if (c == 0 && a < aHi) u[a] = ub[a] - v;
+      }
+      for (int i0 = part * rpl; i0 < n; i0 += rpl * wpn) {
+        const int i = i0 + g;
+        T v = (i < n && c < nv) ? vdot(S[i * nv + c], fc, T(0)) : T(0);
+        for (int o = 1; o < (1 << lg); o <<= 1) v += __shfl_xor_sync(FULL, v, o);
+        if (c == 0 && i < n) t[i] = v;
+      }
+    }
+    // the last sectors whole
+    if (part == wpn - 1) {
+      if (m + lane < ((m + 7) & ~7)) u[m + lane] = T(0);
+      if (n + lane < ((n + 7) & ~7)) t[n + lane] = T(0);
+    }
+  }
+}
+
+// A group, backward: x = t - G^T x_R; a warp a member.
+template <class T>
+__device__ __forceinline__ void item_bgrp(const ApplyArgs<T>& A, const int* hdr0, const int* d, int cnt, const T* data,
+                                          T* wk) {
+  using Vt = typename Vec16<T>::type;
+  constexpr int V = Vec16<T>::V;
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % GW;
+  T* xr = wk + warp * (IW_N + IW_M);
+  for (int q = warp; q < cnt; q += GW) {
+    const int* h = hdr0 + GH * q;
+    const int n = h[0], m = h[1], c0 = h[2], nv = h[7] / V, nq = (n + V - 1) / V;
+    const Vt* G = reinterpret_cast<const Vt*>(data + h[4]);
+    const int* rw = d + h[6];
+    __syncwarp();
+    const T tl = lane < n ? __ldcg(A.t + h[8] + lane) : T(0);
+#pragma unroll 4
+    for (int a = lane; a < m; a += 32) xr[a] = __ldcg(A.w + rw[a]);
+    __syncwarp();
+    const int lg = nq <= 4 ? 2 : nq <= 8 ? 3 : 4;
+    const int c = lane & ((1 << lg) - 1), g = lane >> lg, rpl = 32 >> lg;
+    Vt acc = vzero(T(0));
+    if (c < nq) {
+#pragma unroll 4
+      for (int a = g; a < m; a += rpl) vaxpy(acc, G[a * nv + c], xr[a]);
+    }
+    for (int o = 1 << lg; o < 32; o <<= 1) vshfl_add(acc, o);
+    __syncwarp();
+    if (g == 0 && c < nq) reinterpret_cast<Vt*>(xr)[c] = acc;
+    __syncwarp();
+    if (lane < n) A.w[c0 + lane] = tl - xr[lane];
+  }
+}
+
+// One chunk of a larger interior supernode, forward.
+// hdr: n, rows, c0, u offset (of the chunk's first row), s0, sRows, list, ldk, t offset, whole sectors
+template <class T>
+__device__ __forceinline__ void item_fwd(const ApplyArgs<T>& A, const int* h, const int* d, const int* d2, const T* Gd,
+                                         const T* Sd, T* f, T* ub) {
+  using Vt = typename Vec16<T>::type;
+  constexpr int V = Vec16<T>::V;
+  const int tid = threadIdx.x % GT;
+  const int n = h[0], rows = h[1], c0 = h[2], nv = h[7] / V;
+  // pull lists: the chunk's rows' (rows + 1 offsets, entries) in the descriptor,
+  // the columns' (n + 1 offsets, entries) in the part that the chunks share
+  const bool pull = h[6] != 0;
+  const int* ps = d + h[6];
+  const int* ent = ps + rows + 1;
+  const int* ent2 = d2 + n + 1;
+  for (int t0 = 0; t0 < nv * V; t0 += 2 * GT) {   // two columns and (first pass) one row a thread
+    T v[3];
+    int b[3], e[3];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int t = t0 + tid + i * GT;
+      v[i] = t < n ? __ldcg(A.w + c0 + t) : T(0);
+      b[i] = pull && t < n ? d2[t] : 0;
+      e[i] = pull && t < n ? d2[t + 1] : 0;
+    }
+    const bool in = t0 == 0 && tid < rows;
+    v[2] = T(0);
+    b[2] = pull && in ? ps[tid] : 0;
+    e[2] = pull && in ? ps[tid + 1] : 0;
+    if (pull) {
+      const int* const lists[3] = {ent2, ent2, ent};
+      pull_sums(v, lists, b, e, A.wu);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (t0 + tid + i * GT < nv * V) f[t0 + tid + i * GT] = v[i];
+    if (in) ub[tid] = v[2];
+  }
+  cbar();
+  const Vt* fs = reinterpret_cast<const Vt*>(f);
+  const int R = rows + h[5];   // rows of G, then the chunk's rows of S
+  int lt = 1;                  // threads of a row: 2^lt
+  while (lt < 5 && R << (lt + 1) <= GT) ++lt;
+  const int sub = tid & ((1 << lt) - 1);
+  for (int r0 = 0; r0 < R; r0 += GT >> lt) {
+    const int row = r0 + (tid >> lt);
+    T v = T(0);
+    if (row < R) {
+      const Vt* m = reinterpret_cast<const Vt*>(row < rows ? Gd : Sd) + (size_t)(row < rows ? row : row - rows) * nv;
+#pragma unroll 4
+      for (int c = sub; c < nv; c += 1 << lt) v = vdot(m[c], fs[c], v);
+    }
+    for (int o = 1; o < (1 << lt); o <<= 1) v += __shfl_xor_sync(FULL, v, o);
+    if (sub == 0 && row < R) {
+      if (row < rows) A.wu[h[3] + row] = ub[row] - v;
+      else A.t[h[8] + h[4] + row - rows] = v;
+    }
+  }
+  if (h[9]) {   // chunks of whole sectors: the last ones to their ends
+    constexpr int SE = 32 / (int)sizeof(T);
+    if (tid < (SE - rows % SE) % SE) A.wu[h[3] + rows + tid] = T(0);
+    if (tid < (SE - h[5] % SE) % SE) A.t[h[8] + h[4] + h[5] + tid] = T(0);
+  }
+}
+
+// One chunk of a larger interior supernode, backward: its part of G^T x_R, or
+// x = t - G^T x_R itself when it is the only one (several chunks: item BR).
+// hdr: n, rows, c0, ipOff, chunk, chunks, rows list, ldk, ip stride, t offset
+template <class T>
+__device__ __forceinline__ void item_bwd(const ApplyArgs<T>& A, const int* h, const int* d, const T* Gd, T* xr, T* red) {
+  using Vt = typename Vec16<T>::type;
+  constexpr int V = Vec16<T>::V;
+  const int tid = threadIdx.x % GT, lane = tid & 31, warp = tid >> 5;
+  const int n = h[0], rows = h[1], c0 = h[2], nch = h[5], nv = h[7] / V;
+  if (rows == 0) {   // nothing above: x = t
+    for (int j = tid; j < n; j += GT) A.w[c0 + j] = __ldcg(A.t + h[9] + j);
+    return;
+  }
+  if (tid < rows) xr[tid] = __ldcg(A.w + d[h[6] + tid]);
+  cbar();
+  // 2^lg threads along a row (4 ... 128), the others on further rows
+  int lg = 2;
+  while ((1 << lg) < nv && lg < 7) ++lg;
+  const int wd = 1 << lg, c = tid & (wd - 1), g = tid >> lg, ng = GT >> lg;
+  const Vt* G = reinterpret_cast<const Vt*>(Gd);
+  Vt* rv = reinterpret_cast<Vt*>(red);
+  for (int v0 = 0; v0 < nv; v0 += GT) {
+    Vt acc = vzero(T(0));
+    if (v0 + c < nv) {
+#pragma unroll 4
+      for (int a = g; a < rows; a += ng) vaxpy(acc, G[(size_t)a * nv + v0 + c], xr[a]);
+    }
+    for (int o = wd; o < 32; o <<= 1) vshfl_add(acc, o);
+    const int parts = lg <= 5 ? GW : ng;
+    if (lg > 5) rv[g * wd + c] = acc;
+    else if (lane < wd) rv[warp * wd + lane] = acc;
+    cbar();
+    for (int q = tid; q < max(wd * V, 8); q += GT) {
+      const int j = v0 * V + q;
+      T s = T(0);
+      if (j < n)
+        for (int p = 0; p < parts; ++p) s += red[p * wd * V + q];
+      if (nch > 1) {
+        if (j < h[8]) A.ip[h[3] + (size_t)h[4] * h[8] + j] = s;
+      } else if (j < n) {
+        A.w[c0 + j] = __ldcg(A.t + h[9] + j) - s;
+      }
+    }
+    cbar();
+  }
+}
+
+// Compressed supernode, up: f of a block of columns (added into w) and the
+// block's part of z = W^T f.
+// hdr: c (first column's vector index), h (columns), r, zp row offset, list
+template <class T>
+__device__ __forceinline__ void item_cf(const ApplyArgs<T>& A, const int* h, const int* d, const T* Wd, T* fb, T* red) {
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % GW;
+  const int c0 = h[0], cols = h[1], r = h[2];
+  const int* ps = d + h[4];
+  const int* ent = ps + cols + 1;
+  // a warp per eight rows, lanes along the rows' contribution lists
+  int b[8], e[8];
+  T acc[8], wv[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
-    const T v = warp_sum(acc[q]);
-    if (lane == 0 && i0 + q < n) part[nd.zpOff2 + (size_t)(i0 + q) * nd.ncb + tl.jb] = v;
+    const int i = warp + GW * q;
+    const bool in = i < cols;
+    b[q] = in ? ps[i] + lane : 0;
+    e[q] = in ? ps[i + 1] : 0;
+    wv[q] = (in && lane == 0) ? __ldcg(A.w + c0 + i) : T(0);
+    acc[q] = T(0);
   }
-}
-
-// gs: SOLVE_RB shared.
-template <class T>
-__device__ void cxtile(const SNode<T>& nd, const XTile& tl, const T* gv, T* part, T* gs) {
-  const int n = nd.n, i0 = tl.ib * SOLVE_RB, h = min(SOLVE_RB, n - i0);
-  if (threadIdx.x < SOLVE_RB) gs[threadIdx.x] = (threadIdx.x < h) ? __ldcg(gv + nd.c0 + i0 + threadIdx.x) : T(0);
-  __syncthreads();
-  const int j = tl.jb * XT_COLS + threadIdx.x;
-  if (j < n) {
-    T s = T(0);
-#pragma unroll 16
-    for (int i = 0; i < h; ++i) s += nd.X[(size_t)(i0 + i) * n + j] * gs[i];
-    part[nd.zpOff2 + (size_t)j * nd.nb + tl.ib] = s;
-  }
-  __syncthreads();
-}
-
-// y_i = sum of its tile partials (fixed order) for one 64-row block, then the
-// block's part of z = U^T y; the last block of the supernode to finish sums
-// the parts in fixed order.  yb: SOLVE_RB shared, red: 8 x 256 shared.
-template <class T>
-__device__ void cy_block(const SNode<T>& nd, int b, int* sync, T* zpart, const T* ypart, T* yv, T* wu, T* yb,
-                         T (*red)[256], int* sLast) {
-  const int n = nd.n, i0 = b * SOLVE_RB, h = min(SOLVE_RB, n - i0);
-  if (threadIdx.x < SOLVE_RB) {
-    const int i = threadIdx.x;
-    T s = T(0);
-    if (i < h) {
-      const int jbEnd = min(nd.ncb - 1, (i0 + SOLVE_RB - 1) / XT_COLS);
-      const T* p = ypart + nd.zpOff2 + (size_t)(i0 + i) * nd.ncb;
-      for (int jb = 0; jb <= jbEnd; ++jb) s += __ldcg(p + jb);
-      yv[nd.c0 + i0 + i] = s;
+  bool more = true;
+  while (more) {
+    T v[8], x[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      v[q] = b[q] < e[q] ? __ldcg(A.wu + ent[b[q]]) : T(0);
+      x[q] = b[q] + 32 < e[q] ? __ldcg(A.wu + ent[b[q] + 32]) : T(0);
     }
-    yb[i] = s;
+    more = false;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      acc[q] = (acc[q] + v[q]) + x[q];
+      b[q] += 64;
+      more = more || b[q] - lane < e[q];
+    }
   }
-  __syncthreads();
-  const int r = nd.r;
-  rows_t_gemv<T>(nd.U + (size_t)i0 * r, r, h, r, yb, zpart + nd.zpOff + (size_t)b * r, red);
-  int* done = sync + nd.syncOff;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int i = warp + GW * q;
+    if (i >= cols) break;
+    const T s = warp_sum(acc[q]);
+    if (lane == 0) {
+      const T v = wv[q] + s;
+      A.w[c0 + i] = v;
+      fb[i] = v;
+    }
+  }
+  cbar();
+  if (r > 0) cols_gemv<T>(Wd, r, cols, fb, A.zp + h[3], red);
+}
+
+// acc = the product of this warp's rows (i = warp, warp + GW, ...) of M (row
+// stride r) with the sum of the partial rows.
+template <class T>
+__device__ __forceinline__ void rows_times_parts(const T* M, int r, int rows, const T* part, int parts, T (&acc)[8],
+                                                 T* zs, T* red) {
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % GW;
+  constexpr int KT = GT * Vec16<T>::V;
+  const int rp = (r + 7) & ~7;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) acc[q] = T(0);
+  for (int k0 = 0; k0 < r; k0 += KT) {
+    sum_parts<T>(part, rp, k0, parts, zs, red);
+    const int kn = min(KT, r - k0);
+    const T* m = M + (size_t)warp * r + k0;
+#pragma unroll 2
+    for (int k = lane; k < kn; k += 32) {
+      const T z = zs[k];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (warp + GW * q < rows) acc[q] += m[(size_t)GW * q * r + k] * z;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 8; ++q) acc[q] = warp_sum(acc[q]);
+}
+
+template <class T>
+__global__ void __launch_bounds__(NGRP * GT + 32, 3) apply_kernel(ApplyArgs<T> A) {
+  extern __shared__ __align__(128) unsigned char apsm[];
+  __shared__ __align__(8) unsigned long long bars[2 * NSTAGE];
+  __shared__ __align__(16) ApplyItem sItem[NSTAGE];
+  const int lane = threadIdx.x & 31;
+  int* const err = A.sync;
   if (threadIdx.x == 0) {
-    __threadfence();
-    *sLast = (atomicAdd(done, 1) == nd.nb - 1);
-    __threadfence();
+    for (int s = 0; s < NSTAGE; ++s) {
+      mbar_init(smem_u32(&bars[s]), 1);              // full: the producer's arrival and its bytes
+      mbar_init(smem_u32(&bars[NSTAGE + s]), 1);     // empty: one consumer thread
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  if (!*sLast) return;
-  rows_t_gemv<T>(zpart + nd.zpOff, r, nd.nb, r, nullptr, wu + nd.wuOff, red);
-  if (threadIdx.x == 0) *done = 0;
-  __syncthreads();
-}
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 
-// x_j = sum of its tile partials over the row blocks ib >= 4 jb (fixed order).
-template <class T>
-__device__ void cx_reduce_col(const SNode<T>& nd, int j, const T* xpart, T* w) {
-  const T* p = xpart + nd.zpOff2 + (size_t)j * nd.nb;
-  T s = T(0);
-  for (int ib = (j / XT_COLS) * (XT_COLS / SOLVE_RB); ib < nd.nb; ++ib) s += __ldcg(p + ib);
-  w[nd.c0 + j] = s;
-}
-
-// u_a = -(V z)_a, the supernode's contribution to its ancestors' right-hand
-// sides (one warp).
-template <class T>
-__device__ void cvz_row(const SNode<T>& nd, int a, T* wu) {
-  const int lane = threadIdx.x & 31, r = nd.r;
-  const T* z = wu + nd.wuOff;
-  const T* v = nd.V + (size_t)a * r;
-  T s = T(0);
-  for (int k = lane; k < r; k += 32) s += v[k] * __ldcg(z + k);
-  s = warp_sum(s);
-  if (lane == 0) wu[nd.wuOff + 2 * r + a] = -s;
-}
-
-// s = V^T x_R for one 128-row chunk; the last chunk to finish sums the chunk
-// partials in fixed order.  xs: 128 shared, red: 8 x 256 shared.
-template <class T>
-__device__ void cvtx_chunk(const SNode<T>& nd, int ch, const int* __restrict__ rows, int* sync, T* spart,
-                           const T* w, T* sv, T* xs, T (*red)[256], int* sLast) {
-  const int r = nd.r, a0 = ch * 128, ah = min(128, nd.m - a0);
-  const int* rw = rows + nd.rowsOff + a0;
-  for (int a = threadIdx.x; a < ah; a += blockDim.x) xs[a] = __ldcg(w + rw[a]);
-  __syncthreads();
-  rows_t_gemv<T>(nd.V + (size_t)a0 * r, r, ah, r, xs, spart + nd.spOff + (size_t)ch * r, red);
-  int* done = sync + nd.syncOff + 1;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    *sLast = (atomicAdd(done, 1) == nd.nch - 1);
-    __threadfence();
+  if (threadIdx.x >= NGRP * GT) {   // ---- producer
+    unsigned full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[NSTAGE]);
+    // Tickets are drawn in pairs (one latency for two items) as far ahead as
+    // there are stages -- except in a phase of few items (ApplyItem::shallow),
+    // where a CTA that holds more than a group's worth keeps items from idle
+    // CTAs: there the next single ticket waits for the last item but one
+    // (c2 apply: 0.39 ms in pairs throughout, 0.376 ms so).
+    int have = 0, ends = 0;   // items read ahead (0 ... 2)
+    bool more = true;
+    ApplyItem cur, nxt;
+    for (int k = 0;; ++k) {
+      const int s = k % NSTAGE, use = k / NSTAGE;
+      if (have == 0 && more) {
+        const int want = k > 0 && cur.shallow ? 1 : 2;
+        if (want == 1 && k > 1) mbar_wait(empty0 + 8 * ((k - 2) % NSTAGE), ((k - 2) / NSTAGE) & 1);
+        int tk = 0;
+        if (lane == 0) tk = atomicAdd(A.sync + 1, want);
+        tk = __shfl_sync(FULL, tk, 0);
+        if (tk < A.nItems) {
+          nxt = A.items[tk];
+          have = 1;
+        }
+        more = tk + want <= A.nItems;
+        if (want == 2 && tk + 1 < A.nItems) {
+          cur = nxt;
+          nxt = A.items[tk + 1];
+          have = 2;
+        } else {
+          cur = nxt;
+        }
+      } else if (have == 1) {
+        cur = nxt;
+      }
+      const bool end = have == 0;
+      if (!end) --have;
+      bool ok = true;
+      if (use > 0) ok = mbar_wait(empty0 + 8 * s, (use - 1) & 1);
+      if (!ok && lane == 0) atomicExch(err, 4);
+      if (end || !ok) {   // one end mark per group
+        if (lane == 0) {
+          sItem[s].kind = IT_END;
+          mbar_arrive(full0 + 8 * s);
+        }
+        more = false;
+        have = 0;
+        if (++ends == NGRP) break;
+        continue;
+      }
+      const ApplyItem& it = cur;
+      unsigned char* st = apsm + (size_t)s * ST_BYTES;
+      if (lane == 0) {
+        sItem[s] = it;
+        const int total = it.descBytes + it.desc2Bytes + it.bytes0 + it.bytes1;
+        mbar_expect(full0 + 8 * s, total);
+        if (it.descBytes) bulk_copy(st + ST_DATA, A.blob + it.desc, it.descBytes, full0 + 8 * s);
+        if (it.desc2Bytes) bulk_copy(st + ST_DATA + it.descBytes, A.blob + it.desc2, it.desc2Bytes, full0 + 8 * s);
+      }
+      __syncwarp();
+      if (lane == 0) {
+        if (it.bytes0) bulk_copy(st, it.g0, it.bytes0, full0 + 8 * s);
+        if (it.bytes1) bulk_copy(st + it.bytes0, it.g1, it.bytes1, full0 + 8 * s);
+      }
+    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    return;
   }
-  __syncthreads();
-  if (!*sLast) return;
-  rows_t_gemv<T>(spart + nd.spOff, r, nd.nch, r, nullptr, sv + nd.wuOff + r, red);
-  if (threadIdx.x == 0) *done = 0;
-  __syncthreads();
+
+  // ---- consumers
+  const int grp = threadIdx.x / GT, tid = threadIdx.x % GT, warp = tid >> 5;
+  T* const red = reinterpret_cast<T*>(apsm + NSTAGE * ST_BYTES) + grp * A.work;   // GT vectors (a group item: its buffers)
+  T* const zs = red + GT * Vec16<T>::V;                                           // GT vectors
+  T* const f = zs + GT * Vec16<T>::V;                                             // the widest chunk item's columns
+  for (int k = grp;; k += NGRP) {
+    const int s = k % NSTAGE, use = k / NSTAGE;
+    if (!mbar_wait(smem_u32(&bars[s]), use & 1)) {   // cannot happen while the producer runs
+      if (tid == 0) atomicExch(err, 3);
+      break;
+    }
+    const ApplyItem& it = sItem[s];
+    const int kind = it.kind;
+    if (kind == IT_END) break;
+    const unsigned char* st = apsm + (size_t)s * ST_BYTES;
+    const T* data = reinterpret_cast<const T*>(st);
+    const int* d = it.descBytes ? reinterpret_cast<const int*>(st + ST_DATA) : A.blob + it.desc;
+    const int* h = d + 2 * it.waits;
+    const int* d2 = it.desc2Bytes ? reinterpret_cast<const int*>(st + ST_DATA + it.descBytes) : A.blob + it.desc2;
+    if (warp == 0) wait_list(d, it.waits, A.sync, err);
+    cbar();
+    // pieces too wide for a stage are read where they are
+    const T* g0 = it.bytes0 ? data : reinterpret_cast<const T*>(it.g0);
+    const T* g1 = it.bytes1 ? data + it.bytes0 / sizeof(T) : reinterpret_cast<const T*>(it.g1);
+    switch (kind) {
+      case IT_FGRP: item_fgrp<T>(A, h, d, it.count, data, red); break;
+      case IT_BGRP: item_bgrp<T>(A, h, d, it.count, data, red); break;
+      case IT_FWD: item_fwd<T>(A, h, d, d2, g0, g1, f, zs); break;
+      case IT_BWD: item_bwd<T>(A, h, d, g0, zs, red); break;
+      case IT_BR: {   // hdr: n, c0, ipOff, parts, ip stride, t offset: x = t - the parts of G^T x_R, in order
+        for (int k0 = 0; k0 < h[0]; k0 += GT * Vec16<T>::V) {
+          const int kn = min(GT * Vec16<T>::V, h[0] - k0);
+          T t[Vec16<T>::V];
+#pragma unroll
+          for (int q = 0; q < Vec16<T>::V; ++q) t[q] = tid + q * GT < kn ? __ldcg(A.t + h[5] + k0 + tid + q * GT) : T(0);
+          sum_parts<T>(A.ip + h[2], h[4], k0, h[3], zs, red);
+#pragma unroll
+          for (int q = 0; q < Vec16<T>::V; ++q)
+            if (tid + q * GT < kn) A.w[h[1] + k0 + tid + q * GT] = t[q] - zs[tid + q * GT];
+        }
+        break;
+      }
+      case IT_CF: item_cf<T>(A, h, d, g0, zs, red); break;
+      case IT_CU: {   // hdr: rows, r, zp offset, parts, u offset
+        T acc[8];
+        rows_times_parts<T>(g0, h[1], h[0], A.zp + h[2], h[3], acc, zs, red);
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (lane == 0 && warp + GW * q < ((h[0] + 7) & ~7)) A.wu[h[4] + warp + GW * q] = -acc[q];   // (acc: 0 past the rows)
+        break;
+      }
+      case IT_Y: {   // hdr: c0 + j0, columns, rows, yp offset (block jb, row i0)
+        for (int j = tid; j < Y_COLS<T>; j += GT) red[j] = j < h[1] ? __ldcg(A.w + h[0] + j) : T(0);
+        cbar();
+        T v[Y_ROWS / GW];
+#pragma unroll
+        for (int q = 0; q < Y_ROWS / GW; ++q) v[q] = T(0);
+        for (int j = lane; j < h[1]; j += 32) {
+          const T fj = red[j];
+#pragma unroll
+          for (int q = 0; q < Y_ROWS / GW; ++q)
+            if (warp + GW * q < h[2]) v[q] += data[(warp + GW * q) * Y_COLS<T> + j] * fj;
+        }
+#pragma unroll
+        for (int q = 0; q < Y_ROWS / GW; ++q) {
+          const T y = warp_sum(v[q]);
+          if (lane == 0 && warp + GW * q < ((h[2] + 7) & ~7)) A.yp[h[3] + warp + GW * q] = y;
+        }
+        break;
+      }
+      case IT_XT: {   // hdr: rows, columns, yp offset (row i0), yp stride, i0, xp offset (block ib, column j0), column blocks
+        using Vt = typename Vec16<T>::type;
+        constexpr int V = Vec16<T>::V, TR = T_ROWS<T>, TPR = GT / TR, NV = T_COLS / V, NG = GT / NV;
+        {   // TPR threads a row add its partials of y (fixed order)
+          const int i = tid / TPR, sub = tid - i * TPR;
+          T y = T(0);
+          if (i < h[0]) {
+            const int nj = min(h[6], ((h[4] + i) / Y_ROWS * Y_ROWS + Y_ROWS - 1) / Y_COLS<T> + 1);
+#pragma unroll 4
+            for (int jb = sub; jb < nj; jb += TPR) y += __ldcg(A.yp + h[2] + (size_t)jb * h[3] + i);
+          }
+#pragma unroll
+          for (int o = 1; o < TPR; o <<= 1) y += __shfl_xor_sync(FULL, y, o);
+          if (sub == 0) zs[i] = y;
+        }
+        cbar();
+        const int g = tid / NV, c = tid - g * NV;
+        Vt acc = vzero(T(0));
+        if (g < NG && c * V < h[1])
+          for (int i = g; i < h[0]; i += NG) vaxpy(acc, reinterpret_cast<const Vt*>(data)[i * NV + c], zs[i]);
+        if (g < NG) reinterpret_cast<Vt*>(red)[g * NV + c] = acc;
+        cbar();
+        if (tid < ((h[1] + 7) & ~7)) {
+          T x = T(0);
+#pragma unroll
+          for (int q = 0; q < NG; ++q) x += red[q * T_COLS + tid];
+          A.xp[h[5] + tid] = x;
+        }
+        break;
+      }
+      case IT_CR: {   // hdr: partials' offset (first column), parts, row stride, columns, offset of the sums, 1: of s
+        using Vt = typename Vec16<T>::type;
+        constexpr int V = Vec16<T>::V;
+        T* const base = h[5] ? A.sp : A.zp;
+        const int nv = h[3] / V, ng = GT / nv, g = tid / nv, c = tid - g * nv;
+        const Vt* p = reinterpret_cast<const Vt*>(base + h[0]) + c;
+        const size_t stride = h[2] / V;
+        Vt acc = vzero(T(0));
+        if (g < ng) {
+          for (int i = g; i < h[1]; i += 8 * ng) {
+            Vt v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = i + q * ng < h[1] ? __ldcg(p + (size_t)(i + q * ng) * stride) : vzero(T(0));
+#pragma unroll
+            for (int q = 0; q < 8; ++q) vadd(acc, v[q]);
+          }
+          reinterpret_cast<Vt*>(red)[g * nv + c] = acc;
+        }
+        cbar();
+        if (tid < h[3]) {
+          T x = T(0);
+          for (int q = 0; q < ng; ++q) x += red[q * h[3] + tid];
+          base[h[4] + tid] = x;
+        }
+        break;
+      }
+      case IT_CS: {   // hdr: rows, r, sp offset, rows list
+        if (tid < h[0]) zs[tid] = __ldcg(A.w + d[h[3] + tid]);
+        cbar();
+        cols_gemv<T>(g0, h[1], h[0], zs, A.sp + h[2], red);
+        break;
+      }
+      default: {   // IT_CX; hdr: c, columns, r, sp offset, parts, xp offset (first column), xp stride, j0, first row block, row blocks
+        // t of a column: its tiles' partials from the diagonal down, a lane a
+        // column, the warps' sums added in order
+        const int cols = h[1], ib0 = (h[7] + lane) / T_COLS * T_COLS / T_ROWS<T>;
+        T t = T(0), acc[8];
+#pragma unroll 8
+        for (int ib = h[8] + warp; ib < h[9]; ib += GW)
+          t += (lane < cols && ib >= ib0) ? __ldcg(A.xp + h[5] + (size_t)ib * h[6] + lane) : T(0);
+        if (h[4] > 0) {
+          rows_times_parts<T>(g0, h[2], cols, A.sp + h[3], h[4], acc, zs, red);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) acc[q] = T(0);
+        }
+        cbar();
+        red[warp * 32 + lane] = t;
+        T own = T(0);
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (lane == q) own = acc[q];
+        cbar();
+        const int j = warp + GW * lane;
+        if (lane < 8 && j < cols) {
+          T x = T(0);
+#pragma unroll
+          for (int q = 0; q < GW; ++q) x += red[q * 32 + j];
+          A.w[h[0] + j] = x - own;
+        }
+        break;
+      }
+    }
+    const int sig = it.sig;
+    cbar();   // every consumer has stored and is done with the stage
+    if (tid == GT - 32) {   // not the warp that polls for the next item
+      mbar_arrive(smem_u32(&bars[NSTAGE + s]));
+      __threadfence();
+      atomicAdd(A.sync + sig, 1);
+    }
+  }
 }
 
-// g_i = y_i - (U s)_i in place (one warp).
+// The tiles of X = L11^{-1} that the items read, each packed into one stage's
+// bytes (zeros outside the matrix), so that one bulk copy brings it: a copy per
+// row of a 64 x 64 tile costs its producer 64 issues of about 15 ns.  A block a
+// tile; bound by HBM (X read, and written once per tile shape).
 template <class T>
-__device__ void cg_row(const SNode<T>& nd, int i, const T* sv, T* yv) {
-  const int lane = threadIdx.x & 31, r = nd.r;
-  const T* s = sv + nd.wuOff + r;
-  const T* u = nd.U + (size_t)i * r;
-  T acc = T(0);
-  for (int k = lane; k < r; k += 32) acc += u[k] * __ldcg(s + k);
-  acc = warp_sum(acc);
-  if (lane == 0) yv[nd.c0 + i] = __ldcg(yv + nd.c0 + i) - acc;
+__global__ void __launch_bounds__(256) pack_tiles_kernel(const SNode<T>* __restrict__ nodes,
+                                                         const PackTile* __restrict__ tiles, T* __restrict__ out) {
+  const PackTile p = tiles[blockIdx.x];
+  const SNode<T>& nd = nodes[p.node];
+  T* o = out + (size_t)blockIdx.x * (ST_DATA / sizeof(T));
+  const int lg = 31 - __clz(p.cols);   // columns: a power of two
+#pragma unroll 4
+  for (int e = threadIdx.x; e < ST_DATA / (int)sizeof(T); e += 256) {
+    const int i = p.i0 + (e >> lg), j = p.j0 + (e & (p.cols - 1));
+    o[e] = (i < nd.n && j < nd.n) ? nd.X[(size_t)i * nd.ldx + j] : T(0);
+  }
 }
 
-// One launch per piece and level, chained by programmatic dependent launch.
-// (All levels of a direction as one ticketed launch, with each phase waiting
-// on the previous one through counters, measured slower on c2: 1.19 vs 1.07
-// ms per apply -- the dependent launches already start without gaps; running
-// the y and x reductions at the tail of the tile launches, by the last tile
-// of each block, measured the same: 0.936 vs 0.919 ms.)
-template <class T>
-__global__ void __launch_bounds__(256) compressed_gather_rows(const SNode<T>* __restrict__ nodes,
-                                                              const int* __restrict__ lvl,
-                                                              const long long* __restrict__ cstart,
-                                                              const long long* __restrict__ ent,
-                                                              const T* __restrict__ wu, T* __restrict__ w) {
-  pdl_enter();
-  const SNode<T>& nd = nodes[lvl[blockIdx.y]];
-  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i < nd.n) cgather_row<T>(nd, i, cstart, ent, wu, w);
-}
-
-template <class T>
-__global__ void __launch_bounds__(256) compressed_ytile_kernel(const SNode<T>* __restrict__ nodes,
-                                                               const XTile* __restrict__ tiles,
-                                                               const T* __restrict__ w, T* __restrict__ part) {
-  pdl_enter();
-  const XTile tl = tiles[blockIdx.x];
-  cytile<T>(nodes[tl.node], tl, w, part);
-}
-
-template <class T>
-__global__ void __launch_bounds__(256) compressed_xtile_kernel(const SNode<T>* __restrict__ nodes,
-                                                               const XTile* __restrict__ tiles,
-                                                               const T* __restrict__ gv, T* __restrict__ part) {
-  pdl_enter();
-  __shared__ T gs[SOLVE_RB];
-  const XTile tl = tiles[blockIdx.x];
-  cxtile<T>(nodes[tl.node], tl, gv, part, gs);
-}
-
-template <class T>
-__global__ void __launch_bounds__(256) compressed_y_kernel(const SNode<T>* __restrict__ nodes,
-                                                           const RowBlock* __restrict__ work, int* __restrict__ sync,
-                                                           T* __restrict__ zpart, const T* __restrict__ ypart,
-                                                           T* __restrict__ yv, T* __restrict__ wu) {
-  pdl_enter();
-  __shared__ T yb[SOLVE_RB];
-  __shared__ T red[8][256];
-  __shared__ int sLast;
+// [S; G] of an interior supernode of up to 64 columns from D = L11^{-1} (one
+// block): S = D^T D and G = L21 D share the product (rows) x D with the rows
+// of D^T, then of L21.  A block per 64 rows; a thread per (row, NQ of the 4 NQ
+// columns); D's zeros above the diagonal are skipped in steps of four.
+// Latency-bound: the products of all supernodes are a few GFLOP.
+template <class T, int NQ>
+__global__ void __launch_bounds__(256) interior_ops_kernel(const SNode<T>* __restrict__ nodes,
+                                                           const RowBlock* __restrict__ work) {
+  constexpr int W = 4 * NQ, P = W + 1;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  T (*Ds)[P] = reinterpret_cast<T (*)[P]>(smraw);
+  T (*Rs)[P] = reinterpret_cast<T (*)[P]>(smraw + sizeof(T) * W * P);
   const RowBlock wk = work[blockIdx.x];
-  cy_block<T>(nodes[wk.node], wk.b, sync, zpart, ypart, yv, wu, yb, red, &sLast);
-}
-
-template <class T>
-__global__ void __launch_bounds__(256) compressed_x_reduce(const SNode<T>* __restrict__ nodes,
-                                                           const int* __restrict__ lvl, const T* __restrict__ xpart,
-                                                           T* __restrict__ w) {
-  pdl_enter();
-  const SNode<T>& nd = nodes[lvl[blockIdx.y]];
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < nd.n) cx_reduce_col<T>(nd, j, xpart, w);
-}
-
-template <class T>
-__global__ void __launch_bounds__(256) compressed_vz_kernel(const SNode<T>* __restrict__ nodes,
-                                                            const int* __restrict__ lvl, T* __restrict__ wu) {
-  pdl_enter();
-  const SNode<T>& nd = nodes[lvl[blockIdx.y]];
-  for (int a = blockIdx.x * 8 + (threadIdx.x >> 5); a < nd.m; a += gridDim.x * 8) cvz_row<T>(nd, a, wu);
-}
-
-template <class T>
-__global__ void __launch_bounds__(256) compressed_vtx_kernel(const SNode<T>* __restrict__ nodes,
-                                                             const int* __restrict__ lvl,
-                                                             const int* __restrict__ rows,
-                                                             int* __restrict__ sync, T* __restrict__ spart,
-                                                             const T* __restrict__ w, T* __restrict__ sv) {
-  pdl_enter();
-  __shared__ T xs[128];
-  __shared__ T red[8][256];
-  __shared__ int sLast;
-  const SNode<T>& nd = nodes[lvl[blockIdx.y]];
-  if (blockIdx.x < nd.nch) cvtx_chunk<T>(nd, blockIdx.x, rows, sync, spart, w, sv, xs, red, &sLast);
-}
-
-template <class T>
-__global__ void __launch_bounds__(256) compressed_g_kernel(const SNode<T>* __restrict__ nodes,
-                                                           const int* __restrict__ lvl, const T* __restrict__ sv,
-                                                           T* __restrict__ yv) {
-  pdl_enter();
-  const SNode<T>& nd = nodes[lvl[blockIdx.y]];
-  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i < nd.n && nd.r > 0 && nd.m > 0) cg_row<T>(nd, i, sv, yv);
+  const SNode<T>& nd = nodes[wk.node];
+  const int n = nd.n, R = n + nd.m, r0 = wk.b * 64;
+  for (int idx = threadIdx.x; idx < W * W; idx += 256) {
+    const int i = idx / W, j = idx - i * W;
+    Ds[i][j] = (i < n && j <= i) ? nd.Dinv[(size_t)i * n + j] : T(0);
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < 64 * W; idx += 256) {
+    const int i = idx / W, k = idx - i * W, row = r0 + i;
+    T v = T(0);
+    if (k < n && row < R) v = row < n ? Ds[k][row] : nd.L[(size_t)row * nd.ld + k];
+    Rs[i][k] = v;
+  }
+  __syncthreads();
+  const int i = threadIdx.x >> 2, cg = threadIdx.x & 3;
+  T acc[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) acc[q] = T(0);
+  for (int kb = 0; kb < NQ && 4 * kb < n; ++kb) {
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      const T l = Rs[i][4 * kb + kk];
+#pragma unroll
+      for (int q = 0; q < NQ; ++q)
+        if (q <= kb) acc[q] += l * Ds[4 * kb + kk][cg + 4 * q];
+    }
+  }
+  const int row = r0 + i;
+  if (row < R) {
+    T* out = row < n ? nd.Sg + (size_t)row * nd.ldk : nd.G + (size_t)(row - n) * nd.ldk;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+      if (cg + 4 * q < n) out[cg + 4 * q] = acc[q];
+  }
 }
 
 // Inverse of each lower-triangular diagonal block (column c by thread c,
@@ -695,7 +982,7 @@ __global__ void convert_out_kernel(const T* __restrict__ src, double* __restrict
   pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dst[i] = (double)src[i];
-  if (c) clear_piece(c, count);
+  clear_piece(c, count);
 }
 
 }  // namespace
@@ -713,14 +1000,43 @@ void SolveEngine<T>::plan() {
   const int nn = (int)S.nodes.size();
   nodes_.assign(nn, SNode<T>{});
   std::vector<int> rowsAll, rel, child, lvlNodes;
-  long long wuCur = 0, dinvCur = 0, zpCur = 0, spCur = 0, ipCur = 0, xCur = 0, xpCur = 0;
-  int syncCur = SYNC_GLOBAL;   // error word, ticket and completion counters of the interior launches
-  std::vector<long long> xOff(nn, -1);
-  std::vector<long long> xTaskOff;   // per compressed diagonal-block task: offset in the X arena
+  // the single-vector apply's u and t of a supernode, each on whole 32-byte
+  // sectors: a sector has one writer and is written whole (words stored into
+  // part of a sector long evicted cost its reader a fill from DRAM)
+  long long uCur = 0, tCur = 0;
+  auto take = [](long long& cur, int len) {
+    const long long at = cur;
+    cur += (len + 7) & ~7;
+    if (cur > INT_MAX) throw std::runtime_error("solve plan: a work vector has more than 2^31 entries");
+    return (int)at;
+  };
+  long long wuCur = 0, dinvCur = 0, ipCur = 0, xCur = 0, gCur = 0, sCur = 0, wCur = 0;
+  int syncCur = SYNC_GLOBAL;   // batched apply: error word, tickets and completion counters of the interior launches
+  std::vector<long long> xOff(nn, -1), gOff(nn, 0), sOff(nn, 0), wOff(nn, -1);
+  std::vector<long long> xTaskOff;   // per diagonal-block task: offset in the X arena, or -1
   bytesPerApply_ = 0;
   std::vector<int> pos(S.n, -1);
   std::vector<DinvTask<T>> dinvTasks;
   std::vector<long long> dinvTaskOff, dinvNodeOff(nn, 0);
+  // X = L11^{-1} (n x ldx, upper triangle zero): the inverted 64 x 64 diagonal
+  // blocks go in place
+  auto plan_x = [&](int s) {
+    SNode<T>& sn = nodes_[s];
+    sn.ldx = (sn.n + 3) & ~3;
+    xOff[s] = xCur;
+    for (int b = 0; b * SOLVE_RB < sn.n; ++b) {
+      DinvTask<T> t{};
+      t.L = sn.L + (size_t)b * SOLVE_RB * sn.ld + (size_t)b * SOLVE_RB;
+      t.ld = sn.ld;
+      t.h = std::min(SOLVE_RB, sn.n - b * SOLVE_RB);
+      t.pad = t.h;
+      t.ldD = sn.ldx;
+      dinvTasks.push_back(t);
+      dinvTaskOff.push_back(-1);
+      xTaskOff.push_back(xCur + (long long)b * SOLVE_RB * sn.ldx + (long long)b * SOLVE_RB);
+    }
+    xCur += (long long)sn.n * sn.ldx;
+  };
   for (int s = 0; s < nn; ++s) {
     const Node& nd = S.nodes[s];
     SNode<T>& sn = nodes_[s];
@@ -730,6 +1046,8 @@ void SolveEngine<T>::plan() {
     sn.c0 = nd.c0;
     sn.rowsOff = (long long)rowsAll.size();
     rowsAll.insert(rowsAll.end(), nd.rows.begin(), nd.rows.end());
+    sn.uOff = take(uCur, nd.m());
+    sn.tOff = nd.compressed ? 0 : take(tCur, nd.n);
     if (!nd.compressed) {
       sn.L = F_.interior() + F_.frontOff[s];
       sn.r = 0;
@@ -759,42 +1077,37 @@ void SolveEngine<T>::plan() {
         const int hl = nd.n - (nbI - 1) * SOLVE_RB;
         dinvCur += (long long)(nbI - 1) * SOLVE_RB * SOLVE_RB + (long long)hl * hl;
       }
-      bytesPerApply_ += 2.0 * sizeof(T) * (double)(nd.n * (nd.n + 1) / 2 + (double)nd.m() * nd.n);
+      // FP64: an odd row stride in 16-byte units, so that a lane a row reads
+      // shared memory without bank conflicts
+      sn.ldk = (nd.n + 3) & ~3;
+      if (sizeof(T) == 8 && (sn.ldk = (nd.n + 1) & ~1) % 4 == 0) sn.ldk += 2;
+      if (nd.n > SOLVE_RB) plan_x(s);   // S and G follow from it
+      bytesPerApply_ += sizeof(T) * ((double)nd.n * nd.n + 2.0 * nd.m() * nd.n);
     } else {
       sn.L = F_.compressed() + F_.frontOff[s];
       sn.r = F_.rank[s];
       sn.V = sn.r ? F_.vu() + F_.vOff[s] : nullptr;
       sn.U = sn.r ? F_.vu() + F_.uOff[s] : nullptr;
       sn.wuOff = wuCur;
-      wuCur += 2LL * sn.r + sn.m;   // z | s | u = -V z
+      wuCur += 2LL * sn.r + sn.m;   // z | s | u = -V z (z and s: batched apply)
       sn.nb = (nd.n + SOLVE_RB - 1) / SOLVE_RB;
-      sn.nch = (sn.r > 0 && sn.m > 0) ? (sn.m + 127) / 128 : 0;
-      sn.syncOff = syncCur;
-      syncCur += 2;   // row blocks of y done, V chunks of s done
-      sn.ncb = (nd.n + XT_COLS - 1) / XT_COLS;
-      sn.zpOff2 = xpCur;
-      xpCur += (long long)nd.n * sn.nb;
-      sn.zpOff = zpCur;
-      zpCur += (long long)sn.nb * sn.r;
-      sn.spOff = spCur;
-      spCur += (long long)sn.nch * sn.r;
-      // X = L11^{-1}: the inverted 64 x 64 diagonal blocks go in place
-      xOff[s] = xCur;
-      for (int b = 0; b < sn.nb; ++b) {
-        DinvTask<T> t{};
-        t.L = sn.L + (size_t)b * SOLVE_RB * sn.ld + (size_t)b * SOLVE_RB;
-        t.ld = sn.ld;
-        t.h = std::min(SOLVE_RB, nd.n - b * SOLVE_RB);
-        t.pad = t.h;
-        t.ldD = nd.n;
-        dinvTasks.push_back(t);
-        dinvTaskOff.push_back(-1);
-        xTaskOff.push_back(xCur + (long long)b * SOLVE_RB * nd.n + (long long)b * SOLVE_RB);
-      }
-      xCur += (long long)nd.n * nd.n;
+      wOff[s] = wCur;
+      wCur = (wCur + (long long)nd.n * sn.r + 3) & ~3LL;
+      plan_x(s);
       bytesPerApply_ += 2.0 * sizeof(T) * ((double)nd.n * (nd.n + 1) / 2 + (double)sn.r * (nd.m() + nd.n));
     }
   }
+  // G and S of the interior supernodes, in the order of the levels (the members
+  // of a work item are neighbours)
+  for (auto& lv : F_.interiorLevels)
+    for (int pass = 0; pass < 2; ++pass)
+      for (int s : lv)
+        if (group_member(s) == (pass == 0)) {
+          gOff[s] = gCur;
+          gCur += (long long)nodes_[s].m * nodes_[s].ldk;
+          sOff[s] = sCur;
+          sCur += (long long)nodes_[s].n * nodes_[s].ldk;
+        }
   // interior children and rel maps (target index of each row in the parent front)
   for (int s = 0; s < nn; ++s) {
     const Node& nd = S.nodes[s];
@@ -828,90 +1141,41 @@ void SolveEngine<T>::plan() {
       std::stable_sort(pl[s].begin(), pl[s].end(), [](const SPull& a, const SPull& b) { return a.kind < b.kind; });
   iLevels_.clear();
   cLevels_.clear();
-  smemIF_.clear();
-  smemIB_.clear();
   std::vector<RowBlock> iwork;
   for (auto& lv : F_.interiorLevels) {
     iLevels_.push_back({(long long)iwork.size(), 0});
-    size_t f = 8, b = 8;
-    for (int d : lv) {
+    for (int d : lv)
       for (int c = 0; c < std::max(1, nodes_[d].nch); ++c) iwork.push_back(RowBlock{d, c});
-      f = std::max(f, sizeof(T) * S.nodes[d].n);
-      b = std::max(b, sizeof(T) * (((S.nodes[d].n + 1) & ~1) + ICH));
-    }
     iLevels_.back().second = (int)(iwork.size() - iLevels_.back().first);
-    smemIF_.push_back(f);
-    smemIB_.push_back(b);
   }
   // backward order: the levels top-down
   std::vector<RowBlock> iworkB;
   for (int l = (int)iLevels_.size() - 1; l >= 0; --l)
     iworkB.insert(iworkB.end(), iwork.begin() + iLevels_[l].first,
                   iwork.begin() + iLevels_[l].first + iLevels_[l].second);
-  // the single-vector apply: per level, the small supernodes in groups of
-  // eight (a warp each), then the chunk blocks of the others
-  std::vector<RowBlock> iworkS, iworkSB;
-  std::vector<int> small;
-  {
-    std::vector<std::pair<size_t, size_t>> lvRange;   // per level: [begin, end) in iworkS
-    bool anySmall = false;
-    for (auto& lv : F_.interiorLevels) {
-      const size_t b0 = iworkS.size();
-      std::vector<int> sm;
-      for (int d : lv)
-        if (S.nodes[d].n <= IW_N && S.nodes[d].m() <= ICH) sm.push_back(d);
-      for (size_t g = 0; g < sm.size(); g += 8) {
-        const int cnt = (int)std::min<size_t>(8, sm.size() - g);
-        iworkS.push_back(RowBlock{-1 - (int)(small.size() / 8), cnt});
-        for (int q = 0; q < 8; ++q) small.push_back(q < cnt ? sm[g + q] : -1);
-        anySmall = true;
-      }
-      for (int d : lv)
-        if (!(S.nodes[d].n <= IW_N && S.nodes[d].m() <= ICH))
-          for (int c = 0; c < std::max(1, nodes_[d].nch); ++c) iworkS.push_back(RowBlock{d, c});
-      lvRange.push_back({b0, iworkS.size()});
-    }
-    for (int l = (int)lvRange.size() - 1; l >= 0; --l)
-      iworkSB.insert(iworkSB.end(), iworkS.begin() + lvRange[l].first, iworkS.begin() + lvRange[l].second);
-    smemWarps_ = anySmall ? sizeof(T) * 8 * (IW_N + ICH) : 0;
+  // S and G of the supernodes of up to 64 columns: 64-row blocks of [S; G], by
+  // column class (<= 16, <= 32, <= 64)
+  std::vector<RowBlock> opsWork;
+  for (int cls = 0; cls < 3; ++cls) {
+    const int lo = cls == 0 ? 0 : 8 << cls, hi = 16 << cls;
+    opsClass_[cls].first = (long long)opsWork.size();
+    for (int s = 0; s < nn; ++s)
+      if (!S.nodes[s].compressed && S.nodes[s].n > lo && S.nodes[s].n <= hi)
+        for (int b = 0; b * 64 < S.nodes[s].n + S.nodes[s].m(); ++b) opsWork.push_back(RowBlock{s, b});
+    opsClass_[cls].second = (int)(opsWork.size() - opsClass_[cls].first);
   }
-  for (size_t v : smemIB_)
-    if (v > 200 * 1024) throw std::runtime_error("interior front too large for the shared-memory solve");
-  // compressed levels: (supernode, 64-row block) work lists
-  std::vector<RowBlock> tickF;
-  tickOff_.clear();
-  cBlocks_.clear();
-  cMaxCh_.clear();
-  cVzGrid_.clear();
   cRowGrid_.clear();
-  cColGrid_.clear();
   cMRowGrid_.clear();
-  std::vector<XTile> xtiles;
-  cTiles_.clear();
   for (auto& lv : F_.compressedLevels) {
     cLevels_.push_back({(long long)lvlNodes.size(), (int)lv.size()});
     lvlNodes.insert(lvlNodes.end(), lv.begin(), lv.end());
-    tickOff_.push_back((long long)tickF.size());
-    const long long t0 = (long long)xtiles.size();
-    for (int j : lv)   // tiles with a part on or below the diagonal
-      for (int ib = 0; ib < nodes_[j].nb; ++ib)
-        for (int jb = 0; jb < nodes_[j].ncb && jb * XT_COLS <= ib * SOLVE_RB + SOLVE_RB - 1; ++jb)
-          xtiles.push_back(XTile{j, ib, jb});
-    cTiles_.push_back({t0, (int)((long long)xtiles.size() - t0)});
-    int maxCh = 1, blocks = 0, maxN = 1, maxM = 1;
+    int maxN = 1, maxM = 1;
     for (int j : lv) {
-      maxCh = std::max(maxCh, nodes_[j].nch);
-      blocks += nodes_[j].nb;
       maxN = std::max(maxN, nodes_[j].n);
       maxM = std::max(maxM, nodes_[j].m);
-      for (int b = 0; b < nodes_[j].nb; ++b) tickF.push_back(RowBlock{j, b});
     }
-    cBlocks_.push_back(blocks);
-    cMaxCh_.push_back(maxCh);
-    cVzGrid_.push_back(std::min(64, (maxM + 7) / 8));
     cRowGrid_.push_back((maxN + 7) / 8);
     cMRowGrid_.push_back((maxM + 7) / 8);
-    cColGrid_.push_back((maxN + 255) / 256);
   }
   clk.mark("layout");
   cudaStream_t st = F_.stream;
@@ -919,29 +1183,36 @@ void SolveEngine<T>::plan() {
     b.alloc(std::max<size_t>(bytes, 16));
     if (bytes) RSCHOL_CUDA(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, st));
   };
-  dWu_.alloc(sizeof(T) * std::max(1LL, wuCur));
   dDinv_.alloc(sizeof(T) * std::max(1LL, dinvCur));
-  dZp_.alloc(sizeof(T) * std::max(1LL, zpCur));
-  dSp_.alloc(sizeof(T) * std::max(1LL, spCur));
-  dIp_.alloc(sizeof(T) * std::max(1LL, ipCur));
-  dYi_.alloc(sizeof(T) * std::max(1, S.n));
-  dXp_.alloc(sizeof(T) * std::max(1LL, xpCur));
+  dT_.alloc(sizeof(T) * std::max(8LL, tCur));
   dX_.alloc(sizeof(T) * std::max(1LL, xCur));
-  RSCHOL_CUDA(cudaMemsetAsync(dX_.p, 0, sizeof(T) * std::max(1LL, xCur), st));   // upper triangles stay zero
+  RSCHOL_CUDA(cudaMemsetAsync(dX_.p, 0, sizeof(T) * std::max(1LL, xCur), st));   // upper triangles and padding stay zero
+  dG_.alloc(sizeof(T) * std::max(1LL, gCur));
+  dS_.alloc(sizeof(T) * std::max(1LL, sCur));
+  RSCHOL_CUDA(cudaMemsetAsync(dG_.p, 0, dG_.bytes, st));   // the row padding stays zero
+  RSCHOL_CUDA(cudaMemsetAsync(dS_.p, 0, dS_.bytes, st));
+  dWc_.alloc(sizeof(T) * std::max(4LL, wCur));
   for (size_t q = 0; q < dinvTasks.size(); ++q)
     dinvTasks[q].D = xTaskOff[q] >= 0 ? dX_.as<T>() + xTaskOff[q] : dDinv_.as<T>() + dinvTaskOff[q];
   for (int s = 0; s < nn; ++s) {
-    if (S.nodes[s].compressed) nodes_[s].X = dX_.as<T>() + xOff[s];
-    else nodes_[s].Dinv = dDinv_.as<T>() + dinvNodeOff[s];
+    if (xOff[s] >= 0) nodes_[s].X = dX_.as<T>() + xOff[s];
+    if (S.nodes[s].compressed) {
+      nodes_[s].W = dWc_.as<T>() + wOff[s];
+    } else {
+      nodes_[s].Dinv = dDinv_.as<T>() + dinvNodeOff[s];
+      nodes_[s].G = dG_.as<T>() + gOff[s];
+      nodes_[s].Sg = dS_.as<T>() + sOff[s];
+    }
   }
   nDinv_ = (int)dinvTasks.size();
   clk.mark("arenas");
   plan_inverse(xOff);
   clk.mark("inverse");
   // per-row contribution lists of the compressed supernodes (in source order)
+  std::vector<long long> cstart;
+  std::vector<long long> ents;   // offsets into the batched apply's update-vector arena
+  std::vector<int> entsU;        // and into the single-vector one's
   {
-    std::vector<long long> cstart;
-    std::vector<long long> ents;   // offsets into the update-vector arena
     for (int s = 0; s < nn; ++s) {
       const Node& nd = S.nodes[s];
       if (!nd.compressed) continue;
@@ -953,19 +1224,27 @@ void SolveEngine<T>::plan() {
       nodes_[s].cOff = (long long)cstart.size();
       for (int t = 0; t <= nd.n; ++t) cstart.push_back(base + cnt[t]);
       ents.resize(ents.size() + cnt[nd.n]);
+      entsU.resize(ents.size());
       std::vector<int> fill(cnt.begin(), cnt.end() - 1);
       for (const SPull& P : pl[s]) {
         const SNode<T>& src = nodes_[P.src];
         for (int a = P.a0; a < P.a1; ++a) {
           // interior root: its update vector; compressed: u = -V z
           const long long e = (P.kind == 0) ? src.wuOff + a : src.wuOff + 2 * src.r + a;
-          ents[base + fill[S.nodes[P.src].rows[a] - nd.c0]++] = e;
+          const long long at = base + fill[S.nodes[P.src].rows[a] - nd.c0]++;
+          ents[at] = e;
+          entsU[at] = src.uOff + a;
         }
       }
     }
     up(dCStart_, cstart.data(), cstart.size() * sizeof(long long));
     up(dCEnt_, ents.data(), ents.size() * sizeof(long long));
   }
+  dWu_.alloc(sizeof(T) * std::max(8LL, uCur));
+  RSCHOL_CUDA(cudaMemsetAsync(dWu_.p, 0, dWu_.bytes, st));
+  clk.mark("lists");
+  plan_items(rel, cstart, entsU);
+  clk.mark("items");
   up(dNodes_, nodes_.data(), nodes_.size() * sizeof(SNode<T>));
   up(dRows_, rowsAll.data(), rowsAll.size() * sizeof(int));
   up(dRel_, rel.data(), rel.size() * sizeof(int));
@@ -974,40 +1253,607 @@ void SolveEngine<T>::plan() {
   up(dIWork_, iwork.data(), iwork.size() * sizeof(RowBlock));
   up(dIWorkB_, iworkB.data(), iworkB.size() * sizeof(RowBlock));
   nIWork_ = (int)iwork.size();
-  up(dIWorkS_, iworkS.data(), iworkS.size() * sizeof(RowBlock));
-  up(dIWorkSB_, iworkSB.data(), iworkSB.size() * sizeof(RowBlock));
-  up(dSmall_, small.data(), small.size() * sizeof(int));
-  nIWorkS_ = (int)iworkS.size();
+  up(dOpsWork_, opsWork.data(), opsWork.size() * sizeof(RowBlock));
   wuTotal_ = wuCur;
   ipTotal_ = ipCur;
   maxNI_ = 0;
   for (int s = 0; s < nn; ++s)
     if (!S.nodes[s].compressed) maxNI_ = std::max(maxNI_, S.nodes[s].n);
   kB_ = 0;   // the batched apply re-plans on its next use
-  smemIFmax_ = 8;
-  smemIBmax_ = 8;
-  for (size_t v : smemIF_) smemIFmax_ = std::max(smemIFmax_, v);
-  for (size_t v : smemIB_) smemIBmax_ = std::max(smemIBmax_, v);
-  up(dTickF_, tickF.data(), tickF.size() * sizeof(RowBlock));
-  up(dTiles_, xtiles.data(), xtiles.size() * sizeof(XTile));
   up(dDinvTasks_, dinvTasks.data(), dinvTasks.size() * sizeof(DinvTask<T>));
   syncInts_ = syncCur;
-  dSync_.alloc(sizeof(int) * syncCur);
-  RSCHOL_CUDA(cudaMemsetAsync(dSync_.p, 0, sizeof(int) * syncCur, st));
   if (!std::is_same<T, double>::value) dW_.alloc(sizeof(T) * std::max(1, S.n));
   RSCHOL_CUDA(cudaStreamSynchronize(st));
   clk.mark("upload");
-  const int maxSmem = 200 * 1024;
-  RSCHOL_CUDA(cudaFuncSetAttribute(interior_forward_chunks<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxSmem));
-  RSCHOL_CUDA(cudaFuncSetAttribute(interior_backward_chunks<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxSmem));
-  launchesPerApply_ = (iLevels_.empty() ? 0 : 2) + 8 * (long long)cLevels_.size() - (cLevels_.empty() ? 0 : 1) +
-                      (std::is_same<T, double>::value ? (nIWorkS_ > 0 ? 1 : 0) : 2);
+  launchesPerApply_ = 1 + (std::is_same<T, double>::value ? 1 : 2);
   bytesPerApply_ += 8.0 * 4 * S.n;
+}
+
+// Whether an interior supernode joins a group item: at most a warp's lanes of
+// columns and its S and G within one stage.
+template <class T>
+bool SolveEngine<T>::group_member(int s) const {
+  const SNode<T>& sn = nodes_[s];
+  return sn.n <= IW_N && sn.m <= IW_M && (long long)(sn.n + sn.m) * sn.ldk * (long long)sizeof(T) <= ST_DATA;
+}
+
+// The work items of one application, in ticket order, with their descriptors.
+// rel: target index of each row in the parent front (interior children);
+// cstart / ents: contribution lists of the compressed columns.
+template <class T>
+void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<long long>& cstart,
+                                const std::vector<int>& ents) {
+  const Symbolic& S = F_.S;
+  const int nn = (int)S.nodes.size();
+  cudaStream_t st = F_.stream;
+  std::vector<ApplyItem> items;
+  std::vector<int> blob(4, 0), phaseOf;
+  int phase = 0;
+  const int E = (int)sizeof(T);
+  struct Done {   // "finished" of a supernode in one direction: a counter and its target
+    int ctr = -1, target = 0;
+  };
+  std::vector<Done> up(nn), zDone(nn), solved(nn), tDone(nn), sDone(nn), fDone(nn);
+  std::vector<int> upCount(nn, 0);
+  int nCtr = 2;   // [0] error word, [1] ticket
+  std::vector<int> produced(2, 0);
+  auto counter = [&]() {
+    produced.push_back(0);
+    return nCtr++;
+  };
+  auto pairs_of = [&](std::vector<int>& w, const Done& d) {
+    for (size_t q = 0; q + 1 < w.size(); q += 2)
+      if (w[q] == d.ctr) {
+        w[q + 1] = std::max(w[q + 1], d.target);
+        return;
+      }
+    w.push_back(d.ctr);
+    w.push_back(d.target);
+  };
+  auto i32 = [](long long v) {
+    if (v < 0 || v > INT_MAX) throw std::runtime_error("solve plan: a work vector has more than 2^31 entries");
+    return (int)v;
+  };
+  auto bytes16 = [](long long b) { return (int)((b + 15) & ~15LL); };
+  auto open_part = [&]() {   // the blob's next 16-byte boundary
+    blob.resize((blob.size() + 3) & ~(size_t)3, 0);
+    return i32((long long)blob.size());
+  };
+  // Append an item.  Its descriptor is written straight into the blob: begin
+  // (the waits), then the header and the lists, then end; an offset of a list
+  // in the descriptor is the blob's size then minus it.desc.
+  auto begin = [&](ApplyItem& it, const std::vector<int>& waits) {
+    it.waits = (int)waits.size() / 2;
+    for (size_t q = 0; q < waits.size(); q += 2)   // every wait must be met by earlier items
+      if (produced[waits[q]] < waits[q + 1]) throw std::runtime_error("solve plan: an item waits on a later one");
+    it.desc = open_part();
+    blob.insert(blob.end(), waits.begin(), waits.end());
+  };
+  auto off16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 != 0; };
+  auto end = [&](ApplyItem& it) {
+    const long long db = 4LL * (open_part() - it.desc);
+    it.descBytes = db <= ST_DESC ? (int)db : 0;
+    if (it.descBytes == 0 || it.descBytes + it.desc2Bytes > ST_DESC) it.desc2Bytes = 0;
+    // what a bulk copy needs: 16-byte boundaries, and room in a stage
+    if ((it.bytes0 > 0 && off16(it.g0)) || (it.bytes1 > 0 && off16(it.g1)) || (it.bytes0 | it.bytes1) % 16 != 0 ||
+        it.bytes0 + it.bytes1 > ST_DATA)
+      throw std::runtime_error("solve plan: a piece of the factor does not fit its stage");
+    produced[it.sig]++;
+    items.push_back(it);
+    phaseOf.push_back(phase);
+  };
+  auto push = [&](ApplyItem& it, const std::vector<int>& waits, std::initializer_list<int> header) {
+    begin(it, waits);
+    blob.insert(blob.end(), header.begin(), header.end());
+    end(it);
+  };
+
+  // Row stride of partial sums: whole 32-byte sectors, so that an item stores
+  // no part of one (words into a line long evicted cost its reader a fill from
+  // DRAM: c2, 6 us in every reading item)
+  auto part_ld = [](int n) { return (n + 7) & ~7; };
+  // chunks of the larger interior supernodes: rows of G and of S per item
+  struct Chunks {
+    int nch, rc, per, staged, whole;
+  };
+  std::vector<Chunks> ch(nn);
+  long long ipCur = 0;
+  std::vector<long long> ipOff(nn, 0);
+  fLen_ = 4;
+  for (int s = 0; s < nn; ++s) {
+    const SNode<T>& sn = nodes_[s];
+    if (S.nodes[s].compressed || group_member(s)) continue;
+    fLen_ = std::max(fLen_, sn.ldk);
+    Chunks& c = ch[s];
+    const int maxRows = ST_DATA / (sn.ldk * E);
+    c.staged = maxRows >= 8;
+    const int cap = c.staged ? maxRows : 32;   // too wide for a stage: 32 rows, read in place
+    c.nch = std::max(1, (sn.n + sn.m + cap - 1) / cap);
+    // (multiples of a sector, so that a chunk stores whole sectors of u and t,
+    // where a stage holds two of them)
+    const int al = cap >= 2 * (32 / E) ? 32 / E : 1;
+    c.whole = al > 1;
+    for (;; ++c.nch) {
+      c.rc = ((sn.m + c.nch - 1) / c.nch + al - 1) / al * al;
+      c.per = ((sn.n + c.nch - 1) / c.nch + al - 1) / al * al;
+      if (c.rc + c.per <= cap && c.rc <= 64) break;
+    }
+    ipOff[s] = ipCur;
+    ipCur += (long long)c.nch * part_ld(sn.n);
+  }
+  // groups of small supernodes, per level
+  std::vector<std::vector<std::vector<int>>> groups(F_.interiorLevels.size());
+  std::vector<int> childCount(nn, 0);
+  for (size_t l = 0; l < F_.interiorLevels.size(); ++l) {
+    long long bytes = 0, ints = 0;
+    for (int s : F_.interiorLevels[l]) {
+      if (!group_member(s)) continue;
+      const SNode<T>& sn = nodes_[s];
+      const long long b = (long long)(sn.n + sn.m) * sn.ldk * E;
+      long long q = GH + 8 + sn.n + sn.m + 1;
+      for (int c : S.children[s]) q += nodes_[c].m + 2;
+      auto& g = groups[l];
+      if (g.empty() || (int)g.back().size() == GRP || bytes + b > ST_DATA || 4 * (ints + q) > ST_DESC) {
+        g.push_back({});
+        bytes = ints = 0;
+      }
+      g.back().push_back(s);
+      bytes += b;
+      ints += q;
+    }
+  }
+  // the pull lists of a supernode's columns and rows, in child order ...
+  std::vector<int> pStart, pEnt, pFill;
+  auto pull_prepare = [&](int s) {
+    const int R = nodes_[s].n + nodes_[s].m;
+    pStart.assign(R + 1, 0);
+    for (int c : S.children[s]) {
+      const int* rl = rel.data() + nodes_[c].relOff;
+      for (int a = 0; a < nodes_[c].m; ++a) pStart[rl[a] + 1]++;
+    }
+    for (int t = 0; t < R; ++t) pStart[t + 1] += pStart[t];
+    pEnt.resize(pStart[R]);
+    pFill.assign(pStart.begin(), pStart.end() - 1);
+    for (int c : S.children[s]) {
+      const int* rl = rel.data() + nodes_[c].relOff;
+      for (int a = 0; a < nodes_[c].m; ++a) pEnt[pFill[rl[a]]++] = nodes_[c].uOff + a;
+    }
+  };
+  // ... and those of its rows [r0, r0 + count) of [columns; rows], appended to the
+  // blob as offsets and entries
+  auto pull_lists = [&](int r0, int count) {
+    const int e0 = pStart[r0];
+    for (int i = 0; i <= count; ++i) blob.push_back(pStart[r0 + i] - e0);
+    blob.insert(blob.end(), pEnt.begin() + e0, pEnt.begin() + pStart[r0 + count]);
+  };
+  auto has_pull = [&](int s) {
+    for (int c : S.children[s])
+      if (nodes_[c].m > 0) return true;
+    return false;
+  };
+  std::vector<int> waits;
+  // ---- interior, forward
+  for (size_t l = 0; l < F_.interiorLevels.size(); ++l) {
+    ++phase;
+    for (auto& g : groups[l]) {
+      ApplyItem it{};
+      it.kind = IT_FGRP;
+      it.sig = counter();
+      it.count = (int)g.size();
+      const SNode<T>& first = nodes_[g[0]];
+      it.g0 = first.G;
+      it.g1 = first.Sg;
+      waits.clear();
+      long long gE = 0, sE = 0;
+      for (int s : g) {
+        gE += (long long)nodes_[s].m * nodes_[s].ldk;
+        sE += (long long)nodes_[s].n * nodes_[s].ldk;
+        for (int c : S.children[s]) pairs_of(waits, up[c]);
+      }
+      it.bytes0 = (int)(gE * E);
+      it.bytes1 = (int)(sE * E);
+      begin(it, waits);
+      const size_t h0 = blob.size();
+      blob.resize(h0 + GH * g.size(), 0);
+      for (size_t q = 0; q < g.size(); ++q) {
+        const int s = g[q];
+        const SNode<T>& sn = nodes_[s];
+        int* h = &blob[h0 + GH * q];
+        h[0] = sn.n;
+        h[1] = sn.m;
+        h[2] = sn.c0;
+        h[3] = sn.uOff;
+        h[4] = (int)(sn.G - first.G);
+        h[5] = (int)(gE + (sn.Sg - first.Sg));
+        h[7] = sn.ldk;
+        h[8] = sn.tOff;
+        if (has_pull(s)) {
+          h[6] = (int)blob.size() - it.desc;
+          pull_prepare(s);
+          pull_lists(0, sn.n + sn.m);
+        }
+        up[s] = fDone[s] = Done{it.sig, 1};
+      }
+      end(it);
+    }
+    for (int s : F_.interiorLevels[l]) {
+      if (group_member(s)) continue;
+      const SNode<T>& sn = nodes_[s];
+      const Chunks& c = ch[s];
+      waits.clear();
+      for (int k : S.children[s]) pairs_of(waits, up[k]);
+      up[s] = fDone[s] = Done{counter(), c.nch};
+      const bool pull = has_pull(s);
+      int shared = 0, sharedBytes = 0;
+      if (pull) {   // the columns' lists, once for all chunks
+        pull_prepare(s);
+        shared = open_part();
+        pull_lists(0, sn.n);
+        sharedBytes = 4 * (open_part() - shared);
+      }
+      for (int b = 0; b < c.nch; ++b) {
+        const int a0 = std::min(sn.m, b * c.rc), rows = std::min(c.rc, sn.m - a0);
+        const int s0 = std::min(sn.n, b * c.per), sr = std::min(c.per, sn.n - s0);
+        ApplyItem it{};
+        it.kind = IT_FWD;
+        it.sig = up[s].ctr;
+        it.g0 = sn.G + (size_t)a0 * sn.ldk;
+        it.g1 = sn.Sg + (size_t)s0 * sn.ldk;
+        if (c.staged) {
+          it.bytes0 = rows * sn.ldk * E;
+          it.bytes1 = sr * sn.ldk * E;
+        }
+        it.desc2 = shared;
+        it.desc2Bytes = sharedBytes;
+        begin(it, waits);
+        const int list = pull ? (int)blob.size() - it.desc + 10 : 0;
+        blob.insert(blob.end(), {sn.n, rows, sn.c0, sn.uOff + a0, s0, sr, list, sn.ldk, sn.tOff, c.whole});
+        if (pull) pull_lists(sn.n + a0, rows);
+        end(it);
+      }
+    }
+  }
+  // ---- compressed levels
+  const int L = (int)F_.compressedLevels.size();
+  auto rows_per = [&](int r, int& staged) {   // rows of an r-wide matrix per item
+    if (r == 0) {
+      staged = 0;
+      return ROWS8;
+    }
+    const int fit = ST_DATA / (r * E) & ~7;
+    staged = fit >= 8;
+    return staged ? std::min(ROWS8, fit) : 16;
+  };
+  long long zpCur = 0, spCur = 0, ypCur = 0, xpCur = 0;
+  std::vector<long long> zpOff(nn), spOff(nn), ypOff(nn), xpOff(nn);
+  // Many partials of z or s are added once, by items of CR_COLS columns, before
+  // the items that read the sums: each of those would otherwise add all of them
+  // (c2: 200 partials of s, 8 us in every item; with the extra step 1.5 + 1.5).
+  // Up to CR_MIN partials the extra step costs more than it saves.
+  constexpr int CR_COLS = 16, CR_MIN = 12;
+  auto emit_cr = [&](Done& d, long long& off, int rp, int isS) {
+    const int parts = d.target;
+    if (parts <= CR_MIN) return parts;
+    waits.clear();
+    pairs_of(waits, d);
+    const long long sums = off + (long long)parts * rp;   // the row after the partials
+    const Done all{counter(), (rp + CR_COLS - 1) / CR_COLS};
+    for (int k0 = 0; k0 < rp; k0 += CR_COLS) {
+      ApplyItem it{};
+      it.kind = IT_CR;
+      it.sig = all.ctr;
+      push(it, waits, {i32(off + k0), parts, rp, std::min(CR_COLS, rp - k0), i32(sums + k0), isS});
+    }
+    d = all;
+    off = sums;
+    return 1;
+  };
+  std::vector<int> zParts(nn, 0), sParts(nn, 0);
+  std::vector<int> yBase(nn, -1);   // first of the supernode's per-row-block counters of y
+  constexpr int YR = Y_ROWS, YC = Y_COLS<T>, TR = T_ROWS<T>;
+  for (int j = 0; j < nn; ++j) {
+    if (!S.nodes[j].compressed) continue;
+    const SNode<T>& sn = nodes_[j];
+    int sg = 0;
+    const int cb = rows_per(sn.r, sg), rp = part_ld(sn.r);
+    zpOff[j] = zpCur;
+    zpCur += (long long)((sn.n + cb - 1) / cb + 1) * rp;
+    spOff[j] = spCur;
+    spCur += (long long)((sn.m + cb - 1) / cb + 1) * rp;
+    ypOff[j] = ypCur;
+    ypCur += (long long)part_ld(sn.n) * ((sn.n + YC - 1) / YC);
+    xpOff[j] = xpCur;
+    xpCur += (long long)part_ld(sn.n) * ((sn.n + TR - 1) / TR);
+  }
+  auto emit_cf = [&](int l) {
+    ++phase;
+    for (int j : F_.compressedLevels[l]) {
+      const SNode<T>& sn = nodes_[j];
+      int sg = 0;
+      const int cb = rows_per(sn.r, sg), rp = part_ld(sn.r), nb = (sn.n + cb - 1) / cb;
+      waits.clear();
+      for (int c : S.children[j]) pairs_of(waits, up[c]);
+      zDone[j] = Done{counter(), nb};
+      up[j] = zDone[j];
+      for (int b = 0; b < nb; ++b) {
+        const int j0 = b * cb, cols = std::min(cb, sn.n - j0);
+        ApplyItem it{};
+        it.kind = IT_CF;
+        it.sig = zDone[j].ctr;
+        it.g0 = sn.W + (size_t)j0 * sn.r;
+        it.bytes0 = sg ? bytes16((long long)cols * sn.r * E) : 0;
+        begin(it, waits);
+        const int list = (int)blob.size() - it.desc + 5;
+        blob.insert(blob.end(), {sn.c0 + j0, cols, sn.r, i32(zpOff[j] + (long long)b * rp), list});
+        const long long* cs = &cstart[sn.cOff + j0];
+        for (int i = 0; i <= cols; ++i) blob.push_back(i32(cs[i] - cs[0]));
+        blob.insert(blob.end(), ents.begin() + cs[0], ents.begin() + cs[cols]);
+        end(it);
+      }
+    }
+  };
+  std::vector<Done> zSum(nn);   // z of a supernode ready to be read
+  auto emit_cu = [&](int l) {
+    ++phase;
+    for (int j : F_.compressedLevels[l]) {
+      zSum[j] = zDone[j];
+      if (nodes_[j].m > 0 && nodes_[j].r > 0) zParts[j] = emit_cr(zSum[j], zpOff[j], part_ld(nodes_[j].r), 0);
+    }
+    for (int j : F_.compressedLevels[l]) {
+      const SNode<T>& sn = nodes_[j];
+      if (sn.m == 0 || sn.r == 0) continue;
+      int sg = 0;
+      const int rb = rows_per(sn.r, sg), nb = (sn.m + rb - 1) / rb;
+      waits.clear();
+      pairs_of(waits, zSum[j]);
+      up[j] = Done{counter(), nb};
+      for (int b = 0; b < nb; ++b) {
+        const int a0 = b * rb, rows = std::min(rb, sn.m - a0);
+        ApplyItem it{};
+        it.kind = IT_CU;
+        it.sig = up[j].ctr;
+        it.g0 = sn.V + (size_t)a0 * sn.r;
+        it.bytes0 = sg ? bytes16((long long)rows * sn.r * E) : 0;
+        push(it, waits, {rows, sn.r, i32(zpOff[j]), zParts[j], sn.uOff + a0});
+      }
+    }
+  };
+  // a tile of X: its packed copy, one stage
+  std::vector<PackTile> packs;
+  std::vector<int> packItems;   // items whose g0 is the tile of the same place in packs
+  auto tile_of = [&](ApplyItem& it, int j, int j0, int i0, int boxCols, int boxRows) {
+    packItems.push_back((int)items.size());
+    packs.push_back(PackTile{j, i0, j0, boxCols, boxRows});
+    it.bytes0 = ST_DATA;
+  };
+  auto emit_y = [&](int l) {
+    ++phase;
+    for (int j : F_.compressedLevels[l]) {
+      const SNode<T>& sn = nodes_[j];
+      const int ncb = (sn.n + YC - 1) / YC, nt = (sn.n + TR - 1) / TR;
+      waits.clear();
+      pairs_of(waits, zDone[j]);
+      yBase[j] = nCtr;
+      for (int q = 0; q < nt; ++q) counter();
+      for (int i0 = 0; i0 < sn.n; i0 += YR)
+        for (int jb = 0; jb * YC <= i0 + YR - 1 && jb < ncb; ++jb) {
+          const int j0 = jb * YC, rows = std::min(YR, sn.n - i0);
+          const int cols = std::min({YC, sn.n - j0, i0 + rows - j0});   // up to the diagonal
+          if (cols <= 0) throw std::runtime_error("solve plan: an empty tile");
+          ApplyItem it{};
+          it.kind = IT_Y;
+          it.sig = yBase[j] + i0 / TR;
+          tile_of(it, j, j0, i0, YC, YR);
+          push(it, waits, {sn.c0 + j0, cols, rows, i32(ypOff[j] + (long long)jb * part_ld(sn.n) + i0)});
+        }
+    }
+  };
+  auto emit_t = [&](int l) {
+    ++phase;
+    for (int j : F_.compressedLevels[l]) {
+      const SNode<T>& sn = nodes_[j];
+      const int ncb = (sn.n + YC - 1) / YC, nt = (sn.n + TR - 1) / TR;
+      tDone[j] = Done{counter(), 0};
+      for (int ib = 0; ib < nt; ++ib) {
+        const int i0 = ib * TR, rows = std::min(TR, sn.n - i0);
+        std::vector<int> waits;
+        pairs_of(waits, Done{yBase[j] + ib, produced[yBase[j] + ib]});
+        for (int j0 = 0; j0 <= i0 + TR - 1 && j0 < sn.n; j0 += T_COLS) {
+          const int cols = std::min(T_COLS, sn.n - j0);
+          ApplyItem it{};
+          it.kind = IT_XT;
+          it.sig = tDone[j].ctr;
+          tDone[j].target++;
+          tile_of(it, j, j0, i0, T_COLS, TR);
+          push(it, waits, {rows, cols, i32(ypOff[j] + i0), part_ld(sn.n), i0,
+                                i32(xpOff[j] + (long long)ib * part_ld(sn.n) + j0), ncb});
+        }
+      }
+    }
+  };
+  auto emit_cs = [&](int l) {
+    ++phase;
+    for (int j : F_.compressedLevels[l]) {
+      const SNode<T>& sn = nodes_[j];
+      if (sn.m == 0 || sn.r == 0) continue;
+      int sg = 0;
+      const int rb = rows_per(sn.r, sg), rp = part_ld(sn.r), nb = (sn.m + rb - 1) / rb;
+      waits.clear();
+      pairs_of(waits, solved[S.nodes[j].parent]);
+      sDone[j] = Done{counter(), nb};
+      for (int b = 0; b < nb; ++b) {
+        const int a0 = b * rb, rows = std::min(rb, sn.m - a0);
+        ApplyItem it{};
+        it.kind = IT_CS;
+        it.sig = sDone[j].ctr;
+        it.g0 = sn.V + (size_t)a0 * sn.r;
+        it.bytes0 = sg ? bytes16((long long)rows * sn.r * E) : 0;
+        begin(it, waits);
+        const int list = (int)blob.size() - it.desc + 4;
+        blob.insert(blob.end(), {rows, sn.r, i32(spOff[j] + (long long)b * rp), list});
+        blob.insert(blob.end(), S.nodes[j].rows.begin() + a0, S.nodes[j].rows.begin() + a0 + rows);
+        end(it);
+      }
+    }
+    for (int j : F_.compressedLevels[l])
+      if (sDone[j].ctr >= 0) sParts[j] = emit_cr(sDone[j], spOff[j], part_ld(nodes_[j].r), 1);
+  };
+  auto emit_cx = [&](int l) {
+    ++phase;
+    for (int j : F_.compressedLevels[l]) {
+      const SNode<T>& sn = nodes_[j];
+      int sg = 0;
+      const int cb = rows_per(sn.r, sg), nb = (sn.n + cb - 1) / cb, nt = (sn.n + TR - 1) / TR;
+      waits.clear();
+      pairs_of(waits, tDone[j]);
+      if (sDone[j].ctr >= 0) pairs_of(waits, sDone[j]);
+      solved[j] = Done{counter(), nb};
+      for (int b = 0; b < nb; ++b) {
+        const int j0 = b * cb, cols = std::min(cb, sn.n - j0);
+        ApplyItem it{};
+        it.kind = IT_CX;
+        it.sig = solved[j].ctr;
+        it.g0 = sn.W + (size_t)j0 * sn.r;
+        it.bytes0 = sg && sDone[j].ctr >= 0 ? bytes16((long long)cols * sn.r * E) : 0;
+        push(it, waits, {sn.c0 + j0, cols, sn.r, i32(spOff[j]), sParts[j],
+                              i32(xpOff[j] + j0), part_ld(sn.n), j0, j0 / T_COLS * T_COLS / TR, nt});
+      }
+    }
+  };
+  // The products with X follow their level's up pieces one level behind, so
+  // that the chain up the tree comes first and they fill its gaps.
+  for (int l = 0; l < L; ++l) {
+    emit_cf(l);
+    emit_cu(l);
+    if (l >= 1) emit_y(l - 1);
+    if (l >= 2) emit_t(l - 2);
+  }
+  if (L >= 1) emit_y(L - 1);
+  if (L >= 1) emit_t(L - 1);
+  if (L >= 2) emit_t(L - 2);
+  for (int l = L - 1; l >= 0; --l) {
+    emit_cs(l);
+    emit_cx(l);
+  }
+  // ---- interior, backward
+  for (int l = (int)F_.interiorLevels.size() - 1; l >= 0; --l) {
+    ++phase;
+    auto wait_for = [&](int s, std::vector<int>& waits) {
+      const int p = S.nodes[s].parent;
+      pairs_of(waits, p >= 0 ? solved[p] : fDone[s]);
+    };
+    for (int s : F_.interiorLevels[l]) {
+      if (group_member(s)) continue;
+      const SNode<T>& sn = nodes_[s];
+      const Chunks& c = ch[s];
+      waits.clear();
+      wait_for(s, waits);
+      const int nch = sn.m > 0 ? (sn.m + c.rc - 1) / c.rc : 1;
+      const Done parts{counter(), nch};
+      for (int b = 0; b < nch; ++b) {
+        const int a0 = b * c.rc, rows = std::min(c.rc, sn.m - a0);
+        ApplyItem it{};
+        it.kind = IT_BWD;
+        it.sig = parts.ctr;
+        it.g0 = sn.G + (size_t)a0 * sn.ldk;
+        it.bytes0 = c.staged ? rows * sn.ldk * E : 0;
+        begin(it, waits);
+        const int list = (int)blob.size() - it.desc + 10;
+        blob.insert(blob.end(), {sn.n, rows, sn.c0, i32(ipOff[s]), b, nch, list, sn.ldk, part_ld(sn.n), sn.tOff});
+        blob.insert(blob.end(), S.nodes[s].rows.begin() + a0, S.nodes[s].rows.begin() + a0 + rows);
+        end(it);
+      }
+      solved[s] = parts;
+    }
+    for (auto& g : groups[l]) {
+      ApplyItem it{};
+      it.kind = IT_BGRP;
+      it.sig = counter();
+      it.count = (int)g.size();
+      const SNode<T>& first = nodes_[g[0]];
+      it.g0 = first.G;
+      long long gE = 0;
+      waits.clear();
+      for (int s : g) {
+        gE += (long long)nodes_[s].m * nodes_[s].ldk;
+        wait_for(s, waits);
+      }
+      it.bytes0 = (int)(gE * E);
+      begin(it, waits);
+      const size_t h0 = blob.size();
+      blob.resize(h0 + GH * g.size(), 0);
+      for (size_t q = 0; q < g.size(); ++q) {
+        const SNode<T>& sn = nodes_[g[q]];
+        int* h = &blob[h0 + GH * q];
+        h[0] = sn.n;
+        h[1] = sn.m;
+        h[2] = sn.c0;
+        h[4] = (int)(sn.G - first.G);
+        h[6] = (int)blob.size() - it.desc;
+        h[7] = sn.ldk;
+        h[8] = sn.tOff;
+        blob.insert(blob.end(), S.nodes[g[q]].rows.begin(), S.nodes[g[q]].rows.end());
+        solved[g[q]] = Done{it.sig, 1};
+      }
+      end(it);
+    }
+    ++phase;
+    // the sums of a level's chunks after all of them: next to its chunks such
+    // an item would hold up its group
+    for (int s : F_.interiorLevels[l]) {
+      if (group_member(s) || solved[s].target == 1) continue;
+      ApplyItem it{};
+      it.kind = IT_BR;
+      it.sig = counter();
+      waits.clear();
+      pairs_of(waits, solved[s]);
+      push(it, waits, {nodes_[s].n, nodes_[s].c0, i32(ipOff[s]), solved[s].target, part_ld(nodes_[s].n),
+                            nodes_[s].tOff});
+      solved[s] = Done{it.sig, 1};
+    }
+  }
+  nItems_ = (int)items.size();
+  // shared memory: the stages, and per consumer group two areas of GT vectors
+  // and the f buffer (or a group item's buffers in their place)
+  work_ = (std::max(GW * (IW_N + IW_M), 2 * GT * Vec16<T>::V + fLen_) + 3) & ~3;
+  smem_ = (size_t)NSTAGE * ST_BYTES + NGRP * sizeof(T) * (size_t)work_;
+  if (smem_ > 226 * 1024) throw std::runtime_error("interior front too large for the shared-memory solve");
+  RSCHOL_CUDA(cudaFuncSetAttribute(apply_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_));
+  int dev = 0, sms = 0, per = 0;
+  RSCHOL_CUDA(cudaGetDevice(&dev));
+  RSCHOL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  RSCHOL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, apply_kernel<T>, NGRP * GT + 32, smem_));
+  grid_ = std::min(std::max(1, nItems_), sms * std::max(1, per));
+  // phases that a few items per group work off
+  std::vector<int> count(phase + 1, 0);
+  for (int q : phaseOf) count[q]++;
+  for (size_t q = 0; q < items.size(); ++q) items[q].shallow = count[phaseOf[q]] <= SHALLOW * NGRP * grid_;
+  nSync_ = nCtr;
+  auto upload = [&](DevBuf& b, const void* src, size_t bytes) {
+    b.alloc(std::max<size_t>(bytes, 16));
+    if (bytes) RSCHOL_CUDA(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, st));
+  };
+  nPacks_ = (int)packs.size();
+  upload(dPackTiles_, packs.data(), packs.size() * sizeof(PackTile));
+  dPacked_.alloc(std::max<size_t>(16, packs.size() * (size_t)ST_DATA));
+  for (size_t q = 0; q < packItems.size(); ++q)
+    items[packItems[q]].g0 = dPacked_.as<unsigned char>() + q * (size_t)ST_DATA;
+  upload(dItems_, items.data(), items.size() * sizeof(ApplyItem));
+  upload(dBlob_, blob.data(), blob.size() * sizeof(int));
+  dSync_.alloc(sizeof(int) * nCtr);
+  RSCHOL_CUDA(cudaMemsetAsync(dSync_.p, 0, sizeof(int) * nCtr, st));
+  dZp_.alloc(sizeof(T) * std::max(4LL, zpCur));
+  dSp_.alloc(sizeof(T) * std::max(4LL, spCur));
+  dYp_.alloc(sizeof(T) * std::max(1LL, ypCur));
+  dXp_.alloc(sizeof(T) * std::max(1LL, xpCur));
+  dIp_.alloc(sizeof(T) * std::max(1LL, ipCur));
+  RSCHOL_CUDA(cudaStreamSynchronize(st));   // the host arrays go out of scope
 }
 
 template <class T>
 void SolveEngine<T>::plan_inverse(const std::vector<long long>& xOff) {
-  // X = L11^{-1} of every compressed supernode by recursive doubling: with
+  // X = L11^{-1} of every compressed supernode, and of the interior ones of
+  // more than 64 columns, by recursive doubling: with
   // the diagonal 64 x 64 inverses in place, for block sizes sz = 64, 128, ...
   // every pair (A, B) of consecutive sz-blocks gets X_BA = -X_BB (L_BA X_AA).
   // Both products run by 64-column (64-row) blocks whose K stops at the
@@ -1018,13 +1864,13 @@ void SolveEngine<T>::plan_inverse(const std::vector<long long>& xOff) {
   const int nn = (int)S.nodes.size();
   int maxN = 0;
   for (int s = 0; s < nn; ++s)
-    if (S.nodes[s].compressed) maxN = std::max(maxN, S.nodes[s].n);
+    if (xOff[s] >= 0) maxN = std::max(maxN, S.nodes[s].n);
   long long t1Max = 1;
   for (int sz = SOLVE_RB; sz < maxN; sz *= 2) {
     long long t1 = 0;
     for (int s = 0; s < nn; ++s) {
       const int n = S.nodes[s].n;
-      if (!S.nodes[s].compressed) continue;
+      if (xOff[s] < 0) continue;
       for (int A0 = 0; A0 + sz < n; A0 += 2 * sz) t1 += (long long)std::min(sz, n - A0 - sz) * sz;
     }
     t1Max = std::max(t1Max, t1);
@@ -1073,8 +1919,8 @@ void SolveEngine<T>::plan_inverse(const std::vector<long long>& xOff) {
     std::vector<GemmTask<T>> b1, b2;
     long long t1cur = 0;
     for (int s = 0; s < nn; ++s) {
-      if (!S.nodes[s].compressed) continue;
-      const int n = S.nodes[s].n, ld = nodes_[s].ld;
+      if (xOff[s] < 0) continue;
+      const int n = S.nodes[s].n, ld = nodes_[s].ld, lx = nodes_[s].ldx;
       const T* L = nodes_[s].L;
       T* X = dX_.as<T>() + xOff[s];
       for (int A0 = 0; A0 + sz < n; A0 += 2 * sz) {
@@ -1083,18 +1929,47 @@ void SolveEngine<T>::plan_inverse(const std::vector<long long>& xOff) {
         t1cur += (long long)bsz * sz;
         for (int a = 0; a * SOLVE_RB < sz; ++a)   // T1[:, a] = L_BA[:, a:] X_AA[a:, a]
           b1.push_back(mk(L + (size_t)B0 * ld + A0 + a * SOLVE_RB, ld,
-                          X + (size_t)(A0 + a * SOLVE_RB) * n + A0 + a * SOLVE_RB, n, T1 + a * SOLVE_RB, sz, bsz,
+                          X + (size_t)(A0 + a * SOLVE_RB) * lx + A0 + a * SOLVE_RB, lx, T1 + a * SOLVE_RB, sz, bsz,
                           SOLVE_RB, sz - a * SOLVE_RB, T(1)));
         for (int b = 0; b * SOLVE_RB < bsz; ++b) {   // X_BA[b, :] = -X_BB[b, :b] T1[:b, :]
           const int hb = std::min(SOLVE_RB, bsz - b * SOLVE_RB), K = std::min(bsz, (b + 1) * SOLVE_RB);
-          b2.push_back(mk(X + (size_t)(B0 + b * SOLVE_RB) * n + B0, n, T1, sz,
-                          X + (size_t)(B0 + b * SOLVE_RB) * n + A0, n, hb, sz, K, T(-1)));
+          b2.push_back(mk(X + (size_t)(B0 + b * SOLVE_RB) * lx + B0, lx, T1, sz,
+                          X + (size_t)(B0 + b * SOLVE_RB) * lx + A0, lx, hb, sz, K, T(-1)));
         }
       }
     }
     flush(b1);
     flush(b2);
   }
+  // then the products the apply reads: W = X^T U of the compressed supernodes,
+  // S = X^T X and G = L21 X of the interior ones of more than 64 columns, by
+  // blocks whose K starts at the triangle
+  std::vector<GemmTask<T>> bw, bi;
+  for (int s = 0; s < nn; ++s) {
+    const SNode<T>& sn = nodes_[s];
+    const int n = sn.n, lx = sn.ldx;
+    if (S.nodes[s].compressed) {
+      for (int j0 = 0; sn.r > 0 && j0 < n; j0 += rpt) {
+        GemmTask<T> t = mk(sn.X + (size_t)j0 * lx + j0, lx, sn.U + (size_t)j0 * sn.r, sn.r,
+                           const_cast<T*>(sn.W) + (size_t)j0 * sn.r, sn.r, std::min(rpt, n - j0), sn.r, n - j0, T(1));
+        t.tA = 1;
+        bw.push_back(t);
+      }
+    } else if (xOff[s] >= 0) {
+      for (int i0 = 0; i0 < n; i0 += rpt) {
+        const int h = std::min(rpt, n - i0);
+        GemmTask<T> t = mk(sn.X + (size_t)i0 * lx + i0, lx, sn.X + (size_t)i0 * lx, lx, sn.Sg + (size_t)i0 * sn.ldk,
+                           sn.ldk, h, n, n - i0, T(1));
+        t.tA = 1;
+        bi.push_back(t);
+        if (sn.m > 0)
+          bi.push_back(mk(sn.L + (size_t)n * sn.ld + i0, sn.ld, sn.X + (size_t)i0 * lx + i0, lx, sn.G + i0, sn.ldk,
+                          sn.m, h, n - i0, T(1)));
+      }
+    }
+  }
+  flush(bw);
+  flush(bi);
   dXGemm_.alloc(std::max<size_t>(16, tasks.size() * sizeof(GemmTask<T>)));
   if (!tasks.empty())
     RSCHOL_CUDA(cudaMemcpyAsync(dXGemm_.p, tasks.data(), tasks.size() * sizeof(GemmTask<T>), cudaMemcpyHostToDevice,
@@ -1114,6 +1989,19 @@ int SolveEngine<T>::prepare(cudaStream_t st) {
     RSCHOL_LAUNCH_CHECK();
     ++launches;
   }
+  // S and G of the interior supernodes of up to 64 columns
+  auto ops = [&](auto kernel, int cls, int nq) {
+    if (opsClass_[cls].second == 0) return;
+    const int smem = (int)sizeof(T) * (4 * nq + 64) * (4 * nq + 1);
+    if (smem > 48 * 1024) RSCHOL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kernel<<<opsClass_[cls].second, 256, smem, st>>>(dNodes_.as<SNode<T>>(),
+                                                     dOpsWork_.as<RowBlock>() + opsClass_[cls].first);
+    RSCHOL_LAUNCH_CHECK();
+    ++launches;
+  };
+  ops(interior_ops_kernel<T, 4>, 0, 4);
+  ops(interior_ops_kernel<T, 8>, 1, 8);
+  ops(interior_ops_kernel<T, 16>, 2, 16);
   for (const XStep& x : xSteps_) {
     const GemmTask<T>* d = dXGemm_.as<GemmTask<T>>() + x.off;
     if constexpr (std::is_same<T, float>::value) {
@@ -1122,6 +2010,11 @@ int SolveEngine<T>::prepare(cudaStream_t st) {
     } else {
       launch_gemm<T>(d, x.count, x.tiles, st);
     }
+    ++launches;
+  }
+  if (nPacks_ > 0) {
+    pack_tiles_kernel<T><<<nPacks_, 256, 0, st>>>(dNodes_.as<SNode<T>>(), dPackTiles_.as<PackTile>(), dPacked_.as<T>());
+    RSCHOL_LAUNCH_CHECK();
     ++launches;
   }
   return launches;
@@ -1135,7 +2028,7 @@ int SolveEngine<T>::take_error(cudaStream_t st) {
   RSCHOL_CUDA(cudaStreamSynchronize(st));
   if (e) {
     // a wait gave up: counters and flags are in an unknown state; start over
-    RSCHOL_CUDA(cudaMemsetAsync(dSync_.p, 0, sizeof(int) * syncInts_, st));
+    RSCHOL_CUDA(cudaMemsetAsync(dSync_.p, 0, sizeof(int) * nSync_, st));
     RSCHOL_CUDA(cudaStreamSynchronize(st));
   }
   return e;
@@ -1150,52 +2043,19 @@ void SolveEngine<T>::apply_inplace(double* w64, cudaStream_t st) {
     launch_k(convert_kernel<double, T>, dim3((n + 255) / 256), dim3(256), 0, st, w64, w, n);
     RSCHOL_LAUNCH_CHECK();
   }
-  const int* lvl = dLevelNodes_.as<int>();
   int* sync = dSync_.as<int>();
-  const int epoch = 1;   // completion targets: every apply starts its counters at zero
-  if (nIWorkS_ > 0) {
-    launch_k(interior_forward_chunks<T>, dim3(nIWorkS_), dim3(256), std::max(smemIFmax_, smemWarps_), st, dNodes_.as<SNode<T>>(), dIWorkS_.as<RowBlock>(), dRel_.as<int>(), dChild_.as<int>(), sync, epoch, w, dYi_.as<T>(), dWu_.as<T>(), dSmall_.as<int>());
-    RSCHOL_LAUNCH_CHECK();
-  }
-  T* yv = dYi_.as<T>();
-  for (size_t l = 0; l < cLevels_.size(); ++l) {
-    const int* lv = lvl + cLevels_[l].first;
-    launch_k(compressed_gather_rows<T>, dim3(cRowGrid_[l], cLevels_[l].second), dim3(256), 0, st, dNodes_.as<SNode<T>>(), lv, dCStart_.as<long long>(), dCEnt_.as<long long>(), dWu_.as<T>(), w);
-    RSCHOL_LAUNCH_CHECK();
-    launch_k(compressed_ytile_kernel<T>, dim3(cTiles_[l].second), dim3(256), 0, st, dNodes_.as<SNode<T>>(), dTiles_.as<XTile>() + cTiles_[l].first, w, dXp_.as<T>());
-    RSCHOL_LAUNCH_CHECK();
-    launch_k(compressed_y_kernel<T>, dim3(cBlocks_[l]), dim3(256), 0, st, dNodes_.as<SNode<T>>(), dTickF_.as<RowBlock>() + tickOff_[l], sync, dZp_.as<T>(), dXp_.as<T>(), yv, dWu_.as<T>());
-    RSCHOL_LAUNCH_CHECK();
-    if (l + 1 < cLevels_.size()) {   // the top level's u feeds no one
-      launch_k(compressed_vz_kernel<T>, dim3(cVzGrid_[l], cLevels_[l].second), dim3(256), 0, st, dNodes_.as<SNode<T>>(), lv, dWu_.as<T>());
-      RSCHOL_LAUNCH_CHECK();
-    }
-  }
-  for (int l = (int)cLevels_.size() - 1; l >= 0; --l) {
-    const int* lv = lvl + cLevels_[l].first;
-    launch_k(compressed_vtx_kernel<T>, dim3(cMaxCh_[l], cLevels_[l].second), dim3(256), 0, st, dNodes_.as<SNode<T>>(), lv, dRows_.as<int>(), sync, dSp_.as<T>(), w, dWu_.as<T>());
-    RSCHOL_LAUNCH_CHECK();
-    launch_k(compressed_g_kernel<T>, dim3(cRowGrid_[l], cLevels_[l].second), dim3(256), 0, st, dNodes_.as<SNode<T>>(), lv, dWu_.as<T>(), yv);
-    RSCHOL_LAUNCH_CHECK();
-    launch_k(compressed_xtile_kernel<T>, dim3(cTiles_[l].second), dim3(256), 0, st, dNodes_.as<SNode<T>>(), dTiles_.as<XTile>() + cTiles_[l].first, yv, dXp_.as<T>());
-    RSCHOL_LAUNCH_CHECK();
-    launch_k(compressed_x_reduce<T>, dim3(cColGrid_[l], cLevels_[l].second), dim3(256), 0, st, dNodes_.as<SNode<T>>(), lv, dXp_.as<T>(), w);
-    RSCHOL_LAUNCH_CHECK();
-  }
-  if (nIWorkS_ > 0) {
-    launch_k(interior_backward_chunks<T>, dim3(nIWorkS_), dim3(256), std::max(smemIBmax_, smemWarps_), st, dNodes_.as<SNode<T>>(), dIWorkSB_.as<RowBlock>(), dRows_.as<int>(), sync, epoch, dIp_.as<T>(), dYi_.as<T>(), w, dSmall_.as<int>());
-    RSCHOL_LAUNCH_CHECK();
-  }
-  // the interior counters are cleared by the apply's last kernel
-  int* clr = nIWorkS_ > 0 ? sync + SYNC_GLOBAL : nullptr;
-  const int nClr = nIWorkS_ > 0 ? syncInts_ - SYNC_GLOBAL : 0;
+  const ApplyArgs<T> args{dItems_.as<ApplyItem>(), nItems_,         dBlob_.as<int>(), sync,          w,
+                          dT_.as<T>(),             dWu_.as<T>(),    dZp_.as<T>(),     dSp_.as<T>(),  dYp_.as<T>(),
+                          dXp_.as<T>(),            dIp_.as<T>(),    work_};
+  launch_k(apply_kernel<T>, dim3(grid_), dim3(NGRP * GT + 32), smem_, st, args);
+  RSCHOL_LAUNCH_CHECK();
+  // ticket and counters are cleared by the apply's last kernel
   if (!std::is_same<T, double>::value) {
-    launch_k(convert_out_kernel<T>, dim3((n + 255) / 256), dim3(256), 0, st, (const T*)w, w64, n, clr, nClr);
-    RSCHOL_LAUNCH_CHECK();
-  } else if (nClr > 0) {
-    launch_k(clear_counters, dim3((nClr + 1023) / 1024), dim3(256), 0, st, clr, nClr);
-    RSCHOL_LAUNCH_CHECK();
+    launch_k(convert_out_kernel<T>, dim3((n + 255) / 256), dim3(256), 0, st, (const T*)w, w64, n, sync + 1, nSync_ - 1);
+  } else {
+    launch_k(clear_counters, dim3((nSync_ + 1023) / 1024), dim3(256), 0, st, sync + 1, nSync_ - 1);
   }
+  RSCHOL_LAUNCH_CHECK();
 }
 
 template class SolveEngine<double>;

@@ -8,23 +8,20 @@
 // A_{rest,I} L_I^{-T} L_I^{-1} are stored explicitly), compressed nodes use
 // the (HODLR-expanded) dense L11 and the V U^T off-diagonal.
 //
-// Forward: interior supernodes in one launch, one thread block per
-// (supernode, 128-row chunk of L21) taken in level order from a ticket
-// counter; each waits (bounded) for its children's chunk blocks, assembles
-// their update vectors (extend-add, fixed order) for the supernode's columns
-// and its chunk, solves with L11 and forms its chunk of the update vector.
-// Compressed levels bottom-up: a gather pass adds each row's fixed-order
-// contribution list (interior-root update vectors, u_c = -V_c z_c of
-// compressed descendants, formed by a launch after each level); y = X f with
-// X = L11^{-1}, formed once per factorisation (inverted 64 x 64 diagonal
-// blocks, then recursive doubling X_BA = -X_BB L_BA X_AA with batched GEMMs),
-// so the triangular solve becomes a GEMV with no chain of dependent blocks;
-// z = U^T y is reduced in fixed order by the last row block to finish.
-// Backward mirrors this (s = V^T x_R, g = y - U s, x = X^T g), then the
-// interior supernodes top-down in one launch (each waits for its parent's
-// solve; chunk blocks form parts of L21^T x_R, the last one to finish sums
-// them in fixed order and solves with L11^T).  No atomics touch
-// the numbers: results are bitwise reproducible.
+// Every supernode is applied through products formed once per factorisation,
+// so that no triangular chain lies between the levels of the tree:
+//   interior    S = (L11 L11^T)^{-1}, G = L21 L11^{-1}:
+//               up u = (children's rows) - G f, t = S f; down x = t - G^T x_R
+//   compressed  X = L11^{-1}, W = X^T U (L21 = V U^T):
+//               up z = W^T f, u = -V z; across t = X^T (X f);
+//               down s = V^T x_R, x = t - W s
+// (the same operator up to rounding: L11^{-T} (L11^{-1} f - L21^T x_R)).
+// X by inverted 64 x 64 diagonal blocks and recursive doubling X_BA = -X_BB
+// L_BA X_AA with batched GEMMs; W, and S and G above 64 columns, by batched
+// GEMMs; S and G of the small supernodes by one kernel.
+// One persistent launch works the whole application off as a list of items in
+// topological order (solve.cu).  Every sum has a fixed order and no atomics
+// touch the numbers: results are bitwise reproducible.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -38,7 +35,6 @@
 namespace rschol {
 
 constexpr int SOLVE_RB = 64;   // rows per compressed row block
-constexpr int XT_COLS = 256;   // columns per tile of X = L11^{-1} in the apply GEMVs
 
 template <class T>
 struct SNode {
@@ -46,21 +42,24 @@ struct SNode {
   const T* V;       // compressed: m x r
   const T* U;       // compressed: n x r
   const T* Dinv;    // interior: inverted 64 x 64 diagonal blocks of L11 (the last one h x h)
-  const T* X;       // compressed: L11^{-1} (n x n, row-major, upper triangle zero)
+  const T* X;       // compressed, and interior of n > 64: L11^{-1} (n x ldx, row-major, upper triangle zero)
+  T* G;             // interior: L21 L11^{-1} (m x ldk)
+  T* Sg;            // interior: (L11 L11^T)^{-1} (n x ldk)
+  const T* W;       // compressed: X^T U (n x r)
   int ld, n, m, r, c0;
   int childBegin, childEnd;   // interior: children (range in the child list)
-  int nb, nch;                // compressed: row blocks of L11; both: 128-row chunks of V / L21
-  int syncOff;                // compressed: 2 completion counters; interior: backward chunk
-                              // counter, forward completion count, backward solved flag
+  int nb, nch;                // compressed: 64-row blocks of L11; interior: 128-row chunks of L21 (batched apply)
+  int ldk, ldx;               // row strides of G and Sg, and of X
+  int uOff, tOff;             // single vector: update vector (interior: children's rows - G f, compressed:
+                              // -V z), and t = S f of an interior supernode
+  int syncOff;                // interior (batched apply): backward chunk counter, forward completion
+                              // count, backward solved flag
   int parentI;                // interior: parent if it is interior, else -1
   long long rowsOff;          // rows of this node in the row arena
-  long long wuOff;            // interior: update vector; compressed: z (r), s (r), u = -V z (m)
+  long long wuOff;            // batched apply: interior: update vector; compressed: z (r), s (r), u = -V z (m)
   long long relOff;           // interior: target index in the parent front of each row
   long long cOff;             // compressed: first of its n+1 contribution-list offsets
-  long long zpOff, spOff;     // compressed: partials of z (nb x r) and s (nch x r);
-                              // interior (zpOff): partials of L21^T x_R (nch x n)
-  long long zpOff2;           // compressed: tile partials of X f (n x ncb) and X^T g (n x nb)
-  int ncb;                    // compressed: 256-column blocks of X
+  long long zpOff;            // interior (batched apply): partials of L21^T x_R (nch x n)
 };
 
 struct SPull {       // contribution source of a compressed supernode (plan time)
@@ -73,8 +72,22 @@ struct RowBlock {    // one thread block's work: (supernode, row block or chunk)
   int node, b;
 };
 
-struct XTile {       // a 64 x 256 tile of X = L11^{-1} (row block ib, column block jb)
-  int node, ib, jb;
+struct PackTile {    // a tile of X packed for the apply: rows from i0, columns from j0
+  int node, i0, j0, cols, rows;
+};
+
+struct alignas(16) ApplyItem {   // one work item of the single-vector apply
+  const void* g0;   // its pieces of the factor ...
+  const void* g1;
+  int kind;
+  int bytes0, bytes1;          // ... and their bytes to stage (0: read in place, or none)
+  int desc, descBytes;         // descriptor: offset in the blob (ints), bytes to stage (0: read in place)
+  int waits;                   // (counter, target) pairs at the descriptor's start
+  int sig;                     // counter released when the item is done
+  int count;                   // members of a group
+  int shallow;                 // an item of a phase of few items (ticket draw)
+  int desc2, desc2Bytes;       // a part of the descriptor that several items share
+  int pad;
 };
 
 template <class T>
@@ -129,30 +142,26 @@ class SolveEngine {
   FactorEngine<T>& F_;
   std::vector<SNode<T>> nodes_;
   DevBuf dNodes_, dRows_, dRel_, dChild_, dWu_, dW_, dLevelNodes_, dCStart_, dCEnt_;
-  DevBuf dDinv_, dDinvTasks_, dZp_, dSp_, dIp_, dYi_, dSync_, dTickF_, dIWork_, dIWorkB_;
+  DevBuf dDinv_, dDinvTasks_, dZp_, dSp_, dIp_, dT_, dYp_, dXp_, dSync_, dIWork_, dIWorkB_;
   int nIWork_ = 0;
-  size_t smemIFmax_ = 8, smemIBmax_ = 8;
-  // single-vector apply: work lists with the small interior supernodes in
-  // groups of eight (a warp each; group members in dSmall_)
-  DevBuf dIWorkS_, dIWorkSB_, dSmall_;
-  int nIWorkS_ = 0;
-  size_t smemWarps_ = 0;
-  DevBuf dX_, dT1_, dXGemm_;          // compressed L11^{-1}, its temporaries and GEMM tasks
-  DevBuf dXp_, dTiles_;               // tile partials of the X products, tile lists
-  std::vector<std::pair<long long, int>> cTiles_;   // per compressed level: (offset, count) of tiles
+  // single-vector apply: the work items and their descriptors, the counters
+  // ([0] error word, [1] ticket), the launch shape
+  DevBuf dItems_, dBlob_, dPackTiles_, dPacked_;
+  int nPacks_ = 0;
+  int nItems_ = 0, nSync_ = 0, grid_ = 1, fLen_ = 4, work_ = 0;
+  size_t smem_ = 0;
+  bool group_member(int s) const;
+  void plan_items(const std::vector<int>& rel, const std::vector<long long>& cstart, const std::vector<int>& ents);
+  DevBuf dG_, dS_, dWc_, dOpsWork_;                 // G and S of the interior, W of the compressed supernodes
+  std::pair<long long, int> opsClass_[3];           // work of interior_ops_kernel per column class
+  DevBuf dX_, dT1_, dXGemm_;          // L11^{-1}, its temporaries and GEMM tasks
   std::vector<XStep> xSteps_;
   int nDinv_ = 0;
   int syncInts_ = 0;
-  std::vector<long long> tickOff_;   // per compressed level: first ticket entry
-  std::vector<int> cBlocks_;         // per compressed level: row blocks
-  std::vector<int> cMaxCh_;          // per compressed level: most V chunks of a node
-  std::vector<int> cVzGrid_;         // per compressed level: row blocks of the u = -V z launch
   std::vector<int> cRowGrid_;        // per compressed level: 8-row blocks of the largest supernode
-  std::vector<int> cColGrid_;        // per compressed level: 256-column blocks of the largest supernode
   void plan_inverse(const std::vector<long long>& xOff);   // GEMM schedule of X = L11^{-1}
   std::vector<std::pair<long long, int>> iLevels_;  // (offset, count) into the interior work list
   std::vector<std::pair<long long, int>> cLevels_;  // (offset, count) into the level node list
-  std::vector<size_t> smemIF_, smemIB_;
   long long launchesPerApply_ = 0;
   double bytesPerApply_ = 0;
   // batched apply: work buffers sized for the widest k seen (they only grow,

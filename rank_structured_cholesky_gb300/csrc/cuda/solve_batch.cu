@@ -610,7 +610,7 @@ void SolveEngine<T>::plan_batch(int k, int cwR, int cwC) {
       T* wj = w + (size_t)nd.c0 * k;
       for (int ib = 0; ib < nd.nb; ++ib) {   // Y = X F by row blocks
         const int h = std::min(64, n - ib * 64), K = std::min(n, (ib + 1) * 64);
-        gy.push_back(mk(nd.X + (size_t)ib * 64 * n, n, false, wj, k, yj + (size_t)ib * 64 * k, k, h, k, K, T(1),
+        gy.push_back(mk(nd.X + (size_t)ib * 64 * nd.ldx, nd.ldx, false, wj, k, yj + (size_t)ib * 64 * k, k, h, k, K, T(1),
                         T(0)));
       }
       if (r > 0) {
@@ -623,7 +623,7 @@ void SolveEngine<T>::plan_batch(int k, int cwR, int cwC) {
       }
       for (int jb = 0; jb < nd.nb; ++jb) {   // X = X^T G by column blocks
         const int h = std::min(64, n - jb * 64), K = n - jb * 64;
-        gx.push_back(mk(nd.X + (size_t)jb * 64 * n + jb * 64, n, true, yj + (size_t)jb * 64 * k, k,
+        gx.push_back(mk(nd.X + (size_t)jb * 64 * nd.ldx + jb * 64, nd.ldx, true, yj + (size_t)jb * 64 * k, k,
                         wj + (size_t)jb * 64 * k, k, h, k, K, T(1), T(0)));
       }
     }
