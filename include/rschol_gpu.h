@@ -147,13 +147,13 @@ int rschol_precond_apply_device(rschol_factor* f, const double* d_b, double* d_x
 int rschol_precond_apply_device_noalloc(rschol_factor* f, const double* d_b, double* d_x, int nrhs);
 
 /* Autotuner of the batched apply (no reference counterpart): times the
- * candidate tile shapes (interior (row, column) pair tiles, column groups of
- * the compressed-level products) of every width class (number of
- * right-hand sides rounded up to a power of two) up to max_columns and keeps
- * the fastest for this factor; run it while the GPU is otherwise quiet.  No
- * candidate changes any result: every shape forms each column's sums in the
- * same order.  Untuned classes use fixed shapes.  The choices are listed in
- * rschol_factor_describe ("batch_tuning": class, RA, RC, cwR, cwC, ms). */
+ * candidate launch shapes (persistent thread blocks per SM) of every width
+ * class (number of right-hand sides rounded up to a power of two) up to
+ * max_columns and keeps the fastest for this factor; run it while the GPU is
+ * otherwise quiet.  No candidate changes any result: every shape forms each
+ * column's sums in the same order.  Untuned classes use a fixed shape.  The
+ * choices are listed in rschol_factor_describe ("batch_tuning": class, blocks
+ * per SM, columns per pass, 0, 0, ms). */
 int rschol_factor_autotune(rschol_factor* f, int max_columns);
 
 /* Autotuner of the factor's schedule (no reference counterpart): times

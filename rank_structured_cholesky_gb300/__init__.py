@@ -289,7 +289,7 @@ class GpuFactor:
         return x, (info[0] if nrhs == 1 else info)
 
     def autotune(self, max_columns=64):
-        """Time the batched apply's tile shapes for every width class up to max_columns."""
+        """Time the batched apply's launch shapes for every width class up to max_columns."""
         st = load_library().rschol_factor_autotune(self.h, max_columns)
         if st != RSCHOL_OK:
             raise RscholError(st, self.ctx.last_error())

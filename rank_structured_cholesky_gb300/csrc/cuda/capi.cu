@@ -791,7 +791,7 @@ const char* rschol_factor_describe(rschol_factor* f) {
   }
   o << ", \"batch_tuning\": [";
   bool first = true;
-  for (const auto& row : f->impl->batch_tuning()) {   // per width class: class, RA, RC, cwR, cwC, ms
+  for (const auto& row : f->impl->batch_tuning()) {   // per width class: class, blocks per SM, columns per pass, 0, 0, ms
     o << (first ? "" : ", ") << "[" << row[0] << ", " << row[1] << ", " << row[2] << ", " << row[3] << ", " << row[4]
       << ", " << row[5] << "]";
     first = false;

@@ -4,6 +4,7 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include "apply_dev.cuh"
 #include "solve.cuh"
 #include "solve_dev.cuh"
 
@@ -12,175 +13,6 @@ namespace rschol {
 namespace {
 
 using namespace solvedev;
-
-// 16-byte vectors of the factor's type.
-template <class T> struct Vec16;
-template <> struct Vec16<float> {
-  using type = float4;
-  static constexpr int V = 4;
-};
-template <> struct Vec16<double> {
-  using type = double2;
-  static constexpr int V = 2;
-};
-__device__ __forceinline__ float vdot(float4 a, float4 b, float s) {
-  return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s))));
-}
-__device__ __forceinline__ double vdot(double2 a, double2 b, double s) { return fma(a.y, b.y, fma(a.x, b.x, s)); }
-__device__ __forceinline__ void vaxpy(float4& acc, float4 a, float x) {
-  acc.x = fmaf(a.x, x, acc.x);
-  acc.y = fmaf(a.y, x, acc.y);
-  acc.z = fmaf(a.z, x, acc.z);
-  acc.w = fmaf(a.w, x, acc.w);
-}
-__device__ __forceinline__ void vaxpy(double2& acc, double2 a, double x) {
-  acc.x = fma(a.x, x, acc.x);
-  acc.y = fma(a.y, x, acc.y);
-}
-__device__ __forceinline__ void vadd(float4& a, float4 b) {
-  a.x += b.x;
-  a.y += b.y;
-  a.z += b.z;
-  a.w += b.w;
-}
-__device__ __forceinline__ void vadd(double2& a, double2 b) {
-  a.x += b.x;
-  a.y += b.y;
-}
-__device__ __forceinline__ float4 vzero(float) { return make_float4(0.f, 0.f, 0.f, 0.f); }
-__device__ __forceinline__ double2 vzero(double) { return make_double2(0.0, 0.0); }
-__device__ __forceinline__ void vshfl_add(float4& v, int o) {
-  v.x += __shfl_xor_sync(FULL, v.x, o);
-  v.y += __shfl_xor_sync(FULL, v.y, o);
-  v.z += __shfl_xor_sync(FULL, v.z, o);
-  v.w += __shfl_xor_sync(FULL, v.w, o);
-}
-__device__ __forceinline__ void vshfl_add(double2& v, int o) {
-  v.x += __shfl_xor_sync(FULL, v.x, o);
-  v.y += __shfl_xor_sync(FULL, v.y, o);
-}
-
-// ---------------------------------------------------------------------------
-// The apply engine: one persistent launch runs a whole preconditioner
-// application as a list of work items (ApplyItem) in a topological order.
-//
-// Roles: a CTA is one producer warp and two groups of four consumer warps.  The
-// producer takes the next item from a ticket counter and bulk-copies
-// (cp.async.bulk, completion on an mbarrier) its descriptor and its piece of
-// the factor into one of three shared-memory stages, running ahead of the
-// consumers: the factor does not depend on the right-hand side, so its bytes
-// arrive while earlier items still wait or compute.  The groups take the items
-// in turn: a group waits (bounded) until the counters the item names have
-// reached their targets, gathers the vector entries, forms the products from
-// shared memory, stores, and one thread releases the item's own counter.  An
-// item is about 3 us of dependent steps whatever its bytes, so what counts is
-// the bytes being worked on at once: six groups an SM.
-//
-// Every item waits only on items earlier in the list (checked when the list is
-// built) and a group works its tickets in order, so the smallest unfinished
-// ticket can always proceed, whatever else shares the GPU.  The next kernel
-// (clear_counters / convert_out_kernel) zeroes ticket and counters, so the
-// launch needs no host state and replays inside a CUDA graph.
-//
-// Bound: a chain of hand-overs (release, poll, gather, product: ~3 us each, one
-// or two a tree level and direction), then the factor's bytes.  The triangles X
-// and the products with S lie off that chain and fill its gaps.  Measured, one
-// application (before: a triangular solve per supernode on the chain, two
-// ticketed launches for the interior and eight launches per compressed level):
-// 3D 64^3 FP32 0.914 -> 0.376 ms (591 MB, 0.087 ms at the copy rate), 3D 96^3
-// FP32 2.23 -> 1.18 ms, 2D 193 x 187 FP64 0.632 -> 0.149 ms, 2D 40 x 37 FP64
-// 0.159 -> 0.066 ms.  Two groups of four warps against one of eight (half the
-// items in work at once): 3D 64^3 0.400 against 0.494 ms.
-
-constexpr int ST_DATA = 16384, ST_DESC = 4096, ST_BYTES = ST_DATA + ST_DESC;
-constexpr int NSTAGE = 3;
-constexpr int NGRP = 2, GT = 128, GW = GT / 32;   // consumer groups of a CTA, threads and warps of one
-constexpr int IW_N = 32, IW_M = 128;     // members of a group item: n <= IW_N, m <= IW_M
-constexpr int GRP = 8;                   // most members of a group
-constexpr int GH = 10;                   // header words of a member
-constexpr int SHALLOW = 1;               // phases of up to this many items a group (in all CTAs) draw tickets singly
-constexpr int ROWS8 = 8 * GW;            // most rows of W or V in an item (eight a warp)
-
-enum ItemKind : int { IT_FGRP = 0, IT_FWD, IT_CF, IT_CU, IT_Y, IT_XT, IT_CS, IT_CX, IT_BGRP, IT_BWD, IT_CR, IT_BR, IT_END };
-
-// tile of X of the Y = X f items (rows x columns) and of the t = X^T y items
-constexpr int Y_ROWS = 16, T_COLS = 64;
-template <class T> constexpr int Y_COLS = ST_DATA / Y_ROWS / (int)sizeof(T);
-template <class T> constexpr int T_ROWS = ST_DATA / T_COLS / (int)sizeof(T);
-
-// barrier of the caller's consumer group (bar.sync wants whole warps)
-__device__ __forceinline__ void cbar() {
-  __syncwarp();
-  asm volatile("bar.sync %0, 128;" ::"r"(1 + (int)(threadIdx.x / GT)) : "memory");
-}
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(unsigned bar, int count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect(unsigned bar, int bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_test(unsigned bar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Warp-wide wait for a phase: lane 0 polls, for at most about four seconds;
-// false when it gave up.
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
-  int ok = 1;
-  if ((threadIdx.x & 31) == 0 && !mbar_test(bar, parity)) {
-    unsigned long long t0, t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-    for (int it = 1; !mbar_test(bar, parity); ++it) {
-      if (it > 64) __nanosleep(20);
-      if ((it & 255) == 0) {
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-        if (t - t0 > 4000000000ull) {
-          ok = 0;
-          break;
-        }
-      }
-    }
-  }
-  ok = __shfl_sync(FULL, ok, 0);
-  __syncwarp();   // what lane 0 has seen complete, the others may read
-  return ok != 0;
-}
-// global -> shared, 16-byte aligned addresses and size, completion on bar
-__device__ __forceinline__ void bulk_copy(void* dst, const void* src, int bytes, unsigned bar) {
-  asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
-
-// Warp-wide bounded wait until every listed counter has reached its target
-// (pairs of counter index and target).
-__device__ __forceinline__ void wait_list(const int* pairs, int count, const int* sync, int* err) {
-  const int lane = threadIdx.x & 31;
-  for (int c0 = 0; c0 < count; c0 += 32) {
-    const bool have = c0 + lane < count;
-    const int idx = have ? pairs[2 * (c0 + lane)] : 0, target = have ? pairs[2 * (c0 + lane) + 1] : 0;
-    for (int it = 0;; ++it) {
-      const bool ok = !have || ld_acquire(sync + idx) >= target;
-      if (__all_sync(FULL, ok)) break;
-      if (it >= SPIN_LIMIT) {
-        if (lane == 0) atomicExch(err, 1);
-        return;
-      }
-      if ((it & 63) == 63 && __any_sync(FULL, ld_volatile(err) != 0)) return;
-      if (it) __nanosleep(20);
-    }
-  }
-}
 
 // v[i] + the pull list [b[i], e[i]) of wu entries, in order, for N targets at
 // once: the loads of a round (two entries a target) are all in flight together.
@@ -269,23 +101,6 @@ __device__ __forceinline__ void cols_gemv(const T* M, int r, int h, const T* v, 
     }
   }
 }
-
-template <class T>
-struct ApplyArgs {
-  const ApplyItem* items;
-  int nItems;
-  const int* blob;
-  int* sync;        // [0] error word, [1] ticket, then the counters
-  T* w;             // permuted vector, in place
-  T* t;             // S f of the interior columns
-  T* wu;            // update vectors
-  T* zp;            // partials of z = W^T f
-  T* sp;            // partials of s = V^T x_R
-  T* yp;            // partials of X f
-  T* xp;            // partials of X^T y
-  T* ip;            // partials of G^T x_R
-  int work;         // elements of a group's work area in shared memory
-};
 
 // A group of small interior supernodes, forward: u = (children's rows) - G f
 // and t = S f; a warp a member, or several when there are fewer members.  FP32:
@@ -618,68 +433,7 @@ __global__ void __launch_bounds__(NGRP * GT + 32, 3) apply_kernel(ApplyArgs<T> A
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   if (threadIdx.x >= NGRP * GT) {   // ---- producer
-    unsigned full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[NSTAGE]);
-    // Tickets are drawn in pairs (one latency for two items) as far ahead as
-    // there are stages -- except in a phase of few items (ApplyItem::shallow),
-    // where a CTA that holds more than a group's worth keeps items from idle
-    // CTAs: there the next single ticket waits for the last item but one
-    // (c2 apply: 0.39 ms in pairs throughout, 0.376 ms so).
-    int have = 0, ends = 0;   // items read ahead (0 ... 2)
-    bool more = true;
-    ApplyItem cur, nxt;
-    for (int k = 0;; ++k) {
-      const int s = k % NSTAGE, use = k / NSTAGE;
-      if (have == 0 && more) {
-        const int want = k > 0 && cur.shallow ? 1 : 2;
-        if (want == 1 && k > 1) mbar_wait(empty0 + 8 * ((k - 2) % NSTAGE), ((k - 2) / NSTAGE) & 1);
-        int tk = 0;
-        if (lane == 0) tk = atomicAdd(A.sync + 1, want);
-        tk = __shfl_sync(FULL, tk, 0);
-        if (tk < A.nItems) {
-          nxt = A.items[tk];
-          have = 1;
-        }
-        more = tk + want <= A.nItems;
-        if (want == 2 && tk + 1 < A.nItems) {
-          cur = nxt;
-          nxt = A.items[tk + 1];
-          have = 2;
-        } else {
-          cur = nxt;
-        }
-      } else if (have == 1) {
-        cur = nxt;
-      }
-      const bool end = have == 0;
-      if (!end) --have;
-      bool ok = true;
-      if (use > 0) ok = mbar_wait(empty0 + 8 * s, (use - 1) & 1);
-      if (!ok && lane == 0) atomicExch(err, 4);
-      if (end || !ok) {   // one end mark per group
-        if (lane == 0) {
-          sItem[s].kind = IT_END;
-          mbar_arrive(full0 + 8 * s);
-        }
-        more = false;
-        have = 0;
-        if (++ends == NGRP) break;
-        continue;
-      }
-      const ApplyItem& it = cur;
-      unsigned char* st = apsm + (size_t)s * ST_BYTES;
-      if (lane == 0) {
-        sItem[s] = it;
-        const int total = it.descBytes + it.desc2Bytes + it.bytes0 + it.bytes1;
-        mbar_expect(full0 + 8 * s, total);
-        if (it.descBytes) bulk_copy(st + ST_DATA, A.blob + it.desc, it.descBytes, full0 + 8 * s);
-        if (it.desc2Bytes) bulk_copy(st + ST_DATA + it.descBytes, A.blob + it.desc2, it.desc2Bytes, full0 + 8 * s);
-      }
-      __syncwarp();
-      if (lane == 0) {
-        if (it.bytes0) bulk_copy(st, it.g0, it.bytes0, full0 + 8 * s);
-        if (it.bytes1) bulk_copy(st + it.bytes0, it.g1, it.bytes1, full0 + 8 * s);
-      }
-    }
+    apply_producer<T>(A, apsm, sItem, smem_u32(&bars[0]), smem_u32(&bars[NSTAGE]));
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     return;
   }
@@ -999,7 +753,7 @@ void SolveEngine<T>::plan() {
   const Symbolic& S = F_.S;
   const int nn = (int)S.nodes.size();
   nodes_.assign(nn, SNode<T>{});
-  std::vector<int> rowsAll, rel, child, lvlNodes;
+  std::vector<int> rel;
   // the single-vector apply's u and t of a supernode, each on whole 32-byte
   // sectors: a sector has one writer and is written whole (words stored into
   // part of a sector long evicted cost its reader a fill from DRAM)
@@ -1010,8 +764,7 @@ void SolveEngine<T>::plan() {
     if (cur > INT_MAX) throw std::runtime_error("solve plan: a work vector has more than 2^31 entries");
     return (int)at;
   };
-  long long wuCur = 0, dinvCur = 0, ipCur = 0, xCur = 0, gCur = 0, sCur = 0, wCur = 0;
-  int syncCur = SYNC_GLOBAL;   // batched apply: error word, tickets and completion counters of the interior launches
+  long long dinvCur = 0, xCur = 0, gCur = 0, sCur = 0, wCur = 0;
   std::vector<long long> xOff(nn, -1), gOff(nn, 0), sOff(nn, 0), wOff(nn, -1);
   std::vector<long long> xTaskOff;   // per diagonal-block task: offset in the X arena, or -1
   bytesPerApply_ = 0;
@@ -1044,38 +797,21 @@ void SolveEngine<T>::plan() {
     sn.n = nd.n;
     sn.m = nd.m();
     sn.c0 = nd.c0;
-    sn.rowsOff = (long long)rowsAll.size();
-    rowsAll.insert(rowsAll.end(), nd.rows.begin(), nd.rows.end());
     sn.uOff = take(uCur, nd.m());
     sn.tOff = nd.compressed ? 0 : take(tCur, nd.n);
     if (!nd.compressed) {
       sn.L = F_.interior() + F_.frontOff[s];
       sn.r = 0;
-      sn.wuOff = wuCur;
-      wuCur += nd.m();
-      sn.nch = (nd.m() + ICH - 1) / ICH;
-      sn.syncOff = syncCur;
-      syncCur += 3;   // backward chunk counter, forward completion count, backward solved flag
-      sn.parentI = (nd.parent >= 0 && !S.nodes[nd.parent].compressed) ? nd.parent : -1;
-      sn.zpOff = ipCur;
-      ipCur += (long long)sn.nch * nd.n;
-      // inverted 64 x 64 diagonal blocks, the last one stored h x h
-      const int nbI = (nd.n + SOLVE_RB - 1) / SOLVE_RB;
-      for (int b = 0; b < nbI; ++b) {
+      if (nd.n <= SOLVE_RB) {   // D = L11^{-1} in one block: S and G follow from it
         DinvTask<T> t{};
-        t.L = sn.L + (size_t)b * SOLVE_RB * sn.ld + (size_t)b * SOLVE_RB;
+        t.L = sn.L;
         t.ld = sn.ld;
-        t.h = std::min(SOLVE_RB, nd.n - b * SOLVE_RB);
-        t.pad = t.h;
-        t.ldD = t.h;
+        t.h = t.pad = t.ldD = nd.n;
         dinvTasks.push_back(t);
-        dinvTaskOff.push_back(dinvCur + (long long)b * SOLVE_RB * SOLVE_RB);
+        dinvTaskOff.push_back(dinvCur);
         xTaskOff.push_back(-1);
-      }
-      dinvNodeOff[s] = dinvCur;
-      {
-        const int hl = nd.n - (nbI - 1) * SOLVE_RB;
-        dinvCur += (long long)(nbI - 1) * SOLVE_RB * SOLVE_RB + (long long)hl * hl;
+        dinvNodeOff[s] = dinvCur;
+        dinvCur += (long long)nd.n * nd.n;
       }
       // FP64: an odd row stride in 16-byte units, so that a lane a row reads
       // shared memory without bank conflicts
@@ -1088,9 +824,6 @@ void SolveEngine<T>::plan() {
       sn.r = F_.rank[s];
       sn.V = sn.r ? F_.vu() + F_.vOff[s] : nullptr;
       sn.U = sn.r ? F_.vu() + F_.uOff[s] : nullptr;
-      sn.wuOff = wuCur;
-      wuCur += 2LL * sn.r + sn.m;   // z | s | u = -V z (z and s: batched apply)
-      sn.nb = (nd.n + SOLVE_RB - 1) / SOLVE_RB;
       wOff[s] = wCur;
       wCur = (wCur + (long long)nd.n * sn.r + 3) & ~3LL;
       plan_x(s);
@@ -1108,13 +841,10 @@ void SolveEngine<T>::plan() {
           sOff[s] = sCur;
           sCur += (long long)nodes_[s].n * nodes_[s].ldk;
         }
-  // interior children and rel maps (target index of each row in the parent front)
+  // rel maps (target index of each interior child's row in the parent front)
   for (int s = 0; s < nn; ++s) {
     const Node& nd = S.nodes[s];
     if (nd.compressed) continue;
-    nodes_[s].childBegin = (int)child.size();
-    for (int c : S.children[s]) child.push_back(c);
-    nodes_[s].childEnd = (int)child.size();
     for (int a = 0; a < nd.m(); ++a) pos[nd.rows[a]] = a;
     for (int c : S.children[s]) {
       const Node& cn = S.nodes[c];
@@ -1139,20 +869,6 @@ void SolveEngine<T>::plan() {
   for (int s = 0; s < nn; ++s)
     if (S.nodes[s].compressed)
       std::stable_sort(pl[s].begin(), pl[s].end(), [](const SPull& a, const SPull& b) { return a.kind < b.kind; });
-  iLevels_.clear();
-  cLevels_.clear();
-  std::vector<RowBlock> iwork;
-  for (auto& lv : F_.interiorLevels) {
-    iLevels_.push_back({(long long)iwork.size(), 0});
-    for (int d : lv)
-      for (int c = 0; c < std::max(1, nodes_[d].nch); ++c) iwork.push_back(RowBlock{d, c});
-    iLevels_.back().second = (int)(iwork.size() - iLevels_.back().first);
-  }
-  // backward order: the levels top-down
-  std::vector<RowBlock> iworkB;
-  for (int l = (int)iLevels_.size() - 1; l >= 0; --l)
-    iworkB.insert(iworkB.end(), iwork.begin() + iLevels_[l].first,
-                  iwork.begin() + iLevels_[l].first + iLevels_[l].second);
   // S and G of the supernodes of up to 64 columns: 64-row blocks of [S; G], by
   // column class (<= 16, <= 32, <= 64)
   std::vector<RowBlock> opsWork;
@@ -1163,19 +879,6 @@ void SolveEngine<T>::plan() {
       if (!S.nodes[s].compressed && S.nodes[s].n > lo && S.nodes[s].n <= hi)
         for (int b = 0; b * 64 < S.nodes[s].n + S.nodes[s].m(); ++b) opsWork.push_back(RowBlock{s, b});
     opsClass_[cls].second = (int)(opsWork.size() - opsClass_[cls].first);
-  }
-  cRowGrid_.clear();
-  cMRowGrid_.clear();
-  for (auto& lv : F_.compressedLevels) {
-    cLevels_.push_back({(long long)lvlNodes.size(), (int)lv.size()});
-    lvlNodes.insert(lvlNodes.end(), lv.begin(), lv.end());
-    int maxN = 1, maxM = 1;
-    for (int j : lv) {
-      maxN = std::max(maxN, nodes_[j].n);
-      maxM = std::max(maxM, nodes_[j].m);
-    }
-    cRowGrid_.push_back((maxN + 7) / 8);
-    cMRowGrid_.push_back((maxM + 7) / 8);
   }
   clk.mark("layout");
   cudaStream_t st = F_.stream;
@@ -1210,8 +913,7 @@ void SolveEngine<T>::plan() {
   clk.mark("inverse");
   // per-row contribution lists of the compressed supernodes (in source order)
   std::vector<long long> cstart;
-  std::vector<long long> ents;   // offsets into the batched apply's update-vector arena
-  std::vector<int> entsU;        // and into the single-vector one's
+  std::vector<int> ents;   // offsets into the update-vector arena
   {
     for (int s = 0; s < nn; ++s) {
       const Node& nd = S.nodes[s];
@@ -1224,44 +926,26 @@ void SolveEngine<T>::plan() {
       nodes_[s].cOff = (long long)cstart.size();
       for (int t = 0; t <= nd.n; ++t) cstart.push_back(base + cnt[t]);
       ents.resize(ents.size() + cnt[nd.n]);
-      entsU.resize(ents.size());
       std::vector<int> fill(cnt.begin(), cnt.end() - 1);
       for (const SPull& P : pl[s]) {
         const SNode<T>& src = nodes_[P.src];
         for (int a = P.a0; a < P.a1; ++a) {
-          // interior root: its update vector; compressed: u = -V z
-          const long long e = (P.kind == 0) ? src.wuOff + a : src.wuOff + 2 * src.r + a;
-          const long long at = base + fill[S.nodes[P.src].rows[a] - nd.c0]++;
-          ents[at] = e;
-          entsU[at] = src.uOff + a;
+          ents[base + fill[S.nodes[P.src].rows[a] - nd.c0]++] = src.uOff + a;
         }
       }
     }
-    up(dCStart_, cstart.data(), cstart.size() * sizeof(long long));
-    up(dCEnt_, ents.data(), ents.size() * sizeof(long long));
   }
   dWu_.alloc(sizeof(T) * std::max(8LL, uCur));
   RSCHOL_CUDA(cudaMemsetAsync(dWu_.p, 0, dWu_.bytes, st));
   clk.mark("lists");
-  plan_items(rel, cstart, entsU);
+  plan_items(rel, cstart, ents);
   clk.mark("items");
   up(dNodes_, nodes_.data(), nodes_.size() * sizeof(SNode<T>));
-  up(dRows_, rowsAll.data(), rowsAll.size() * sizeof(int));
-  up(dRel_, rel.data(), rel.size() * sizeof(int));
-  up(dChild_, child.data(), child.size() * sizeof(int));
-  up(dLevelNodes_, lvlNodes.data(), lvlNodes.size() * sizeof(int));
-  up(dIWork_, iwork.data(), iwork.size() * sizeof(RowBlock));
-  up(dIWorkB_, iworkB.data(), iworkB.size() * sizeof(RowBlock));
-  nIWork_ = (int)iwork.size();
   up(dOpsWork_, opsWork.data(), opsWork.size() * sizeof(RowBlock));
-  wuTotal_ = wuCur;
-  ipTotal_ = ipCur;
-  maxNI_ = 0;
-  for (int s = 0; s < nn; ++s)
-    if (!S.nodes[s].compressed) maxNI_ = std::max(maxNI_, S.nodes[s].n);
-  kB_ = 0;   // the batched apply re-plans on its next use
+  kAllocB_ = 0;   // the batched apply's buffers follow the new plan
+  dSyncB_.release();
+  ++batchGen_;
   up(dDinvTasks_, dinvTasks.data(), dinvTasks.size() * sizeof(DinvTask<T>));
-  syncInts_ = syncCur;
   if (!std::is_same<T, double>::value) dW_.alloc(sizeof(T) * std::max(1, S.n));
   RSCHOL_CUDA(cudaStreamSynchronize(st));
   clk.mark("upload");
@@ -1819,11 +1503,11 @@ void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<l
   smem_ = (size_t)NSTAGE * ST_BYTES + NGRP * sizeof(T) * (size_t)work_;
   if (smem_ > 226 * 1024) throw std::runtime_error("interior front too large for the shared-memory solve");
   RSCHOL_CUDA(cudaFuncSetAttribute(apply_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_));
-  int dev = 0, sms = 0, per = 0;
+  int dev = 0, per = 0;
   RSCHOL_CUDA(cudaGetDevice(&dev));
-  RSCHOL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  RSCHOL_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
   RSCHOL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, apply_kernel<T>, NGRP * GT + 32, smem_));
-  grid_ = std::min(std::max(1, nItems_), sms * std::max(1, per));
+  grid_ = std::min(std::max(1, nItems_), sms_ * std::max(1, per));
   // phases that a few items per group work off
   std::vector<int> count(phase + 1, 0);
   for (int q : phaseOf) count[q]++;

@@ -41,25 +41,17 @@ struct SNode {
   const T* L;       // interior: [L11; L21] panel; compressed: L11 (HODLR expanded)
   const T* V;       // compressed: m x r
   const T* U;       // compressed: n x r
-  const T* Dinv;    // interior: inverted 64 x 64 diagonal blocks of L11 (the last one h x h)
+  const T* Dinv;    // interior of n <= 64: L11^{-1} (n x n)
   const T* X;       // compressed, and interior of n > 64: L11^{-1} (n x ldx, row-major, upper triangle zero)
   T* G;             // interior: L21 L11^{-1} (m x ldk)
   T* Sg;            // interior: (L11 L11^T)^{-1} (n x ldk)
   const T* W;       // compressed: X^T U (n x r)
   int ld, n, m, r, c0;
-  int childBegin, childEnd;   // interior: children (range in the child list)
-  int nb, nch;                // compressed: 64-row blocks of L11; interior: 128-row chunks of L21 (batched apply)
   int ldk, ldx;               // row strides of G and Sg, and of X
-  int uOff, tOff;             // single vector: update vector (interior: children's rows - G f, compressed:
-                              // -V z), and t = S f of an interior supernode
-  int syncOff;                // interior (batched apply): backward chunk counter, forward completion
-                              // count, backward solved flag
-  int parentI;                // interior: parent if it is interior, else -1
-  long long rowsOff;          // rows of this node in the row arena
-  long long wuOff;            // batched apply: interior: update vector; compressed: z (r), s (r), u = -V z (m)
+  int uOff, tOff;             // update vector (interior: children's rows - G f, compressed: -V z), and
+                              // t = S f of an interior supernode
   long long relOff;           // interior: target index in the parent front of each row
   long long cOff;             // compressed: first of its n+1 contribution-list offsets
-  long long zpOff;            // interior (batched apply): partials of L21^T x_R (nch x n)
 };
 
 struct SPull {       // contribution source of a compressed supernode (plan time)
@@ -68,7 +60,7 @@ struct SPull {       // contribution source of a compressed supernode (plan time
   int kind;          // 0: interior root update vector, 1: compressed V z
 };
 
-struct RowBlock {    // one thread block's work: (supernode, row block or chunk)
+struct RowBlock {    // one thread block's work: (supernode, row block)
   int node, b;
 };
 
@@ -76,7 +68,7 @@ struct PackTile {    // a tile of X packed for the apply: rows from i0, columns 
   int node, i0, j0, cols, rows;
 };
 
-struct alignas(16) ApplyItem {   // one work item of the single-vector apply
+struct alignas(16) ApplyItem {   // one work item of an application
   const void* g0;   // its pieces of the factor ...
   const void* g1;
   int kind;
@@ -99,13 +91,11 @@ struct DinvTask {    // invert one lower-triangular diagonal block (h x h, h <= 
   T* D;
 };
 
-struct XStep {       // one batched GEMM launch (X = L11^{-1} doubling, batched apply)
+struct XStep {       // one batched GEMM launch (X = L11^{-1} doubling, W, S and G)
   long long off;
   int count, tiles;
-  int tc;            // on the tensor cores (batched apply: the transposed skinny form)
-  int bn = 64;       // tensor-core tile width of the launch (X doubling)
-  long long redOff = 0;   // batched apply: K-slice sums after the launch (first, count, grid); tiles = units
-  int redCount = 0, redGrid = 0;
+  int tc;            // on the tensor cores
+  int bn = 64;       // tensor-core tile width of the launch
 };
 
 template <class T>
@@ -125,13 +115,13 @@ class SolveEngine {
   // contiguous) := M^{-1} W with one pass over the factor; k <=
   // batch_capacity().  take_error_batch: as take_error, for the batched path.
   void apply_batch(double* d_W, int k, cudaStream_t s);
-  // Time the candidate tile shapes of every width class up to kmax on this
+  // Time the candidate launch shapes of every width class up to kmax on this
   // stream (run it while the GPU is otherwise quiet) and keep the fastest.
   void autotune_batch(int kmax, cudaStream_t s);
-  // the tile shapes chosen for each width class so far: (class, RA, RC, cwR, cwC, ms) rows
+  // the shapes chosen for each width class so far: (class, blocks per SM, columns per pass, 0, 0, ms) rows
   std::vector<std::array<double, 6>> batch_tuning() const;
   int batch_capacity() const;
-  // bumped whenever the batched apply's buffers are reallocated or its tile
+  // bumped whenever the batched apply's buffers are reallocated or its
   // shapes retuned (a graph that captured an apply must then be captured again)
   long long batch_generation() const { return batchGen_; }
   int take_error_batch(cudaStream_t s);
@@ -141,14 +131,13 @@ class SolveEngine {
  private:
   FactorEngine<T>& F_;
   std::vector<SNode<T>> nodes_;
-  DevBuf dNodes_, dRows_, dRel_, dChild_, dWu_, dW_, dLevelNodes_, dCStart_, dCEnt_;
-  DevBuf dDinv_, dDinvTasks_, dZp_, dSp_, dIp_, dT_, dYp_, dXp_, dSync_, dIWork_, dIWorkB_;
-  int nIWork_ = 0;
-  // single-vector apply: the work items and their descriptors, the counters
-  // ([0] error word, [1] ticket), the launch shape
+  DevBuf dNodes_, dWu_, dW_;
+  DevBuf dDinv_, dDinvTasks_, dZp_, dSp_, dIp_, dT_, dYp_, dXp_, dSync_;
+  // the work items and their descriptors, the counters ([0] error word,
+  // [1] ticket), the single-vector launch's shape
   DevBuf dItems_, dBlob_, dPackTiles_, dPacked_;
   int nPacks_ = 0;
-  int nItems_ = 0, nSync_ = 0, grid_ = 1, fLen_ = 4, work_ = 0;
+  int nItems_ = 0, nSync_ = 0, sms_ = 1, grid_ = 1, fLen_ = 4, work_ = 0;
   size_t smem_ = 0;
   bool group_member(int s) const;
   void plan_items(const std::vector<int>& rel, const std::vector<long long>& cstart, const std::vector<int>& ents);
@@ -157,44 +146,26 @@ class SolveEngine {
   DevBuf dX_, dT1_, dXGemm_;          // L11^{-1}, its temporaries and GEMM tasks
   std::vector<XStep> xSteps_;
   int nDinv_ = 0;
-  int syncInts_ = 0;
-  std::vector<int> cRowGrid_;        // per compressed level: 8-row blocks of the largest supernode
   void plan_inverse(const std::vector<long long>& xOff);   // GEMM schedule of X = L11^{-1}
-  std::vector<std::pair<long long, int>> iLevels_;  // (offset, count) into the interior work list
-  std::vector<std::pair<long long, int>> cLevels_;  // (offset, count) into the level node list
   long long launchesPerApply_ = 0;
   double bytesPerApply_ = 0;
-  // batched apply: work buffers sized for the widest k seen (they only grow,
-  // so a changing width frees nothing and never synchronises the device);
-  // the GEMM task lists are built once per width and kept
-  // Tile shapes of the batched apply (none changes any column's arithmetic):
-  // the interior (row, column) pair tile RA x RC and the column groups of the
-  // two skinny product forms, per width class (k rounded up to a power of
-  // two).  Fixed heuristics unless the class was tuned by autotune_batch
-  // (or, with RSCHOL_AUTOTUNE=1, on first use).
+  // batched apply: work buffers sized for the widest block seen, and per width
+  // class (columns rounded up to a power of two) the persistent blocks per SM
+  // (fixed unless tuned by autotune_batch or, with RSCHOL_AUTOTUNE=1, on first
+  // use); no choice changes any column's arithmetic
   struct BatchCfg {
-    int ra = 1, rc = 1, cwR = 1, cwC = 1;
+    int blocks = 2;
     double ms = 0;   // the winning candidate's time (0: not timed)
   };
-  BatchCfg heuristic_cfg(int kp) const;
   const BatchCfg& config_for(int k, cudaStream_t s, bool tune);
   int width_class(int k) const;
   void apply_batch_cfg(double* W64, int k, cudaStream_t s, const BatchCfg& c);
   std::map<int, BatchCfg> tuned_;
   bool autotune_ = true;
-  void plan_batch(int k, int cwR, int cwC);
-  long long wuTotal_ = 0, ipTotal_ = 0;
-  int maxNI_ = 0;                      // largest interior supernode width
-  std::vector<int> cMRowGrid_;         // per compressed level: 8-row blocks of the largest m
-  int kB_ = 0, kAllocB_ = 0;
+  void plan_batch(int kp);
+  int kAllocB_ = 0;
   long long batchGen_ = 0;
-  DevBuf dWuB_, dYB_, dIpB_, dSyncB_, dWB_;
-  struct BatchPlan {
-    DevBuf tasks, sums, ws;   // GEMM tasks, K-slice sums and their slice products
-    std::vector<std::vector<XStep>> steps;   // [6 * level + phase]
-  };
-  std::map<int, BatchPlan> bPlans_;
-  const BatchPlan* bPlan_ = nullptr;
+  DevBuf dWuB_, dTB_, dZpB_, dSpB_, dYpB_, dXpB_, dIpB_, dSyncB_, dWB_;
 };
 
 }  // namespace rschol

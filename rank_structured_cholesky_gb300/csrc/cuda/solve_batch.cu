@@ -1,21 +1,31 @@
 // Batched preconditioner apply: W (n x k, row-major, the k right-hand sides
 // of a row contiguous) := M^{-1} W with one pass over the factor.
 //
-// Same operator and schedule as SolveEngine::apply_inplace, with every vector
-// widened to k columns: the interior supernodes run in one ticketed launch
-// per direction (a thread per (row, right-hand side) pair), and the
-// compressed levels become batched GEMMs on the factor's GEMM kernels:
-//   forward   Y = X F (row blocks of X stop at the diagonal), Z = U^T Y,
-//             U_c = -V Z;
-//   backward  S = V^T X_R, G = Y - U S, X = X^T G (column blocks of X start at
-//             the diagonal).
-// Factor bytes are read once per apply whatever k is; vector bytes scale
-// with k.
+// The work items, their pieces of the factor and their order are those of the
+// single-vector apply (solve.cu); only the products change: the pieces of the
+// factor lie in shared memory, so a thread forms a tile of rows (or columns)
+// of the piece times one 16-byte vector of right-hand sides.  A pass of an item
+// covers up to KC columns (four vectors); wider blocks take several passes with
+// the staged piece.  Factor bytes are read once per apply whatever k is; vector
+// bytes scale with k.
+//
+// Width invariance: every (row, column) sum runs serially over the piece in one
+// order, or in splits fixed by the piece alone; how threads cover (row, column)
+// pairs depends on k, the arithmetic of a column does not.
+//
+// Bound: the latency of the items' gathers (a pass of an item is about 5 us of
+// dependent loads whatever its bytes), FP64 its 1/64 rate.  Measured, one
+// application against the earlier kernels (a triangular solve with a thread per
+// (row, column) pair, six launches per compressed level): 2D 1024^2 FP32 k = 64
+// 10.50 -> 5.99 ms, k = 8 3.62 -> 0.85 ms; 3D 40^3 FP32 k = 32 1.99 -> 1.06 ms,
+// k = 8 1.81 -> 0.47 ms; 3D 64^3 FP32 k = 16 3.23 -> 1.10 ms; 3D 44x40x47 FP64
+// k = 8 2.78 -> 1.84 ms.
 #include <algorithm>
 #include <mutex>
 #include <stdexcept>
 #include <type_traits>
 
+#include "apply_dev.cuh"
 #include "solve.cuh"
 #include "solve_dev.cuh"
 
@@ -25,660 +35,705 @@ namespace {
 
 using namespace solvedev;
 
-// Every (row, right-hand side) pair of the interior solves is a dot product
-// formed serially in a fixed order, so each column's arithmetic is the same
-// whatever k is.  pair_dots runs such a family: for r < rows, c < k,
-// acc = init(r, c), then for j = lo(r) .. hi(r) - 1 in order
-// acc += a(r, j) * F(j, c) (acc -= ... when SUB), then out(r, c, acc).  A
-// thread takes a tile of RA rows x RC columns (consecutive threads take
-// consecutive column tiles): 1 x 1 spreads the pairs over all threads at
-// small k, 4 x 4 reuses every load of A and F four times at large k.  The
-// tiling only changes which thread forms a pair, not its arithmetic.
-template <class T, int RA, int RC, bool SUB, class AE, class FV, class Init, class Lo, class Hi, class Out>
-__device__ __forceinline__ void pair_dots(int rows, int k, AE a, FV fv, Init init, Lo lo, Hi hi, Out out) {
-  const int ct = (k + RC - 1) / RC, rt = (rows + RA - 1) / RA;
-  for (int tile = threadIdx.x; tile < rt * ct; tile += blockDim.x) {
-    const int tr = tile / ct;
-    const int r0 = tr * RA, c0 = (tile - tr * ct) * RC;
-    T acc[RA][RC];
-    int l[RA], h[RA];
-    int jlo = 0x7fffffff, jhi = -0x7fffffff;
+constexpr int FB = 8192;   // bytes of a group's buffer of right-hand-side vectors
+constexpr int FV = FB / 16;
+// Persistent blocks per SM: two with 112 registers a thread; three with 72 spill
+// in FP32 (2D 1024^2, k = 64: 5.99 against 7.06 ms an application)
+constexpr int BATCH_BLOCKS = 2;
+// rows (columns) of a piece a thread holds: FP64 pieces of a stage have half as
+// many
+template <class T> constexpr int NR = sizeof(T) == 8 ? 2 : 4;
+
+template <class T>
+struct Pass {   // one pass over up to four vectors of right-hand sides
+  using Vt = typename Vec16<T>::type;
+  const ApplyArgs<T>* A;
+  int kp;        // row stride of the blocks (right-hand sides, padded to a vector)
+  int cgN;       // vectors of the pass, rounded up to 1, 2 or 4
+  int col;       // this thread's first column
+  bool act;      // its vector holds columns of the block
+  int cg, rg, nrg, tid;
+  __device__ __forceinline__ Vt ld(const T* base, long long idx) const {
+    return act ? __ldcg(reinterpret_cast<const Vt*>(base + idx * kp + col)) : vzero(T(0));
+  }
+  __device__ __forceinline__ void st(T* base, long long idx, Vt v) const {
+    if (act) *reinterpret_cast<Vt*>(base + idx * kp + col) = v;
+  }
+};
+
+__device__ __forceinline__ void vsub(float4& a, float4 b) {
+  a.x -= b.x;
+  a.y -= b.y;
+  a.z -= b.z;
+  a.w -= b.w;
+}
+__device__ __forceinline__ void vsub(double2& a, double2 b) {
+  a.x -= b.x;
+  a.y -= b.y;
+}
+
+// v[i] + the entries [b[i], e[i]) of a pull list, in order, for N targets at
+// once: the loads of a round (two entries a target) are all in flight together.
+template <class T, int N>
+__device__ __forceinline__ void pulls(const Pass<T>& p, typename Vec16<T>::type (&v)[N], const int* ent, int (&b)[N],
+                                      const int (&e)[N]) {
+  bool more = true;
+  while (more) {
+    typename Vec16<T>::type x[N], y[N];
 #pragma unroll
-    for (int r = 0; r < RA; ++r) {
-      const bool rv = r0 + r < rows;
-      l[r] = rv ? lo(r0 + r) : 0;
-      h[r] = rv ? hi(r0 + r) : 0;
-#pragma unroll
-      for (int q = 0; q < RC; ++q) acc[r][q] = (rv && c0 + q < k) ? init(r0 + r, c0 + q) : T(0);
-      if (rv) {
-        jlo = min(jlo, l[r]);
-        jhi = max(jhi, h[r]);
-      }
+    for (int i = 0; i < N; ++i) {
+      x[i] = b[i] < e[i] ? p.ld(p.A->wu, ent[b[i]]) : vzero(T(0));
+      y[i] = b[i] + 1 < e[i] ? p.ld(p.A->wu, ent[b[i] + 1]) : vzero(T(0));
     }
-    bool same = true;   // every row of the tile runs over [jlo, jhi)
+    more = false;
 #pragma unroll
-    for (int r = 0; r < RA; ++r) same = same && (r0 + r >= rows || (l[r] == jlo && h[r] == jhi));
-    if (same) {
-      for (int j = jlo; j < jhi; ++j) {
-        T f[RC];
+    for (int i = 0; i < N; ++i) {
+      vadd(v[i], x[i]);
+      vadd(v[i], y[i]);
+      b[i] += 2;
+      more = more || b[i] < e[i];
+    }
+  }
+}
+
+// f of the columns [j0, j0 + jn) (offsets ps[j], entries ent; ps null: no
+// children) into F, the caller's threads rg, rg + nrg, ... of every vector
+template <class T>
+__device__ __forceinline__ void gather_f(const Pass<T>& p, int c0, int j0, int jn, const int* ps, const int* ent,
+                                         int rg, int nrg, typename Vec16<T>::type* F) {
+  constexpr int N = 4;
+  constexpr int V = Vec16<T>::V;
+  const int jp = (jn + V - 1) / V * V;   // zeros up to a vector
+  for (int jb = rg; jb < jp; jb += N * nrg) {
+    typename Vec16<T>::type v[N];
+    int b[N], e[N];
 #pragma unroll
-        for (int q = 0; q < RC; ++q) f[q] = (RC == 1 || c0 + q < k) ? fv(j, c0 + q) : T(0);
+    for (int i = 0; i < N; ++i) {
+      const int j = jb + i * nrg;
+      const bool in = j < jn;
+      v[i] = in ? p.ld(p.A->w, c0 + j0 + j) : vzero(T(0));
+      b[i] = ps && in ? ps[j0 + j] : 0;
+      e[i] = ps && in ? ps[j0 + j + 1] : 0;
+    }
+    if (ps) pulls<T, N>(p, v, ent, b, e);
 #pragma unroll
-        for (int r = 0; r < RA; ++r) {
-          const T av = (RA == 1 || r0 + r < rows) ? a(r0 + r, j) : T(0);
+    for (int i = 0; i < N; ++i)
+      if (jb + i * nrg < jp) F[(jb + i * nrg) * p.cgN + p.cg] = v[i];
+  }
+}
+
+__device__ __forceinline__ void vstep(float4& acc, const float4& m, const float4* F, int fs) {
+  vaxpy(acc, F[0], m.x);
+  vaxpy(acc, F[fs], m.y);
+  vaxpy(acc, F[2 * fs], m.z);
+  vaxpy(acc, F[3 * fs], m.w);
+}
+__device__ __forceinline__ void vstep(double2& acc, const double2& m, const double2* F, int fs) {
+  vaxpy(acc, F[0], m.x);
+  vaxpy(acc, F[fs], m.y);
+}
+
+// acc[i] += sum_k M_i[k] F[k], k < kn in order, for the thread's rows M_i = M +
+// off[i] (off < 0: none); F: vectors, row stride fs.  ALIGNED: rows on 16-byte
+// boundaries, zeros behind them (and in F) up to a vector: read in vectors -- the
+// eight rows of a warp lie 16 floats apart in the commonest supernodes, four
+// deep in the same banks when read by words.
+template <class T, bool ALIGNED>
+__device__ __forceinline__ void rows_dot(const T* M, const int (&off)[NR<T>], int k0, int kn,
+                                         const typename Vec16<T>::type* F, int fs,
+                                         typename Vec16<T>::type (&acc)[NR<T>]) {
+  using Vt = typename Vec16<T>::type;
+  constexpr int V = Vec16<T>::V;
+  if constexpr (ALIGNED) {
+#pragma unroll 2
+    for (int k = 0; k < kn; k += V) {
 #pragma unroll
-          for (int q = 0; q < RC; ++q) {
-            if (SUB) acc[r][q] -= av * f[q];
-            else acc[r][q] += av * f[q];
-          }
+      for (int i = 0; i < NR<T>; ++i)
+        if (off[i] >= 0) vstep(acc[i], *reinterpret_cast<const Vt*>(M + off[i] + k0 + k), F + k * fs, fs);
+    }
+  } else {
+#pragma unroll 4
+    for (int k = 0; k < kn; ++k) {
+      const Vt f = F[k * fs];
+#pragma unroll
+      for (int i = 0; i < NR<T>; ++i)
+        if (off[i] >= 0) vaxpy(acc[i], f, M[off[i] + k0 + k]);
+    }
+  }
+}
+
+// out(j, sum_{a < h} M[a * ld + j] X[a * xs]) for the thread's columns j < nc
+template <class T, class Out>
+__device__ __forceinline__ void cols_dot(const T* M, int ld, int h, int nc, const typename Vec16<T>::type* X, int xs,
+                                         int j0, int step, Out out) {
+  for (int jb = j0; jb < nc; jb += NR<T> * step) {
+    typename Vec16<T>::type acc[NR<T>];
+    const T* m[NR<T>];
+#pragma unroll
+    for (int i = 0; i < NR<T>; ++i) {
+      acc[i] = vzero(T(0));
+      m[i] = jb + i * step < nc ? M + jb + i * step : nullptr;
+    }
+#pragma unroll 4
+    for (int a = 0; a < h; ++a) {
+      const typename Vec16<T>::type x = X[a * xs];
+#pragma unroll
+      for (int i = 0; i < NR<T>; ++i)
+        if (m[i]) vaxpy(acc[i], x, m[i][(size_t)a * ld]);
+    }
+#pragma unroll
+    for (int i = 0; i < NR<T>; ++i)
+      if (jb + i * step < nc) out(jb + i * step, acc[i]);
+  }
+}
+
+// A group's members, a warp each; lanes over (row group, vector).
+template <class T>
+__device__ __forceinline__ void fgrp_k(const Pass<T>& p, const int* h0, const int* d, int cnt, const T* data,
+                                       typename Vec16<T>::type* buf) {
+  using Vt = typename Vec16<T>::type;
+  const int lane = threadIdx.x & 31, warp = p.tid >> 5;
+  const int rg = lane / p.cgN, nrg = 32 / p.cgN;
+  Vt* F = buf + warp * 32 * p.cgN;
+  for (int q = warp; q < cnt; q += GW) {
+    const int* h = h0 + GH * q;
+    const int n = h[0], m = h[1], c0 = h[2], ldk = h[7];
+    const bool has = h[6] != 0;
+    const int* ps = d + h[6];
+    const int* ent = ps + n + m + 1;
+    __syncwarp();
+    gather_f<T>(p, c0, 0, n, has ? ps : nullptr, ent, rg, nrg, F);
+    __syncwarp();
+    for (int r0 = 0; r0 < m + n; r0 += NR<T> * nrg) {   // rows of G, then of S
+      Vt acc[NR<T>];
+      int off[NR<T>];
+#pragma unroll
+      for (int i = 0; i < NR<T>; ++i) {
+        const int r = r0 + rg + i * nrg;
+        off[i] = r < m ? h[4] + r * ldk : r < m + n ? h[5] + (r - m) * ldk : -1;
+        acc[i] = vzero(T(0));
+      }
+      rows_dot<T, true>(data, off, 0, n, F + p.cg, p.cgN, acc);
+      Vt u[NR<T>];
+      if (has && r0 < m) {
+        int b[NR<T>], e[NR<T>];
+#pragma unroll
+        for (int i = 0; i < NR<T>; ++i) {
+          const int r = r0 + rg + i * nrg;
+          u[i] = vzero(T(0));
+          b[i] = r < m ? ps[n + r] : 0;
+          e[i] = r < m ? ps[n + r + 1] : 0;
+        }
+        pulls<T, NR<T>>(p, u, ent, b, e);
+      } else {
+#pragma unroll
+        for (int i = 0; i < NR<T>; ++i) u[i] = vzero(T(0));
+      }
+#pragma unroll
+      for (int i = 0; i < NR<T>; ++i) {
+        const int r = r0 + rg + i * nrg;
+        if (r < m) {
+          vsub(u[i], acc[i]);
+          p.st(p.A->wu, h[3] + r, u[i]);
+        } else if (r < m + n) {
+          p.st(p.A->t, h[8] + r - m, acc[i]);
         }
       }
-    } else {
-      for (int j = jlo; j < jhi; ++j) {
-        T f[RC];
+    }
+  }
+}
+
+template <class T>
+__device__ __forceinline__ void bgrp_k(const Pass<T>& p, const int* h0, const int* d, int cnt, const T* data,
+                                       typename Vec16<T>::type* buf) {
+  using Vt = typename Vec16<T>::type;
+  const int lane = threadIdx.x & 31, warp = p.tid >> 5;
+  const int rg = lane / p.cgN, nrg = 32 / p.cgN;
+  Vt* X = buf + warp * 128;   // 128 vectors: NR<T> rows a lane
+  for (int q = warp; q < cnt; q += GW) {
+    const int* h = h0 + GH * q;
+    const int n = h[0], m = h[1], c0 = h[2], ldk = h[7];
+    const T* G = data + h[4];
+    const int* rw = d + h[6];
+    // the thread's columns j = rg + i nrg: 32 columns in 1, 2 or 4 sweeps of them
+    const int tile = NR<T> * nrg;   // rows of x_R a tile
+    for (int jb = 0; jb < n; jb += NR<T> * nrg) {
+      Vt acc[NR<T>], nx[NR<T>];
+      const T* g[NR<T>];
 #pragma unroll
-        for (int q = 0; q < RC; ++q) f[q] = (RC == 1 || c0 + q < k) ? fv(j, c0 + q) : T(0);
+      for (int i = 0; i < NR<T>; ++i) {
+        acc[i] = vzero(T(0));
+        g[i] = jb + rg + i * nrg < n ? G + jb + rg + i * nrg : nullptr;
+        nx[i] = rg + i * nrg < m ? p.ld(p.A->w, rw[rg + i * nrg]) : vzero(T(0));
+      }
+      for (int a0 = 0; a0 < m; a0 += tile) {
+        __syncwarp();
 #pragma unroll
-        for (int r = 0; r < RA; ++r)
-          if (j >= l[r] && j < h[r]) {
-            const T av = a(r0 + r, j);
+        for (int i = 0; i < NR<T>; ++i) X[(rg + i * nrg) * p.cgN + p.cg] = nx[i];
+        __syncwarp();
 #pragma unroll
-            for (int q = 0; q < RC; ++q) {
-              if (SUB) acc[r][q] -= av * f[q];
-              else acc[r][q] += av * f[q];
+        for (int i = 0; i < NR<T>; ++i) {   // the next tile's loads under this one's products
+          const int a = a0 + tile + rg + i * nrg;
+          nx[i] = a < m ? p.ld(p.A->w, rw[a]) : vzero(T(0));
+        }
+        const int an = min(tile, m - a0);
+#pragma unroll 4
+        for (int a = 0; a < an; ++a) {
+          const Vt x = X[a * p.cgN + p.cg];
+#pragma unroll
+          for (int i = 0; i < NR<T>; ++i)
+            if (g[i]) vaxpy(acc[i], x, g[i][(size_t)(a0 + a) * ldk]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < NR<T>; ++i) {
+        const int j = jb + rg + i * nrg;
+        if (j < n) {
+          Vt v = p.ld(p.A->t, h[8] + j);
+          vsub(v, acc[i]);
+          p.st(p.A->w, c0 + j, v);
+        }
+      }
+    }
+  }
+}
+
+// One chunk: the rows of G, then of S (in a stage they follow each other; a
+// supernode too wide for one is read where it is, G's rows and S's in turn).
+template <class T>
+__device__ __forceinline__ void fwd_k(const Pass<T>& p, const int* h, const int* d, const int* d2, const T* Gd,
+                                      const T* Sd, bool staged, typename Vec16<T>::type* F) {
+  using Vt = typename Vec16<T>::type;
+  constexpr int V = Vec16<T>::V;
+  const int n = h[0], rows = h[1], c0 = h[2], ldk = h[7];
+  const bool has = h[6] != 0;
+  const int* ps = d + h[6];
+  const int* ent = ps + rows + 1;
+  const int* ent2 = d2 + n + 1;
+  const int ft = FV / p.cgN / V * V;   // rows of f a tile
+  for (int part = 0; part < (staged ? 1 : 2); ++part) {
+    const T* M = part ? Sd : Gd;
+    const int first = part ? rows : 0, cnt = staged ? rows + h[5] : part ? h[5] : rows;
+    for (int r0 = 0; r0 < cnt; r0 += NR<T> * p.nrg) {   // one sweep for the chunk heights in use
+      Vt acc[NR<T>];
+      int off[NR<T>];
+#pragma unroll
+      for (int i = 0; i < NR<T>; ++i) {
+        const int r = r0 + p.rg + i * p.nrg;
+        off[i] = r < cnt ? r * ldk : -1;
+        acc[i] = vzero(T(0));
+      }
+      for (int j0 = 0; j0 < n; j0 += ft) {
+        const int jn = min(ft, n - j0);
+        if (j0 > 0 || r0 > 0 || part > 0) cbar();
+        gather_f<T>(p, c0, j0, jn, has ? d2 : nullptr, ent2, p.rg, p.nrg, F);
+        cbar();
+        rows_dot<T, true>(M, off, j0, jn, F + p.cg, p.cgN, acc);
+      }
+      Vt u[NR<T>];
+      int b[NR<T>], e[NR<T>];
+#pragma unroll
+      for (int i = 0; i < NR<T>; ++i) {
+        const int r = first + r0 + p.rg + i * p.nrg;
+        u[i] = vzero(T(0));
+        b[i] = has && r < rows ? ps[r] : 0;
+        e[i] = has && r < rows ? ps[r + 1] : 0;
+      }
+      if (has) pulls<T, NR<T>>(p, u, ent, b, e);
+#pragma unroll
+      for (int i = 0; i < NR<T>; ++i) {
+        const int r = first + r0 + p.rg + i * p.nrg;
+        if (off[i] < 0) continue;
+        if (r < rows) {
+          vsub(u[i], acc[i]);
+          p.st(p.A->wu, h[3] + r, u[i]);
+        } else {
+          p.st(p.A->t, h[8] + h[4] + r - rows, acc[i]);
+        }
+      }
+    }
+  }
+}
+
+// F[kk] = sum of `parts` partial rows at idx0 + q * rp + kk, kk < kn
+template <class T>
+__device__ __forceinline__ void parts_k(const Pass<T>& p, const T* base, long long idx0, int rp, int kn, int parts,
+                                        typename Vec16<T>::type* F) {
+  using Vt = typename Vec16<T>::type;
+  for (int kk = p.rg; kk < kn; kk += p.nrg) {
+    Vt v = vzero(T(0));
+    for (int q0 = 0; q0 < parts; q0 += 4) {
+      Vt x[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) x[q] = q0 + q < parts ? p.ld(base, idx0 + (long long)(q0 + q) * rp + kk) : vzero(T(0));
+#pragma unroll
+      for (int q = 0; q < 4; ++q) vadd(v, x[q]);
+    }
+    F[kk * p.cgN + p.cg] = v;
+  }
+}
+
+// out(i, sum_k M[i * r + k] y[k]) for the item's rows i < rows, y the sum of the
+// partial rows
+template <class T, class Out>
+__device__ __forceinline__ void rows_parts_k(const Pass<T>& p, const T* Mx, int r, int rows, const T* base,
+                                             long long idx0, int parts, typename Vec16<T>::type* F, Out out) {
+  using Vt = typename Vec16<T>::type;
+  const int rp = (r + 7) & ~7, ft = FV / p.cgN;
+  for (int r0 = 0; r0 < rows; r0 += NR<T> * p.nrg) {
+    Vt acc[NR<T>];
+    int off[NR<T>];
+#pragma unroll
+    for (int i = 0; i < NR<T>; ++i) {
+      const int q = r0 + p.rg + i * p.nrg;
+      off[i] = q < rows ? q * r : -1;
+      acc[i] = vzero(T(0));
+    }
+    for (int k0 = 0; k0 < r; k0 += ft) {
+      const int kn = min(ft, r - k0);
+      cbar();
+      parts_k<T>(p, base, idx0 + k0, rp, kn, parts, F);
+      cbar();
+      rows_dot<T, false>(Mx, off, k0, kn, F + p.cg, p.cgN, acc);
+    }
+#pragma unroll
+    for (int i = 0; i < NR<T>; ++i)
+      if (r0 + p.rg + i * p.nrg < rows) out(r0 + p.rg + i * p.nrg, acc[i]);
+  }
+}
+
+// red[s * cnt + o] (o < cnt outputs of a vector each, s < SP splits) added over s
+// in order; every thread of the group must call it
+template <class T, int SP, class Part, class Out>
+__device__ __forceinline__ void split_sum(const Pass<T>& p, int outs, typename Vec16<T>::type* red, Part part, Out out) {
+  using Vt = typename Vec16<T>::type;
+  for (int e = p.rg; e < outs * SP; e += p.nrg) red[e * p.cgN + p.cg] = part(e / SP, e % SP);
+  cbar();
+  for (int o = p.rg; o < outs; o += p.nrg) {
+    Vt v = vzero(T(0));
+#pragma unroll
+    for (int s = 0; s < SP; ++s) vadd(v, red[(o * SP + s) * p.cgN + p.cg]);
+    out(o, v);
+  }
+}
+
+template <class T>
+__global__ void __launch_bounds__(NGRP * GT + 32, BATCH_BLOCKS) apply_batch_kernel(ApplyArgs<T> A, int kp) {
+  using Vt = typename Vec16<T>::type;
+  constexpr int V = Vec16<T>::V, KC = 4 * V;
+  extern __shared__ __align__(128) unsigned char absm[];
+  __shared__ __align__(8) unsigned long long bars[2 * NSTAGE];
+  __shared__ __align__(16) ApplyItem sItem[NSTAGE];
+  int* const err = A.sync;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NSTAGE; ++s) {
+      mbar_init(smem_u32(&bars[s]), 1);
+      mbar_init(smem_u32(&bars[NSTAGE + s]), 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  if (threadIdx.x >= NGRP * GT) {
+    apply_producer<T>(A, absm, sItem, smem_u32(&bars[0]), smem_u32(&bars[NSTAGE]));
+    return;
+  }
+  const int grp = threadIdx.x / GT, tid = threadIdx.x % GT, warp = tid >> 5;
+  Vt* const F = reinterpret_cast<Vt*>(absm + NSTAGE * ST_BYTES + grp * FB);
+  for (int k = grp;; k += NGRP) {
+    const int s = k % NSTAGE, use = k / NSTAGE;
+    if (!mbar_wait(smem_u32(&bars[s]), use & 1)) {   // cannot happen while the producer runs
+      if (tid == 0) atomicExch(err, 3);
+      break;
+    }
+    const ApplyItem& it = sItem[s];
+    const int kind = it.kind;
+    if (kind == IT_END) break;
+    const unsigned char* st = absm + (size_t)s * ST_BYTES;
+    const T* data = reinterpret_cast<const T*>(st);
+    const int* d = it.descBytes ? reinterpret_cast<const int*>(st + ST_DATA) : A.blob + it.desc;
+    const int* h = d + 2 * it.waits;
+    const int* d2 = it.desc2Bytes ? reinterpret_cast<const int*>(st + ST_DATA + it.descBytes) : A.blob + it.desc2;
+    if (warp == 0) wait_list(d, it.waits, A.sync, err);
+    cbar();
+    const T* g0 = it.bytes0 ? data : reinterpret_cast<const T*>(it.g0);
+    const T* g1 = it.bytes1 ? data + it.bytes0 / sizeof(T) : reinterpret_cast<const T*>(it.g1);
+    for (int col0 = 0; col0 < kp; col0 += KC) {
+      Pass<T> p;
+      p.A = &A;
+      p.kp = kp;
+      const int rem = (kp - col0) / V;
+      p.cgN = rem >= 3 ? 4 : rem;
+      p.tid = tid;
+      p.cg = tid % p.cgN;
+      p.rg = tid / p.cgN;
+      p.nrg = GT / p.cgN;
+      p.col = col0 + p.cg * V;
+      p.act = p.col < kp;
+      if (col0 > 0) cbar();   // the buffers of the last pass
+      switch (kind) {
+        case IT_FGRP: fgrp_k<T>(p, h, d, it.count, data, F); break;
+        case IT_BGRP: bgrp_k<T>(p, h, d, it.count, data, F); break;
+        case IT_FWD: fwd_k<T>(p, h, d, d2, it.bytes0 + it.bytes1 > 0 ? data : g0, g1, it.bytes0 + it.bytes1 > 0, F); break;
+        case IT_BWD: {
+          const int n = h[0], rows = h[1];
+          if (rows == 0) {
+            for (int j = p.rg; j < n; j += p.nrg) p.st(A.w, h[2] + j, p.ld(A.t, h[9] + j));
+            break;
+          }
+#pragma unroll 2
+          for (int a = p.rg; a < rows; a += p.nrg) F[a * p.cgN + p.cg] = p.ld(A.w, d[h[6] + a]);
+          cbar();
+          cols_dot<T>(g0, h[7], rows, n, F + p.cg, p.cgN, p.rg, p.nrg, [&](int j, Vt v) {
+            if (h[5] > 1) {
+              p.st(A.ip, h[3] + (long long)h[4] * h[8] + j, v);
+            } else {
+              Vt t = p.ld(A.t, h[9] + j);
+              vsub(t, v);
+              p.st(A.w, h[2] + j, t);
+            }
+          });
+          break;
+        }
+        case IT_BR: {
+          for (int j = p.rg; j < h[0]; j += p.nrg) {
+            Vt t = p.ld(A.t, h[5] + j), x = vzero(T(0));
+            for (int q0 = 0; q0 < h[3]; q0 += 8) {
+              Vt v[8];
+#pragma unroll
+              for (int q = 0; q < 8; ++q)
+                v[q] = q0 + q < h[3] ? p.ld(A.ip, h[2] + (long long)(q0 + q) * h[4] + j) : vzero(T(0));
+#pragma unroll
+              for (int q = 0; q < 8; ++q) vadd(x, v[q]);
+            }
+            vsub(t, x);
+            p.st(A.w, h[1] + j, t);
+          }
+          break;
+        }
+        case IT_CF: {
+          const int cols = h[1], r = h[2];
+          const int* ps = d + h[4];
+          const int* ent = ps + cols + 1;
+          for (int i = p.rg; i < cols; i += p.nrg) {   // (a column a thread: its list eight entries at a time)
+            Vt v = p.ld(A.w, h[0] + i);
+            const int e = ps[i + 1];
+            for (int b = ps[i]; b < e; b += 8) {
+              Vt x[8];
+#pragma unroll
+              for (int q = 0; q < 8; ++q) x[q] = b + q < e ? p.ld(A.wu, ent[b + q]) : vzero(T(0));
+#pragma unroll
+              for (int q = 0; q < 8; ++q) vadd(v, x[q]);
+            }
+            p.st(A.w, h[0] + i, v);
+            F[i * p.cgN + p.cg] = v;
+          }
+          cbar();
+          if (r > 0)
+            cols_dot<T>(g0, r, cols, r, F + p.cg, p.cgN, p.rg, p.nrg, [&](int j, Vt v) { p.st(A.zp, h[3] + j, v); });
+          break;
+        }
+        case IT_CU:
+          rows_parts_k<T>(p, g0, h[1], h[0], A.zp, h[2], h[3], F, [&](int i, Vt v) {
+            Vt u = vzero(T(0));
+            vsub(u, v);
+            p.st(A.wu, h[4] + i, u);
+          });
+          break;
+        case IT_CR: {   // columns of partials, eight splits of the partials a column
+          T* const base = h[5] ? A.sp : A.zp;
+          split_sum<T, 8>(
+              p, h[3], F,
+              [&](int o, int sp) {
+                Vt x = vzero(T(0));
+                for (int q0 = sp; q0 < h[1]; q0 += 64) {
+                  Vt v[8];
+#pragma unroll
+                  for (int q = 0; q < 8; ++q)
+                    v[q] = q0 + 8 * q < h[1] ? p.ld(base, h[0] + (long long)(q0 + 8 * q) * h[2] + o) : vzero(T(0));
+#pragma unroll
+                  for (int q = 0; q < 8; ++q) vadd(x, v[q]);
+                }
+                return x;
+              },
+              [&](int o, Vt v) { p.st(base, h[4] + o, v); });
+          break;
+        }
+        case IT_Y: {
+          // the tile's rows in two halves of its columns (fixed), f in tiles
+          const int cols = h[1], rows = h[2], ft = FV / p.cgN / 2;
+          const int half = Y_COLS<T> / 2;
+          Vt acc[2] = {vzero(T(0)), vzero(T(0))};   // (row, half) pairs rg, rg + nrg: 32 of them
+          for (int j0 = 0; j0 < half; j0 += ft) {
+            const int jn = min(ft, half - j0);
+            cbar();
+            for (int e = p.rg; e < 2 * jn; e += p.nrg) {   // both halves' rows of f
+              const int hh = e >= jn, j = (hh ? e - jn : e) + j0 + hh * half;
+              F[(hh * ft + (hh ? e - jn : e)) * p.cgN + p.cg] = j < cols ? p.ld(A.w, h[0] + j) : vzero(T(0));
+            }
+            cbar();
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const int e = p.rg + i * p.nrg, row = e >> 1, hh = e & 1;
+              if (e < 2 * Y_ROWS && row < rows) {
+                const T* m = data + row * Y_COLS<T> + hh * half + j0;
+                const Vt* f = F + hh * ft * p.cgN + p.cg;
+#pragma unroll 2
+                for (int j = 0; j < jn; j += V)
+                  vstep(acc[i], *reinterpret_cast<const Vt*>(m + j), f + j * p.cgN, p.cgN);
+              }
             }
           }
+          cbar();
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            if (p.rg + i * p.nrg < 2 * Y_ROWS) F[(p.rg + i * p.nrg) * p.cgN + p.cg] = acc[i];
+          cbar();
+          for (int i = p.rg; i < rows; i += p.nrg) {
+            Vt v = F[2 * i * p.cgN + p.cg];
+            vadd(v, F[(2 * i + 1) * p.cgN + p.cg]);
+            p.st(A.yp, h[3] + i, v);
+          }
+          break;
+        }
+        case IT_XT: {
+          for (int i = p.rg; i < h[0]; i += p.nrg) {
+            const int nj = min(h[6], ((h[4] + i) / Y_ROWS * Y_ROWS + Y_ROWS - 1) / Y_COLS<T> + 1);
+            Vt y = vzero(T(0));
+            for (int j0 = 0; j0 < nj; j0 += 8) {
+              Vt v[8];
+#pragma unroll
+              for (int q = 0; q < 8; ++q)
+                v[q] = j0 + q < nj ? p.ld(A.yp, h[2] + (long long)(j0 + q) * h[3] + i) : vzero(T(0));
+#pragma unroll
+              for (int q = 0; q < 8; ++q) vadd(y, v[q]);
+            }
+            F[i * p.cgN + p.cg] = y;
+          }
+          cbar();
+          cols_dot<T>(data, T_COLS, h[0], h[1], F + p.cg, p.cgN, p.rg, p.nrg,
+                      [&](int j, Vt v) { p.st(A.xp, h[5] + j, v); });
+          break;
+        }
+        case IT_CS: {
+#pragma unroll 2
+          for (int a = p.rg; a < h[0]; a += p.nrg) F[a * p.cgN + p.cg] = p.ld(A.w, d[h[3] + a]);
+          cbar();
+          cols_dot<T>(g0, h[1], h[0], h[1], F + p.cg, p.cgN, p.rg, p.nrg,
+                      [&](int j, Vt v) { p.st(A.sp, h[2] + j, v); });
+          break;
+        }
+        default: {   // IT_CX: t first (four splits of the row blocks), stored in place of x
+          const int cols = h[1];
+          split_sum<T, 4>(
+              p, cols, F,
+              [&](int j, int sp) {
+                Vt x = vzero(T(0));
+                const int first = max(h[8], (h[7] + j) / T_COLS * T_COLS / T_ROWS<T>);
+                for (int i0 = h[8] + sp; i0 < h[9]; i0 += 32) {
+                  Vt v[8];
+#pragma unroll
+                  for (int q = 0; q < 8; ++q) {
+                    const int ib = i0 + 4 * q;
+                    v[q] = ib < h[9] && ib >= first ? p.ld(A.xp, h[5] + (long long)ib * h[6] + j) : vzero(T(0));
+                  }
+#pragma unroll
+                  for (int q = 0; q < 8; ++q) vadd(x, v[q]);
+                }
+                return x;
+              },
+              [&](int j, Vt v) { p.st(A.w, h[0] + j, v); });
+          if (h[4] > 0) {
+            cbar();
+            rows_parts_k<T>(p, g0, h[2], cols, A.sp, h[3], h[4], F, [&](int j, Vt v) {
+              Vt x = p.ld(A.w, h[0] + j);
+              vsub(x, v);
+              p.st(A.w, h[0] + j, x);
+            });
+          }
+          break;
+        }
       }
     }
-#pragma unroll
-    for (int r = 0; r < RA; ++r)
-#pragma unroll
-      for (int q = 0; q < RC; ++q)
-        if (r0 + r < rows && c0 + q < k) out(r0 + r, c0 + q, acc[r][q]);
-  }
-}
-
-// f := L^{-1} f for k right-hand sides (f: n x k in shared memory, row
-// stride k) with the inverted 64 x 64 diagonal blocks of L; t: 64 x k
-// shared.
-template <class T, int RA, int RC>
-__device__ void trsv_dinv_k(const T* __restrict__ L, int ld, int n, const T* __restrict__ D, T* f, T* t, int k) {
-  for (int i0 = 0; i0 < n; i0 += 64) {
-    const int h = min(64, n - i0);
-    pair_dots<T, RA, RC, true>(
-        h, k, [&](int i, int j) { return L[(size_t)(i0 + i) * ld + j]; },
-        [&](int j, int c) { return f[(size_t)j * k + c]; }, [&](int i, int c) { return f[(size_t)(i0 + i) * k + c]; },
-        [](int) { return 0; }, [&](int) { return i0; }, [&](int i, int c, T v) { t[(size_t)i * k + c] = v; });
-    __syncthreads();
-    const T* Db = D + (size_t)i0 * 64;
-    pair_dots<T, RA, RC, false>(
-        h, k, [&](int i, int j) { return Db[(size_t)i * h + j]; }, [&](int j, int c) { return t[(size_t)j * k + c]; },
-        [](int, int) { return T(0); }, [](int) { return 0; }, [](int i) { return i + 1; },
-        [&](int i, int c, T v) { f[(size_t)(i0 + i) * k + c] = v; });
-    __syncthreads();
-  }
-}
-
-// f := L^{-T} f for k right-hand sides, same blocks.
-template <class T, int RA, int RC>
-__device__ void trsv_dinv_t_k(const T* __restrict__ L, int ld, int n, const T* __restrict__ D, T* f, T* t, int k) {
-  if (n <= 0) return;
-  for (int i0 = ((n - 1) / 64) * 64; i0 >= 0; i0 -= 64) {
-    const int h = min(64, n - i0);
-    pair_dots<T, RA, RC, true>(
-        h, k, [&](int j, int i) { return L[(size_t)i * ld + i0 + j]; },
-        [&](int i, int c) { return f[(size_t)i * k + c]; }, [&](int j, int c) { return f[(size_t)(i0 + j) * k + c]; },
-        [&](int) { return i0 + h; }, [&](int) { return n; }, [&](int j, int c, T v) { t[(size_t)j * k + c] = v; });
-    __syncthreads();
-    const T* Db = D + (size_t)i0 * 64;
-    pair_dots<T, RA, RC, false>(
-        h, k, [&](int j, int i) { return Db[(size_t)i * h + j]; }, [&](int i, int c) { return t[(size_t)i * k + c]; },
-        [](int, int) { return T(0); }, [](int j) { return j; }, [&](int) { return h; },
-        [&](int j, int c, T v) { f[(size_t)(i0 + j) * k + c] = v; });
-    __syncthreads();
-  }
-}
-
-template <class T, int RA, int RC>
-__global__ void __launch_bounds__(256) interior_forward_k(const SNode<T>* __restrict__ nodes,
-                                                          const RowBlock* __restrict__ work,
-                                                          const int* __restrict__ rel, const int* __restrict__ child,
-                                                          int* __restrict__ sync, int epoch, int k,
-                                                          const T* __restrict__ w, T* __restrict__ yout,
-                                                          T* __restrict__ wu) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ int sTicket;
-  int* err = sync;
-  if (threadIdx.x == 0) sTicket = atomicAdd(&sync[SYNC_TICK_F], 1);
-  __syncthreads();
-  if (sTicket >= (int)gridDim.x) {   // counters not reset: report, touch nothing
-    if (threadIdx.x == 0) atomicExch(err, 2);
-    return;
-  }
-  const RowBlock wk = work[sTicket];
-  const SNode<T>& nd = nodes[wk.node];
-  const int n = nd.n, a0 = wk.b * ICH, a1 = min(nd.m, a0 + ICH);
-  const int warp = threadIdx.x >> 5;
-  T* f = reinterpret_cast<T*>(smraw);   // n x k
-  T* t = f + (size_t)n * k;             // 64 x k
-  T* wud = wu + nd.wuOff * k;
-  if (warp == 0)
-    for (int c = nd.childBegin; c < nd.childEnd; ++c) {
-      const SNode<T>& cn = nodes[child[c]];
-      if (!wait_geq(sync + cn.syncOff + 1, epoch * max(1, cn.nch), err)) break;
-    }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < n * k; idx += blockDim.x) f[idx] = w[(size_t)nd.c0 * k + idx];
-  for (int idx = a0 * k + threadIdx.x; idx < a1 * k; idx += blockDim.x) wud[idx] = T(0);
-  __syncthreads();
-  for (int c = nd.childBegin; c < nd.childEnd; ++c) {
-    const SNode<T>& cn = nodes[child[c]];
-    const T* wuc = wu + cn.wuOff * k;
-    const int* rl = rel + cn.relOff;
-    for (int idx = threadIdx.x; idx < cn.m * k; idx += blockDim.x) {
-      const int a = idx / k, q = idx - a * k;
-      const int tr = rl[a];
-      const T v = __ldcg(wuc + idx);
-      if (tr < n) f[(size_t)tr * k + q] += v;
-      else if (tr - n >= a0 && tr - n < a1) wud[(size_t)(tr - n) * k + q] += v;
-    }
-    __syncthreads();
-  }
-  trsv_dinv_k<T, RA, RC>(nd.L, nd.ld, n, nd.Dinv, f, t, k);
-  if (wk.b == 0)
-    for (int idx = threadIdx.x; idx < n * k; idx += blockDim.x) yout[(size_t)nd.c0 * k + idx] = f[idx];
-  // wud[a][c] -= L21[a] . y[:, c]
-  {
-    const T* L21 = nd.L + (size_t)(n + a0) * nd.ld;
-    const int ld = nd.ld;
-    pair_dots<T, RA, RC, false>(
-        a1 - a0, k, [&](int a, int j) { return L21[(size_t)a * ld + j]; },
-        [&](int j, int c) { return f[(size_t)j * k + c]; }, [](int, int) { return T(0); }, [](int) { return 0; },
-        [&](int) { return n; }, [&](int a, int c, T v) { wud[(size_t)(a0 + a) * k + c] -= v; });
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(sync + nd.syncOff + 1, 1);
-  }
-  launch_done(&sync[SYNC_TICK_F], &sync[SYNC_DONE_F]);
-}
-
-template <class T, int RA, int RC>
-__global__ void __launch_bounds__(256) interior_backward_k(const SNode<T>* __restrict__ nodes,
-                                                           const RowBlock* __restrict__ work,
-                                                           const int* __restrict__ rows, int* __restrict__ sync,
-                                                           int epoch, int k, T* __restrict__ ipart,
-                                                           const T* __restrict__ yin, T* __restrict__ w) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ int sLast, sTicket;
-  int* err = sync;
-  if (threadIdx.x == 0) sTicket = atomicAdd(&sync[SYNC_TICK_B], 1);
-  __syncthreads();
-  if (sTicket >= (int)gridDim.x) {
-    if (threadIdx.x == 0) atomicExch(err, 2);
-    return;
-  }
-  const RowBlock wk = work[sTicket];
-  const SNode<T>& nd = nodes[wk.node];
-  if (nd.parentI >= 0 && (threadIdx.x >> 5) == 0) wait_geq(sync + nodes[nd.parentI].syncOff + 2, epoch, err);
-  __syncthreads();
-  const int n = nd.n, a0 = wk.b * ICH, a1 = min(nd.m, a0 + ICH);
-  T* f = reinterpret_cast<T*>(smraw);   // n x k
-  T* t = f + (size_t)n * k;             // 64 x k
-  const int nch = (nd.m + ICH - 1) / ICH;
-  if (nch > 0) {
-    // part[j][c] = sum_{a in chunk} L21[a][j] x_{rows[a]}[c] (x written by
-    // other blocks of this launch: loads bypass L1)
-    const int* rw = rows + nd.rowsOff;
-    const T* L21 = nd.L + (size_t)n * nd.ld;
-    const int ld = nd.ld;
-    T* part = ipart + (nd.zpOff + (size_t)wk.b * n) * k;
-    pair_dots<T, RA, RC, false>(
-        n, k, [&](int j, int a) { return L21[(size_t)a * ld + j]; },
-        [&](int a, int c) { return __ldcg(w + (size_t)rw[a] * k + c); }, [](int, int) { return T(0); },
-        [&](int) { return a0; }, [&](int) { return a1; }, [&](int j, int c, T v) { part[(size_t)j * k + c] = v; });
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    const int sig = it.sig;
+    cbar();   // every consumer has stored and is done with the stage
+    if (tid == GT - 32) {
+      mbar_arrive(smem_u32(&bars[NSTAGE + s]));
       __threadfence();
-      sLast = (atomicAdd(sync + nd.syncOff, 1) == nch - 1);
-      __threadfence();
-    }
-    __syncthreads();
-    if (!sLast) {
-      launch_done(&sync[SYNC_TICK_B], &sync[SYNC_DONE_B]);
-      return;
+      atomicAdd(A.sync + sig, 1);
     }
   }
-  for (int idx = threadIdx.x; idx < n * k; idx += blockDim.x) {
-    T s = T(0);
-    for (int c = 0; c < nch; ++c) s += __ldcg(ipart + (nd.zpOff + (size_t)c * n) * k + idx);
-    f[idx] = yin[(size_t)nd.c0 * k + idx] - s;
-  }
-  __syncthreads();
-  trsv_dinv_t_k<T, RA, RC>(nd.L, nd.ld, n, nd.Dinv, f, t, k);
-  for (int idx = threadIdx.x; idx < n * k; idx += blockDim.x) w[(size_t)nd.c0 * k + idx] = f[idx];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    if (nch > 0) sync[nd.syncOff] = 0;
-    st_release(sync + nd.syncOff + 2, epoch);
-  }
-  launch_done(&sync[SYNC_TICK_B], &sync[SYNC_DONE_B]);
 }
 
-// w[c0 + i][c] += fixed-order sum of row i's contributions (a warp per row).
+// W64 (n x k) to the working block (n x kp, zeros in the padding)
 template <class T>
-__global__ void __launch_bounds__(256) compressed_gather_k(const SNode<T>* __restrict__ nodes,
-                                                           const int* __restrict__ lvl,
-                                                           const long long* __restrict__ cstart,
-                                                           const long long* __restrict__ ent, int k,
-                                                           const T* __restrict__ wu, T* __restrict__ w) {
-  const SNode<T>& nd = nodes[lvl[blockIdx.y]];
-  const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= nd.n) return;
-  const long long* cs = cstart + nd.cOff;
-  for (int c = lane; c < k; c += 32) {
-    T acc = T(0);
-    for (long long e = cs[i]; e < cs[i + 1]; ++e) acc += wu[ent[e] * k + c];
-    w[(size_t)(nd.c0 + i) * k + c] += acc;
+__global__ void __launch_bounds__(256) widen_kernel(const double* __restrict__ src, T* __restrict__ dst, long long n,
+                                                    int k, int kp) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n * kp; i += (long long)gridDim.x * blockDim.x) {
+    const long long r = i / kp;
+    const int c = (int)(i - r * kp);
+    dst[i] = c < k ? (T)src[r * k + c] : T(0);
   }
 }
 
-// X_R (m x k) of every compressed supernode of a level into its u region.
+// and back; the last kernel of a batched apply also zeroes the ticket and the
+// counters (their last reader, the apply kernel, has finished)
 template <class T>
-__global__ void __launch_bounds__(256) compressed_gather_xr_k(const SNode<T>* __restrict__ nodes,
-                                                              const int* __restrict__ lvl,
-                                                              const int* __restrict__ rows, int k,
-                                                              const T* __restrict__ w, T* __restrict__ wu) {
-  const SNode<T>& nd = nodes[lvl[blockIdx.y]];
-  const int lane = threadIdx.x & 31;
-  const int a = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (a >= nd.m || nd.r == 0) return;
-  const int g = rows[nd.rowsOff + a];
-  T* dst = wu + (nd.wuOff + 2 * nd.r + a) * k;
-  for (int c = lane; c < k; c += 32) dst[c] = w[(size_t)g * k + c];
-}
-
-// Products of the compressed levels: C (M x k) = alpha op(A) B + beta C
-// with B (K x k, row stride ldb) the block of right-hand sides.  With k <= 64
-// these are streaming products over the factor's X, U and V, so they run on
-// SIMT kernels that read A once, coalesced.  Each output column's sum has a
-// fixed order that depends on K alone (not on k); tasks are cut into units
-// (one block each) of a row group and a group of CW columns (skinny_cw),
-// numbered from each task's unitBase.
-template <class T>
-struct SkinnyTask {
-  const T* A;
-  const T* B;
-  T* C;
-  int M, K, lda, ldb, ldc;
-  T alpha, beta;
-  int unitBase;
-};
-
-template <class T>
-__device__ __forceinline__ int find_skinny(const SkinnyTask<T>* __restrict__ tasks, int count, int u) {
-  int lo = 0, hi = count - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (tasks[mid].unitBase <= u) lo = mid;
-    else hi = mid - 1;
+__global__ void __launch_bounds__(256) narrow_kernel(const T* __restrict__ src, double* __restrict__ dst, long long n,
+                                                     int k, int kp, int* __restrict__ clr, int nClr) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n * k; i += (long long)gridDim.x * blockDim.x) {
+    const long long r = i / k;
+    const int c = (int)(i - r * k);
+    dst[i] = (double)src[r * kp + c];
   }
-  return lo;
-}
-
-// Row form, A row-major M x K.  A block per (16 rows, column group), a warp
-// per two rows; lane l adds kk = l, l + 32, ... in order (zeros past K),
-// then the lanes meet in a fixed butterfly.  Chunks of 256 rows of B are
-// staged in shared memory transposed, so lane l reads its kk without bank
-// conflicts, and each staged value serves both rows of the warp.
-constexpr int SK_CHUNK = 256;   // kk per staged chunk of B (8 per lane)
-
-template <class T, int CW>
-__global__ void __launch_bounds__(256) skinny_rows_kernel(const SkinnyTask<T>* __restrict__ tasks, int count, int k) {
-  __shared__ T Bs[CW][SK_CHUNK + 1];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int u = blockIdx.x;
-  const SkinnyTask<T> t = tasks[find_skinny(tasks, count, u)];
-  const int cg = (k + CW - 1) / CW;
-  const int local = u - t.unitBase, rb = local / cg, c0 = (local - rb * cg) * CW;
-  const int i0 = rb * 16 + warp * 2;
-  T acc[2][CW];
-#pragma unroll
-  for (int q = 0; q < CW; ++q) acc[0][q] = acc[1][q] = T(0);
-  const T* a0 = t.A + (size_t)min(i0, t.M - 1) * t.lda;
-  const T* a1 = t.A + (size_t)min(i0 + 1, t.M - 1) * t.lda;
-  for (int kk0 = 0; kk0 < t.K; kk0 += SK_CHUNK) {
-    T av[2][SK_CHUNK / 32];
-#pragma unroll
-    for (int s = 0; s < SK_CHUNK / 32; ++s) {
-      const int kk = kk0 + lane + 32 * s;
-      av[0][s] = kk < t.K ? a0[kk] : T(0);
-      av[1][s] = kk < t.K ? a1[kk] : T(0);
-    }
-    for (int e = threadIdx.x; e < SK_CHUNK * CW; e += blockDim.x) {
-      const int l = e / CW, q = e - l * CW;
-      Bs[q][l] = (kk0 + l < t.K && c0 + q < k) ? t.B[(size_t)(kk0 + l) * t.ldb + c0 + q] : T(0);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int s = 0; s < SK_CHUNK / 32; ++s)
-#pragma unroll
-      for (int q = 0; q < CW; ++q) {
-        const T b = Bs[q][lane + 32 * s];
-        acc[0][q] += av[0][s] * b;
-        acc[1][q] += av[1][s] * b;
-      }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const int i = i0 + r;
-#pragma unroll
-    for (int q = 0; q < CW; ++q) {
-      const T v = warp_sum(acc[r][q]);
-      if (lane == q && i < t.M && c0 + q < k) {
-        T* c = t.C + (size_t)i * t.ldc + c0 + q;
-        T o = t.alpha * v;
-        if (t.beta != T(0)) o += t.beta * *c;
-        *c = o;
-      }
-    }
-  }
-}
-
-// Transposed form, A stored K x M (op(A)[i][kk] = A[kk][i]).  A block per
-// (64 rows, column group): lanes take rows i0 + lane and i0 + lane + 32
-// (coalesced along A's rows), warp w adds kk = w, w + 8, ... in order, and
-// the 8 warp partials are added in warp order.
-template <class T, int CW>
-__global__ void __launch_bounds__(256) skinny_cols_kernel(const SkinnyTask<T>* __restrict__ tasks, int count, int k) {
-  // warp partials go through shared memory QB columns at a time (<= 32 KB)
-  constexpr int QB = sizeof(T) * 8 * 64 * CW > 32768 ? CW / 2 : CW;
-  __shared__ T red[8][64][QB];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int u = blockIdx.x;
-  const SkinnyTask<T> t = tasks[find_skinny(tasks, count, u)];
-  const int cg = (k + CW - 1) / CW;
-  const int local = u - t.unitBase, rb = local / cg, c0 = (local - rb * cg) * CW;
-  const int i0 = rb * 64;
-  const bool v0 = i0 + lane < t.M, v1 = i0 + lane + 32 < t.M;
-  T acc[2][CW];
-#pragma unroll
-  for (int q = 0; q < CW; ++q) acc[0][q] = acc[1][q] = T(0);
-#pragma unroll 8
-  for (int kk = warp; kk < t.K; kk += 8) {
-    const T* arow = t.A + (size_t)kk * t.lda + i0;
-    const T a0 = v0 ? arow[lane] : T(0), a1 = v1 ? arow[lane + 32] : T(0);
-    const T* b = t.B + (size_t)kk * t.ldb + c0;
-#pragma unroll
-    for (int q = 0; q < CW; ++q) {
-      const T bv = c0 + q < k ? b[q] : T(0);
-      acc[0][q] += a0 * bv;
-      acc[1][q] += a1 * bv;
-    }
-  }
-#pragma unroll
-  for (int qb = 0; qb < CW; qb += QB) {
-#pragma unroll
-    for (int q = 0; q < QB; ++q) {
-      red[warp][lane][q] = acc[0][qb + q];
-      red[warp][lane + 32][q] = acc[1][qb + q];
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < 64 * QB; e += blockDim.x) {
-      const int r = e / QB, q = e - r * QB;
-      if (i0 + r >= t.M || c0 + qb + q >= k) continue;
-      T v = T(0);
-#pragma unroll
-      for (int w = 0; w < 8; ++w) v += red[w][r][q];
-      T* c = t.C + (size_t)(i0 + r) * t.ldc + c0 + qb + q;
-      T o = t.alpha * v;
-      if (t.beta != T(0)) o += t.beta * *c;
-      *c = o;
-    }
-    __syncthreads();
-  }
-}
-
-// Long-K products of the batched apply run as K slices (each slice's product
-// to its own block of a workspace, so many more tiles are in flight at small
-// k); this kernel then forms C = alpha * (slice 0 + slice 1 + ...) + beta * C,
-// slices added in order.  The slicing depends on K alone, so the arithmetic of
-// a column does not depend on how many columns the block has.
-template <class T>
-struct SliceSum {
-  T* C;
-  const T* ws;   // slices x M x N, row stride N
-  int ldc, M, N, slices;
-  T alpha, beta;
-};
-
-template <class T>
-__global__ void __launch_bounds__(256) slice_sum_kernel(const SliceSum<T>* __restrict__ sums) {
-  const SliceSum<T> t = sums[blockIdx.y];
-  const long long mn = (long long)t.M * t.N;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < mn; e += (long long)gridDim.x * blockDim.x) {
-    T s = T(0);
-    for (int q = 0; q < t.slices; ++q) s += t.ws[q * mn + e];
-    const int i = (int)(e / t.N), j = (int)(e - (long long)i * t.N);
-    T* c = t.C + (size_t)i * t.ldc + j;
-    T v = t.alpha * s;
-    if (t.beta != T(0)) v += t.beta * *c;
-    *c = v;
-  }
-}
-
-template <class A, class B>
-__global__ void convert_k_kernel(const A* __restrict__ src, B* __restrict__ dst, long long count,
-                                 int* __restrict__ clr = nullptr, int nClr = 0) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x)
-    dst[i] = (B)src[i];
-  // the last kernel of a batched apply also zeroes the interior completion
-  // counters (their last reader, the backward launch, has finished)
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nClr; i += gridDim.x * blockDim.x) clr[i] = 0;
 }
-
-int skinny_width(int k) {
-  int p = 1;
-  while (p < k) p <<= 1;
-  return p;
-}
-
-// columns per unit: k rounded up to a power of two, at most 16 (row form) or
-// 8 (transposed form, whose B values are broadcast loads)
-int skinny_cw(int k, bool cols) { return std::min(cols ? 8 : 16, skinny_width(k)); }
 
 }  // namespace
 
 template <class T>
 int SolveEngine<T>::batch_capacity() const {
-  const size_t per = sizeof(T) * (size_t)(maxNI_ + 64);
-  const int bySmem = (int)std::min<size_t>(64, (200 * 1024) / std::max<size_t>(per, 1));
-  return std::max(1, bySmem);
+  return 64;
 }
 
+// Buffers for blocks of kp columns; they only grow, so a changing width frees
+// nothing and never synchronises the device.
 template <class T>
-void SolveEngine<T>::plan_batch(int k, int cwR, int cwC) {
-  const int key = k * 256 + cwR * 16 + cwC;   // cwR <= 16, cwC <= 8
-  if (key == kB_) return;
-  const Symbolic& S = F_.S;
+void SolveEngine<T>::plan_batch(int kp) {
+  if (kp <= kAllocB_) return;
   cudaStream_t st = F_.stream;
-  if (k > kAllocB_) {
-    dWuB_.alloc(sizeof(T) * std::max(1LL, wuTotal_ * k));
-    dYB_.alloc(sizeof(T) * std::max<long long>(1, (long long)S.n * k));
-    dIpB_.alloc(sizeof(T) * std::max(1LL, ipTotal_ * k));
-    if (!dSyncB_.p) {
-      dSyncB_.alloc(sizeof(int) * syncInts_);
-      RSCHOL_CUDA(cudaMemsetAsync(dSyncB_.p, 0, sizeof(int) * syncInts_, st));
-    }
-    dWB_.alloc(sizeof(T) * std::max<long long>(1, (long long)S.n * k));   // the working copy of W
-    kAllocB_ = k;
-    ++batchGen_;
-    bPlans_.clear();   // the task lists point into the old buffers
+  auto widen = [&](DevBuf& b, const DevBuf& single) { b.alloc(single.bytes * (size_t)kp); };
+  widen(dWuB_, dWu_);
+  widen(dTB_, dT_);
+  widen(dZpB_, dZp_);
+  widen(dSpB_, dSp_);
+  widen(dYpB_, dYp_);
+  widen(dXpB_, dXp_);
+  widen(dIpB_, dIp_);
+  dWB_.alloc(sizeof(T) * (size_t)std::max(1, F_.S.n) * kp);   // the working copy of W
+  if (!dSyncB_.p) {
+    dSyncB_.alloc(sizeof(int) * nSync_);
+    RSCHOL_CUDA(cudaMemsetAsync(dSyncB_.p, 0, sizeof(int) * nSync_, st));
   }
-  auto found = bPlans_.find(key);
-  if (found != bPlans_.end()) {
-    bPlan_ = &found->second;
-    kB_ = key;
-    return;
-  }
-  BatchPlan& plan = bPlans_[key];
-  // products of the compressed levels (skinny SIMT kernels)
-  std::vector<SkinnyTask<T>> tasks;
-  auto& steps = plan.steps;
-  steps.assign(6 * cLevels_.size(), {});
-  T* wu = dWuB_.as<T>();
-  T* yb = dYB_.as<T>();
-  T* w = dWB_.as<T>();
-  // column groups of the two product forms
-  const int cgR = (k + cwR - 1) / cwR;
-  const int cgC = (k + cwC - 1) / cwC;
-  struct Prod {   // one product before it is cut into units
-    const T* A;
-    const T* B;
-    T* C;
-    int M, K, lda, ldb, ldc;
-    bool tA;
-    T alpha, beta;
-  };
-  auto mk = [&](const T* A, int lda, bool tA, const T* B, int ldb, T* C, int ldc, int M, int, int K, T alpha,
-                T beta) { return Prod{A, B, C, M, K, lda, ldb, ldc, tA, alpha, beta}; };
-  // K slicing of the transposed form (a thread runs down K): tasks with K
-  // above kSliceMin run as slices of kSlice into a workspace, then a
-  // fixed-order sum; the slicing depends on K alone
-  constexpr int kSlice = 512, kSliceMin = 768;
-  std::vector<SliceSum<T>> sums;
-  std::vector<std::pair<size_t, long long>> taskWs;   // (task, workspace offset) to patch
-  std::vector<std::pair<size_t, long long>> sumWs;    // (sum, workspace offset) to patch
-  long long wsTotal = 0;
-  auto flush = [&](std::vector<Prod>& batch, int slot) {
-    if (batch.empty()) return;
-    const bool cols = batch[0].tA;   // a flush holds one form
-    std::vector<SkinnyTask<T>> run;
-    const long long sum0 = (long long)sums.size();
-    long long maxMN = 0, wsStep = 0;
-    auto add = [&](const Prod& g, T* C, int ldc, T alpha, T beta) {
-      run.push_back(SkinnyTask<T>{g.A, g.B, C, g.M, g.K, g.lda, g.ldb, ldc, alpha, beta, 0});
-    };
-    for (const Prod& g : batch) {
-      if (!cols || g.K <= kSliceMin) {
-        add(g, g.C, g.ldc, g.alpha, g.beta);
-        continue;
-      }
-      const int ns = (g.K + kSlice - 1) / kSlice;
-      const long long mn = (long long)g.M * k;
-      sumWs.push_back({sums.size(), wsStep});
-      sums.push_back(SliceSum<T>{g.C, nullptr, g.ldc, g.M, k, ns, g.alpha, g.beta});
-      for (int q = 0; q < ns; ++q) {
-        Prod t = g;
-        t.K = std::min(kSlice, g.K - q * kSlice);
-        t.A = g.A + (size_t)q * kSlice * g.lda;
-        t.B = g.B + (size_t)q * kSlice * g.ldb;
-        taskWs.push_back({tasks.size() + run.size(), wsStep + q * mn});
-        add(t, nullptr, k, T(1), T(0));
-      }
-      wsStep += ns * mn;
-      maxMN = std::max(maxMN, mn);
-    }
-    wsTotal = std::max(wsTotal, wsStep);   // every step's slices start at the workspace base
-    int units = 0;   // one block per unit: (16 rows | 64 rows, column group)
-    for (auto& t : run) {
-      t.unitBase = units;
-      units += cols ? (t.M + 63) / 64 * cgC : (t.M + 15) / 16 * cgR;
-    }
-    XStep xs{(long long)tasks.size(), (int)run.size(), units, cols ? 1 : 0};
-    xs.redOff = sum0;
-    xs.redCount = (int)(sums.size() - sum0);
-    xs.redGrid = (int)std::min<long long>(64, (maxMN + 255) / 256);
-    steps[slot].push_back(xs);
-    tasks.insert(tasks.end(), run.begin(), run.end());
-    batch.clear();
-  };
-  const int L = (int)cLevels_.size();
-  for (int l = 0; l < L; ++l) {
-    std::vector<Prod> gy, gz, gu, gs, gg, gx;
-    for (int q = 0; q < cLevels_[l].second; ++q) {
-      const int j = F_.compressedLevels[l][q];
-      const SNode<T>& nd = nodes_[j];
-      const int n = nd.n, m = nd.m, r = nd.r;
-      T* z = wu + nd.wuOff * k;
-      T* sv = wu + (nd.wuOff + r) * k;
-      T* u = wu + (nd.wuOff + 2 * r) * k;
-      T* yj = yb + (size_t)nd.c0 * k;
-      T* wj = w + (size_t)nd.c0 * k;
-      for (int ib = 0; ib < nd.nb; ++ib) {   // Y = X F by row blocks
-        const int h = std::min(64, n - ib * 64), K = std::min(n, (ib + 1) * 64);
-        gy.push_back(mk(nd.X + (size_t)ib * 64 * nd.ldx, nd.ldx, false, wj, k, yj + (size_t)ib * 64 * k, k, h, k, K, T(1),
-                        T(0)));
-      }
-      if (r > 0) {
-        gz.push_back(mk(nd.U, r, true, yj, k, z, k, r, k, n, T(1), T(0)));
-        if (m > 0 && l + 1 < L) gu.push_back(mk(nd.V, r, false, z, k, u, k, m, k, r, T(-1), T(0)));
-        if (m > 0) {
-          gs.push_back(mk(nd.V, r, true, u, k, sv, k, r, k, m, T(1), T(0)));
-          gg.push_back(mk(nd.U, r, false, sv, k, yj, k, n, k, r, T(-1), T(1)));
-        }
-      }
-      for (int jb = 0; jb < nd.nb; ++jb) {   // X = X^T G by column blocks
-        const int h = std::min(64, n - jb * 64), K = n - jb * 64;
-        gx.push_back(mk(nd.X + (size_t)jb * 64 * nd.ldx + jb * 64, nd.ldx, true, yj + (size_t)jb * 64 * k, k,
-                        wj + (size_t)jb * 64 * k, k, h, k, K, T(1), T(0)));
-      }
-    }
-    flush(gy, 6 * l + 0);
-    flush(gz, 6 * l + 1);
-    flush(gu, 6 * l + 2);
-    flush(gs, 6 * l + 3);
-    flush(gg, 6 * l + 4);
-    flush(gx, 6 * l + 5);
-  }
-  plan.ws.alloc(sizeof(T) * std::max(1LL, wsTotal));
-  T* ws = plan.ws.template as<T>();
-  for (auto& tw : taskWs) tasks[tw.first].C = ws + tw.second;
-  for (auto& sw : sumWs) sums[sw.first].ws = ws + sw.second;
-  plan.sums.alloc(std::max<size_t>(16, sums.size() * sizeof(SliceSum<T>)));
-  if (!sums.empty())
-    RSCHOL_CUDA(cudaMemcpyAsync(plan.sums.p, sums.data(), sums.size() * sizeof(SliceSum<T>), cudaMemcpyHostToDevice,
-                                st));
-  plan.tasks.alloc(std::max<size_t>(16, tasks.size() * sizeof(SkinnyTask<T>)));
-  if (!tasks.empty())
-    RSCHOL_CUDA(cudaMemcpyAsync(plan.tasks.p, tasks.data(), tasks.size() * sizeof(SkinnyTask<T>),
-                                cudaMemcpyHostToDevice, st));
-  RSCHOL_CUDA(cudaStreamSynchronize(st));
-  bPlan_ = &plan;
-  kB_ = key;
+  kAllocB_ = kp;
+  ++batchGen_;
 }
 
-template <class T>
-typename SolveEngine<T>::BatchCfg SolveEngine<T>::heuristic_cfg(int kp) const {
-  // what the tuner picks on 2D and 3D diffusion factors of 0.26 - 1 M
-  // unknowns: 1 x 1 pair tiles up to 16 columns, 2 x 4 above; row-form groups
-  // of up to 16 columns; transposed-form groups of 4, 8 from 16 columns on
-  BatchCfg c;
-  if (kp >= 32) c.ra = 2, c.rc = 4;
-  c.cwR = std::min(16, skinny_width(kp));
-  c.cwC = std::min(kp >= 16 ? 8 : 4, skinny_width(kp));
-  return c;
-}
-
-// The width class of k is kp = k rounded up to a power of two (<= the batch
-// capacity); its shapes are timed once, at k = kp, on a zero block: first the
-// interior pair tile, then the row-form and the transposed-form column
-// groups, each over a handful of candidates, the fastest of two timed
-// applies after one warm-up.
 template <class T>
 int SolveEngine<T>::width_class(int k) const {
-  return std::min(skinny_width(k), std::max(k, batch_capacity()));
+  int p = 1;
+  while (p < k) p <<= 1;
+  return p;
 }
 
+// The width class of k is k rounded up to a power of two.  Its one shape, the
+// persistent blocks per SM, is timed at the full width on a zero block: fewer
+// blocks leave fewer items waiting on one another at small widths.
 template <class T>
 const typename SolveEngine<T>::BatchCfg& SolveEngine<T>::config_for(int k, cudaStream_t st, bool tune) {
   const int kp = width_class(k);
   auto it = tuned_.find(kp);
   if (it != tuned_.end() && (it->second.ms > 0 || !tune)) return it->second;
-  BatchCfg best = heuristic_cfg(kp);
+  BatchCfg best;
   if (tune) {
     const size_t bytes = sizeof(double) * (size_t)std::max(1, F_.S.n) * kp;
     DevBuf zero;
@@ -688,7 +743,7 @@ const typename SolveEngine<T>::BatchCfg& SolveEngine<T>::config_for(int k, cudaS
     RSCHOL_CUDA(cudaEventCreate(&e0));
     RSCHOL_CUDA(cudaEventCreate(&e1));
     auto time_cfg = [&](const BatchCfg& c) {
-      apply_batch_cfg(zero.as<double>(), kp, st, c);   // warm-up (plans this shape)
+      apply_batch_cfg(zero.as<double>(), kp, st, c);   // warm-up
       float bestMs = 1e30f;
       for (int rep = 0; rep < 2; ++rep) {
         RSCHOL_CUDA(cudaEventRecord(e0, st));
@@ -702,32 +757,16 @@ const typename SolveEngine<T>::BatchCfg& SolveEngine<T>::config_for(int k, cudaS
       return (double)bestMs;
     };
     best.ms = time_cfg(best);
-    auto consider = [&](BatchCfg c) {
-      if (c.ra == best.ra && c.rc == best.rc && c.cwR == best.cwR && c.cwC == best.cwC) return;
+    for (int b = 1; b < best.blocks; ++b) {
+      BatchCfg c;
+      c.blocks = b;
       c.ms = time_cfg(c);
       if (c.ms < best.ms) best = c;
-    };
-    const int tiles[4][2] = {{1, 1}, {1, 4}, {2, 4}, {4, 4}};
-    for (auto& tl : tiles) {
-      BatchCfg c = best;
-      c.ra = tl[0];
-      c.rc = tl[1];
-      consider(c);
-    }
-    for (int cw = 4; cw <= std::min(16, kp); cw *= 2) {
-      BatchCfg c = best;
-      c.cwR = cw;
-      consider(c);
-    }
-    for (int cw = 2; cw <= std::min(8, kp); cw *= 2) {
-      BatchCfg c = best;
-      c.cwC = cw;
-      consider(c);
     }
     RSCHOL_CUDA(cudaEventDestroy(e0));
     RSCHOL_CUDA(cudaEventDestroy(e1));
   }
-  ++batchGen_;   // new tile shapes: a captured apply would use the old ones
+  ++batchGen_;   // a new shape: a captured apply would use the old one
   return tuned_[kp] = best;
 }
 
@@ -741,8 +780,7 @@ template <class T>
 std::vector<std::array<double, 6>> SolveEngine<T>::batch_tuning() const {
   std::vector<std::array<double, 6>> out;
   for (const auto& kv : tuned_)
-    out.push_back({(double)kv.first, (double)kv.second.ra, (double)kv.second.rc, (double)kv.second.cwR,
-                   (double)kv.second.cwC, kv.second.ms});
+    out.push_back({(double)kv.first, (double)kv.second.blocks, 4.0 * Vec16<T>::V, 0.0, 0.0, kv.second.ms});
   return out;
 }
 
@@ -755,101 +793,26 @@ void SolveEngine<T>::apply_batch(double* W64, int k, cudaStream_t st) {
 
 template <class T>
 void SolveEngine<T>::apply_batch_cfg(double* W64, int k, cudaStream_t st, const BatchCfg& cfg) {
-  plan_batch(k, cfg.cwR, cfg.cwC);
-  const int n = F_.S.n;
-  const long long nk = (long long)n * k;
-  T* w = dWB_.as<T>();
-  convert_k_kernel<double, T><<<(unsigned)std::min<long long>((nk + 255) / 256, 4096), 256, 0, st>>>(W64, w, nk);
-  RSCHOL_LAUNCH_CHECK();
-  // completion targets: every apply starts its counters at zero (they are
-  // cleared by its last kernel), so the apply keeps no host state and replays
-  // inside CUDA graphs
-  const int epoch = 1;
-  int* sync = dSyncB_.as<int>();
-  const size_t smem = sizeof(T) * (size_t)(maxNI_ + 64) * k;
+  constexpr int V = Vec16<T>::V;
+  const int kp = (k + V - 1) / V * V;
+  plan_batch(kp);
+  constexpr int smem = NSTAGE * ST_BYTES + NGRP * FB;
   static std::once_flag once;
   std::call_once(once, [] {
-    const int sm = 200 * 1024;
-#define RSCHOL_SMEM_ATTR(RA, RC)                                                                                \
-  RSCHOL_CUDA(cudaFuncSetAttribute(interior_forward_k<T, RA, RC>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm)); \
-  RSCHOL_CUDA(cudaFuncSetAttribute(interior_backward_k<T, RA, RC>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))
-    RSCHOL_SMEM_ATTR(1, 1);
-    RSCHOL_SMEM_ATTR(1, 4);
-    RSCHOL_SMEM_ATTR(2, 4);
-    RSCHOL_SMEM_ATTR(4, 4);
-#undef RSCHOL_SMEM_ATTR
+    RSCHOL_CUDA(cudaFuncSetAttribute(apply_batch_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   });
-  // register tiles of (row, column) pairs (BatchCfg)
-  using IF = decltype(&interior_forward_k<T, 1, 1>);
-  using IB = decltype(&interior_backward_k<T, 1, 1>);
-  IF fwd = interior_forward_k<T, 1, 1>;
-  IB bwd = interior_backward_k<T, 1, 1>;
-  if (cfg.ra == 4) {
-    fwd = interior_forward_k<T, 4, 4>;
-    bwd = interior_backward_k<T, 4, 4>;
-  } else if (cfg.ra == 2) {
-    fwd = interior_forward_k<T, 2, 4>;
-    bwd = interior_backward_k<T, 2, 4>;
-  } else if (cfg.rc == 4) {
-    fwd = interior_forward_k<T, 1, 4>;
-    bwd = interior_backward_k<T, 1, 4>;
-  }
-  if (nIWork_ > 0) {
-    fwd<<<nIWork_, 256, smem, st>>>(dNodes_.as<SNode<T>>(), dIWork_.as<RowBlock>(), dRel_.as<int>(), dChild_.as<int>(),
-                                    sync, epoch, k, w, dYB_.as<T>(), dWuB_.as<T>());
-    RSCHOL_LAUNCH_CHECK();
-  }
-  const int* lvl = dLevelNodes_.as<int>();
-  const SkinnyTask<T>* bg = bPlan_->tasks.template as<SkinnyTask<T>>();
-  auto gemm = [&](int slot) {
-    for (const XStep& x : bPlan_->steps[slot]) {
-      const SkinnyTask<T>* tk = bg + x.off;
-      const int cw = x.tc ? cfg.cwC : cfg.cwR;
-#define RSCHOL_SKINNY(CW)                                                     \
-  if (x.tc) skinny_cols_kernel<T, CW><<<x.tiles, 256, 0, st>>>(tk, x.count, k); \
-  else skinny_rows_kernel<T, CW><<<x.tiles, 256, 0, st>>>(tk, x.count, k)
-      switch (cw) {
-        case 1: RSCHOL_SKINNY(1); break;
-        case 2: RSCHOL_SKINNY(2); break;
-        case 4: RSCHOL_SKINNY(4); break;
-        case 8: RSCHOL_SKINNY(8); break;
-        default: RSCHOL_SKINNY(16); break;
-      }
-#undef RSCHOL_SKINNY
-      RSCHOL_LAUNCH_CHECK();
-      if (x.redCount > 0) {
-        slice_sum_kernel<T><<<dim3(x.redGrid, x.redCount), 256, 0, st>>>(bPlan_->sums.template as<SliceSum<T>>() +
-                                                                         x.redOff);
-        RSCHOL_LAUNCH_CHECK();
-      }
-    }
-  };
-  const int L = (int)cLevels_.size();
-  for (int l = 0; l < L; ++l) {
-    const int* lv = lvl + cLevels_[l].first;
-    compressed_gather_k<T><<<dim3(cRowGrid_[l], cLevels_[l].second), 256, 0, st>>>(
-        dNodes_.as<SNode<T>>(), lv, dCStart_.as<long long>(), dCEnt_.as<long long>(), k, dWuB_.as<T>(), w);
-    RSCHOL_LAUNCH_CHECK();
-    gemm(6 * l + 0);
-    gemm(6 * l + 1);
-    gemm(6 * l + 2);
-  }
-  for (int l = L - 1; l >= 0; --l) {
-    const int* lv = lvl + cLevels_[l].first;
-    compressed_gather_xr_k<T><<<dim3(cMRowGrid_[l], cLevels_[l].second), 256, 0, st>>>(
-        dNodes_.as<SNode<T>>(), lv, dRows_.as<int>(), k, w, dWuB_.as<T>());
-    RSCHOL_LAUNCH_CHECK();
-    gemm(6 * l + 3);
-    gemm(6 * l + 4);
-    gemm(6 * l + 5);
-  }
-  if (nIWork_ > 0) {
-    bwd<<<nIWork_, 256, smem, st>>>(dNodes_.as<SNode<T>>(), dIWorkB_.as<RowBlock>(), dRows_.as<int>(), sync, epoch,
-                                    k, dIpB_.as<T>(), dYB_.as<T>(), w);
-    RSCHOL_LAUNCH_CHECK();
-  }
-  convert_k_kernel<T, double><<<(unsigned)std::min<long long>((nk + 255) / 256, 4096), 256, 0, st>>>(
-      w, W64, nk, nIWork_ > 0 ? sync + SYNC_GLOBAL : nullptr, nIWork_ > 0 ? syncInts_ - SYNC_GLOBAL : 0);
+  const long long n = F_.S.n;
+  T* w = dWB_.as<T>();
+  const unsigned grid = (unsigned)std::min<long long>((n * kp + 255) / 256, 4096);
+  widen_kernel<T><<<grid, 256, 0, st>>>(W64, w, n, k, kp);
+  RSCHOL_LAUNCH_CHECK();
+  int* sync = dSyncB_.as<int>();
+  const ApplyArgs<T> args{dItems_.as<ApplyItem>(), nItems_,         dBlob_.as<int>(), sync,           w,
+                          dTB_.as<T>(),            dWuB_.as<T>(),   dZpB_.as<T>(),    dSpB_.as<T>(),  dYpB_.as<T>(),
+                          dXpB_.as<T>(),           dIpB_.as<T>(),   0};
+  apply_batch_kernel<T><<<std::min(std::max(1, nItems_), sms_ * cfg.blocks), NGRP * GT + 32, smem, st>>>(args, kp);
+  RSCHOL_LAUNCH_CHECK();
+  narrow_kernel<T><<<grid, 256, 0, st>>>(w, W64, n, k, kp, sync + 1, nSync_ - 1);
   RSCHOL_LAUNCH_CHECK();
 }
 
@@ -860,31 +823,24 @@ int SolveEngine<T>::take_error_batch(cudaStream_t st) {
   RSCHOL_CUDA(cudaMemcpyAsync(&e, dSyncB_.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   RSCHOL_CUDA(cudaStreamSynchronize(st));
   if (e) {
-    RSCHOL_CUDA(cudaMemsetAsync(dSyncB_.p, 0, sizeof(int) * syncInts_, st));
+    RSCHOL_CUDA(cudaMemsetAsync(dSyncB_.p, 0, sizeof(int) * nSync_, st));
     RSCHOL_CUDA(cudaStreamSynchronize(st));
   }
   return e;
 }
 
-template int SolveEngine<double>::batch_capacity() const;
-template int SolveEngine<float>::batch_capacity() const;
-template void SolveEngine<double>::plan_batch(int, int, int);
-template void SolveEngine<float>::plan_batch(int, int, int);
-template SolveEngine<double>::BatchCfg SolveEngine<double>::heuristic_cfg(int) const;
-template SolveEngine<float>::BatchCfg SolveEngine<float>::heuristic_cfg(int) const;
-template const SolveEngine<double>::BatchCfg& SolveEngine<double>::config_for(int, cudaStream_t, bool);
-template const SolveEngine<float>::BatchCfg& SolveEngine<float>::config_for(int, cudaStream_t, bool);
-template int SolveEngine<double>::width_class(int) const;
-template int SolveEngine<float>::width_class(int) const;
-template void SolveEngine<double>::autotune_batch(int, cudaStream_t);
-template void SolveEngine<float>::autotune_batch(int, cudaStream_t);
-template void SolveEngine<double>::apply_batch_cfg(double*, int, cudaStream_t, const BatchCfg&);
-template void SolveEngine<float>::apply_batch_cfg(double*, int, cudaStream_t, const BatchCfg&);
-template std::vector<std::array<double, 6>> SolveEngine<double>::batch_tuning() const;
-template std::vector<std::array<double, 6>> SolveEngine<float>::batch_tuning() const;
-template void SolveEngine<double>::apply_batch(double*, int, cudaStream_t);
-template void SolveEngine<float>::apply_batch(double*, int, cudaStream_t);
-template int SolveEngine<double>::take_error_batch(cudaStream_t);
-template int SolveEngine<float>::take_error_batch(cudaStream_t);
+#define RSCHOL_INST(T)                                                                               \
+  template int SolveEngine<T>::batch_capacity() const;                                               \
+  template void SolveEngine<T>::plan_batch(int);                                                     \
+  template const SolveEngine<T>::BatchCfg& SolveEngine<T>::config_for(int, cudaStream_t, bool);      \
+  template int SolveEngine<T>::width_class(int) const;                                               \
+  template void SolveEngine<T>::autotune_batch(int, cudaStream_t);                                   \
+  template void SolveEngine<T>::apply_batch_cfg(double*, int, cudaStream_t, const BatchCfg&);        \
+  template std::vector<std::array<double, 6>> SolveEngine<T>::batch_tuning() const;                  \
+  template void SolveEngine<T>::apply_batch(double*, int, cudaStream_t);                             \
+  template int SolveEngine<T>::take_error_batch(cudaStream_t);
+RSCHOL_INST(double)
+RSCHOL_INST(float)
+#undef RSCHOL_INST
 
 }  // namespace rschol

@@ -49,18 +49,5 @@ __device__ __forceinline__ bool wait_geq_lim(const int* p, int target, int* err,
   return wait_geq(p, target, err, __ldcg(limitP));
 }
 
-// Every block of a ticketed launch calls this once when it is done; the last
-// one resets the ticket and completion counters for the next launch.
-__device__ __forceinline__ void launch_done(int* tick, int* done) {
-  __syncthreads();
-  if (threadIdx.x == 0 && atomicAdd(done, 1) == (int)gridDim.x - 1) {
-    atomicExch(tick, 0);
-    atomicExch(done, 0);
-  }
-}
-
-constexpr int ICH = 128;   // off-diagonal rows per interior chunk block
-constexpr int SYNC_TICK_F = 1, SYNC_DONE_F = 2, SYNC_TICK_B = 3, SYNC_DONE_B = 4, SYNC_GLOBAL = 5;
-
 }  // namespace solvedev
 }  // namespace rschol
