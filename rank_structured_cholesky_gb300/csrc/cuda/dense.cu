@@ -120,6 +120,91 @@ __device__ void gemm_tile(const GemmTask<T>& t, int row0, int col0, T (*As)[BK][
   }
 }
 
+// FP64: one 32 x 32 tile.  The FP64 unit is the limit (two multiply-adds a
+// clock and SM), so the tile is small enough to spread a launch over the SMs and
+// the 16 x 16 blocks outside C are skipped; K in slices of 32, the next one
+// loaded into registers under the current one's products.  Each C entry's K
+// order is the plain ascending one.  (3D 37x41x35 FP64: the GEMM steps of a
+// factorisation 18.0 ms in 64 x 64 tiles, 7.2 so.)
+__device__ void gemm_tile_f64(const GemmTask<double>& t, int row0, int col0, double (*As)[32][33],
+                              double (*Bs)[32][33]) {
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int nI = min(2, (t.M - row0 + 15) >> 4), nJ = min(2, (t.N - col0 + 15) >> 4);
+  double acc[2][2] = {{0, 0}, {0, 0}}, cpre[2][2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int gi = row0 + ty + 16 * i, gj = col0 + tx + 16 * j;
+      cpre[i][j] = (t.beta != 0 && gi < t.M && gj < t.N) ? __ldcg(t.C + (size_t)gi * t.ldc + gj) : 0.0;
+    }
+  double ra[4], rb[4];
+  const int f = tid & 31, s0 = tid >> 5;   // fast and slow index of a thread's four elements (slow: s0 + 8 q)
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int s = s0 + 8 * q;
+      const int gi = row0 + (t.tA ? f : s), ka = k0 + (t.tA ? s : f);
+      ra[q] = (gi < t.M && ka < t.K) ? __ldcg(t.A + (t.tA ? (size_t)ka * t.lda + gi : (size_t)gi * t.lda + ka)) : 0.0;
+      const int gj = col0 + (t.tB ? s : f), kb = k0 + (t.tB ? f : s);
+      rb[q] = (gj < t.N && kb < t.K) ? __ldcg(t.B + (t.tB ? (size_t)gj * t.ldb + kb : (size_t)kb * t.ldb + gj)) : 0.0;
+    }
+  };
+  auto store = [&](int st) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int s = s0 + 8 * q;
+      if (t.tA) As[st][f][s] = ra[q];
+      else As[st][s][f] = ra[q];
+      if (t.tB) Bs[st][s][f] = rb[q];
+      else Bs[st][f][s] = rb[q];
+    }
+  };
+  if (t.K > 0) {
+    load(0);
+    store(0);
+  }
+  __syncthreads();
+  int st = 0;
+  for (int k0 = 0; k0 < t.K; k0 += 32) {
+    const bool more = k0 + 32 < t.K;
+    if (more) load(k0 + 32);
+    const int kn = min(32, t.K - k0);
+    if (nI == 2 && nJ == 2) {
+#pragma unroll 4
+      for (int k = 0; k < kn; ++k) {
+        const double a0 = As[st][ty][k], a1 = As[st][ty + 16][k], b0 = Bs[st][tx][k], b1 = Bs[st][tx + 16][k];
+        acc[0][0] = fma(a0, b0, acc[0][0]);
+        acc[0][1] = fma(a0, b1, acc[0][1]);
+        acc[1][0] = fma(a1, b0, acc[1][0]);
+        acc[1][1] = fma(a1, b1, acc[1][1]);
+      }
+    } else {
+#pragma unroll 4
+      for (int k = 0; k < kn; ++k) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            if (i < nI && j < nJ) acc[i][j] = fma(As[st][ty + 16 * i][k], Bs[st][tx + 16 * j][k], acc[i][j]);
+      }
+    }
+    if (more) store(st ^ 1);
+    __syncthreads();
+    st ^= 1;
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int gi = row0 + ty + 16 * i, gj = col0 + tx + 16 * j;
+      if (gi >= t.M || gj >= t.N) continue;
+      double v = t.alpha * acc[i][j];
+      if (t.beta != 0) v = fma(t.beta, cpre[i][j], v);
+      t.C[(size_t)gi * t.ldc + gj] = v;
+    }
+}
+
 template <class T>
 __global__ void __launch_bounds__(GEMM_THREADS) gemm_kernel(const GemmTask<T>* __restrict__ tasks, int nTasks) {
   int lo = 0, hi = nTasks - 1;
@@ -132,11 +217,18 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_kernel(const GemmTask<T>* _
   const GemmTask<T> t = tasks[lo];
   const int local = b - t.tileBase;
   const int ti = local / t.tilesN, tj = local - ti * t.tilesN;
-  const int row0 = ti * BM, col0 = tj * BN;
-  if (t.lower && row0 + BM - 1 < col0) return;
-  __shared__ T As[2][BK][BM + 1];
-  __shared__ T Bs[2][BK][BN + 1];
-  gemm_tile<T>(t, row0, col0, As, Bs);
+  constexpr int TL = simt_tile<T>;
+  const int row0 = ti * TL, col0 = tj * TL;
+  if (t.lower && row0 + TL - 1 < col0) return;
+  if constexpr (std::is_same<T, double>::value) {
+    __shared__ double As[2][32][33];
+    __shared__ double Bs[2][32][33];
+    gemm_tile_f64(t, row0, col0, As, Bs);
+  } else {
+    __shared__ T As[2][BK][BM + 1];
+    __shared__ T Bs[2][BK][BN + 1];
+    gemm_tile<T>(t, row0, col0, As, Bs);
+  }
 }
 
 template <class T>
@@ -533,6 +625,184 @@ __device__ void tile_abt_f32(const float* A, int lda, const float* B, int ldb, f
   __syncthreads();
 }
 
+// The FP64 pieces of the fused Cholesky, tiles of up to 32 x 32, 256 threads as
+// 16 x 16.  The FP64 unit is the limit, so each piece forms the 16 x 16 blocks it
+// needs and no more, and divisions and square roots (tens of FP64 instructions
+// each) are done once a column by one warp.  (Against 64 x 64 tiles, whose
+// POTRF -> TRSM -> update chain took 130 us a panel: Cholesky steps of 3D
+// 37x41x35 23.1 -> 12.0 ms, the whole FP64 factorisation of a 61x53 grid 1.36 ->
+// 0.81 ms.)
+//   C := C - A B^T (sub), C := A B^T otherwise; C (M x N), A (M x K), B (N x K).
+// lower: C's blocks above the diagonal are not wanted; tri: B is lower
+// triangular (its columns stop at the row).  A and C may alias: all of A is read
+// before the barrier that precedes the stores.
+__device__ void tile_abt_f64(const double* A, int lda, const double* B, int ldb, double* C, int ldc, int M, int N,
+                             int K, bool sub, bool lower, bool tri, double* smem) {
+  double (*As)[33] = reinterpret_cast<double (*)[33]>(smem);
+  double (*Bs)[33] = reinterpret_cast<double (*)[33]>(smem + 32 * 33);
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, f = tid & 31, s0 = tid >> 5;
+  double ra[4], rb[4], c[2][2];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int i = s0 + 8 * q;
+    ra[q] = (i < M && f < K) ? __ldcg(A + (size_t)i * lda + f) : 0.0;
+    rb[q] = (i < N && f < K) ? __ldcg(B + (size_t)i * ldb + f) : 0.0;
+  }
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const int i = ty + 16 * a, j = tx + 16 * b;
+      c[a][b] = (sub && i < M && j < N) ? __ldcg(C + (size_t)i * ldc + j) : 0.0;
+    }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    As[s0 + 8 * q][f] = ra[q];
+    Bs[s0 + 8 * q][f] = rb[q];
+  }
+  __syncthreads();
+  const bool m1 = M > 16, n1 = N > 16;
+  const bool w01 = n1 && !lower, w10 = m1, w11 = m1 && n1;   // blocks wanted besides (0, 0)
+  double acc[2][2] = {{0, 0}, {0, 0}};
+  const int k0 = tri ? min(K, 16) : K;   // K of the first 16 columns
+#pragma unroll 4
+  for (int k = 0; k < K; ++k) {
+    const double a0 = As[ty][k], a1 = As[ty + 16][k], b0 = Bs[tx][k], b1 = Bs[tx + 16][k];
+    if (k < k0) {
+      acc[0][0] = fma(a0, b0, acc[0][0]);
+      if (w10) acc[1][0] = fma(a1, b0, acc[1][0]);
+    }
+    if (w01) acc[0][1] = fma(a0, b1, acc[0][1]);
+    if (w11) acc[1][1] = fma(a1, b1, acc[1][1]);
+  }
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const int i = ty + 16 * a, j = tx + 16 * b;
+      if (i < M && j < N && (!lower || b <= a)) C[(size_t)i * ldc + j] = sub ? c[a][b] - acc[a][b] : acc[a][b];
+    }
+  __syncthreads();
+}
+
+// Right-looking Cholesky of one n x n (n <= 32) tile, as potrf_tile_reg: column j
+// published unscaled with the reciprocal of its pivot, one barrier a column.
+__device__ void potrf_tile_f64(double* A, int ld, int n, int code, int* flag) {
+  __shared__ double col[2][32], rpv[2], piv[32], dia[32], rdia[32];
+  __shared__ int bad;
+  const int tid = threadIdx.x, ti = tid >> 4, tk = tid & 15;
+  double v[2][2];
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const int i = ti + 16 * a, k = tk + 16 * b;
+      v[a][b] = (i < n && k <= i) ? __ldcg(A + (size_t)i * ld + k) : 0.0;
+    }
+  if (tid == 0) bad = 0;
+  __syncthreads();
+  const bool two = n > 16;
+#pragma unroll
+  for (int b0 = 0; b0 < 2; ++b0) {
+    for (int jj = 0; jj < 16 && 16 * b0 + jj < n; ++jj) {
+      const int j = 16 * b0 + jj, buf = j & 1;
+      if (tk == jj) {   // the owners of column j: rows ti, ti + 16
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+          const int i = ti + 16 * a;
+          double u = v[a][b0];
+          if (i == j) {
+            if (!(u > 0.0)) {   // not positive definite (or NaN): keep going, report
+              bad = 1;
+              u = 1.0;
+            }
+            piv[j] = u;
+            rpv[buf] = pivot_recip(u);
+          }
+          col[buf][i] = i <= j ? 0.0 : u;
+        }
+      }
+      __syncthreads();
+      const double rp = rpv[buf];
+      const double r1 = two ? col[buf][ti + 16] * rp : 0.0;
+      if (b0 == 0) {
+        const double r0 = col[buf][ti] * rp, c0 = col[buf][tk];
+        v[0][0] -= r0 * c0;
+        if (two) v[1][0] -= r1 * c0;
+      }
+      if (two) v[1][1] -= r1 * col[buf][tk + 16];
+    }
+  }
+  __syncthreads();
+  if (tid < n) {
+    const double d = sqrt(piv[tid]);
+    dia[tid] = d;
+    rdia[tid] = 1.0 / d;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const int i = ti + 16 * a, k = tk + 16 * b;
+      if (b <= a && i < n && k <= i) A[(size_t)i * ld + k] = (k == i) ? dia[k] : v[a][b] * rdia[k];
+    }
+  if (tid == 0 && bad) atomicMin(flag, code);
+  __syncthreads();
+}
+
+// out (32 x 32) := L^{-1}, L the w x w (w <= 32) lower tile at Lg padded with a
+// unit diagonal: the 16 x 16 diagonal inverses by forward substitution (a warp
+// each, lane c keeps column c), then the block below the diagonal.
+__device__ void tile_inverse_f64(const double* Lg, int ldl, int w, double* out, double* smem) {
+  double (*L)[33] = reinterpret_cast<double (*)[33]>(smem);
+  double (*Li)[33] = reinterpret_cast<double (*)[33]>(smem + 32 * 33);
+  __shared__ double Tm[16][17], rd[32];
+  const int tid = threadIdx.x;
+#pragma unroll
+  for (int idx = tid; idx < 1024; idx += 256) {
+    const int i = idx >> 5, j = idx & 31;
+    L[i][j] = (i < w && j <= i) ? __ldcg(Lg + (size_t)i * ldl + j) : (i == j ? 1.0 : 0.0);
+    Li[i][j] = 0.0;
+  }
+  __syncthreads();
+  if (tid < 32) rd[tid] = 1.0 / L[tid][tid];
+  __syncthreads();
+  const int nb = (w + 15) >> 4;
+  {
+    const int wb = tid >> 5, c = tid & 15;
+    if (wb < nb && (tid & 31) < 16) {
+      const int o = 16 * wb;
+      double x[16];
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {
+        double s = (r == c) ? 1.0 : 0.0;
+#pragma unroll
+        for (int k = 0; k < r; ++k) s -= L[o + r][o + k] * x[k];
+        x[r] = s * rd[o + r];
+      }
+#pragma unroll
+      for (int r = 0; r < 16; ++r) Li[o + r][o + c] = x[r];
+    }
+  }
+  __syncthreads();
+  if (nb == 2) {
+    const int i = tid >> 4, j = tid & 15;
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) s += L[16 + i][k] * Li[k][j];
+    Tm[i][j] = s;
+    __syncthreads();
+    s = 0.0;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) s += Li[16 + i][16 + k] * Tm[k][j];
+    Li[16 + i][j] = -s;
+    __syncthreads();
+  }
+#pragma unroll
+  for (int idx = tid; idx < 1024; idx += 256) out[idx] = Li[idx >> 5][idx & 31];
+}
+
 template <class T>
 __global__ void __launch_bounds__(256) trsm_inv_kernel(const TrsmTask<T>* __restrict__ tasks, int nTasks) {
   // B (64-row chunk x w) := B L^{-T}: the block inverts its w x w tile and
@@ -561,9 +831,9 @@ __global__ void __launch_bounds__(256) trsm_inv_kernel(const TrsmTask<T>* __rest
 
 // Blocked partial Cholesky of every front of a level in one launch.  A job
 // factors the first nDiag columns of a front F (rows x rows, lower, row-major)
-// in panels: the first w0 = nDiag - 64 (P - 1) wide, the others 64, so that
-// every later panel and every trailing block is aligned to the tile grid
-// b(0) = 0, b(t) = w0 + 64 (t - 1).  Panel p is one POTRF of tile (p, p)
+// in panels: the first w0 = nDiag - NB (P - 1) wide, the others NB (64, FP64 32),
+// so that every later panel and every trailing block is aligned to the tile grid
+// b(0) = 0, b(t) = w0 + NB (t - 1).  Panel p is one POTRF of tile (p, p)
 // (which also stores the tile's inverse), one TRSM per row tile a > p, and
 // one update C(a, b) -= X(a) X(b)^T (K = panel width) per lower tile of the
 // trailing block with column tile b below nUpd.  Each piece is a work item;
@@ -614,8 +884,9 @@ __global__ void __launch_bounds__(256) chol_fused_kernel(const CholFusedJob<T>* 
   int* pdone = tdone + j.TR;       // P: POTRF of panel p done
   const int p = it.p, a = it.a, b = it.b;
   const int* lim = flag + 2;   // polls before a wait gives up (set with the flags before the factorisation)
-  auto bnd = [&](int t) { return t == 0 ? 0 : j.w0 + 64 * (t - 1); };      // columns (and Cholesky rows)
-  auto rbnd = [&](int t) { return t == 0 ? 0 : j.r1 + 64 * (t - 1); };     // rows
+  constexpr int NB = chol_nb<T>;
+  auto bnd = [&](int t) { return t == 0 ? 0 : j.w0 + NB * (t - 1); };      // columns (and Cholesky rows)
+  auto rbnd = [&](int t) { return t == 0 ? 0 : j.r1 + NB * (t - 1); };     // rows
   const int c0 = bnd(p), wp = bnd(p + 1) - c0;
   if ((threadIdx.x >> 5) == 0) {
     bool ok;
@@ -640,65 +911,44 @@ __global__ void __launch_bounds__(256) chol_fused_kernel(const CholFusedJob<T>* 
     // Cholesky job: factor the diagonal tile; TRSM job: L is factored already
     T* A = j.L ? const_cast<T*>(j.L) + (size_t)c0 * j.ldl + c0 : F + (size_t)c0 * ld + c0;
     const int lda = j.L ? j.ldl : ld;
-    if (!j.L) potrf_tile_reg<T>(A, ld, wp, j.code, flag);
-    if (j.L || c0 + wp < j.nRows) {   // rows below: the TRSM items multiply by the inverse
-      T (*L)[65] = reinterpret_cast<T (*)[65]>(cf_smem);
-      T (*Li)[65] = reinterpret_cast<T (*)[65]>(cf_smem + sizeof(T) * 64 * 65);
-      T (*Tm)[16][17] = reinterpret_cast<T (*)[16][17]>(cf_smem + 2 * sizeof(T) * 64 * 65);
-      tile_inverse<T>(A, lda, wp, L, Li, Tm);
-      T* out = ws + j.inv + (size_t)p * 4096;
+    T* out = ws + j.inv + (size_t)p * NB * NB;
+    const bool below = j.L || c0 + wp < j.nRows;   // rows below: the TRSM items multiply by the inverse
+    if constexpr (std::is_same<T, double>::value) {
+      if (!j.L) potrf_tile_f64(A, ld, wp, j.code, flag);
+      if (below) tile_inverse_f64(A, lda, wp, out, reinterpret_cast<double*>(cf_smem));
+    } else {
+      if (!j.L) potrf_tile_reg<T>(A, ld, wp, j.code, flag);
+      if (below) {
+        T (*L)[65] = reinterpret_cast<T (*)[65]>(cf_smem);
+        T (*Li)[65] = reinterpret_cast<T (*)[65]>(cf_smem + sizeof(T) * 64 * 65);
+        T (*Tm)[16][17] = reinterpret_cast<T (*)[16][17]>(cf_smem + 2 * sizeof(T) * 64 * 65);
+        tile_inverse<T>(A, lda, wp, L, Li, Tm);
 #pragma unroll
-      for (int idx = threadIdx.x; idx < 64 * 64; idx += 256) out[idx] = Li[idx >> 6][idx & 63];
+        for (int idx = threadIdx.x; idx < 64 * 64; idx += 256) out[idx] = Li[idx >> 6][idx & 63];
+      }
     }
     done = pdone + p;
     doneVal = 1;
-  } else if (it.kind == CHOL_TRSM && std::is_same<T, float>::value) {
+  } else if (it.kind == CHOL_TRSM) {
     // X(a) := X(a) Li(p)^T with the panel's inverse tile straight from the workspace
     const int r0 = rbnd(a), nr = min(rbnd(a + 1), j.nRows) - r0;
-    float* X = reinterpret_cast<float*>(F) + (size_t)r0 * ld + c0;
-    const float* Li = reinterpret_cast<const float*>(ws) + j.inv + (size_t)p * 4096;
-    tile_abt_f32(X, ld, Li, 64, X, ld, nr, wp, wp, false, reinterpret_cast<float*>(cf_smem));
+    T* X = F + (size_t)r0 * ld + c0;
+    const T* Li = ws + j.inv + (size_t)p * NB * NB;
+    if constexpr (std::is_same<T, double>::value)
+      tile_abt_f64(X, ld, Li, NB, X, ld, nr, wp, wp, false, false, true, reinterpret_cast<double*>(cf_smem));
+    else tile_abt_f32(X, ld, Li, NB, X, ld, nr, wp, wp, false, reinterpret_cast<float*>(cf_smem));
     done = tdone + a;
     doneVal = p + 1;
-  } else if (it.kind == CHOL_TRSM) {
-    T (*X)[65] = reinterpret_cast<T (*)[65]>(cf_smem);
-    T (*Li)[65] = reinterpret_cast<T (*)[65]>(cf_smem + sizeof(T) * 64 * 65);
-    const T* in = ws + j.inv + (size_t)p * 4096;
-#pragma unroll
-    for (int idx = threadIdx.x; idx < 64 * 64; idx += 256) Li[idx >> 6][idx & 63] = __ldcg(in + idx);
-    __syncthreads();
-    const int r0 = rbnd(a);
-    trsm_chunk_mul<T>(F + (size_t)r0 * ld + c0, ld, min(rbnd(a + 1), j.nRows) - r0, wp, X, Li);
-    done = tdone + a;
-    doneVal = p + 1;
-  } else if (std::is_same<T, float>::value) {   // update of tile (a, b) by panel p
+  } else {   // update of tile (a, b) by panel p
     const int r0 = rbnd(a), q0 = bnd(b);
-    float* Ff = reinterpret_cast<float*>(F);
-    const float* Bp = j.L ? reinterpret_cast<const float*>(j.L) + (size_t)q0 * j.ldl + c0 : Ff + (size_t)q0 * ld + c0;
+    const T* Bp = j.L ? j.L + (size_t)q0 * j.ldl + c0 : F + (size_t)q0 * ld + c0;   // TRSM job: X(a) L(b, p)^T
     const int m = min(rbnd(a + 1), j.nRows) - r0, n = min(bnd(b + 1), j.nUpd) - q0, ldb = j.L ? j.ldl : ld;
-    tile_abt_f32(Ff + (size_t)r0 * ld + c0, ld, Bp, ldb, Ff + (size_t)r0 * ld + q0, ld, m, n, wp, true,
-                 reinterpret_cast<float*>(cf_smem));
-    done = cnt + a * j.TU + b;
-    doneVal = p + 1;
-  } else {
-    const int r0 = rbnd(a), q0 = bnd(b);
-    GemmTask<T> g;
-    g.A = F + (size_t)r0 * ld + c0;
-    g.B = j.L ? j.L + (size_t)q0 * j.ldl + c0 : F + (size_t)q0 * ld + c0;   // TRSM job: X(a) L(b, p)^T
-    g.C = F + (size_t)r0 * ld + q0;
-    g.M = min(rbnd(a + 1), j.nRows) - r0;
-    g.N = min(bnd(b + 1), j.nUpd) - q0;
-    g.K = wp;
-    g.lda = g.ldc = ld;
-    g.ldb = j.L ? j.ldl : ld;
-    g.tA = 0;
-    g.tB = 1;
-    g.lower = 0;
-    g.alpha = T(-1);
-    g.beta = T(1);
-    T (*As)[BK][BM + 1] = reinterpret_cast<T (*)[BK][BM + 1]>(cf_smem);
-    T (*Bs)[BK][BN + 1] = reinterpret_cast<T (*)[BK][BN + 1]>(cf_smem + 2 * sizeof(T) * BK * (BM + 1));
-    gemm_tile<T>(g, 0, 0, As, Bs);
+    if constexpr (std::is_same<T, double>::value)
+      tile_abt_f64(F + (size_t)r0 * ld + c0, ld, Bp, ldb, F + (size_t)r0 * ld + q0, ld, m, n, wp, true, !j.L && a == b,
+                   false, reinterpret_cast<double*>(cf_smem));
+    else
+      tile_abt_f32(F + (size_t)r0 * ld + c0, ld, Bp, ldb, F + (size_t)r0 * ld + q0, ld, m, n, wp, true,
+                   reinterpret_cast<float*>(cf_smem));
     done = cnt + a * j.TU + b;
     doneVal = p + 1;
   }
@@ -1250,7 +1500,8 @@ void launch_chol_fused(const CholFusedJob<T>* jobs, const CholItem* items, int n
                        T* ws, int* flag, unsigned long long* trace, cudaStream_t s) {
   if (nItems <= 0) return;
   RSCHOL_CUDA(cudaMemsetAsync(sync, 0, sizeof(int) * (size_t)syncInts, s));
-  const int smem = (int)(sizeof(T) * (3 * 64 * 65 + 3 * 16 * 17));
+  const int smem = std::is_same<T, double>::value ? (int)(sizeof(T) * 2 * 32 * 33)
+                                                  : (int)(sizeof(T) * (3 * 64 * 65 + 3 * 16 * 17));
   static std::once_flag once;
   std::call_once(once, [&] {
     RSCHOL_CUDA(cudaFuncSetAttribute(chol_fused_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));

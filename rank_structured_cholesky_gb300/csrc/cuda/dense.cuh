@@ -72,20 +72,20 @@ struct TrsmTask {
 // Blocked partial Cholesky of several fronts in one launch (tile-level
 // dependencies, ticketed work items): job = the first nDiag columns of the
 // nRows x nRows lower front F; trailing updates reach the columns below nUpd.
-// Panels: the first w0 = nDiag - 64 (P - 1) wide, then 64; tile t spans rows
-// [b(t), b(t + 1)), b(0) = 0, b(t) = w0 + 64 (t - 1); TR / TU tiles cover
+// Panels: the first w0 = nDiag - NB (P - 1) wide, then NB = chol_nb<T>; tile t
+// spans rows [b(t), b(t + 1)), b(0) = 0, b(t) = w0 + NB (t - 1); TR / TU tiles cover
 // nRows / nUpd.
 // A TRSM job (L != null) is the same launch's B := B L^{-T} for a factored
 // w x w lower L (ld ldl) and F = B (nRows x w, ld): "POTRF" items only
 // invert L's diagonal tiles (no wait), the updates are X(a) L(b, p)^T, and B's
-// rows are cut at 0, r1 = 64, 128, ... (a Cholesky job has r1 = w0).
+// rows are cut at 0, r1 = NB, 2 NB, ... (a Cholesky job has r1 = w0).
 template <class T>
 struct CholFusedJob {
   T* F;
   int ld, nDiag, nRows, nUpd, code;
   int w0, P, TR, TU;
   int cnt;          // offset of the job's TR x TU + TR + P counters after the ticket
-  long long inv;    // element offset of the job's P inverse tiles (64 x 64) in the workspace
+  long long inv;    // element offset of the job's P inverse tiles (NB x NB) in the workspace
   const T* L;       // TRSM job: the factored triangle (null for a Cholesky job)
   int ldl, r1;      // r1: height of the first row tile
 };
@@ -124,6 +124,13 @@ struct ExtAddRow {
   T* Frow;             // target row
   int segBegin, segEnd;
 };
+
+// Tile (rows and columns) of the SIMT GEMM, and panel and tile width of the fused
+// Cholesky.  FP64 runs at 1/64 of the FP32 rate -- two multiply-adds a clock and
+// SM -- so a 64 x 64 x 64 product holds its SM for 64 us and leaves the others
+// idle wherever a launch has few of them: FP64 tiles are 32 wide.
+template <class T> constexpr int simt_tile = std::is_same<T, double>::value ? 32 : 64;
+template <class T> constexpr int chol_nb = std::is_same<T, double>::value ? 32 : 64;
 
 template <class T> void launch_gemm(const GemmTask<T>* dTasks, int nTasks, int totalTiles, cudaStream_t s);
 // The lower triangle of an n x n FP32 block (leading dimension ld) to FP64

@@ -16,7 +16,7 @@ namespace rschol {
 
 namespace {
 constexpr int NB = 64;           // tile width of the blocked factorisations
-int tiles_of(int M, int N, int rowsPerTile) { return ((M + rowsPerTile - 1) / rowsPerTile) * ((N + 63) / 64); }
+int tiles_of(int M, int N, int tile) { return ((M + tile - 1) / tile) * ((N + tile - 1) / tile); }
 
 // FP32 factors run their GEMMs on the tensor cores unless
 // RSCHOL_TENSOR_CORES=0 (the SIMT kernel then serves both precisions).
@@ -92,8 +92,8 @@ void FactorEngine<T>::flush_gemm(std::vector<GemmTask<T>>& batch, int) {
   if (tc && prm.schur_bf16)
     for (auto& t : batch) bf = bf || t.split != 0;
   const int kAlign = bf ? 64 : 32;   // K per pipeline stage: split-K slices start on one
-  const int rowsPerTile = tc ? 128 : 64;
-  const int bn = tc ? tc_tile_n(maxN) : 64;   // tile width: 128 x bn on the tensor cores
+  const int rowsPerTile = tc ? 128 : simt_tile<T>;
+  const int bn = tc ? tc_tile_n(maxN) : simt_tile<T>;   // tile width: 128 x bn on the tensor cores
   long long baseTiles = 0;
   for (auto& t : batch) baseTiles += (long long)((t.M + rowsPerTile - 1) / rowsPerTile) * ((t.N + bn - 1) / bn);
   const long long want = 2LL * 152;   // two blocks per SM
@@ -144,7 +144,7 @@ template <class T>
 void FactorEngine<T>::push_gemm(const GemmTask<T>& t0, int& tiles, std::vector<GemmTask<T>>& batch) {
   if (t0.M <= 0 || t0.N <= 0) return;
   GemmTask<T> t = t0;
-  tiles += tiles_of(t.M, t.N, 64);   // tiles and bases are fixed when the batch is flushed
+  tiles += tiles_of(t.M, t.N, simt_tile<T>);   // tiles and bases are fixed when the batch is flushed
   batch.push_back(t);
   double f = 2.0 * t.M * t.N * std::max(t.K, 0);
   if (t.lower && t.M == t.N) f *= 0.5;
@@ -188,6 +188,7 @@ template <class T>
 template <class U>
 void FactorEngine<T>::emit_fused(const std::vector<CholJob<U>>& jobs, int kind, std::vector<CholFusedJob<U>>& cjobs,
                                  std::vector<CholItem>& items, long long& syncMax, long long& wsMax) {
+  constexpr int NB = chol_nb<U>;
   Step st{kind, (long long)items.size(), 0, 0};
   const double flops0 = flops;
   const int j0 = (int)cjobs.size();
@@ -400,6 +401,7 @@ void FactorEngine<T>::emit_l21(const std::vector<TrsmJob<T>>& jobs) {
 template <class T>
 void FactorEngine<T>::emit_trsm(const std::vector<TrsmJob<T>>& jobs) {
   if (fusedChol_) {   // one ticketed launch (TRSM jobs of the fused Cholesky kernel)
+    constexpr int NB = chol_nb<T>;
     Step st{ST_CHOL, (long long)cholItems_.size(), 0, 0};
     const double flops0 = flops;
     const int j0 = (int)cholJobs_.size();

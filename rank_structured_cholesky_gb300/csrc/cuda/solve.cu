@@ -1544,7 +1544,7 @@ void SolveEngine<T>::plan_inverse(const std::vector<long long>& xOff) {
   // triangle, so the work is n^3 / 3 per supernode.
   const Symbolic& S = F_.S;
   const bool tc = std::is_same<T, float>::value && F_.tensor_cores();
-  const int rpt = tc ? 128 : 64;
+  const int rpt = tc ? 128 : simt_tile<T>;
   const int nn = (int)S.nodes.size();
   int maxN = 0;
   for (int s = 0; s < nn; ++s)
@@ -1575,7 +1575,6 @@ void SolveEngine<T>::plan_inverse(const std::vector<long long>& xOff) {
     t.ldc = ldc;
     t.alpha = alpha;
     t.beta = T(0);
-    t.tilesN = (N + 63) / 64;
     t.split = 1;
     t.kSplit = 1;
     t.kLen = K;
@@ -1585,7 +1584,7 @@ void SolveEngine<T>::plan_inverse(const std::vector<long long>& xOff) {
     if (batch.empty()) return;
     int maxN = 0;
     for (auto& t : batch) maxN = std::max(maxN, t.N);
-    const int bn = tc ? tc_tile_n(maxN) : 64;
+    const int bn = tc ? tc_tile_n(maxN) : simt_tile<T>;
     int tiles = 0;
     for (auto& t : batch) {
       t.tilesN = (t.N + bn - 1) / bn;
@@ -1629,19 +1628,20 @@ void SolveEngine<T>::plan_inverse(const std::vector<long long>& xOff) {
   // S = X^T X and G = L21 X of the interior ones of more than 64 columns, by
   // blocks whose K starts at the triangle
   std::vector<GemmTask<T>> bw, bi;
+  const int blk = rpt;
   for (int s = 0; s < nn; ++s) {
     const SNode<T>& sn = nodes_[s];
     const int n = sn.n, lx = sn.ldx;
     if (S.nodes[s].compressed) {
-      for (int j0 = 0; sn.r > 0 && j0 < n; j0 += rpt) {
+      for (int j0 = 0; sn.r > 0 && j0 < n; j0 += blk) {
         GemmTask<T> t = mk(sn.X + (size_t)j0 * lx + j0, lx, sn.U + (size_t)j0 * sn.r, sn.r,
-                           const_cast<T*>(sn.W) + (size_t)j0 * sn.r, sn.r, std::min(rpt, n - j0), sn.r, n - j0, T(1));
+                           const_cast<T*>(sn.W) + (size_t)j0 * sn.r, sn.r, std::min(blk, n - j0), sn.r, n - j0, T(1));
         t.tA = 1;
         bw.push_back(t);
       }
     } else if (xOff[s] >= 0) {
-      for (int i0 = 0; i0 < n; i0 += rpt) {
-        const int h = std::min(rpt, n - i0);
+      for (int i0 = 0; i0 < n; i0 += blk) {
+        const int h = std::min(blk, n - i0);
         GemmTask<T> t = mk(sn.X + (size_t)i0 * lx + i0, lx, sn.X + (size_t)i0 * lx, lx, sn.Sg + (size_t)i0 * sn.ldk,
                            sn.ldk, h, n, n - i0, T(1));
         t.tA = 1;
