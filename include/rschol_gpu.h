@@ -239,6 +239,12 @@ int rschol_step_timing(rschol_factor* f, int enable, double* out);
  * 1 when the operands were staged by TMA (A M x K and B N x K row-major,
  * aligned, TF32), 0 when through registers.  out holds 3 values. */
 int rschol_selftest_gemm(int M, int N, int K, int tA, int tB, int split, int lower, double* out);
+/* Diagnostics: the FP64 GEMM kernel, split into `slices` along K, against a host
+ * product: out[0] = largest error relative to sum_k |a b| + |beta c|. */
+int rschol_selftest_gemm64(int M, int N, int K, int tA, int tB, int slices, double* out);
+/* Diagnostics: thin Householder QR of `tasks` random n x r matrices (column r / 2
+ * zero): out[0] = max |Q^T Q - I|, out[1] = max over columns |y - Q Q^T y| / |y|. */
+int rschol_selftest_qr(int n, int r, int tasks, int fp64, double* out);
 
 /* Diagnostics (no reference counterpart): *ms = average device time of one
  * tensor-core launch C (M x N) -= A (M x K) B^T (A, B row-major, the

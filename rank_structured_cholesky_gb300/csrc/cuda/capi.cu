@@ -936,6 +936,143 @@ extern "C" int rschol_selftest_gemm(int M, int N, int K, int tA, int tB, int spl
   return RSCHOL_OK;
 }
 
+// ---- diagnostics: the FP64 GEMM (slices > 1: split along K) against a host product --
+extern "C" int rschol_selftest_gemm64(int M, int N, int K, int tA, int tB, int slices, double* out) {
+  if (M <= 0 || N <= 0 || K <= 0 || slices <= 0 || slices > K || !out) return RSCHOL_E_BAD_INPUT;
+  int count = 0;
+  if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0) return RSCHOL_E_NO_DEVICE;
+  try {
+    std::vector<double> A((size_t)M * K), B((size_t)K * N), C((size_t)M * N), C0((size_t)M * N);
+    uint64_t st = 0x9E3779B97F4A7C15ull;
+    for (auto* v : {&A, &B, &C0})
+      for (auto& x : *v) {
+        st = st * 6364136223846793005ull + 1442695040888963407ull;
+        x = (double)(st >> 11) * (1.0 / 9007199254740992.0) * 2.0 - 1.0;
+      }
+    DevBuf dA, dB, dC, dT, dW, dIds, dBase;
+    dA.alloc(sizeof(double) * A.size());
+    dB.alloc(sizeof(double) * B.size());
+    dC.alloc(sizeof(double) * C.size());
+    dT.alloc(sizeof(GemmTask<double>));
+    RSCHOL_CUDA(cudaMemcpy(dA.p, A.data(), sizeof(double) * A.size(), cudaMemcpyHostToDevice));
+    RSCHOL_CUDA(cudaMemcpy(dB.p, B.data(), sizeof(double) * B.size(), cudaMemcpyHostToDevice));
+    RSCHOL_CUDA(cudaMemcpy(dC.p, C0.data(), sizeof(double) * C.size(), cudaMemcpyHostToDevice));
+    GemmTask<double> t{};
+    t.A = dA.as<double>();
+    t.B = dB.as<double>();
+    t.C = dC.as<double>();
+    t.M = M;
+    t.N = N;
+    t.K = K;
+    t.lda = tA ? M : K;
+    t.ldb = tB ? K : N;
+    t.ldc = N;
+    t.tA = tA;
+    t.tB = tB;
+    t.alpha = -1.25;
+    t.beta = 0.5;
+    t.tilesN = (N + simt_tile<double> - 1) / simt_tile<double>;
+    t.kLen = (K + slices - 1) / slices;
+    t.kSplit = (K + t.kLen - 1) / t.kLen;
+    const int tilesPer = ((M + simt_tile<double> - 1) / simt_tile<double>)*t.tilesN;
+    dW.alloc(sizeof(double) * (size_t)t.kSplit * tilesPer * simt_tile<double> * simt_tile<double>);
+    t.ws = dW.as<float>();
+    RSCHOL_CUDA(cudaMemcpy(dT.p, &t, sizeof(t), cudaMemcpyHostToDevice));
+    launch_gemm(dT.as<GemmTask<double>>(), 1, tilesPer * t.kSplit, 0);
+    if (t.kSplit > 1) {
+      const int id = 0;
+      const long long base[2] = {0, (long long)M * N};
+      dIds.alloc(sizeof(int));
+      dBase.alloc(sizeof(base));
+      RSCHOL_CUDA(cudaMemcpy(dIds.p, &id, sizeof(int), cudaMemcpyHostToDevice));
+      RSCHOL_CUDA(cudaMemcpy(dBase.p, base, sizeof(base), cudaMemcpyHostToDevice));
+      launch_gemm_splitk_reduce(dT.as<GemmTask<double>>(), dIds.as<int>(), 1, dBase.as<long long>(), base[1], 0);
+    }
+    RSCHOL_CUDA(cudaDeviceSynchronize());
+    RSCHOL_CUDA(cudaMemcpy(C.data(), dC.p, sizeof(double) * C.size(), cudaMemcpyDeviceToHost));
+    double worst = 0;
+    for (int i = 0; i < M; ++i)
+      for (int j = 0; j < N; ++j) {
+        double s = 0, mag = 0;
+        for (int k = 0; k < K; ++k) {
+          const double p = A[tA ? (size_t)k * M + i : (size_t)i * K + k] * B[tB ? (size_t)j * K + k : (size_t)k * N + j];
+          s += p;
+          mag += std::fabs(p);
+        }
+        const double c0 = 0.5 * C0[(size_t)i * N + j];
+        worst = std::max(worst, std::fabs(C[(size_t)i * N + j] - (c0 - 1.25 * s)) / (1.25 * mag + std::fabs(c0)));
+      }
+    out[0] = worst;
+  } catch (const std::exception&) {
+    return RSCHOL_E_CUDA;
+  }
+  return RSCHOL_OK;
+}
+
+// ---- diagnostics: the thin Householder QR -------------------------------------
+namespace {
+template <class T>
+void selftest_qr(int n, int r, int tasks, double* out) {
+  std::vector<T> Y((size_t)tasks * n * r), Q(Y.size());
+  uint64_t st = 0x9E3779B97F4A7C15ull;
+  for (size_t e = 0; e < Y.size(); ++e) {
+    st = st * 6364136223846793005ull + 1442695040888963407ull;
+    // column r / 2 is zero where there are three or more
+    Y[e] = (r >= 3 && (int)(e % r) == r / 2) ? T(0) : (T)((double)(st >> 11) * (1.0 / 9007199254740992.0) * 2.0 - 1.0);
+  }
+  DevBuf dY, dW, dT, dS;
+  dY.alloc(sizeof(T) * Y.size());
+  dW.alloc(sizeof(T) * Y.size());
+  dS.alloc(sizeof(T) * std::max(1LL, householder_qr_workspace(tasks, n, r)));
+  std::vector<QrTask<T>> t;
+  for (int q = 0; q < tasks; ++q)
+    t.push_back(QrTask<T>{dY.as<T>() + (size_t)q * n * r, dW.as<T>() + (size_t)q * n * r, n, r});
+  dT.alloc(sizeof(QrTask<T>) * t.size());
+  RSCHOL_CUDA(cudaMemcpy(dY.p, Y.data(), sizeof(T) * Y.size(), cudaMemcpyHostToDevice));
+  RSCHOL_CUDA(cudaMemcpy(dT.p, t.data(), sizeof(QrTask<T>) * t.size(), cudaMemcpyHostToDevice));
+  launch_householder_qr<T>(dT.as<QrTask<T>>(), tasks, n, r, dS.as<T>(), 0);
+  RSCHOL_CUDA(cudaDeviceSynchronize());
+  RSCHOL_CUDA(cudaMemcpy(Q.data(), dY.p, sizeof(T) * Y.size(), cudaMemcpyDeviceToHost));
+  out[0] = out[1] = 0;
+  std::vector<double> G((size_t)r * r), H((size_t)r * r);
+  for (int q = 0; q < tasks; ++q) {
+    const T *y = Y.data() + (size_t)q * n * r, *x = Q.data() + (size_t)q * n * r;
+    std::fill(G.begin(), G.end(), 0.0);   // Q^T Q
+    std::fill(H.begin(), H.end(), 0.0);   // Q^T Y
+    for (int i = 0; i < n; ++i)
+      for (int a = 0; a < r; ++a)
+        for (int b = 0; b < r; ++b) {
+          G[(size_t)a * r + b] += (double)x[(size_t)i * r + a] * (double)x[(size_t)i * r + b];
+          H[(size_t)a * r + b] += (double)x[(size_t)i * r + a] * (double)y[(size_t)i * r + b];
+        }
+    for (int a = 0; a < r; ++a)
+      for (int b = 0; b < r; ++b) out[0] = std::max(out[0], std::fabs(G[(size_t)a * r + b] - (a == b ? 1.0 : 0.0)));
+    for (int b = 0; b < r; ++b) {
+      double num = 0, den = 0;
+      for (int i = 0; i < n; ++i) {
+        double s = (double)y[(size_t)i * r + b];
+        den += s * s;
+        for (int a = 0; a < r; ++a) s -= (double)x[(size_t)i * r + a] * H[(size_t)a * r + b];
+        num += s * s;
+      }
+      if (den > 0) out[1] = std::max(out[1], std::sqrt(num / den));
+    }
+  }
+}
+}  // namespace
+extern "C" int rschol_selftest_qr(int n, int r, int tasks, int fp64, double* out) {
+  if (r <= 0 || n < r || tasks <= 0 || !out) return RSCHOL_E_BAD_INPUT;
+  int count = 0;
+  if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0) return RSCHOL_E_NO_DEVICE;
+  try {
+    if (fp64) selftest_qr<double>(n, r, tasks, out);
+    else selftest_qr<float>(n, r, tasks, out);
+  } catch (const std::exception&) {
+    return RSCHOL_E_CUDA;
+  }
+  return RSCHOL_OK;
+}
+
 // ---- diagnostics: device time of one tensor-core GEMM launch -----------------
 extern "C" int rschol_bench_gemm(int M, int N, int K, int split, int reps, double* ms) {
   if (M <= 0 || N <= 0 || K <= 0 || reps <= 0 || !ms || split < 0 || split > 2) return RSCHOL_E_BAD_INPUT;

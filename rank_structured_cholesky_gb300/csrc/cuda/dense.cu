@@ -125,9 +125,11 @@ __device__ void gemm_tile(const GemmTask<T>& t, int row0, int col0, T (*As)[BK][
 // the 16 x 16 blocks outside C are skipped; K in slices of 32, the next one
 // loaded into registers under the current one's products.  Each C entry's K
 // order is the plain ascending one.  (3D 37x41x35 FP64: the GEMM steps of a
-// factorisation 18.0 ms in 64 x 64 tiles, 7.2 so.)
-__device__ void gemm_tile_f64(const GemmTask<double>& t, int row0, int col0, double (*As)[32][33],
-                              double (*Bs)[32][33]) {
+// factorisation 18.0 ms in 64 x 64 tiles, 7.2 so, 5.1 with the launches of few
+// tiles split along K.)
+// part != null: the slice [kb, ke) of K, its plain product into part (32 x 32).
+__device__ void gemm_tile_f64(const GemmTask<double>& t, int row0, int col0, int kb, int ke, double* part,
+                              double (*As)[32][33], double (*Bs)[32][33]) {
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int nI = min(2, (t.M - row0 + 15) >> 4), nJ = min(2, (t.N - col0 + 15) >> 4);
   double acc[2][2] = {{0, 0}, {0, 0}}, cpre[2][2];
@@ -136,7 +138,7 @@ __device__ void gemm_tile_f64(const GemmTask<double>& t, int row0, int col0, dou
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const int gi = row0 + ty + 16 * i, gj = col0 + tx + 16 * j;
-      cpre[i][j] = (t.beta != 0 && gi < t.M && gj < t.N) ? __ldcg(t.C + (size_t)gi * t.ldc + gj) : 0.0;
+      cpre[i][j] = (t.beta != 0 && !part && gi < t.M && gj < t.N) ? __ldcg(t.C + (size_t)gi * t.ldc + gj) : 0.0;
     }
   double ra[4], rb[4];
   const int f = tid & 31, s0 = tid >> 5;   // fast and slow index of a thread's four elements (slow: s0 + 8 q)
@@ -145,9 +147,9 @@ __device__ void gemm_tile_f64(const GemmTask<double>& t, int row0, int col0, dou
     for (int q = 0; q < 4; ++q) {
       const int s = s0 + 8 * q;
       const int gi = row0 + (t.tA ? f : s), ka = k0 + (t.tA ? s : f);
-      ra[q] = (gi < t.M && ka < t.K) ? __ldcg(t.A + (t.tA ? (size_t)ka * t.lda + gi : (size_t)gi * t.lda + ka)) : 0.0;
-      const int gj = col0 + (t.tB ? s : f), kb = k0 + (t.tB ? f : s);
-      rb[q] = (gj < t.N && kb < t.K) ? __ldcg(t.B + (t.tB ? (size_t)gj * t.ldb + kb : (size_t)kb * t.ldb + gj)) : 0.0;
+      ra[q] = (gi < t.M && ka < ke) ? __ldcg(t.A + (t.tA ? (size_t)ka * t.lda + gi : (size_t)gi * t.lda + ka)) : 0.0;
+      const int gj = col0 + (t.tB ? s : f), kk = k0 + (t.tB ? f : s);
+      rb[q] = (gj < t.N && kk < ke) ? __ldcg(t.B + (t.tB ? (size_t)gj * t.ldb + kk : (size_t)kk * t.ldb + gj)) : 0.0;
     }
   };
   auto store = [&](int st) {
@@ -160,16 +162,16 @@ __device__ void gemm_tile_f64(const GemmTask<double>& t, int row0, int col0, dou
       else Bs[st][f][s] = rb[q];
     }
   };
-  if (t.K > 0) {
-    load(0);
+  if (ke > kb) {
+    load(kb);
     store(0);
   }
   __syncthreads();
   int st = 0;
-  for (int k0 = 0; k0 < t.K; k0 += 32) {
-    const bool more = k0 + 32 < t.K;
+  for (int k0 = kb; k0 < ke; k0 += 32) {
+    const bool more = k0 + 32 < ke;
     if (more) load(k0 + 32);
-    const int kn = min(32, t.K - k0);
+    const int kn = min(32, ke - k0);
     if (nI == 2 && nJ == 2) {
 #pragma unroll 4
       for (int k = 0; k < kn; ++k) {
@@ -199,6 +201,10 @@ __device__ void gemm_tile_f64(const GemmTask<double>& t, int row0, int col0, dou
     for (int j = 0; j < 2; ++j) {
       const int gi = row0 + ty + 16 * i, gj = col0 + tx + 16 * j;
       if (gi >= t.M || gj >= t.N) continue;
+      if (part) {
+        part[(ty + 16 * i) * 32 + tx + 16 * j] = acc[i][j];
+        continue;
+      }
       double v = t.alpha * acc[i][j];
       if (t.beta != 0) v = fma(t.beta, cpre[i][j], v);
       t.C[(size_t)gi * t.ldc + gj] = v;
@@ -215,7 +221,12 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_kernel(const GemmTask<T>* _
     else hi = mid - 1;
   }
   const GemmTask<T> t = tasks[lo];
-  const int local = b - t.tileBase;
+  int local = b - t.tileBase, slice = 0;
+  if (std::is_same<T, double>::value && t.kSplit > 1) {   // K slices: the tiles of each in turn
+    const int tilesPer = ((t.M + 31) / 32) * t.tilesN;
+    slice = local / tilesPer;
+    local -= slice * tilesPer;
+  }
   const int ti = local / t.tilesN, tj = local - ti * t.tilesN;
   constexpr int TL = simt_tile<T>;
   const int row0 = ti * TL, col0 = tj * TL;
@@ -223,12 +234,42 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_kernel(const GemmTask<T>* _
   if constexpr (std::is_same<T, double>::value) {
     __shared__ double As[2][32][33];
     __shared__ double Bs[2][32][33];
-    gemm_tile_f64(t, row0, col0, As, Bs);
+    double* part = nullptr;
+    if (t.kSplit > 1)
+      part = reinterpret_cast<double*>(t.ws) + ((size_t)slice * ((t.M + 31) / 32) * t.tilesN + local) * 1024;
+    gemm_tile_f64(t, row0, col0, t.kSplit > 1 ? slice * t.kLen : 0,
+                  t.kSplit > 1 ? min(t.K, (slice + 1) * t.kLen) : t.K, part, As, Bs);
   } else {
     __shared__ T As[2][BK][BM + 1];
     __shared__ T Bs[2][BK][BN + 1];
     gemm_tile<T>(t, row0, col0, As, Bs);
   }
+}
+
+// C = alpha * (sum of the K-slice products, in slice order) + beta * C for the
+// split FP64 tasks of a launch; one thread per element of C.
+__global__ void gemm_splitk_reduce_f64(const GemmTask<double>* __restrict__ tasks, const int* __restrict__ ids,
+                                       int nIds, const long long* __restrict__ elemBase) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= elemBase[nIds]) return;
+  int lo = 0, hi = nIds - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (elemBase[mid] <= e) lo = mid;
+    else hi = mid - 1;
+  }
+  const GemmTask<double> t = tasks[ids[lo]];
+  const long long le = e - elemBase[lo];
+  const int i = (int)(le / t.N), j = (int)(le - (long long)i * t.N);
+  const size_t tilesPer = (size_t)((t.M + 31) / 32) * t.tilesN;
+  const double* p = reinterpret_cast<const double*>(t.ws) + ((size_t)(i >> 5) * t.tilesN + (j >> 5)) * 1024 +
+                    (i & 31) * 32 + (j & 31);
+  double s = 0.0;
+  for (int sl = 0; sl < t.kSplit; ++sl) s += p[sl * tilesPer * 1024];
+  double* c = t.C + (size_t)i * t.ldc + j;
+  double v = t.alpha * s;
+  if (t.beta != 0) v = fma(t.beta, *c, v);
+  *c = v;
 }
 
 template <class T>
@@ -860,10 +901,10 @@ __device__ __forceinline__ unsigned smid() {
 // (Four blocks per SM -- 64 registers, small spills -- measured slower: the
 // c2 factor 27.3 vs 27.0 ms; the critical POTRF chain pays for the spills.)
 template <class T>
-__global__ void __launch_bounds__(256) chol_fused_kernel(const CholFusedJob<T>* __restrict__ jobs,
-                                                         const CholItem* __restrict__ items, int nItems,
-                                                         int* __restrict__ sync, T* __restrict__ ws, int* flag,
-                                                         unsigned long long* __restrict__ trace) {
+__global__ void __launch_bounds__(256, 3) chol_fused_kernel(const CholFusedJob<T>* __restrict__ jobs,
+                                                            const CholItem* __restrict__ items, int nItems,
+                                                            int* __restrict__ sync, T* __restrict__ ws, int* flag,
+                                                            unsigned long long* __restrict__ trace) {
   extern __shared__ __align__(16) unsigned char cf_smem[];
   __shared__ int sTicket, sOk;
   __shared__ unsigned long long tStart, tReady;
@@ -1172,12 +1213,10 @@ __global__ void __launch_bounds__(QRP_THREADS) qr_panel_kernel(const QrTask<T>* 
 }
 
 // The same panel factorisation with the panel in registers (FP32, at most
-// 512 R rows): thread t keeps rows t + 512 q (q < R) of the 16 panel
-// columns, so a column step touches shared memory only for its three block
+// 512 rows): thread t keeps row t of the 16 panel columns, so a column step touches shared memory only for its three block
 // reductions (|x|^2 below the diagonal with row kk, the 16 dot products
 // s_c = v^T P[:, c], the T column) -- three barriers per column.  Reflectors,
 // T factor and layout as qr_panel_kernel (the sums run in another fixed order).
-template <int R>
 __global__ void __launch_bounds__(QRP_THREADS, 1) qr_panel_reg_kernel(const QrTask<float>* __restrict__ tasks,
                                                                       int j0) {
   constexpr int NW = QRP_THREADS / 32;
@@ -1191,30 +1230,21 @@ __global__ void __launch_bounds__(QRP_THREADS, 1) qr_panel_reg_kernel(const QrTa
   const int pw = min(QR_PB, r - j0), nr = n - j0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* Wg = t.W + (size_t)j0 * n + j0;   // panel element (i, c) at Wg[c * n + i]
-  float a[R][QR_PB];
+  float a[QR_PB];
 #pragma unroll
-  for (int q = 0; q < R; ++q) {
-    const int i = tid + QRP_THREADS * q;
-#pragma unroll
-    for (int c = 0; c < QR_PB; ++c) a[q][c] = (i < nr && c < pw) ? Wg[(size_t)c * n + i] : 0.f;
-  }
+  for (int c = 0; c < QR_PB; ++c) a[c] = (tid < nr && c < pw) ? Wg[(size_t)c * n + tid] : 0.f;
   for (int idx = tid; idx < QR_PB * (QR_PB + 1); idx += QRP_THREADS) (&Ts[0][0])[idx] = 0.f;
   if (tid < QR_PB) sred[tid] = 0.f;   // columns beyond pw keep s = 0
 #pragma unroll
   for (int kk = 0; kk < QR_PB; ++kk) {
     if (kk >= pw) break;
     // |x|^2 below the diagonal; row kk published (alpha and the unit row of the reflector)
-    float x2 = 0.f;
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      const int i = tid + QRP_THREADS * q;
-      if (i > kk && i < nr) x2 += a[q][kk] * a[q][kk];
-    }
-    x2 = warp_sum_d(x2);
+    const bool below = tid > kk && tid < nr;
+    float x2 = warp_sum_d(below ? a[kk] * a[kk] : 0.f);
     if (lane == 0) redA[kk & 1][warp] = x2;
     if (tid == kk)
 #pragma unroll
-      for (int c = 0; c < QR_PB; ++c) rowk[c] = a[0][c];
+      for (int c = 0; c < QR_PB; ++c) rowk[c] = a[c];
     __syncthreads();
     x2 = 0.f;
 #pragma unroll
@@ -1226,21 +1256,12 @@ __global__ void __launch_bounds__(QRP_THREADS, 1) qr_panel_reg_kernel(const QrTa
       tau = (beta - alpha) / beta;
       scal = 1.f / (alpha - beta);
     }
-    float v[R];
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      const int i = tid + QRP_THREADS * q;
-      v[q] = (i > kk && i < nr) ? a[q][kk] * scal : 0.f;
-      if (i > kk && i < nr) a[q][kk] = v[q];
-    }
+    const float v = below ? a[kk] * scal : 0.f;
+    if (below) a[kk] = v;
     // s_c = P[kk][c] + sum_{i > kk} v_i P[i][c]
     float part[QR_PB];
 #pragma unroll
-    for (int c = 0; c < QR_PB; ++c) {
-      part[c] = 0.f;
-#pragma unroll
-      for (int q = 0; q < R; ++q) part[c] += v[q] * a[q][c];
-    }
+    for (int c = 0; c < QR_PB; ++c) part[c] = v * a[c];
     const float ws = warp_transpose_sum16(part);
     if (lane < QR_PB) redC[warp][lane] = ws;
     __syncthreads();
@@ -1263,25 +1284,151 @@ __global__ void __launch_bounds__(QRP_THREADS, 1) qr_panel_reg_kernel(const QrTa
 #pragma unroll
       for (int c = kk + 1; c < QR_PB; ++c) {
         const float w = tau * sred[c];
-#pragma unroll
-        for (int q = 0; q < R; ++q) a[q][c] -= w * v[q];
-        if (tid == kk) a[0][c] -= w;
+        a[c] -= w * v;
+        if (tid == kk) a[c] -= w;
       }
     }
   }
+  if (tid < nr)
 #pragma unroll
-  for (int q = 0; q < R; ++q) {
-    const int i = tid + QRP_THREADS * q;
-    if (i < nr)
-#pragma unroll
-      for (int c = 0; c < QR_PB; ++c)
-        if (c < pw) Wg[(size_t)c * n + i] = a[q][c];
-  }
+    for (int c = 0; c < QR_PB; ++c)
+      if (c < pw) Wg[(size_t)c * n + tid] = a[c];
   __syncthreads();
   // T over the upper triangle of the diagonal block
   for (int idx = tid; idx < pw * pw; idx += QRP_THREADS) {
     const int ra = idx / pw, cb = idx - ra * pw;
     if (ra <= cb) Wg[(size_t)cb * n + ra] = Ts[ra][cb];
+  }
+}
+
+// The panel factorisation over a cluster of eight blocks, the panel's rows split
+// between them in registers (thread t of block b: rows b rp + t + 256 q, q < R).
+// One exchange a column: with x = column kk below the diagonal, the 16 products
+// S_c = x^T P[:, c] give |x|^2 = S_kk and v^T P[:, c] = scal S_c + P[kk][c], so a
+// column is one local reduction, one store of 16 partials into every block's
+// shared memory, one cluster barrier, and the scalars (a square root, two
+// divisions) by one warp.  Reflectors, T factor and layout as qr_panel_kernel.
+// For FP64, whose adds and divisions run at 1/64 of the FP32 rate (every one of
+// 512 threads forming the scalars and 16-term sums held the SM: QR steps of 3D
+// 37x41x35 4.6 -> 1.7 ms), and for FP32 panels of more than 512 rows (those above
+// 2048 went through shared memory or L2: 3D 96^3 24.7 -> 9.0 ms).
+constexpr int QC = 8, QC_THREADS = 256;   // blocks of a cluster, threads of a block
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+template <class T>
+__device__ __forceinline__ void st_cluster(T* local, unsigned rank, T v) {
+  unsigned a = (unsigned)__cvta_generic_to_shared(local), r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  if constexpr (sizeof(T) == 8) asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(r), "d"((double)v) : "memory");
+  else asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(r), "f"((float)v) : "memory");
+}
+
+template <class T, int R>
+__global__ void __cluster_dims__(QC, 1, 1) __launch_bounds__(QC_THREADS)
+    qr_panel_cluster_kernel(const QrTask<T>* __restrict__ tasks, int j0) {
+  constexpr int NW = QC_THREADS / 32;
+  __shared__ T wsum[NW][QR_PB];
+  __shared__ T parts[2][QC][QR_PB], rowk[2][QR_PB];   // written by every block of the cluster / by block 0
+  __shared__ T own[QR_PB], wv[QR_PB], sc[2];
+  __shared__ T Ts[QR_PB][QR_PB + 1];
+  const unsigned rank = blockIdx.x % QC;
+  const QrTask<T> t = tasks[blockIdx.x / QC];
+  const int n = t.n, r = t.r;
+  if (j0 >= r) return;   // (every block of the cluster)
+  const int pw = min(QR_PB, r - j0), nr = n - j0;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rp = max(QR_PB, (nr + QC - 1) / QC), row0 = (int)rank * rp;   // <= QC_THREADS R rows a block
+  const int rows = max(0, min(rp, nr - row0));
+  const int nw = min(NW, (rows + 31) >> 5);   // warps that hold rows
+  T* Wg = t.W + (size_t)j0 * n + j0;          // panel element (i, c) at Wg[c * n + i]
+  T a[R][QR_PB];
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    const int l = tid + QC_THREADS * q;
+#pragma unroll
+    for (int c = 0; c < QR_PB; ++c) a[q][c] = (l < rows && c < pw) ? Wg[(size_t)c * n + row0 + l] : T(0);
+  }
+  for (int idx = tid; idx < QR_PB * (QR_PB + 1); idx += QC_THREADS) (&Ts[0][0])[idx] = T(0);
+  cluster_sync_all();   // every block runs before its shared memory is written
+#pragma unroll
+  for (int kk = 0; kk < QR_PB; ++kk) {
+    if (kk >= pw) break;
+    const int buf = kk & 1;
+    if (warp < nw) {
+      T part[QR_PB];
+#pragma unroll
+      for (int c = 0; c < QR_PB; ++c) part[c] = T(0);
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const int l = tid + QC_THREADS * q;
+        const T x = (l < rows && row0 + l > kk) ? a[q][kk] : T(0);
+#pragma unroll
+        for (int c = 0; c < QR_PB; ++c) part[c] += x * a[q][c];
+      }
+      const T s = warp_transpose_sum16(part);
+      if (lane < QR_PB) wsum[warp][lane] = s;
+    }
+    if (rank == 0 && tid == kk)
+#pragma unroll
+      for (int c = 0; c < QR_PB; ++c) own[c] = a[0][c];
+    __syncthreads();
+    if (tid < QC * QR_PB) {   // a thread per (block, column)
+      const int c = tid % QR_PB;
+      T s = T(0);
+      for (int w = 0; w < nw; ++w) s += wsum[w][c];
+      st_cluster(&parts[buf][rank][c], (unsigned)(tid / QR_PB), s);
+      if (rank == 0) st_cluster(&rowk[buf][c], (unsigned)(tid / QR_PB), own[c]);
+    }
+    cluster_sync_all();
+    if (warp == 0) {
+      const int c = lane % QR_PB;
+      T s = T(0);
+#pragma unroll
+      for (int b = 0; b < QC; ++b) s += parts[buf][b][c];
+      const T x2 = __shfl_sync(0xffffffffu, s, kk), alpha = rowk[buf][kk];
+      T tau = T(0), scal = T(1);
+      if (x2 > T(0)) {
+        const T beta = -copysign(sqrt(alpha * alpha + x2), alpha);
+        tau = (beta - alpha) / beta;
+        scal = T(1) / (alpha - beta);
+      }
+      const T y = scal * s + rowk[buf][c];   // v^T P[:, c]
+      if (lane < QR_PB) wv[c] = tau * y;
+      if (lane == 0) sc[buf] = scal;
+      if (rank == 0) {   // T column kk (dlarft): T[p][kk] = -tau sum_{q=p}^{kk-1} T[p][q] y_q
+        T sum = T(0);
+        for (int q = 0; q < kk; ++q) {
+          const T yq = __shfl_sync(0xffffffffu, y, q);
+          if (lane < kk && q >= lane) sum += Ts[lane][q] * yq;
+        }
+        __syncwarp();
+        if (lane < kk) Ts[lane][kk] = -tau * sum;
+        if (lane == kk) Ts[kk][kk] = tau;
+      }
+    }
+    __syncthreads();
+    if (warp < nw) {   // v = scal x; the columns right of kk
+      const T scal = sc[buf];
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const int l = tid + QC_THREADS * q;
+        if (l < rows && row0 + l > kk) {
+          const T v = a[q][kk] * scal;
+          a[q][kk] = v;
+#pragma unroll
+          for (int c = kk + 1; c < QR_PB; ++c) a[q][c] -= wv[c] * v;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    const int l = tid + QC_THREADS * q;
+    if (l < rows)
+#pragma unroll
+      for (int c = 0; c < QR_PB; ++c)   // (T over the upper triangle of the diagonal block)
+        if (c < pw) Wg[(size_t)c * n + row0 + l] = row0 + l <= c ? Ts[row0 + l][c] : a[q][c];
   }
 }
 
@@ -1471,6 +1618,12 @@ template <class T> void launch_gemm(const GemmTask<T>* d, int n, int tiles, cuda
   gemm_kernel<T><<<tiles, GEMM_THREADS, 0, s>>>(d, n);
   RSCHOL_LAUNCH_CHECK();
 }
+void launch_gemm_splitk_reduce(const GemmTask<double>* d, const int* ids, int nIds, const long long* elemBase,
+                               long long elems, cudaStream_t s) {
+  if (nIds <= 0 || elems <= 0) return;
+  gemm_splitk_reduce_f64<<<(unsigned)((elems + 255) / 256), 256, 0, s>>>(d, ids, nIds, elemBase);
+  RSCHOL_LAUNCH_CHECK();
+}
 template <class T> void launch_potrf(const PotrfTask<T>* d, int n, int* flag, cudaStream_t s) {
   if (n <= 0) return;
   if constexpr (std::is_same<T, float>::value) potrf_reg_kernel<T><<<n, 256, 0, s>>>(d, flag);
@@ -1583,12 +1736,18 @@ int launch_householder_qr(const QrTask<T>* d, int n, int maxRows, int maxR, T* w
   for (int p = 0; p < panels; ++p) {
     const int j0 = p * QR_PB;
     if constexpr (std::is_same<T, float>::value) {
-      if (maxRows <= QRP_THREADS) qr_panel_reg_kernel<1><<<n, QRP_THREADS, 0, s>>>(d, j0);
-      else if (maxRows <= 2 * QRP_THREADS) qr_panel_reg_kernel<2><<<n, QRP_THREADS, 0, s>>>(d, j0);
-      else if (maxRows <= 4 * QRP_THREADS) qr_panel_reg_kernel<4><<<n, QRP_THREADS, 0, s>>>(d, j0);
+      // up to 512 rows one block's registers hold the panel and a column costs three
+      // block barriers; above, a cluster's one exchange a column is quicker (3D 64^3,
+      // up to 2048 rows: 2.50 against 2.64 ms of QR steps)
+      if (maxRows <= QRP_THREADS) qr_panel_reg_kernel<<<n, QRP_THREADS, 0, s>>>(d, j0);
+      else if (maxRows <= QC * QC_THREADS) qr_panel_cluster_kernel<T, 1><<<QC * n, QC_THREADS, 0, s>>>(d, j0);
+      else if (maxRows <= 2 * QC * QC_THREADS) qr_panel_cluster_kernel<T, 2><<<QC * n, QC_THREADS, 0, s>>>(d, j0);
+      else if (maxRows <= 4 * QC * QC_THREADS) qr_panel_cluster_kernel<T, 4><<<QC * n, QC_THREADS, 0, s>>>(d, j0);
       else qr_panel_kernel<T><<<n, QRP_THREADS, smem, s>>>(d, j0, smemElems);
-    } else {
-      qr_panel_kernel<T><<<n, QRP_THREADS, smem, s>>>(d, j0, smemElems);
+    } else {   // what a cluster's registers hold, else the panel in shared or global memory
+      if (maxRows <= QC * QC_THREADS) qr_panel_cluster_kernel<T, 1><<<QC * n, QC_THREADS, 0, s>>>(d, j0);
+      else if (maxRows <= 2 * QC * QC_THREADS) qr_panel_cluster_kernel<T, 2><<<QC * n, QC_THREADS, 0, s>>>(d, j0);
+      else qr_panel_kernel<T><<<n, QRP_THREADS, smem, s>>>(d, j0, smemElems);
     }
     RSCHOL_LAUNCH_CHECK();
     ++launches;

@@ -30,9 +30,9 @@ struct GemmTask {
   int tilesN;
   int tileBase;   // first tile of this task in the launch
   int split;      // tensor-core path: split-precision (3 x TF32) products
-  int kSplit;     // tensor-core path: K slices (1: none); slices write partials to ws
+  int kSplit;     // tensor-core path and FP64: K slices (1: none); slices write partials to ws
   int kLen;       // K per slice (a multiple of 32)
-  float* ws;      // kSplit x tiles x 128 x bn partials (kSplit > 1)
+  float* ws;      // kSplit x tiles x 128 x bn partials (kSplit > 1; FP64: doubles, x 32 x 32)
   int bn;         // tensor-core path: output tile width of the launch (64 or 128; 0: 64)
   // tensor-core path: device addresses of the TMA tensor maps of A and B
   // (K-major operands, 16-byte aligned), or null for register staging
@@ -161,6 +161,9 @@ inline int tc_tile_n(int maxN) { return maxN > 64 ? 128 : 64; }
 // C = alpha * sum of the K-slice partials + beta * C for the split tasks
 // ids[0..nIds) (elemBase: prefix sums of their M x N, elemBase[nIds] = elems).
 void launch_gemm_splitk_reduce(const GemmTask<float>* dTasks, const int* ids, int nIds, const long long* elemBase,
+                               long long elems, cudaStream_t s);
+// The same for FP64 tasks (32 x 32 tiles; ws holds doubles).
+void launch_gemm_splitk_reduce(const GemmTask<double>* dTasks, const int* ids, int nIds, const long long* elemBase,
                                long long elems, cudaStream_t s);
 template <class T> void launch_potrf(const PotrfTask<T>* dTasks, int nTasks, int* dFlag, cudaStream_t s);
 template <class T> void launch_trsm(const TrsmTask<T>* dTasks, int nTasks, int totalChunks, cudaStream_t s);

@@ -66,6 +66,11 @@ void FactorEngine<float>::gemm_launch(const Step& st) {
 
 template <>
 void FactorEngine<double>::gemm_launch(const Step& st) {
+  if (st.kind == ST_GEMM_REDUCE) {
+    launch_gemm_splitk_reduce(dGemm_.as<GemmTask<double>>(), dSplitIds_.as<int>() + st.off, st.count,
+                              dSplitBase_.as<long long>() + st.aux, st.elems, stream);
+    return;
+  }
   launch_gemm<double>(dGemm_.as<GemmTask<double>>() + st.off, st.count, st.grid, stream);
 }
 
@@ -98,6 +103,7 @@ void FactorEngine<T>::flush_gemm(std::vector<GemmTask<T>>& batch, int) {
   for (auto& t : batch) baseTiles += (long long)((t.M + rowsPerTile - 1) / rowsPerTile) * ((t.N + bn - 1) / bn);
   const long long want = 2LL * 152;   // two blocks per SM
   int tiles = 0;
+  long long wsCur = 0;   // (each launch's reduction follows it: all share one workspace)
   std::vector<int> ids;
   std::vector<long long> base{0};
   const long long first = (long long)gemm_.size();
@@ -109,14 +115,19 @@ void FactorEngine<T>::flush_gemm(std::vector<GemmTask<T>>& batch, int) {
     t.kSplit = 1;
     t.kLen = t.K;
     long long wsOff = -1;
-    if (tc && !t.lower && t.K >= 256 && baseTiles < want) {
-      int ks = (int)std::min<long long>(16, std::min<long long>(t.K / 128, (want + baseTiles - 1) / baseTiles));
+    // FP64: a tile holds its SM's FP64 unit in proportion to K, so the aim is
+    // several short ones per SM, for an even last wave (slices of at least 64)
+    constexpr bool f64 = std::is_same<T, double>::value;
+    const long long aim = f64 ? 8LL * 152 : want;
+    const int minK = f64 ? 128 : 256, minSlice = f64 ? 64 : 128;
+    if ((tc || f64) && !t.lower && t.K >= minK && baseTiles < aim) {
+      int ks = (int)std::min<long long>(16, std::min<long long>(t.K / minSlice, (aim + baseTiles - 1) / baseTiles));
       if (ks > 1) {
         const int kl = ((t.K + ks - 1) / ks + kAlign - 1) / kAlign * kAlign;
         t.kSplit = (t.K + kl - 1) / kl;
         t.kLen = kl;
-        wsOff = wsCur_;
-        wsCur_ += (long long)t.kSplit * tilesPer * 128 * bn;
+        wsOff = wsCur;
+        wsCur += (long long)t.kSplit * tilesPer * rowsPerTile * bn;
         ids.push_back((int)(first + q));
         base.push_back(base.back() + (long long)t.M * t.N);
       }
@@ -125,6 +136,7 @@ void FactorEngine<T>::flush_gemm(std::vector<GemmTask<T>>& batch, int) {
     tiles += tilesPer * t.kSplit;
     gemmWsOff_.push_back(wsOff);
   }
+  wsCur_ = std::max(wsCur_, wsCur);
   Step st{ST_GEMM, first, (int)batch.size(), tiles};
   st.aux = tc ? bn | (bf ? 1 << 16 : 0) : 0;   // the tile width, and BF16 splits in bit 16
   gemm_.insert(gemm_.end(), batch.begin(), batch.end());
@@ -1151,7 +1163,7 @@ void FactorEngine<T>::plan() {
   };
   up(dInts_, ints_.data(), ints_.size() * sizeof(int));
   for (auto& s : eaS_) s.rowRel = dInts_.as<int>() + reinterpret_cast<size_t>(s.rowRel);
-  dSplitWs_.alloc(sizeof(float) * std::max(1LL, wsCur_));
+  dSplitWs_.alloc(sizeof(T) * std::max(1LL, wsCur_));
   dQrWs_.alloc(sizeof(T) * std::max(1LL, qrWs_));
   dCholSync_.alloc(sizeof(int) * std::max(1LL, cholSync_));
   dCholWs_.alloc(sizeof(T) * std::max(1LL, cholWs_));
@@ -1162,7 +1174,7 @@ void FactorEngine<T>::plan() {
     dCholTrace_.alloc(tp && tp[0] && !cholItems_.empty() ? 4 * sizeof(unsigned long long) * cholItems_.size() : 0);
   }
   for (size_t q = 0; q < gemm_.size(); ++q)
-    if (gemmWsOff_[q] >= 0) gemm_[q].ws = dSplitWs_.as<float>() + gemmWsOff_[q];
+    if (gemmWsOff_[q] >= 0) gemm_[q].ws = reinterpret_cast<float*>(dSplitWs_.as<T>() + gemmWsOff_[q]);
   up(dSplitIds_, splitIds_.data(), splitIds_.size() * sizeof(int));
   up(dSplitBase_, splitBase_.data(), splitBase_.size() * sizeof(long long));
   // every task pointer must now be a device address, not a plan-time offset
