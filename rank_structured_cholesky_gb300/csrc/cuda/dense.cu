@@ -13,6 +13,7 @@ namespace rschol {
 
 namespace {
 
+using solvedev::ld_acquire;
 using solvedev::st_release;
 using solvedev::wait_geq;
 using solvedev::wait_geq_lim;
@@ -407,9 +408,17 @@ __global__ void __launch_bounds__(256) trsm_kernel(const TrsmTask<T>* __restrict
 // non-positive pivot is replaced by 1 and reported as atomicMin(flag, code).
 // 1 / p on a POTRF's critical path: the fast reciprocal (MUFU-based,
 // __fdividef, within 2 ulp) in FP32, whose factor carries larger rounding
-// errors anyway; exact division in FP64.
+// errors anyway.
 __device__ __forceinline__ float pivot_recip(float p) { return __fdividef(1.0f, p); }
-__device__ __forceinline__ double pivot_recip(double p) { return 1.0 / p; }
+// FP64: the 20-bit estimate and two Newton steps y += y (1 - p y), four dependent
+// multiply-adds (a division is about three times as many on the chain).
+__device__ __forceinline__ double pivot_recip(double p) {
+  if (!(p > 1e-290 && p < 1e290)) return 1.0 / p;
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(p));
+  y = fma(y, fma(-p, y, 1.0), y);
+  return fma(y, fma(-p, y, 1.0), y);
+}
 
 template <class T>
 __device__ void potrf_tile_reg(T* A, int ld, int n, int code, int* flag) {
@@ -598,198 +607,239 @@ __device__ void trsm_chunk_mul(T* B, int ldb, int nr, int w, T (*X)[65], T (*Li)
   __syncthreads();
 }
 
-// One FP32 tile product of the fused Cholesky, 256 threads:
-//   C := C - A B^T (sub) or C := A B^T,
-// C (M x N), A (M x K), B (N x K) row-major, M, N, K <= 64.  Every global
-// load of a thread is issued before the first use (one latency round instead
-// of one per K slice); a warp's load instruction covers 4 rows x 8 columns
-// (four full 32-byte sectors).  A and B land k-major in shared memory with a
-// pitch of 68 floats -- conflict-free stores, and a thread's four rows (four
-// columns) are one 16-byte shared load -- so a K step is 2 shared loads for
-// 16 FMAs (the 64 x 65 layout took 8).  Each thread owns rows 4 ty + a and
-// columns 4 tx + b; the products are summed in ascending k and subtracted
-// from C at the end.  A and C may alias (the TRSM items overwrite their
-// input): all of A is read before the barrier that precedes the stores.
-__device__ void tile_abt_f32(const float* A, int lda, const float* B, int ldb, float* C, int ldc, int M, int N,
-                             int K, bool sub, float* smem) {
-  constexpr int PITCH = 68;
-  float (*As)[PITCH] = reinterpret_cast<float (*)[PITCH]>(smem);
-  float (*Bs)[PITCH] = reinterpret_cast<float (*)[PITCH]>(smem + 64 * PITCH);
+// Factor and invert one FP32 tile on the chain of the fused Cholesky: S (64 x 68
+// shared) holds the n x n lower tile, padded with a unit diagonal; on return its L,
+// and in Li (64 x 68) the inverse's lower blocks.  A column at a time (potrf_tile_reg
+// and tile_inverse) every column costs a block barrier and a round through shared
+// memory, 22 us a tile.  Here in blocks of 16: one warp eliminates the diagonal
+// block and the identity beside it with shuffles, the rows below are multiplied by
+// the inverse, and the same warp updates and eliminates the next diagonal block
+// while the others update the rest and form the inverse's finished block row -- two
+// barriers a block, 10 us a tile.  A pivot that is not positive (or NaN) is
+// replaced by 1 and reported as atomicMin(flag, code).
+__device__ __noinline__ void potrf_inverse_f32(float (*S)[68], float (*Li)[68], float (*Tm)[16][17], int n, bool invert,
+                                               int code, int* flag) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int tx = tid & 15, ty = tid >> 4;
-  float ra[16], rb[16], c[4][4];
+  const int nb = (n + 15) >> 4;
+  const int lj = lane & 15, hi = lane >> 4;
+  bool bad = false;
+  // warp 0: the 16 x 16 block at o; lane r (and r + 16) holds row r in v, and row r
+  // of the inverse of the unit lower factor in e
+  auto diag = [&](int o, float (&v)[16]) {
+    float e[16], pd = 1.f;
 #pragma unroll
-  for (int q = 0; q < 16; ++q) {
-    const int pr = q * 8 + warp, i = 4 * (pr & 15) + (lane & 3), k = 8 * (pr >> 4) + (lane >> 2);
-    ra[q] = (i < M && k < K) ? __ldcg(A + (size_t)i * lda + k) : 0.f;
-    rb[q] = (i < N && k < K) ? __ldcg(B + (size_t)i * ldb + k) : 0.f;
-  }
+    for (int k = 0; k < 16; ++k) e[k] = k == lj ? 1.f : 0.f;
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+    for (int j = 0; j < 16; ++j) {
+      float p = __shfl_sync(0xffffffffu, v[j], j, 16);
+      bad |= !(p > 0.f);
+      p = p > 0.f ? p : 1.f;
+      pd = lj == j ? p : pd;
+      const float l = lj > j ? v[j] * pivot_recip(p) : 0.f;
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int i = 4 * ty + a, j = 4 * tx + b;
-      c[a][b] = (sub && i < M && j < N) ? __ldcg(C + (size_t)i * ldc + j) : 0.f;
+      for (int k = j + 1; k < 16; ++k) v[k] -= l * __shfl_sync(0xffffffffu, v[j], k, 16);
+#pragma unroll
+      for (int k = 0; k < j; ++k) e[k] -= l * __shfl_sync(0xffffffffu, e[k], j, 16);
+      e[j] -= l;
+    }
+    const float d = sqrtf(pd), rd = 1.f / d;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const float rk = __shfl_sync(0xffffffffu, rd, k, 16);
+      if (hi == 0) {
+        Li[o + lj][o + k] = e[k] * rd;
+        if (k <= lj) S[o + lj][o + k] = k == lj ? d : v[k] * rk;
+      }
+    }
+  };
+  // a warp: block (R, C) of the inverse, -Li[R][R] sum_{C <= K < R} L[R][K] Li[K][C];
+  // lane: column lj, rows 2 q + hi
+  auto inv_block = [&](int R, int C) {
+    float t[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) t[q] = 0.f;
+    for (int k = 16 * C; k < 16 * R; k += 4) {
+      float y[4];
+#pragma unroll
+      for (int z = 0; z < 4; ++z) y[z] = Li[k + z][16 * C + lj];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float4 x = *reinterpret_cast<const float4*>(&S[16 * R + 2 * q + hi][k]);
+        t[q] = fmaf(x.w, y[3], fmaf(x.z, y[2], fmaf(x.y, y[1], fmaf(x.x, y[0], t[q]))));
+      }
     }
 #pragma unroll
-  for (int q = 0; q < 16; ++q) {
-    const int pr = q * 8 + warp, i = 4 * (pr & 15) + (lane & 3), k = 8 * (pr >> 4) + (lane >> 2);
-    As[k][i] = ra[q];
-    Bs[k][i] = rb[q];
-  }
-  __syncthreads();
-  float acc[4][4];
+    for (int q = 0; q < 8; ++q) Tm[C][2 * q + hi][lj] = t[q];
+    __syncwarp();
+    float y[16];
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+    for (int k = 0; k < 16; ++k) y[k] = Tm[C][k][lj];
 #pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
-#pragma unroll 4
-  for (int k = 0; k < K; ++k) {
-    const float4 av = *reinterpret_cast<const float4*>(&As[k][4 * ty]);
-    const float4 bv = *reinterpret_cast<const float4*>(&Bs[k][4 * tx]);
-    const float ar[4] = {av.x, av.y, av.z, av.w}, br[4] = {bv.x, bv.y, bv.z, bv.w};
+    for (int q = 0; q < 8; ++q) {
+      float x = 0.f;
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(ar[a], br[b], acc[a][b]);
-  }
-#pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int i = 4 * ty + a;
-    if (i >= M) continue;
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int j = 4 * tx + b;
-      if (j < N) C[(size_t)i * ldc + j] = sub ? c[a][b] - acc[a][b] : acc[a][b];
+      for (int k = 0; k < 16; ++k) x = fmaf(Li[16 * R + 2 * q + hi][16 * R + k], y[k], x);
+      Li[16 * R + 2 * q + hi][16 * C + lj] = -x;
     }
+  };
+  if (warp == 0) {
+    float v[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = S[lj][k];
+    diag(0, v);
   }
   __syncthreads();
+  for (int kb = 0; kb + 1 < nb; ++kb) {
+    const int o = 16 * kb, left = nb - kb - 1;   // blocks below
+    {   // X := A Li(kb)^T: a half warp owns a row
+      const int c = tid & 15, rr = tid >> 4;
+      float lc[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) lc[k] = Li[o + c][o + k];
+      for (int a = 1; a <= left; ++a) {
+        const int i = o + 16 * a + rr;
+        float x = 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) x = fmaf(S[i][o + k], lc[k], x);
+        __syncwarp();
+        S[i][o + c] = x;
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {   // the next diagonal block: each half warp forms eight columns of every row
+      const int q = o + 16;
+      float xr[16], w[8], v[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) xr[k] = S[q + lj][o + k];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) s = fmaf(xr[k], S[q + 8 * hi + c][o + k], s);
+        w[c] = S[q + lj][q + 8 * hi + c] - s;
+      }
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float other = __shfl_xor_sync(0xffffffffu, w[c], 16);
+        v[c] = hi ? other : w[c];
+        v[8 + c] = hi ? w[c] : other;
+      }
+      diag(q, v);
+    } else {   // block row kb of the inverse; the other lower blocks (a, b) in units of 8 rows x 16 columns
+      const int ni = invert ? kb : 0, units = left * (left + 1) - 2;
+      for (int w = warp - 1; w < ni + units; w += 7) {
+        if (w < ni) {
+          inv_block(kb, w);
+          continue;
+        }
+        const int u = w - ni;
+        int a = 1, t = u >> 1;   // block t of (1, 0), (1, 1), (2, 0), ...
+        while (t > a) t -= ++a;
+        const int rb = o + 16 + 16 * a + 8 * (u & 1) + hi, cb = o + 16 + 16 * t + lj;
+        float xj[16], s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int k = 0; k < 16; ++k) xj[k] = S[cb][o + k];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int k = 0; k < 16; ++k) s[q] = fmaf(S[rb + 2 * q][o + k], xj[k], s[q]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) S[rb + 2 * q][cb] -= s[q];
+      }
+    }
+    __syncthreads();
+  }
+  if (invert && warp < nb - 1) inv_block(nb - 1, warp);
+  if (tid == 0 && bad) atomicMin(flag, code);
 }
 
-// The FP64 pieces of the fused Cholesky, tiles of up to 32 x 32, 256 threads as
-// 16 x 16.  The FP64 unit is the limit, so each piece forms the 16 x 16 blocks it
-// needs and no more, and divisions and square roots (tens of FP64 instructions
-// each) are done once a column by one warp.  (Against 64 x 64 tiles, whose
-// POTRF -> TRSM -> update chain took 130 us a panel: Cholesky steps of 3D
-// 37x41x35 23.1 -> 12.0 ms, the whole FP64 factorisation of a 61x53 grid 1.36 ->
-// 0.81 ms.)
-//   C := C - A B^T (sub), C := A B^T otherwise; C (M x N), A (M x K), B (N x K).
-// lower: C's blocks above the diagonal are not wanted; tri: B is lower
-// triangular (its columns stop at the row).  A and C may alias: all of A is read
-// before the barrier that precedes the stores.
-__device__ void tile_abt_f64(const double* A, int lda, const double* B, int ldb, double* C, int ldc, int M, int N,
-                             int K, bool sub, bool lower, bool tri, double* smem) {
-  double (*As)[33] = reinterpret_cast<double (*)[33]>(smem);
-  double (*Bs)[33] = reinterpret_cast<double (*)[33]>(smem + 32 * 33);
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, f = tid & 31, s0 = tid >> 5;
-  double ra[4], rb[4], c[2][2];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int i = s0 + 8 * q;
-    ra[q] = (i < M && f < K) ? __ldcg(A + (size_t)i * lda + f) : 0.0;
-    rb[q] = (i < N && f < K) ? __ldcg(B + (size_t)i * ldb + f) : 0.0;
-  }
-#pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      const int i = ty + 16 * a, j = tx + 16 * b;
-      c[a][b] = (sub && i < M && j < N) ? __ldcg(C + (size_t)i * ldc + j) : 0.0;
-    }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    As[s0 + 8 * q][f] = ra[q];
-    Bs[s0 + 8 * q][f] = rb[q];
-  }
-  __syncthreads();
-  const bool m1 = M > 16, n1 = N > 16;
-  const bool w01 = n1 && !lower, w10 = m1, w11 = m1 && n1;   // blocks wanted besides (0, 0)
-  double acc[2][2] = {{0, 0}, {0, 0}};
-  const int k0 = tri ? min(K, 16) : K;   // K of the first 16 columns
-#pragma unroll 4
-  for (int k = 0; k < K; ++k) {
-    const double a0 = As[ty][k], a1 = As[ty + 16][k], b0 = Bs[tx][k], b1 = Bs[tx + 16][k];
-    if (k < k0) {
-      acc[0][0] = fma(a0, b0, acc[0][0]);
-      if (w10) acc[1][0] = fma(a1, b0, acc[1][0]);
-    }
-    if (w01) acc[0][1] = fma(a0, b1, acc[0][1]);
-    if (w11) acc[1][1] = fma(a1, b1, acc[1][1]);
-  }
-#pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      const int i = ty + 16 * a, j = tx + 16 * b;
-      if (i < M && j < N && (!lower || b <= a)) C[(size_t)i * ldc + j] = sub ? c[a][b] - acc[a][b] : acc[a][b];
-    }
-  __syncthreads();
-}
-
-// Right-looking Cholesky of one n x n (n <= 32) tile, as potrf_tile_reg: column j
-// published unscaled with the reciprocal of its pivot, one barrier a column.
-__device__ void potrf_tile_f64(double* A, int ld, int n, int code, int* flag) {
+// The same for one FP64 tile (n <= 32; S, Li 32 x 33, Tm 16 x 17 shared).  A warp's
+// multiply-add holds its quarter of the FP64 unit for 64 clocks, so what counts is
+// how many each warp issues: warp w keeps rows 4 w .. 4 w + 3 (a thread: one row, every eighth
+// column), skips columns right of them and everything finished, and a row's
+// multiplier is formed once; column j is published unscaled with the reciprocal of
+// its pivot, one barrier a column.  Square roots and their reciprocals by one
+// warp; the inverse's two 16 x 16 diagonal blocks by one warp, a column a lane.
+// (Cholesky steps of 3D 37x41x35 FP64 12.3 -> 12.0 ms against every
+// thread forming all its products on every column.)
+__device__ __noinline__ void potrf_inverse_f64(double (*S)[33], double (*Li)[33], double (*Tm)[17], int n, bool invert,
+                                               int code, int* flag) {
   __shared__ double col[2][32], rpv[2], piv[32], dia[32], rdia[32];
   __shared__ int bad;
-  const int tid = threadIdx.x, ti = tid >> 4, tk = tid & 15;
-  double v[2][2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int i = 4 * warp + (lane >> 3), kc = lane & 7, rLast = 4 * warp + 3;
+  double v[4];
 #pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      const int i = ti + 16 * a, k = tk + 16 * b;
-      v[a][b] = (i < n && k <= i) ? __ldcg(A + (size_t)i * ld + k) : 0.0;
-    }
+  for (int c = 0; c < 4; ++c) v[c] = S[i][kc + 8 * c];
   if (tid == 0) bad = 0;
+  if (tid < 32) piv[tid] = 1.0;
   __syncthreads();
-  const bool two = n > 16;
 #pragma unroll
-  for (int b0 = 0; b0 < 2; ++b0) {
-    for (int jj = 0; jj < 16 && 16 * b0 + jj < n; ++jj) {
-      const int j = 16 * b0 + jj, buf = j & 1;
-      if (tk == jj) {   // the owners of column j: rows ti, ti + 16
-#pragma unroll
-        for (int a = 0; a < 2; ++a) {
-          const int i = ti + 16 * a;
-          double u = v[a][b0];
-          if (i == j) {
-            if (!(u > 0.0)) {   // not positive definite (or NaN): keep going, report
-              bad = 1;
-              u = 1.0;
-            }
-            piv[j] = u;
-            rpv[buf] = pivot_recip(u);
+  for (int c0 = 0; c0 < 4; ++c0) {
+    for (int jj = 0; jj < 8 && 8 * c0 + jj < n; ++jj) {
+      const int j = 8 * c0 + jj, buf = j & 1;
+      if (kc == jj) {
+        double u = v[c0];
+        if (i == j) {
+          if (!(u > 0.0)) {   // not positive definite (or NaN): keep going, report
+            bad = 1;
+            u = 1.0;
           }
-          col[buf][i] = i <= j ? 0.0 : u;
+          piv[j] = u;
+          rpv[buf] = pivot_recip(u);
         }
+        col[buf][i] = i <= j ? 0.0 : u;
       }
       __syncthreads();
-      const double rp = rpv[buf];
-      const double r1 = two ? col[buf][ti + 16] * rp : 0.0;
-      if (b0 == 0) {
-        const double r0 = col[buf][ti] * rp, c0 = col[buf][tk];
-        v[0][0] -= r0 * c0;
-        if (two) v[1][0] -= r1 * c0;
+      if (rLast > j) {
+        const double l = col[buf][i] * rpv[buf];
+#pragma unroll
+        for (int c = c0; c < 4; ++c)
+          if (8 * c <= rLast) v[c] -= l * col[buf][kc + 8 * c];
       }
-      if (two) v[1][1] -= r1 * col[buf][tk + 16];
     }
   }
   __syncthreads();
-  if (tid < n) {
+  if (tid < 32) {
     const double d = sqrt(piv[tid]);
     dia[tid] = d;
     rdia[tid] = 1.0 / d;
   }
   __syncthreads();
 #pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      const int i = ti + 16 * a, k = tk + 16 * b;
-      if (b <= a && i < n && k <= i) A[(size_t)i * ld + k] = (k == i) ? dia[k] : v[a][b] * rdia[k];
-    }
+  for (int c = 0; c < 4; ++c) {
+    const int k = kc + 8 * c;
+    if (8 * c <= rLast && k <= i) S[i][k] = k == i ? dia[i] : v[c] * rdia[k];
+  }
   if (tid == 0 && bad) atomicMin(flag, code);
+  if (!invert) return;   // (uniform; the caller's barrier follows)
   __syncthreads();
+  if (warp == 0) {
+    const int c = lane & 15, o = lane & 16;
+    double x[16];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) x[r] = r == c ? 1.0 : 0.0;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      x[k] *= rdia[o + k];
+#pragma unroll
+      for (int r = k + 1; r < 16; ++r) x[r] -= S[o + r][o + k] * x[k];
+    }
+#pragma unroll
+    for (int r = 0; r < 16; ++r) Li[o + r][o + c] = x[r];
+  }
+  __syncthreads();
+  if (n <= 16) return;
+  {   // Li21 = -Li22 (L21 Li11): warp w columns 2 w, 2 w + 1 (zero above them), then rows 2 w, 2 w + 1
+    const int f = lane & 15, p = 2 * warp + (lane >> 4);
+    double t = 0.0;
+    for (int k = 2 * warp; k < 16; ++k) t = fma(S[16 + f][k], Li[k][p], t);
+    Tm[f][p] = t;
+    __syncthreads();
+    t = 0.0;
+    for (int k = 0; k <= 2 * warp + 1; ++k) t = fma(Li[16 + p][16 + k], Tm[k][f], t);
+    Li[16 + p][f] = -t;
+  }
 }
 
 // out (32 x 32) := L^{-1}, L the w x w (w <= 32) lower tile at Lg padded with a
@@ -836,7 +886,8 @@ __device__ void tile_inverse_f64(const double* Lg, int ldl, int w, double* out, 
     __syncthreads();
     s = 0.0;
 #pragma unroll
-    for (int k = 0; k < 16; ++k) s += Li[16 + i][16 + k] * Tm[k][j];
+    for (int k = 0; k < 16; ++k)
+      if (k <= (i | 1)) s += Li[16 + i][16 + k] * Tm[k][j];   // (lower; i | 1: the same for a warp)
     Li[16 + i][j] = -s;
     __syncthreads();
   }
@@ -874,16 +925,21 @@ __global__ void __launch_bounds__(256) trsm_inv_kernel(const TrsmTask<T>* __rest
 // factors the first nDiag columns of a front F (rows x rows, lower, row-major)
 // in panels: the first w0 = nDiag - NB (P - 1) wide, the others NB (64, FP64 32),
 // so that every later panel and every trailing block is aligned to the tile grid
-// b(0) = 0, b(t) = w0 + NB (t - 1).  Panel p is one POTRF of tile (p, p)
-// (which also stores the tile's inverse), one TRSM per row tile a > p, and
-// one update C(a, b) -= X(a) X(b)^T (K = panel width) per lower tile of the
-// trailing block with column tile b below nUpd.  Each piece is a work item;
-// a block takes the next item from a ticket counter (the items are listed in
-// a topological order, so a block only waits on items taken before its own) and
-// waits, bounded, on per-tile completion counters:
-//   POTRF(p)       tile (p, p) updated by the p earlier panels
-//   TRSM(p, a)     POTRF(p) done; tile (a, p) updated by the p earlier panels
-//   GEMM(p, a, b)  TRSM(p, a) and TRSM(p, b) done; tile (a, b) updated by the p earlier panels
+// b(0) = 0, b(t) = w0 + NB (t - 1).  A work item is one lower tile (a, b) from its
+// input to its result (left-looking): it subtracts X(a, q) X(b, q)^T of the panels
+// q < min(b, P) in order, as they appear, from the tile in registers -- read once,
+// before any wait, and written once -- and then
+//   POTRF(p)      a = b = p: factors the tile and stores its inverse
+//   TRSM(a, b)    b < P: multiplies by the inverse of tile b
+//   GEMM(a, b)    b >= P: a tile of the trailing block, nothing more.
+// A block takes the next item from a ticket counter; the items are listed in a
+// topological order, so a block only waits, bounded, on items taken before its
+// own: tdone[a] panels of row tile a stored, pdone[p] inverse p stored.
+// What bounds it is the chain POTRF(p) -> TRSM(p + 1, p) -> POTRF(p + 1); as one
+// item a tile and panel (right-looking) it was 36 us a panel, 22 of them the tile's
+// factor and inverse, 5 the three hand-overs; now it is 23, and the updates read
+// and write their tiles once (Cholesky steps of a factorisation: 3D 64^3 10.3 -> 8.1
+// ms, 96^3 49.2 -> 36.8 ms, elasticity 30^3 6.3 -> 4.9 ms).
 // sync[0] is the ticket, the counters follow (zeroed before every launch);
 // a wait that gives up sets flag[1].  Data written by other blocks is read
 // through L2 (ld.global.cg).
@@ -898,20 +954,93 @@ __device__ __forceinline__ unsigned smid() {
   return r;
 }
 
-// (Four blocks per SM -- 64 registers, small spills -- measured slower: the
-// c2 factor 27.3 vs 27.0 ms; the critical POTRF chain pays for the spills.)
+// A tile's registers and staging: 16 x 16 threads, R x R entries each -- FP32 rows
+// 4 ty + a and columns 4 tx + b, so that a K step is two 16-byte shared loads for
+// 16 FMAs; FP64 rows ty + 16 a and columns tx + 16 b, so that the 16 x 16 blocks
+// outside the matrix or above the diagonal are skipped.  A panel's products are
+// summed in ascending k and subtracted from the tile together.
+template <class T>
+struct CholTile;
+// (c0, c1) += a (b0, b1): two FP32 multiply-adds in one instruction
+__device__ __forceinline__ void fma2(float& c0, float& c1, float a, float b0, float b1) {
+  asm("{\n.reg .b64 pa, pb, pc;\nmov.b64 pa, {%2, %2};\nmov.b64 pb, {%3, %4};\nmov.b64 pc, {%0, %1};\n"
+      "fma.rn.f32x2 pc, pa, pb, pc;\nmov.b64 {%0, %1}, pc;\n}"
+      : "+f"(c0), "+f"(c1)
+      : "f"(a), "f"(b0), "f"(b1));
+}
+template <>
+struct CholTile<float> {
+  static constexpr int NB = 64, R = 4, Q = 8;
+  typedef float Stage[32][68];   // k-major: conflict-free stores, 16-byte loads
+  // element q of a thread in a 64 x 32 slice (a warp: 4 rows x 8 columns, full sectors)
+  static __device__ int row(int q) { return 4 * ((q * 8 + ((int)threadIdx.x >> 5)) & 15) + (threadIdx.x & 3); }
+  static __device__ int col(int q) { return 8 * ((q * 8 + ((int)threadIdx.x >> 5)) >> 4) + ((threadIdx.x & 31) >> 2); }
+  static __device__ int ti(int a) { return 4 * (threadIdx.x >> 4) + a; }
+  static __device__ int tj(int b) { return 4 * (threadIdx.x & 15) + b; }
+  static __device__ float& at(Stage& s, int i, int k) { return s[k][i]; }
+  static __device__ void mul(const Stage& A, const Stage& B, int kn, float (&acc)[4][4], bool, bool, bool) {
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll 4
+    for (int k = 0; k < kn; ++k) {
+      const float4 av = *reinterpret_cast<const float4*>(&A[k][4 * ty]);
+      const float4 bv = *reinterpret_cast<const float4*>(&B[k][4 * tx]);
+      const float ar[4] = {av.x, av.y, av.z, av.w};
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        fma2(acc[a][0], acc[a][1], ar[a], bv.x, bv.y);
+        fma2(acc[a][2], acc[a][3], ar[a], bv.z, bv.w);
+      }
+    }
+  }
+};
+template <>
+struct CholTile<double> {
+  static constexpr int NB = 32, R = 2, Q = 4;
+  typedef double Stage[32][33];
+  static __device__ int row(int q) { return (threadIdx.x >> 5) + 8 * q; }
+  static __device__ int col(int) { return threadIdx.x & 31; }
+  static __device__ int ti(int a) { return (threadIdx.x >> 4) + 16 * a; }
+  static __device__ int tj(int b) { return (threadIdx.x & 15) + 16 * b; }
+  static __device__ double& at(Stage& s, int i, int k) { return s[i][k]; }
+  // w01, w10, w11: the blocks wanted besides (0, 0); kLeft: the K of the left ones
+  static __device__ void mul(const Stage& A, const Stage& B, int kn, double (&acc)[2][2], bool w01, bool w10, bool w11,
+                             int kLeft = 32) {
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll 4
+    for (int k = 0; k < kn; ++k) {
+      const double a0 = A[ty][k], a1 = A[ty + 16][k], b0 = B[tx][k], b1 = B[tx + 16][k];
+      if (k < kLeft) {
+        acc[0][0] = fma(a0, b0, acc[0][0]);
+        if (w10) acc[1][0] = fma(a1, b0, acc[1][0]);
+      }
+      if (w01) acc[0][1] = fma(a0, b1, acc[0][1]);
+      if (w11) acc[1][1] = fma(a1, b1, acc[1][1]);
+    }
+  }
+};
+// dynamic shared memory: two stages of A and B, the TRSM's operands, or the POTRF's tiles
+template <class T> constexpr int chol_smem = 4 * (int)sizeof(typename CholTile<T>::Stage) +
+                                             (std::is_same<T, float>::value ? 3 * 16 * 17 * 4 : 0);
+
 template <class T>
 __global__ void __launch_bounds__(256, 3) chol_fused_kernel(const CholFusedJob<T>* __restrict__ jobs,
                                                             const CholItem* __restrict__ items, int nItems,
                                                             int* __restrict__ sync, T* __restrict__ ws, int* flag,
                                                             unsigned long long* __restrict__ trace) {
+  typedef CholTile<T> C;
+  typedef typename C::Stage Stage;
+  constexpr int NB = C::NB, R = C::R;
+  static_assert(NB == chol_nb<T>, "tile width");
   extern __shared__ __align__(16) unsigned char cf_smem[];
-  __shared__ int sTicket, sOk;
+  Stage* As = reinterpret_cast<Stage*>(cf_smem);   // [2]
+  Stage* Bs = As + 2;                              // [2]
+  __shared__ int sTicket, sReady;
   __shared__ unsigned long long tStart, tReady;
   int* err = flag + 1;
+  const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
     sTicket = atomicAdd(sync, 1);
-    if (trace) tStart = globaltimer_ns();
+    if (trace) tStart = tReady = globaltimer_ns();
   }
   __syncthreads();
   if (sTicket >= nItems) {   // counters not reset: report, touch nothing
@@ -920,83 +1049,237 @@ __global__ void __launch_bounds__(256, 3) chol_fused_kernel(const CholFusedJob<T
   }
   const CholItem it = items[sTicket];
   const CholFusedJob<T> j = jobs[it.job];
-  int* cnt = sync + 1 + j.cnt;     // TR x TU: panels applied to tile (a, b)
-  int* tdone = cnt + j.TR * j.TU;  // TR: panels whose TRSM of row tile a is done
-  int* pdone = tdone + j.TR;       // P: POTRF of panel p done
-  const int p = it.p, a = it.a, b = it.b;
+  int* tdone = sync + 1 + j.cnt;   // TR: panels of row tile a stored
+  int* pdone = tdone + j.TR;       // P: inverse of panel p stored
+  const int a = it.a, b = it.b;
   const int* lim = flag + 2;   // polls before a wait gives up (set with the flags before the factorisation)
-  constexpr int NB = chol_nb<T>;
   auto bnd = [&](int t) { return t == 0 ? 0 : j.w0 + NB * (t - 1); };      // columns (and Cholesky rows)
   auto rbnd = [&](int t) { return t == 0 ? 0 : j.r1 + NB * (t - 1); };     // rows
-  const int c0 = bnd(p), wp = bnd(p + 1) - c0;
-  if ((threadIdx.x >> 5) == 0) {
-    bool ok;
-    if (it.kind == CHOL_POTRF) ok = j.L ? true : wait_geq_lim(cnt + p * j.TU + p, p, err, lim);
-    else if (it.kind == CHOL_TRSM)
-      ok = wait_geq_lim(pdone + p, 1, err, lim) && wait_geq_lim(cnt + a * j.TU + p, p, err, lim);
-    else
-      ok = wait_geq_lim(tdone + a, p + 1, err, lim) && (j.L || wait_geq_lim(tdone + b, p + 1, err, lim)) &&
-           wait_geq_lim(cnt + a * j.TU + b, p, err, lim);
-    if (threadIdx.x == 0) {
-      sOk = ok;
-      if (trace) tReady = globaltimer_ns();
-    }
-  }
-  __syncthreads();
-  if (!sOk) return;
   T* F = j.F;
-  const int ld = j.ld;
-  int* done;
-  int doneVal;
-  if (it.kind == CHOL_POTRF) {
-    // Cholesky job: factor the diagonal tile; TRSM job: L is factored already
-    T* A = j.L ? const_cast<T*>(j.L) + (size_t)c0 * j.ldl + c0 : F + (size_t)c0 * ld + c0;
-    const int lda = j.L ? j.ldl : ld;
-    T* out = ws + j.inv + (size_t)p * NB * NB;
-    const bool below = j.L || c0 + wp < j.nRows;   // rows below: the TRSM items multiply by the inverse
+  const int ld = j.ld, q0 = bnd(b);
+  int* done = nullptr;
+  int doneVal = 0;
+  if (it.kind == CHOL_POTRF && j.L) {   // TRSM job: L is factored already, invert its diagonal tile
+    const T* A = j.L + (size_t)q0 * j.ldl + q0;
+    T* out = ws + j.inv + (size_t)b * NB * NB;
+    const int w = bnd(b + 1) - q0;
     if constexpr (std::is_same<T, double>::value) {
-      if (!j.L) potrf_tile_f64(A, ld, wp, j.code, flag);
-      if (below) tile_inverse_f64(A, lda, wp, out, reinterpret_cast<double*>(cf_smem));
+      tile_inverse_f64(A, j.ldl, w, out, reinterpret_cast<double*>(cf_smem));
     } else {
-      if (!j.L) potrf_tile_reg<T>(A, ld, wp, j.code, flag);
-      if (below) {
-        T (*L)[65] = reinterpret_cast<T (*)[65]>(cf_smem);
-        T (*Li)[65] = reinterpret_cast<T (*)[65]>(cf_smem + sizeof(T) * 64 * 65);
-        T (*Tm)[16][17] = reinterpret_cast<T (*)[16][17]>(cf_smem + 2 * sizeof(T) * 64 * 65);
-        tile_inverse<T>(A, lda, wp, L, Li, Tm);
+      T (*L)[65] = reinterpret_cast<T (*)[65]>(cf_smem);
+      T (*Li)[65] = L + 64;
+      T (*Tm)[16][17] = reinterpret_cast<T (*)[16][17]>(Li + 64);
+      tile_inverse<T>(A, j.ldl, w, L, Li, Tm);
 #pragma unroll
-        for (int idx = threadIdx.x; idx < 64 * 64; idx += 256) out[idx] = Li[idx >> 6][idx & 63];
-      }
+      for (int idx = threadIdx.x; idx < 64 * 64; idx += 256) out[idx] = Li[idx >> 6][idx & 63];
     }
-    done = pdone + p;
+    done = pdone + b;
     doneVal = 1;
-  } else if (it.kind == CHOL_TRSM) {
-    // X(a) := X(a) Li(p)^T with the panel's inverse tile straight from the workspace
-    const int r0 = rbnd(a), nr = min(rbnd(a + 1), j.nRows) - r0;
-    T* X = F + (size_t)r0 * ld + c0;
-    const T* Li = ws + j.inv + (size_t)p * NB * NB;
-    if constexpr (std::is_same<T, double>::value)
-      tile_abt_f64(X, ld, Li, NB, X, ld, nr, wp, wp, false, false, true, reinterpret_cast<double*>(cf_smem));
-    else tile_abt_f32(X, ld, Li, NB, X, ld, nr, wp, wp, false, reinterpret_cast<float*>(cf_smem));
-    done = tdone + a;
-    doneVal = p + 1;
-  } else {   // update of tile (a, b) by panel p
-    const int r0 = rbnd(a), q0 = bnd(b);
-    const T* Bp = j.L ? j.L + (size_t)q0 * j.ldl + c0 : F + (size_t)q0 * ld + c0;   // TRSM job: X(a) L(b, p)^T
-    const int m = min(rbnd(a + 1), j.nRows) - r0, n = min(bnd(b + 1), j.nUpd) - q0, ldb = j.L ? j.ldl : ld;
-    if constexpr (std::is_same<T, double>::value)
-      tile_abt_f64(F + (size_t)r0 * ld + c0, ld, Bp, ldb, F + (size_t)r0 * ld + q0, ld, m, n, wp, true, !j.L && a == b,
-                   false, reinterpret_cast<double*>(cf_smem));
-    else
-      tile_abt_f32(F + (size_t)r0 * ld + c0, ld, Bp, ldb, F + (size_t)r0 * ld + q0, ld, m, n, wp, true,
-                   reinterpret_cast<float*>(cf_smem));
-    done = cnt + a * j.TU + b;
-    doneVal = p + 1;
+  } else {
+    const int r0 = rbnd(a), m = min(rbnd(a + 1), j.nRows) - r0;
+    const int n = (b < j.P ? bnd(b + 1) : min(bnd(b + 1), j.nUpd)) - q0;
+    const bool same = !j.L && a == b;   // a diagonal tile: A = B, its upper blocks not wanted
+    const int npan = min(b, j.P);
+    T c[R][R];
+#pragma unroll
+    for (int x = 0; x < R; ++x)
+#pragma unroll
+      for (int y = 0; y < R; ++y) {
+        const int i = C::ti(x), k = C::tj(y);
+        c[x][y] = (i < m && k < n) ? __ldcg(F + (size_t)(r0 + i) * ld + q0 + k) : T(0);
+      }
+    const T* Ap = F + (size_t)r0 * ld;
+    const T* Bp = j.L ? j.L + (size_t)q0 * j.ldl : F + (size_t)q0 * ld;   // TRSM job: X(a) L(b, q)^T
+    const int ldb = j.L ? j.ldl : ld;
+    const bool w01 = n > 16 && !same, w10 = m > 16, w11 = m > 16 && n > 16;   // (FP64)
+    T ra[C::Q], rb[C::Q];
+    auto load = [&](int k0, int k1) {
+#pragma unroll
+      for (int q = 0; q < C::Q; ++q) {
+        const int i = C::row(q), k = k0 + C::col(q);
+        ra[q] = (i < m && k < k1) ? __ldcg(Ap + (size_t)i * ld + k) : T(0);
+        if (!same) rb[q] = (i < n && k < k1) ? __ldcg(Bp + (size_t)i * ldb + k) : T(0);
+      }
+    };
+    auto store = [&](int st) {
+#pragma unroll
+      for (int q = 0; q < C::Q; ++q) {
+        C::at(As[st], C::row(q), C::col(q)) = ra[q];
+        if (!same) C::at(Bs[st], C::row(q), C::col(q)) = rb[q];
+      }
+    };
+    // The panels that are there, in one pipelined pass; then wait for more.  (Tiles
+    // far from their turn waiting for four panels at a time, out of step with each
+    // other, to be less in the way of the next panel's: no gain.)
+    for (int q = 0; q < npan;) {
+      if (warp == 0) {
+        const bool ok = wait_geq_lim(tdone + a, q + 1, err, lim) &&
+                        (same || j.L || wait_geq_lim(tdone + b, q + 1, err, lim));
+        if (threadIdx.x == 0) {
+          int r = min(npan, ld_acquire(tdone + a));
+          if (!same && !j.L) r = min(r, ld_acquire(tdone + b));
+          sReady = ok ? r : -1;
+          if (trace) tReady = globaltimer_ns();
+        }
+      }
+      __syncthreads();
+      const int r = sReady;
+      if (r < 0) return;
+      const int kEnd = bnd(r);
+      int k0 = bnd(q), pe = bnd(q + 1), st = 0;   // pe: end of the current panel
+      T acc[R][R];
+#pragma unroll
+      for (int x = 0; x < R; ++x)
+#pragma unroll
+        for (int y = 0; y < R; ++y) acc[x][y] = T(0);
+      if (std::is_same<T, float>::value && same && r == q + 1 && pe - k0 == NB) {
+        // one panel of a diagonal tile -- the chain's last: both slices in one round of loads
+#pragma unroll
+        for (int e = 0; e < C::Q; ++e) {
+          const int i = C::row(e), k = k0 + C::col(e);
+          ra[e] = i < m ? __ldcg(Ap + (size_t)i * ld + k) : T(0);
+          rb[e] = i < m ? __ldcg(Ap + (size_t)i * ld + k + 32) : T(0);
+        }
+#pragma unroll
+        for (int e = 0; e < C::Q; ++e) {
+          C::at(As[0], C::row(e), C::col(e)) = ra[e];
+          C::at(As[1], C::row(e), C::col(e)) = rb[e];
+        }
+        __syncthreads();
+        C::mul(As[0], As[0], 32, acc, w01, w10, w11);
+        C::mul(As[1], As[1], 32, acc, w01, w10, w11);
+#pragma unroll
+        for (int x = 0; x < R; ++x)
+#pragma unroll
+          for (int y = 0; y < R; ++y) c[x][y] -= acc[x][y];
+        __syncthreads();
+        q = r;
+        continue;
+      }
+      load(k0, min(k0 + 32, pe));
+      store(0);
+      __syncthreads();
+      while (true) {
+        const int k1 = min(k0 + 32, pe);
+        const bool last = k1 == pe, more = k1 < kEnd;
+        const int peNext = last ? pe + NB : pe;
+        if (more) load(k1, min(k1 + 32, peNext));
+        C::mul(As[st], same ? As[st] : Bs[st], k1 - k0, acc, w01, w10, w11);
+        if (last)
+#pragma unroll
+          for (int x = 0; x < R; ++x)
+#pragma unroll
+            for (int y = 0; y < R; ++y) {
+              c[x][y] -= acc[x][y];
+              acc[x][y] = T(0);
+            }
+        if (more) store(st ^ 1);
+        __syncthreads();
+        if (!more) break;
+        k0 = k1;
+        pe = peNext;
+        st ^= 1;
+      }
+      q = r;
+    }
+    if (it.kind == CHOL_POTRF) {
+      T* out = ws + j.inv + (size_t)b * NB * NB;
+      const bool below = q0 + n < j.nRows;   // rows below: the TRSM items multiply by the inverse
+      constexpr int PITCH = std::is_same<T, double>::value ? 33 : 68;
+      T (*S)[PITCH] = reinterpret_cast<T (*)[PITCH]>(cf_smem);
+      T (*Li)[PITCH] = S + NB;
+#pragma unroll
+      for (int x = 0; x < R; ++x)
+#pragma unroll
+        for (int y = 0; y < R; ++y) {
+          const int i = C::ti(x), k = C::tj(y);
+          S[i][k] = (k <= i && i < n) ? c[x][y] : (i == k ? T(1) : T(0));
+        }
+      __syncthreads();
+      if constexpr (std::is_same<T, double>::value)
+        potrf_inverse_f64(S, Li, reinterpret_cast<T (*)[17]>(Li + NB), n, below, j.code, flag);
+      else potrf_inverse_f32(S, Li, reinterpret_cast<T (*)[16][17]>(Li + NB), n, below, j.code, flag);
+      __syncthreads();
+      if (below) {   // published before the tile itself, which no item of this launch reads
+#pragma unroll
+        for (int idx = threadIdx.x; idx < NB * NB; idx += 256) {
+          const int i = idx / NB, k = idx % NB;
+          out[idx] = k <= i && i < n ? Li[i][k] : T(0);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+          __threadfence();
+          st_release(pdone + b, 1);
+        }
+      }
+#pragma unroll
+      for (int idx = threadIdx.x; idx < NB * NB; idx += 256) {
+        const int i = idx / NB, k = idx % NB;
+        if (k <= i && i < n) F[(size_t)(r0 + i) * ld + q0 + k] = S[i][k];
+      }
+    } else if (it.kind == CHOL_TRSM) {   // X := C Li(b)^T, the inverse tile from the workspace
+#pragma unroll
+      for (int x = 0; x < R; ++x)
+#pragma unroll
+        for (int y = 0; y < R; ++y) {
+          const int k = C::tj(y);   // C as the A operand: its columns are the k of the product
+          C::at(As[k >> 5], C::ti(x), k & 31) = k < n ? c[x][y] : T(0);
+        }
+      if (warp == 0) {
+        const bool ok = wait_geq_lim(pdone + b, 1, err, lim);
+        if (threadIdx.x == 0) {
+          sReady = ok;
+          if (trace) tReady = globaltimer_ns();
+        }
+      }
+      __syncthreads();
+      if (!sReady) return;
+      const T* Li = ws + j.inv + (size_t)b * NB * NB;
+      T acc[R][R], rl[NB / 32][C::Q];
+#pragma unroll
+      for (int h = 0; h < NB / 32; ++h)
+#pragma unroll
+        for (int q = 0; q < C::Q; ++q) rl[h][q] = __ldcg(Li + C::row(q) * NB + 32 * h + C::col(q));
+#pragma unroll
+      for (int h = 0; h < NB / 32; ++h)
+#pragma unroll
+        for (int q = 0; q < C::Q; ++q) C::at(Bs[h], C::row(q), C::col(q)) = rl[h][q];
+#pragma unroll
+      for (int x = 0; x < R; ++x)
+#pragma unroll
+        for (int y = 0; y < R; ++y) acc[x][y] = T(0);
+      __syncthreads();
+      if constexpr (std::is_same<T, double>::value) {
+        C::mul(As[0], Bs[0], n, acc, n > 16, m > 16, m > 16 && n > 16, 16);   // the inverse is lower triangular
+      } else {
+        C::mul(As[0], Bs[0], min(32, n), acc, true, true, true);
+        if (n > 32) C::mul(As[1], Bs[1], n - 32, acc, true, true, true);
+      }
+#pragma unroll
+      for (int x = 0; x < R; ++x)
+#pragma unroll
+        for (int y = 0; y < R; ++y) {
+          const int i = C::ti(x), k = C::tj(y);
+          if (i < m && k < n) F[(size_t)(r0 + i) * ld + q0 + k] = acc[x][y];
+        }
+      done = tdone + a;
+      doneVal = b + 1;
+    } else {   // a tile of the trailing block
+#pragma unroll
+      for (int x = 0; x < R; ++x)
+#pragma unroll
+        for (int y = 0; y < R; ++y) {
+          const int i = C::ti(x), k = C::tj(y);
+          if (i < m && k < n && (!same || k <= i)) F[(size_t)(r0 + i) * ld + q0 + k] = c[x][y];
+        }
+    }
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();
-    st_release(done, doneVal);
+    if (done) {
+      __threadfence();
+      st_release(done, doneVal);
+    }
     if (trace) {   // diagnostics: when the item started, was ready, ended (ns), and its SM
       unsigned long long* r = trace + 4 * (size_t)sTicket;
       r[0] = tStart;
@@ -1653,8 +1936,7 @@ void launch_chol_fused(const CholFusedJob<T>* jobs, const CholItem* items, int n
                        T* ws, int* flag, unsigned long long* trace, cudaStream_t s) {
   if (nItems <= 0) return;
   RSCHOL_CUDA(cudaMemsetAsync(sync, 0, sizeof(int) * (size_t)syncInts, s));
-  const int smem = std::is_same<T, double>::value ? (int)(sizeof(T) * 2 * 32 * 33)
-                                                  : (int)(sizeof(T) * (3 * 64 * 65 + 3 * 16 * 17));
+  const int smem = chol_smem<T>;
   static std::once_flag once;
   std::call_once(once, [&] {
     RSCHOL_CUDA(cudaFuncSetAttribute(chol_fused_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));

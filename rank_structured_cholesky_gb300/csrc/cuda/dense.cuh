@@ -84,13 +84,13 @@ struct CholFusedJob {
   T* F;
   int ld, nDiag, nRows, nUpd, code;
   int w0, P, TR, TU;
-  int cnt;          // offset of the job's TR x TU + TR + P counters after the ticket
+  int cnt;          // offset of the job's TR + P counters after the ticket
   long long inv;    // element offset of the job's P inverse tiles (NB x NB) in the workspace
   const T* L;       // TRSM job: the factored triangle (null for a Cholesky job)
   int ldl, r1;      // r1: height of the first row tile
 };
 constexpr int CHOL_POTRF = 0, CHOL_TRSM = 1, CHOL_GEMM = 2;
-struct CholItem {   // one piece of panel p: POTRF, TRSM of row tile a, update of tile (a, b)
+struct CholItem {   // one lower tile (a, b): POTRF a = b < P, TRSM b < P, GEMM b >= P; p = b
   int job, kind, p, a, b;
 };
 // sync: syncInts ints (zeroed here, on the stream, before the launch); ws:

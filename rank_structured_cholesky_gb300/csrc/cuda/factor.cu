@@ -222,7 +222,7 @@ void FactorEngine<T>::emit_fused(const std::vector<CholJob<U>>& jobs, int kind, 
     c.TU = tiles(jb.nUpd);
     c.r1 = c.w0;
     c.cnt = (int)(sync - 1);
-    sync += (long long)c.TR * c.TU + c.TR + c.P;
+    sync += c.TR + c.P;
     c.inv = ws;
     ws += (long long)c.P * NB * NB;
     maxP = std::max(maxP, c.P);
@@ -240,27 +240,20 @@ void FactorEngine<T>::emit_fused(const std::vector<CholJob<U>>& jobs, int kind, 
     }
   }
   const int j1 = (int)cjobs.size();
-  // Item order (a topological one, with a look-ahead of one panel): stage p
-  // lists the POTRFs and TRSMs of panel p, the rest R(p - 1) of the previous
-  // panel's updates (column tiles >= p + 1), then L(p), panel p's updates of
-  // column tile p + 1 -- all that POTRF(p + 1) and its TRSMs wait for.  So
-  // the next panel's critical pieces are taken long before the bulk of the
-  // current updates is done.
-  auto updates = [&](int q, int p, int bLo, int bHi) {
-    const CholFusedJob<U>& c = cjobs[q];
-    for (int b = std::max(bLo, p + 1); b < std::min(bHi, c.TU); ++b)
-      for (int a = b; a < c.TR; ++a) items.push_back(CholItem{q, CHOL_GEMM, p, a, b});
-  };
-  for (int p = 0; p <= maxP; ++p) {
+  // Item order (a topological one): the tiles of column 0 of every job, of column
+  // 1, ...; then the trailing tiles.  Blocks that wait hold tiles of the next
+  // columns, which take in each panel as it appears.
+  for (int p = 0; p < maxP; ++p) {
     for (int q = j0; q < j1; ++q)
       if (p < cjobs[q].P) items.push_back(CholItem{q, CHOL_POTRF, p, p, p});
     for (int q = j0; q < j1; ++q)
       if (p < cjobs[q].P)
         for (int a = p + 1; a < cjobs[q].TR; ++a) items.push_back(CholItem{q, CHOL_TRSM, p, a, p});
-    for (int q = j0; q < j1; ++q)
-      if (p >= 1 && p <= cjobs[q].P) updates(q, p - 1, p + 1, INT_MAX);   // R(p - 1)
-    for (int q = j0; q < j1; ++q)
-      if (p < cjobs[q].P) updates(q, p, p + 1, p + 2);                    // L(p)
+  }
+  for (int q = j0; q < j1; ++q) {
+    const CholFusedJob<U>& c = cjobs[q];
+    for (int b = c.P; b < c.TU; ++b)
+      for (int a = b; a < c.TR; ++a) items.push_back(CholItem{q, CHOL_GEMM, b, a, b});
   }
   if (dropItemTest_ && !droppedItem_) {   // test switch: one POTRF whose TRSMs then wait in vain
     for (size_t k = (size_t)st.off; k < items.size(); ++k)
@@ -435,7 +428,7 @@ void FactorEngine<T>::emit_trsm(const std::vector<TrsmJob<T>>& jobs) {
       c.TR = (jb.rows + NB - 1) / NB;
       c.TU = c.P;
       c.cnt = (int)(sync - 1);
-      sync += (long long)c.TR * c.TU + c.TR + c.P;
+      sync += c.TR + c.P;
       c.inv = ws;
       ws += (long long)c.P * NB * NB;
       maxP = std::max(maxP, c.P);
@@ -448,24 +441,13 @@ void FactorEngine<T>::emit_trsm(const std::vector<TrsmJob<T>>& jobs) {
       }
     }
     const int j1 = (int)cholJobs_.size();
-    // all diagonal inverses first (no waits), then stage p: the TRSMs of panel
-    // p, the rest of panel p - 1's updates, panel p's updates of column tile p + 1
+    // all diagonal inverses first (no waits), then the tiles by columns
     for (int q = j0; q < j1; ++q)
       for (int p = 0; p < cholJobs_[q].P; ++p) cholItems_.push_back(CholItem{q, CHOL_POTRF, p, p, p});
-    auto updates = [&](int q, int p, int bLo, int bHi) {
-      const CholFusedJob<T>& c = cholJobs_[q];
-      for (int b = std::max(bLo, p + 1); b < std::min(bHi, c.TU); ++b)
-        for (int a = 0; a < c.TR; ++a) cholItems_.push_back(CholItem{q, CHOL_GEMM, p, a, b});
-    };
-    for (int p = 0; p <= maxP; ++p) {
+    for (int p = 0; p < maxP; ++p)
       for (int q = j0; q < j1; ++q)
         if (p < cholJobs_[q].P)
           for (int a = 0; a < cholJobs_[q].TR; ++a) cholItems_.push_back(CholItem{q, CHOL_TRSM, p, a, p});
-      for (int q = j0; q < j1; ++q)
-        if (p >= 1 && p <= cholJobs_[q].P) updates(q, p - 1, p + 1, INT_MAX);
-      for (int q = j0; q < j1; ++q)
-        if (p < cholJobs_[q].P) updates(q, p, p + 1, p + 2);
-    }
     st.count = st.grid = (int)(cholItems_.size() - st.off);
     st.elems = sync;
     st.flops = flops - flops0;
