@@ -160,10 +160,11 @@ int rschol_factor_autotune(rschol_factor* f, int max_columns);
  * `repeats` numeric factorisations of the factor's current values under each
  * candidate -- FP32 GEMM steps on the tensor cores (128 x 64 or 128 x 128
  * tiles) from K >= 32, 64, 96, 128 or 256, or none (64 x 64 SIMT tiles);
- * the blocked Cholesky
+ * * the blocked Cholesky
  * and TRSM chains of a level as one fused launch of 64 x 64 tile items or as
  * one launch per 64-column panel -- keeps the fastest and leaves the factor
- * refactored with it.  The candidates differ only in rounding.  Run it while
+ * refactored with it (within 3 % of each other the earlier one stays, 128 first).
+ * The candidates differ only in rounding.  Run it while
  * the GPU is otherwise quiet, before creating sessions on the factor.  The
  * choice is listed in rschol_factor_describe ("schedule": tc_min_k (-1: none),
  * fused, tuned_ms). */

@@ -1235,7 +1235,9 @@ extern "C" int rschol_factor_tune_schedule(rschol_factor* f, int repeats) {
     RSCHOL_CUDA(cudaEventCreate(&e0));
     RSCHOL_CUDA(cudaEventCreate(&e1));
     std::vector<int> ks = {INT_MAX};
-    if (f->precision == RSCHOL_MIXED) ks = {32, 64, 96, 128, 256, INT_MAX};
+    // the default first: a candidate displaces one before it by 3 % or more, what two
+    // timings of a schedule differ by (a 16^3 grid: 1.18 ms at 64, 96 and 128 alike)
+    if (f->precision == RSCHOL_MIXED) ks = {128, 256, INT_MAX, 96, 64, 32};
     int bestK = f->impl->tc_min_k();
     bool bestFused = f->impl->fused_chol();
     double best = 1e300;
@@ -1257,7 +1259,7 @@ extern "C" int rschol_factor_tune_schedule(rschol_factor* f, int repeats) {
           RSCHOL_CUDA(cudaEventElapsedTime(&t, e0, e1));
           ms += t;
         }
-        if (ok && ms / repeats < best) {
+        if (ok && ms / repeats < 0.97 * best) {
           best = ms / repeats;
           bestK = k;
           bestFused = fused;

@@ -59,90 +59,106 @@ using namespace tcdev;
 //              (tcgen05.ld, 32 lanes each) -> shared rows -> C (or the
 //              K-slice partials) in coalesced rows, by all threads.
 // NS stages keep NS K tiles in flight, so loads, conversion and MMAs of
-// different stages overlap.  The producers' global-load latency bounds a
-// stage: the c2 factor took 25.49 ms with four producer warps, 24.39 with
-// eight, 24.27 with sixteen.  (Measured
-// against it on the c2 factor's GEMM steps: both operands' loads issued
-// before either is stored, with L2 prefetches of the tiles ahead, 4.33 vs
-// 4.15 ms; asynchronous 16-byte copies into three raw stages converted into
-// two MMA stages, 5.15 ms.)  Every wait is bounded; a wait that gives up sets
+// different stages overlap.  The producers' global-load latency bounds a stage:
+// with the sixteen warps as two groups that take K tiles in turn, and both
+// operands' loads in flight before the wait for the stage, the GEMM steps of a
+// 3D 64^3 factor take 5.3 ms, of 96^3 30.6; all sixteen on one tile at a time, one
+// operand after the other, 6.4 and 38.5.  (Asynchronous 16-byte copies into three
+// raw stages converted into two MMA stages were slower.)
+// Every wait is bounded; a wait that gives up sets
 // *err, stops the loops, waits (bounded) for the CTA's issued MMAs and frees
 // the TMEM before returning.
 // ---------------------------------------------------------------------------
 constexpr int WS_PW = 16;                         // producer warps
 constexpr int WS_PT = 32 * WS_PW;                 // producer threads
+// Producer groups of the register staging: group g takes the K tiles g, g + WS_NG,
+// ...  No more groups than stages: a group's wait for its tile's stage is by phase
+// parity, and only its own last tile, WS_NG before, tells it how far the stage is.
+constexpr int WS_NG = 2, WS_GT = WS_PT / WS_NG;
 constexpr int WS_THREADS = WS_PT + 128;           // + the MMA / epilogue warpgroup
 
-// One ROWS x 32 K tile of an operand into the stage's swizzled K-major
-// buffers (hi at dst, lo at dst + loOff when split).  Element (r, k) of the
-// tile is src[(row0 + r) * ld + k0 + k] (kContig) or src[(k0 + k) * ld + row0
-// + r]; rows >= nRows and k >= kEnd read as zero.  vec: the 16-byte loads
-// along the contiguous dimension are aligned (checked per task).  BF: the
-// tile is stored as BF16 (hi = bf16(a), lo = bf16(a - hi)) at element
-// positions kPos .. kPos + 31 of the 64-element (128-byte) rows; otherwise as
-// TF32 filling the 32-element rows.
-template <int ROWS, bool BF>
-__device__ __forceinline__ void ws_load_tile(const float* __restrict__ src, int ld, bool kContig, bool vec, int row0,
-                                             int nRows, int k0, int kEnd, uint32_t dst, uint32_t loOff, bool split,
-                                             int tid, int kPos = 0) {
-  constexpr int PER = ROWS * 32 / 4 / WS_PT;   // float4 groups per producer thread
+// One ROWS x 32 K tile of an operand, by the threads (tid) of a producer group:
+// ws_load into registers, ws_store into the stage's swizzled K-major buffers (hi at
+// dst, lo at dst + loOff when split).  Element (r, k) of the tile is
+// src[(row0 + r) * ld + k0 + k] (kContig) or src[(k0 + k) * ld + row0 + r]; rows >=
+// nRows and k >= kEnd read as zero.  vec: the 16-byte loads along the contiguous
+// dimension are aligned (checked per task).  BF: the tile is stored as BF16 (hi =
+// bf16(a), lo = bf16(a - hi)) at element positions kPos .. kPos + 31 of the
+// 64-element (128-byte) rows; otherwise as TF32 filling the 32-element rows.
+// Along K a warp takes 4 rows x 32 k.  Along the rows it takes 16 k x 8 rows (whole
+// 32-byte sectors): stored a word at a time, those fall into 32 different banks --
+// rows r and r + 4 swizzle to different halves -- where 128 rows of one k met in
+// two chunks, 16 stores to a bank.
+template <int ROWS>
+struct WsTile {
+  static constexpr int PER = ROWS * 32 / 4 / WS_GT;   // float4 groups per thread
   float4 v[PER];
+};
+template <int ROWS>
+__device__ __forceinline__ int2 ws_pos(bool kContig, int tid, int q) {   // (row, k) of a thread's q-th group
   if (kContig) {
-    // group g: row g >> 3, k 4 (g & 7) .. +3
+    const int g = tid + WS_GT * q;
+    return make_int2(g >> 3, (g & 7) * 4);
+  }
+  const int w = tid >> 5, lane = tid & 31;
+  return make_int2(8 * ((w >> 1) * WsTile<ROWS>::PER + q) + 4 * (lane & 1), 16 * (w & 1) + (lane >> 1));
+}
+template <int ROWS>
+__device__ __forceinline__ void ws_load(WsTile<ROWS>& t, const float* __restrict__ src, int ld, bool kContig, bool vec,
+                                        int row0, int nRows, int k0, int kEnd, int tid) {
 #pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      const int g = tid + WS_PT * q, r = g >> 3, kk = (g & 7) * 4;
-      const int gr = row0 + r, gk = k0 + kk;
+  for (int q = 0; q < WsTile<ROWS>::PER; ++q) {
+    const int2 rk = ws_pos<ROWS>(kContig, tid, q);
+    const int gr = row0 + rk.x, gk = k0 + rk.y;
+    float4& v = t.v[q];
+    if (kContig) {
       const float* p = src + (size_t)gr * ld + gk;
       if (gr < nRows && vec && gk + 3 < kEnd) {
-        v[q] = __ldg(reinterpret_cast<const float4*>(p));
+        v = __ldg(reinterpret_cast<const float4*>(p));
       } else {
-        v[q].x = (gr < nRows && gk < kEnd) ? __ldg(p) : 0.f;
-        v[q].y = (gr < nRows && gk + 1 < kEnd) ? __ldg(p + 1) : 0.f;
-        v[q].z = (gr < nRows && gk + 2 < kEnd) ? __ldg(p + 2) : 0.f;
-        v[q].w = (gr < nRows && gk + 3 < kEnd) ? __ldg(p + 3) : 0.f;
+        v.x = (gr < nRows && gk < kEnd) ? __ldg(p) : 0.f;
+        v.y = (gr < nRows && gk + 1 < kEnd) ? __ldg(p + 1) : 0.f;
+        v.z = (gr < nRows && gk + 2 < kEnd) ? __ldg(p + 2) : 0.f;
+        v.w = (gr < nRows && gk + 3 < kEnd) ? __ldg(p + 3) : 0.f;
+      }
+    } else {
+      const float* p = src + (size_t)gk * ld + gr;
+      if (gk < kEnd && vec && gr + 3 < nRows) {
+        v = __ldg(reinterpret_cast<const float4*>(p));
+      } else {
+        v.x = (gk < kEnd && gr < nRows) ? __ldg(p) : 0.f;
+        v.y = (gk < kEnd && gr + 1 < nRows) ? __ldg(p + 1) : 0.f;
+        v.z = (gk < kEnd && gr + 2 < nRows) ? __ldg(p + 2) : 0.f;
+        v.w = (gk < kEnd && gr + 3 < nRows) ? __ldg(p + 3) : 0.f;
       }
     }
+  }
+}
+template <int ROWS, bool BF>
+__device__ __forceinline__ void ws_store(const WsTile<ROWS>& t, bool kContig, uint32_t dst, uint32_t loOff, bool split,
+                                         int tid, int kPos) {
 #pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      const int g = tid + WS_PT * q, r = g >> 3, kk = (g & 7) * 4;
+  for (int q = 0; q < WsTile<ROWS>::PER; ++q) {
+    const int2 rk = ws_pos<ROWS>(kContig, tid, q);
+    const int r = rk.x, kk = rk.y;
+    const float4 v = t.v[q];
+    if (kContig) {
       if constexpr (BF) {
         const uint32_t off = tc_off16(r, kPos + kk);
         float l[4];
-        const uint32_t h01 = split_bf16x2(v[q].x, v[q].y, l[0], l[1]), h23 = split_bf16x2(v[q].z, v[q].w, l[2], l[3]);
+        const uint32_t h01 = split_bf16x2(v.x, v.y, l[0], l[1]), h23 = split_bf16x2(v.z, v.w, l[2], l[3]);
         st_shared_v2(dst + off, h01, h23);
         if (split) st_shared_v2(dst + loOff + off, pack_bf16x2(l[0], l[1]), pack_bf16x2(l[2], l[3]));
       } else {
         const uint32_t off = tc_off(r, kk);
-        const uint32_t h0 = to_tf32(v[q].x), h1 = to_tf32(v[q].y), h2 = to_tf32(v[q].z), h3 = to_tf32(v[q].w);
+        const uint32_t h0 = to_tf32(v.x), h1 = to_tf32(v.y), h2 = to_tf32(v.z), h3 = to_tf32(v.w);
         st_shared_v4(dst + off, h0, h1, h2, h3);
         if (split)
-          st_shared_v4(dst + loOff + off, to_tf32(v[q].x - __uint_as_float(h0)),
-                       to_tf32(v[q].y - __uint_as_float(h1)), to_tf32(v[q].z - __uint_as_float(h2)),
-                       to_tf32(v[q].w - __uint_as_float(h3)));
+          st_shared_v4(dst + loOff + off, to_tf32(v.x - __uint_as_float(h0)), to_tf32(v.y - __uint_as_float(h1)),
+                       to_tf32(v.z - __uint_as_float(h2)), to_tf32(v.w - __uint_as_float(h3)));
       }
-    }
-  } else {
-    // group g: k g / (ROWS / 4), rows 4 (g mod ROWS / 4) .. +3
-    constexpr int GR = ROWS / 4;
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      const int g = tid + WS_PT * q, kk = g / GR, r = (g % GR) * 4;
-      const int gr = row0 + r, gk = k0 + kk;
-      const float* p = src + (size_t)gk * ld + gr;
-      if (gk < kEnd && vec && gr + 3 < nRows) {
-        v[q] = __ldg(reinterpret_cast<const float4*>(p));
-      } else {
-        v[q].x = (gk < kEnd && gr < nRows) ? __ldg(p) : 0.f;
-        v[q].y = (gk < kEnd && gr + 1 < nRows) ? __ldg(p + 1) : 0.f;
-        v[q].z = (gk < kEnd && gr + 2 < nRows) ? __ldg(p + 2) : 0.f;
-        v[q].w = (gk < kEnd && gr + 3 < nRows) ? __ldg(p + 3) : 0.f;
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      const int g = tid + WS_PT * q, kk = g / GR, r = (g % GR) * 4;
-      const float e[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+    } else {
+      const float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         if constexpr (BF) {
@@ -219,7 +235,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) gemm_tc_kernel(const GemmTask<f
   if constexpr (!BF) viaTma = t.tmA != nullptr && t.tmB != nullptr;
   if (tid == 0) {
     for (int st = 0; st < NS; ++st) {
-      mbar_init(full0 + 8u * st, viaTma ? WS_PT - 32 : WS_PT);   // TMA staging: warp 0 issues, the rest convert
+      mbar_init(full0 + 8u * st, viaTma ? WS_PT - 32 : WS_GT);   // TMA staging: warp 0 issues, the rest convert
       mbar_init(empty0 + 8u * st, 1);
       mbar_init(tma0 + 8u * st, 1);
     }
@@ -279,22 +295,31 @@ __global__ void __launch_bounds__(WS_THREADS, 1) gemm_tc_kernel(const GemmTask<f
     const bool aK = !t.tA, bK = t.tB != 0;   // K contiguous in memory
     const bool aVec = ((reinterpret_cast<uintptr_t>(t.A) & 15u) == 0) && (t.lda & 3) == 0;
     const bool bVec = ((reinterpret_cast<uintptr_t>(t.B) & 15u) == 0) && (t.ldb & 3) == 0;
-    for (int kt = 0; kt < nk; ++kt) {
+    static_assert(WS_NG <= NS, "producer groups");
+    const int gtid = tid % WS_GT;
+    for (int kt = tid / WS_GT; kt < nk; kt += WS_NG) {
       const int st = kt % NS, use = kt / NS;
-      if (use > 0 && !mbar_wait(empty0 + 8u * st, (uint32_t)((use - 1) & 1))) {
-        atomicExch(err, 1);
-        sAbort = 1;
-      }
-      if (sAbort) break;
       const uint32_t a = sbase + (uint32_t)(st * STAGE), b = a + 2 * A_BYTES;
       const int k0 = kBeg + kt * SK;
+      bool stop = false;
 #pragma unroll
       for (int h = 0; h < SK / TC_BK; ++h) {
-        ws_load_tile<TC_BM, BF>(t.A, t.lda, aK, aVec, row0, t.M, k0 + TC_BK * h, kEnd, a, A_BYTES, split, tid,
-                                TC_BK * h);
-        ws_load_tile<BN, BF>(t.B, t.ldb, bK, bVec, col0, t.N, k0 + TC_BK * h, kEnd, b, B_BYTES, split, tid,
-                             TC_BK * h);
+        WsTile<TC_BM> ta;   // both operands in flight, before the wait for the stage
+        WsTile<BN> tb;
+        ws_load(ta, t.A, t.lda, aK, aVec, row0, t.M, k0 + TC_BK * h, kEnd, gtid);
+        ws_load(tb, t.B, t.ldb, bK, bVec, col0, t.N, k0 + TC_BK * h, kEnd, gtid);
+        if (h == 0) {
+          if (use > 0 && !mbar_wait(empty0 + 8u * st, (uint32_t)((use - 1) & 1))) {
+            atomicExch(err, 1);
+            sAbort = 1;
+          }
+          stop = sAbort;
+        }
+        if (stop) break;
+        ws_store<TC_BM, BF>(ta, aK, a, A_BYTES, split, gtid, TC_BK * h);
+        ws_store<BN, BF>(tb, bK, b, B_BYTES, split, gtid, TC_BK * h);
       }
+      if (stop) break;
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       mbar_arrive(full0 + 8u * st);
     }
