@@ -10,21 +10,24 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int VEC_THREADS = 256;
-constexpr int VEC_BLOCKS = 152 * 8;   // fixed grid: 8 CTAs per SM on 152 SMs
+constexpr int VEC_BLOCKS = 152 * 8;   // at most 8 CTAs per SM on 152 SMs
 
 enum { S_DELTA = 0, S_ALPHA, S_BETA, S_RREL, S_BNORM, S_DQ, S_DELTA_NEW, S_BREAK, S_ITERS, S_TRUE, S_COUNT };
 enum { F_ALPHA = 0, F_RNORM, F_BETA, F_DELTA0, F_BNORM, F_TRUE };
 
-__device__ __forceinline__ double block_sum(double v) {
-  __shared__ double ws[32];
+// A warp's FP64 add holds its quarter of the SM's FP64 unit for 64 clocks, so the
+// adds of the reductions are counted: 5 a warp and log2(warps) in the end.
+__device__ __forceinline__ double block_sum(double v) {   // of VEC_THREADS threads
+  constexpr int NW = VEC_THREADS / 32;
+  __shared__ double ws[NW];
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0) ws[warp] = v;
   __syncthreads();
   double t = 0;
   if (warp == 0) {
-    t = (lane < (int)(blockDim.x >> 5)) ? ws[lane] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(FULL, t, o);
+    t = ws[lane % NW];
+    for (int o = NW / 2; o > 0; o >>= 1) t += __shfl_xor_sync(FULL, t, o);
   }
   return t;   // valid in thread 0
 }
@@ -34,17 +37,21 @@ __global__ void spmv_kernel(int n, const int* __restrict__ rp, const int* __rest
                             const double* __restrict__ v, const double* __restrict__ x, double* __restrict__ y,
                             double* __restrict__ part, int withDot) {
   pdl_enter();
-  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int row = (int)(g / TPR), lane = (int)(g % TPR);
-  double s = 0.0;
-  if (row < n)
-    for (int p = rp[row] + lane; p < rp[row + 1]; p += TPR) s += v[p] * x[ci[p]];
-#pragma unroll
-  for (int o = TPR / 2; o > 0; o >>= 1) s += __shfl_down_sync(FULL, s, o, TPR);
+  const int lane = threadIdx.x % TPR;
+  const int groups = gridDim.x * (VEC_THREADS / TPR);   // rows in step
   double dq = 0.0;
-  if (lane == 0 && row < n) {
-    y[row] = s;
-    dq = x[row] * s;
+  // (whole warps together: the shuffles below)
+  for (int first = blockIdx.x * (VEC_THREADS / TPR) + (threadIdx.x & ~31) / TPR; first < n; first += groups) {
+    const int row = first + (threadIdx.x & 31) / TPR;
+    double s = 0.0;
+    if (row < n)
+      for (int p = rp[row] + lane; p < rp[row + 1]; p += TPR) s += v[p] * x[ci[p]];
+#pragma unroll
+    for (int o = TPR / 2; o > 0; o >>= 1) s += __shfl_down_sync(FULL, s, o, TPR);
+    if (lane == 0 && row < n) {
+      y[row] = s;
+      dq += x[row] * s;
+    }
   }
   if (withDot) {
     double t = block_sum(dq);
@@ -189,15 +196,22 @@ PcgEngine::PcgEngine(int n_, const std::vector<int>& rowptr, const std::vector<i
   RSCHOL_CUDA(cudaMemcpyAsync(colind_.p, colind.data(), sizeof(int) * colind.size(), cudaMemcpyHostToDevice, s));
   RSCHOL_CUDA(cudaMemcpyAsync(vals_.p, vals.data(), sizeof(double) * vals.size(), cudaMemcpyHostToDevice, s));
   const double avg = n > 0 ? (double)colind.size() / n : 1.0;
-  // threads per row: one (each thread's loads all in flight at once) up to 12
-  // entries per row -- the c2 PCG took 20.84 ms at one, 20.99 at two, 21.14
-  // at four, 21.64 at eight -- then more for longer rows
-  tpr_ = avg <= 12 ? 1 : avg <= 40 ? 16 : 32;
+  // Threads per row: every one costs the warp adds in the row's sum, and those are
+  // FP64.  One up to 12 entries per row (3D 64^3, 7 entries: 15.6 us an SpMV at one,
+  // 20 at two, 22 at four, 33 at eight); longer rows two, or as many as give the
+  // device 1024 threads an SM (elasticity 30^3, 80 entries: 32 us at two, 35 at
+  // eight, 51 at one and at sixteen, 84 at thirty-two).
+  tpr_ = 1;
+  if (avg > 12)
+    for (tpr_ = 2; tpr_ < 32 && (long long)n * tpr_ < 152 * 1024; tpr_ *= 2) {}
   if (const char* e = std::getenv("RSCHOL_SPMV_TPR")) {   // threads per row of the SpMV (1 ... 32)
     const int t = std::atoi(e);
     if (t == 1 || t == 2 || t == 4 || t == 8 || t == 16 || t == 32) tpr_ = t;
   }
-  nblk_ = (int)(((long long)n * tpr_ + VEC_THREADS - 1) / VEC_THREADS);
+  nblk_ = (int)std::min<long long>(VEC_BLOCKS, ((long long)n * tpr_ + VEC_THREADS - 1) / VEC_THREADS);
+  // four elements a thread, for fewer block sums; two blocks an SM at least
+  nvec_ = (int)std::min<long long>(
+      VEC_BLOCKS, std::max<long long>(VEC_BLOCKS / 4, (n + 4LL * VEC_THREADS - 1) / (4 * VEC_THREADS)));
   for (auto* b : {&r_, &d_, &q_, &s_}) b->alloc(sizeof(double) * std::max(1, n));
   part_.alloc(sizeof(double) * std::max(nblk_, VEC_BLOCKS));
   scal_.alloc(sizeof(double) * S_COUNT);
@@ -252,12 +266,12 @@ void PcgEngine::prologue(const double* b, double* x, const std::function<void(do
   RSCHOL_CUDA(cudaMemsetAsync(sc, 0, sizeof(double) * S_COUNT, st));
   RSCHOL_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * n, st));
   RSCHOL_CUDA(cudaMemcpyAsync(r, b, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
-  launch_k(dot_kernel, dim3(VEC_BLOCKS), dim3(VEC_THREADS), 0, st, b, b, n, part);
-  launch_k(finish_kernel, dim3(1), dim3(1024), 0, st, part, VEC_BLOCKS, sc, F_BNORM);
+  launch_k(dot_kernel, dim3(nvec_), dim3(VEC_THREADS), 0, st, b, b, n, part);
+  launch_k(finish_kernel, dim3(1), dim3(VEC_THREADS), 0, st, part, nvec_, sc, F_BNORM);
   RSCHOL_CUDA(cudaMemcpyAsync(s, r, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
   apply(s);
-  launch_k(dot_kernel, dim3(VEC_BLOCKS), dim3(VEC_THREADS), 0, st, r, s, n, part);
-  launch_k(finish_kernel, dim3(1), dim3(1024), 0, st, part, VEC_BLOCKS, sc, F_DELTA0);
+  launch_k(dot_kernel, dim3(nvec_), dim3(VEC_THREADS), 0, st, r, s, n, part);
+  launch_k(finish_kernel, dim3(1), dim3(VEC_THREADS), 0, st, part, nvec_, sc, F_DELTA0);
   RSCHOL_CUDA(cudaMemcpyAsync(d, s, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
   launches += 4;
   RSCHOL_LAUNCH_CHECK();
@@ -274,13 +288,13 @@ void PcgEngine::iteration(double* x, const std::function<void(double*)>& apply) 
   double* sc = scal_.as<double>();
   cudaStream_t st = stream_;
   spmv(d, q);
-  launch_k(finish_kernel, dim3(1), dim3(1024), 0, st, part, nblk_, sc, F_ALPHA);
-  launch_k(update_xr_kernel, dim3(VEC_BLOCKS), dim3(VEC_THREADS), 0, st, x, r, d, q, sc, n, part, s);
-  launch_k(finish_kernel, dim3(1), dim3(1024), 0, st, part, VEC_BLOCKS, sc, F_RNORM);
+  launch_k(finish_kernel, dim3(1), dim3(VEC_THREADS), 0, st, part, nblk_, sc, F_ALPHA);
+  launch_k(update_xr_kernel, dim3(nvec_), dim3(VEC_THREADS), 0, st, x, r, d, q, sc, n, part, s);
+  launch_k(finish_kernel, dim3(1), dim3(VEC_THREADS), 0, st, part, nvec_, sc, F_RNORM);
   apply(s);
-  launch_k(dot_kernel, dim3(VEC_BLOCKS), dim3(VEC_THREADS), 0, st, r, s, n, part);
-  launch_k(finish_kernel, dim3(1), dim3(1024), 0, st, part, VEC_BLOCKS, sc, F_BETA);
-  launch_k(update_d_kernel, dim3(VEC_BLOCKS), dim3(VEC_THREADS), 0, st, d, s, sc, n);
+  launch_k(dot_kernel, dim3(nvec_), dim3(VEC_THREADS), 0, st, r, s, n, part);
+  launch_k(finish_kernel, dim3(1), dim3(VEC_THREADS), 0, st, part, nvec_, sc, F_BETA);
+  launch_k(update_d_kernel, dim3(nvec_), dim3(VEC_THREADS), 0, st, d, s, sc, n);
   RSCHOL_LAUNCH_CHECK();
   launches += 6;
 }
@@ -291,8 +305,8 @@ void PcgEngine::epilogue(const double* b, const double* x) {
   double* part = part_.as<double>();
   double* sc = scal_.as<double>();
   spmv(x, q);
-  launch_k(residual_kernel, dim3(VEC_BLOCKS), dim3(VEC_THREADS), 0, stream_, b, q, n, part);
-  launch_k(finish_kernel, dim3(1), dim3(1024), 0, stream_, part, VEC_BLOCKS, sc, F_TRUE);
+  launch_k(residual_kernel, dim3(nvec_), dim3(VEC_THREADS), 0, stream_, b, q, n, part);
+  launch_k(finish_kernel, dim3(1), dim3(VEC_THREADS), 0, stream_, part, nvec_, sc, F_TRUE);
   RSCHOL_LAUNCH_CHECK();
   launches += 2;
 }

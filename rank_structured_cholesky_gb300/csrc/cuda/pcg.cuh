@@ -82,7 +82,7 @@ class PcgEngine {
   DevBuf ctl_;                 // eps, maxit of the current solve (read by the graph's control kernels)
   double* hCtl_ = nullptr;     // pinned
   bool useGraph_ = true;
-  int nblk_ = 0;
+  int nblk_ = 0, nvec_ = 0;   // blocks of the SpMV and of the vector kernels
   int tpr_ = 8;
   // batched solves (allocated for kB_ right-hand sides on first use)
   int kB_ = 0;
