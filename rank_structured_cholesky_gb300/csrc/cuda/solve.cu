@@ -41,12 +41,13 @@ __device__ __forceinline__ void pull_sums(T (&v)[N], const int* const (&ent)[N],
 // the columns [k0, k0 + GT vectors), in a fixed order: groups of threads take
 // every ng-th row, the groups are added in order.
 template <class T>
-__device__ __forceinline__ void sum_parts(const T* __restrict__ part, int rp, int k0, int parts, T* zs, T* redT) {
+__device__ __forceinline__ void sum_parts(const T* __restrict__ part, int rp, int cols, int k0, int parts, T* zs,
+                                          T* redT) {
   using Vt = typename Vec16<T>::type;
   constexpr int V = Vec16<T>::V;
   Vt* red = reinterpret_cast<Vt*>(redT);
   const int tid = threadIdx.x % GT;
-  const int nv = min(GT, (rp - k0) / V);
+  const int nv = min(GT, (cols - k0 + V - 1) / V);
   int ng = GT / nv;
   if (ng > parts) ng = parts;
   const int g = tid / nv, c = tid - g * nv;
@@ -400,7 +401,7 @@ __device__ __forceinline__ void rows_times_parts(const T* M, int r, int rows, co
 #pragma unroll
   for (int q = 0; q < 8; ++q) acc[q] = T(0);
   for (int k0 = 0; k0 < r; k0 += KT) {
-    sum_parts<T>(part, rp, k0, parts, zs, red);
+    sum_parts<T>(part, rp, rp, k0, parts, zs, red);
     const int kn = min(KT, r - k0);
     const T* m = M + (size_t)warp * r + k0;
 #pragma unroll 2
@@ -473,7 +474,7 @@ __global__ void __launch_bounds__(NGRP * GT + 32, 3) apply_kernel(ApplyArgs<T> A
           T t[Vec16<T>::V];
 #pragma unroll
           for (int q = 0; q < Vec16<T>::V; ++q) t[q] = tid + q * GT < kn ? __ldcg(A.t + h[5] + k0 + tid + q * GT) : T(0);
-          sum_parts<T>(A.ip + h[2], h[4], k0, h[3], zs, red);
+          sum_parts<T>(A.ip + h[2], h[4], h[0], k0, h[3], zs, red);
 #pragma unroll
           for (int q = 0; q < Vec16<T>::V; ++q)
             if (tid + q * GT < kn) A.w[h[1] + k0 + tid + q * GT] = t[q] - zs[tid + q * GT];
@@ -1491,9 +1492,13 @@ void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<l
       it.sig = counter();
       waits.clear();
       pairs_of(waits, solved[s]);
-      push(it, waits, {nodes_[s].n, nodes_[s].c0, i32(ipOff[s]), solved[s].target, part_ld(nodes_[s].n),
-                            nodes_[s].tOff});
-      solved[s] = Done{it.sig, 1};
+      // many parts: by columns, 1024 entries an item, so that a block of right-hand
+      // sides has no item that reads megabytes (3D 40^3, k = 32: an item of 100 parts
+      // of 400 columns held the level up for 130 - 180 us)
+      const int n = nodes_[s].n, parts = solved[s].target, w = std::max(16, 1024 / parts & ~15);
+      for (int c = 0; c < n; c += w)
+        push(it, waits, {std::min(w, n - c), nodes_[s].c0 + c, i32(ipOff[s] + c), parts, part_ld(n), nodes_[s].tOff + c});
+      solved[s] = Done{it.sig, (n + w - 1) / w};
     }
   }
   nItems_ = (int)items.size();

@@ -17,9 +17,9 @@
 // dependent loads whatever its bytes), FP64 its 1/64 rate.  Measured, one
 // application against the earlier kernels (a triangular solve with a thread per
 // (row, column) pair, six launches per compressed level): 2D 1024^2 FP32 k = 64
-// 10.50 -> 5.99 ms, k = 8 3.62 -> 0.85 ms; 3D 40^3 FP32 k = 32 1.99 -> 1.06 ms,
-// k = 8 1.81 -> 0.47 ms; 3D 64^3 FP32 k = 16 3.23 -> 1.10 ms; 3D 44x40x47 FP64
-// k = 8 2.78 -> 1.84 ms.
+// 10.50 -> 5.99 ms, k = 8 3.62 -> 0.85 ms; 3D 40^3 FP32 k = 32 1.99 -> 0.82 ms,
+// k = 8 1.81 -> 0.42 ms; 3D 64^3 FP32 k = 16 3.23 -> 1.09 ms; 3D 44x40x47 FP64
+// k = 8 2.78 -> 1.75 ms.
 #include <algorithm>
 #include <mutex>
 #include <stdexcept>
@@ -497,13 +497,13 @@ __global__ void __launch_bounds__(NGRP * GT + 32, BATCH_BLOCKS) apply_batch_kern
         case IT_BR: {
           for (int j = p.rg; j < h[0]; j += p.nrg) {
             Vt t = p.ld(A.t, h[5] + j), x = vzero(T(0));
-            for (int q0 = 0; q0 < h[3]; q0 += 8) {
-              Vt v[8];
+            for (int q0 = 0; q0 < h[3]; q0 += 16) {
+              Vt v[16];
 #pragma unroll
-              for (int q = 0; q < 8; ++q)
+              for (int q = 0; q < 16; ++q)
                 v[q] = q0 + q < h[3] ? p.ld(A.ip, h[2] + (long long)(q0 + q) * h[4] + j) : vzero(T(0));
 #pragma unroll
-              for (int q = 0; q < 8; ++q) vadd(x, v[q]);
+              for (int q = 0; q < 16; ++q) vadd(x, v[q]);
             }
             vsub(t, x);
             p.st(A.w, h[1] + j, t);
