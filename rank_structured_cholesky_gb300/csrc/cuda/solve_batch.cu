@@ -17,9 +17,9 @@
 // dependent loads whatever its bytes), FP64 its 1/64 rate.  Measured, one
 // application against the earlier kernels (a triangular solve with a thread per
 // (row, column) pair, six launches per compressed level): 2D 1024^2 FP32 k = 64
-// 10.50 -> 5.99 ms, k = 8 3.62 -> 0.85 ms; 3D 40^3 FP32 k = 32 1.99 -> 0.82 ms,
-// k = 8 1.81 -> 0.42 ms; 3D 64^3 FP32 k = 16 3.23 -> 1.09 ms; 3D 44x40x47 FP64
-// k = 8 2.78 -> 1.75 ms.
+// 10.50 -> 5.99 ms, k = 8 3.62 -> 0.85 ms; 3D 40^3 FP32 k = 32 1.99 -> 0.78 ms,
+// k = 8 1.81 -> 0.39 ms; 3D 64^3 FP32 k = 16 3.23 -> 1.09 ms; 3D 44x40x47 FP64
+// k = 8 2.78 -> 1.47 ms.
 #include <algorithm>
 #include <mutex>
 #include <stdexcept>
@@ -314,6 +314,51 @@ __device__ __forceinline__ void fwd_k(const Pass<T>& p, const int* h, const int*
   for (int part = 0; part < (staged ? 1 : 2); ++part) {
     const T* M = part ? Sd : Gd;
     const int first = part ? rows : 0, cnt = staged ? rows + h[5] : part ? h[5] : rows;
+    // A wide supernode's chunk has few rows (300 columns in FP64: seven): K split over
+    // nrg / slots threads a row and vector, their sums added in order.  (With a
+    // thread for all of K one warp of four had the work, FP64 at that: 3D 44x40x47,
+    // k = 8, 1.75 -> 1.47 ms an application, k = 2 1.33 -> 0.81.  The gather of f,
+    // done over by every chunk, costs little beside: once for all chunks, in items
+    // of its own, it gained nothing.)
+    int slots = 1;
+    while (slots < cnt) slots <<= 1;
+    if (2 * slots <= p.nrg) {
+      const int row = p.rg & (slots - 1), sl = p.rg / slots, ns = p.nrg / slots;
+      Vt acc[NR<T>];
+      int off[NR<T>];
+#pragma unroll
+      for (int i = 0; i < NR<T>; ++i) {
+        off[i] = -1;
+        acc[i] = vzero(T(0));
+      }
+      if (row < cnt) off[0] = row * ldk;
+      for (int j0 = 0; j0 < n; j0 += ft) {
+        const int jn = min(ft, n - j0), jp = (jn + V - 1) / V * V;
+        const int per = ((jp / V + ns - 1) / ns) * V, ka = min(jp, sl * per), kb = min(jp, ka + per);
+        if (j0 > 0 || part > 0) cbar();
+        gather_f<T>(p, c0, j0, jn, has ? d2 : nullptr, ent2, p.rg, p.nrg, F);
+        cbar();
+        rows_dot<T, true>(M, off, j0 + ka, kb - ka, F + ka * p.cgN + p.cg, p.cgN, acc);
+      }
+      cbar();
+      F[p.rg * p.cgN + p.cg] = acc[0];
+      cbar();
+      if (p.rg < cnt) {
+        Vt v = F[row * p.cgN + p.cg], u[1] = {vzero(T(0))};
+        for (int q = 1; q < ns; ++q) vadd(v, F[(q * slots + row) * p.cgN + p.cg]);
+        const int r = first + row;
+        int b[1] = {has && r < rows ? ps[r] : 0};
+        const int e[1] = {has && r < rows ? ps[r + 1] : 0};
+        pulls<T, 1>(p, u, ent, b, e);
+        if (r < rows) {
+          vsub(u[0], v);
+          p.st(p.A->wu, h[3] + r, u[0]);
+        } else {
+          p.st(p.A->t, h[8] + h[4] + r - rows, v);
+        }
+      }
+      continue;
+    }
     for (int r0 = 0; r0 < cnt; r0 += NR<T> * p.nrg) {   // one sweep for the chunk heights in use
       Vt acc[NR<T>];
       int off[NR<T>];
