@@ -243,6 +243,8 @@ int rschol_selftest_gemm(int M, int N, int K, int tA, int tB, int split, int low
 /* Diagnostics: the FP64 GEMM kernel, split into `slices` along K, against a host
  * product: out[0] = largest error relative to sum_k |a b| + |beta c|. */
 int rschol_selftest_gemm64(int M, int N, int K, int tA, int tB, int slices, double* out);
+/* The same for the FP32 SIMT kernels, with tiles of 64 or 128 rows. */
+int rschol_selftest_gemm32(int M, int N, int K, int tA, int tB, int rows, double* out);
 /* Diagnostics: thin Householder QR of `tasks` random n x r matrices (column r / 2
  * zero): out[0] = max |Q^T Q - I|, out[1] = max over columns |y - Q Q^T y| / |y|. */
 int rschol_selftest_qr(int n, int r, int tasks, int fp64, double* out);

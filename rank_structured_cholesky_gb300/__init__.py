@@ -33,6 +33,7 @@ EXPORTED = [
     "rschol_check_structure",
     "rschol_refactor", "rschol_refactor_device", "rschol_stream", "rschol_profile", "rschol_factor_free", "rschol_precond_apply", "rschol_precond_apply_device",
     "rschol_precond_apply_device_noalloc", "rschol_selftest_gemm", "rschol_selftest_gemm64",
+    "rschol_selftest_gemm32",
     "rschol_selftest_qr", "rschol_bench_gemm", "rschol_step_timing", "rschol_pcg",
     "rschol_pcg_device", "rschol_pcg_pysolve", "rschol_factor_n", "rschol_factor_device_bytes", "rschol_factor_num_nodes",
     "rschol_factor_node_info", "rschol_factor_node_l11", "rschol_factor_node_l21", "rschol_factor_perm",
@@ -98,6 +99,7 @@ def load_library():
         "rschol_precond_apply_device_noalloc": (I, [P, P, P, I]),
         "rschol_selftest_gemm": (I, [I, I, I, I, I, I, I, pD]),
         "rschol_selftest_gemm64": (I, [I, I, I, I, I, I, pD]),
+        "rschol_selftest_gemm32": (I, [I, I, I, I, I, I, pD]),
         "rschol_selftest_qr": (I, [I, I, I, I, pD]),
         "rschol_bench_gemm": (I, [I, I, I, I, I, pD]),
         "rschol_step_timing": (I, [P, I, P]),

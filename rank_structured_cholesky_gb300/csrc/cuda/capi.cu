@@ -936,31 +936,33 @@ extern "C" int rschol_selftest_gemm(int M, int N, int K, int tA, int tB, int spl
   return RSCHOL_OK;
 }
 
-// ---- diagnostics: the FP64 GEMM (slices > 1: split along K) against a host product --
-extern "C" int rschol_selftest_gemm64(int M, int N, int K, int tA, int tB, int slices, double* out) {
-  if (M <= 0 || N <= 0 || K <= 0 || slices <= 0 || slices > K || !out) return RSCHOL_E_BAD_INPUT;
+// ---- diagnostics: the SIMT GEMMs against a host product -------------------------
+// FP64: split along K into `slices`; FP32: tiles of `rows` rows
+namespace {
+template <class T>
+int selftest_simt(int M, int N, int K, int tA, int tB, int slices, int rows, double* out) {
   int count = 0;
   if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0) return RSCHOL_E_NO_DEVICE;
   try {
-    std::vector<double> A((size_t)M * K), B((size_t)K * N), C((size_t)M * N), C0((size_t)M * N);
+    std::vector<T> A((size_t)M * K), B((size_t)K * N), C((size_t)M * N), C0((size_t)M * N);
     uint64_t st = 0x9E3779B97F4A7C15ull;
     for (auto* v : {&A, &B, &C0})
       for (auto& x : *v) {
         st = st * 6364136223846793005ull + 1442695040888963407ull;
-        x = (double)(st >> 11) * (1.0 / 9007199254740992.0) * 2.0 - 1.0;
+        x = (T)((double)(st >> 11) * (1.0 / 9007199254740992.0) * 2.0 - 1.0);
       }
     DevBuf dA, dB, dC, dT, dW, dIds, dBase;
-    dA.alloc(sizeof(double) * A.size());
-    dB.alloc(sizeof(double) * B.size());
-    dC.alloc(sizeof(double) * C.size());
-    dT.alloc(sizeof(GemmTask<double>));
-    RSCHOL_CUDA(cudaMemcpy(dA.p, A.data(), sizeof(double) * A.size(), cudaMemcpyHostToDevice));
-    RSCHOL_CUDA(cudaMemcpy(dB.p, B.data(), sizeof(double) * B.size(), cudaMemcpyHostToDevice));
-    RSCHOL_CUDA(cudaMemcpy(dC.p, C0.data(), sizeof(double) * C.size(), cudaMemcpyHostToDevice));
-    GemmTask<double> t{};
-    t.A = dA.as<double>();
-    t.B = dB.as<double>();
-    t.C = dC.as<double>();
+    dA.alloc(sizeof(T) * A.size());
+    dB.alloc(sizeof(T) * B.size());
+    dC.alloc(sizeof(T) * C.size());
+    dT.alloc(sizeof(GemmTask<T>));
+    RSCHOL_CUDA(cudaMemcpy(dA.p, A.data(), sizeof(T) * A.size(), cudaMemcpyHostToDevice));
+    RSCHOL_CUDA(cudaMemcpy(dB.p, B.data(), sizeof(T) * B.size(), cudaMemcpyHostToDevice));
+    RSCHOL_CUDA(cudaMemcpy(dC.p, C0.data(), sizeof(T) * C.size(), cudaMemcpyHostToDevice));
+    GemmTask<T> t{};
+    t.A = dA.as<T>();
+    t.B = dB.as<T>();
+    t.C = dC.as<T>();
     t.M = M;
     t.N = N;
     t.K = K;
@@ -969,16 +971,19 @@ extern "C" int rschol_selftest_gemm64(int M, int N, int K, int tA, int tB, int s
     t.ldc = N;
     t.tA = tA;
     t.tB = tB;
-    t.alpha = -1.25;
-    t.beta = 0.5;
-    t.tilesN = (N + simt_tile<double> - 1) / simt_tile<double>;
+    t.alpha = T(-1.25);
+    t.beta = T(0.5);
+    t.tilesN = (N + simt_tile<T> - 1) / simt_tile<T>;
     t.kLen = (K + slices - 1) / slices;
     t.kSplit = (K + t.kLen - 1) / t.kLen;
-    const int tilesPer = ((M + simt_tile<double> - 1) / simt_tile<double>)*t.tilesN;
-    dW.alloc(sizeof(double) * (size_t)t.kSplit * tilesPer * simt_tile<double> * simt_tile<double>);
+    const int tilesPer = (M + rows - 1) / rows * t.tilesN;
+    dW.alloc(sizeof(T) * (size_t)t.kSplit * tilesPer * rows * simt_tile<T>);
     t.ws = dW.as<float>();
     RSCHOL_CUDA(cudaMemcpy(dT.p, &t, sizeof(t), cudaMemcpyHostToDevice));
-    launch_gemm(dT.as<GemmTask<double>>(), 1, tilesPer * t.kSplit, 0);
+    if constexpr (std::is_same<T, float>::value) {
+      if (rows == 128) launch_gemm_rows128(dT.as<GemmTask<T>>(), 1, tilesPer, 0);
+    }
+    if (rows == simt_tile<T>) launch_gemm(dT.as<GemmTask<T>>(), 1, tilesPer * t.kSplit, 0);
     if (t.kSplit > 1) {
       const int id = 0;
       const long long base[2] = {0, (long long)M * N};
@@ -986,16 +991,16 @@ extern "C" int rschol_selftest_gemm64(int M, int N, int K, int tA, int tB, int s
       dBase.alloc(sizeof(base));
       RSCHOL_CUDA(cudaMemcpy(dIds.p, &id, sizeof(int), cudaMemcpyHostToDevice));
       RSCHOL_CUDA(cudaMemcpy(dBase.p, base, sizeof(base), cudaMemcpyHostToDevice));
-      launch_gemm_splitk_reduce(dT.as<GemmTask<double>>(), dIds.as<int>(), 1, dBase.as<long long>(), base[1], 0);
+      launch_gemm_splitk_reduce(dT.as<GemmTask<T>>(), dIds.as<int>(), 1, dBase.as<long long>(), base[1], 0);
     }
     RSCHOL_CUDA(cudaDeviceSynchronize());
-    RSCHOL_CUDA(cudaMemcpy(C.data(), dC.p, sizeof(double) * C.size(), cudaMemcpyDeviceToHost));
+    RSCHOL_CUDA(cudaMemcpy(C.data(), dC.p, sizeof(T) * C.size(), cudaMemcpyDeviceToHost));
     double worst = 0;
     for (int i = 0; i < M; ++i)
       for (int j = 0; j < N; ++j) {
         double s = 0, mag = 0;
         for (int k = 0; k < K; ++k) {
-          const double p = A[tA ? (size_t)k * M + i : (size_t)i * K + k] * B[tB ? (size_t)j * K + k : (size_t)k * N + j];
+          const double p = (double)A[tA ? (size_t)k * M + i : (size_t)i * K + k] * (double)B[tB ? (size_t)j * K + k : (size_t)k * N + j];
           s += p;
           mag += std::fabs(p);
         }
@@ -1007,6 +1012,15 @@ extern "C" int rschol_selftest_gemm64(int M, int N, int K, int tA, int tB, int s
     return RSCHOL_E_CUDA;
   }
   return RSCHOL_OK;
+}
+}  // namespace
+extern "C" int rschol_selftest_gemm64(int M, int N, int K, int tA, int tB, int slices, double* out) {
+  if (M <= 0 || N <= 0 || K <= 0 || slices <= 0 || slices > K || !out) return RSCHOL_E_BAD_INPUT;
+  return selftest_simt<double>(M, N, K, tA, tB, slices, simt_tile<double>, out);
+}
+extern "C" int rschol_selftest_gemm32(int M, int N, int K, int tA, int tB, int rows, double* out) {
+  if (M <= 0 || N <= 0 || K <= 0 || (rows != 64 && rows != 128) || !out) return RSCHOL_E_BAD_INPUT;
+  return selftest_simt<float>(M, N, K, tA, tB, 1, rows, out);
 }
 
 // ---- diagnostics: the thin Householder QR -------------------------------------

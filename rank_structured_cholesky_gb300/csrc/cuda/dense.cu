@@ -212,6 +212,126 @@ __device__ void gemm_tile_f64(const GemmTask<double>& t, int row0, int col0, int
     }
 }
 
+// FP32, launches of many tiles: 128 x 64 of C a block, 8 x 4 a thread.  What bounds
+// the 64 x 64 tile is its instructions -- eight shared loads for 16 multiply-adds, and
+// the addresses of a tile's loads and C -- (ncu: issue slots 70 % busy, FMA pipe
+// 46 %); this one has three shared loads for 32.  Rows 4 ty + a and 64 + 4 ty + a,
+// columns 2 tx + b and 32 + 2 tx + b; the sums as there, ascending in K.
+// (Updates of rank 32 - 112: 3D 96^3 9.1 -> 7.6 ms a factorisation, 64^3 1.9 -> 1.6.)
+constexpr int G2_ROWS = 128, G2_BK = 16;
+__global__ void __launch_bounds__(GEMM_THREADS, 2) gemm_rows128_kernel(const GemmTask<float>* __restrict__ tasks,
+                                                                       int nTasks) {
+  __shared__ __align__(16) float As[2][G2_BK][132], Bs[2][G2_BK][68];
+  int lo = 0, hi = nTasks - 1;
+  const int bid = blockIdx.x;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (tasks[mid].tileBase <= bid) lo = mid;
+    else hi = mid - 1;
+  }
+  const GemmTask<float> t = tasks[lo];
+  const int local = bid - t.tileBase, ti = local / t.tilesN, tj = local - ti * t.tilesN;
+  const int row0 = ti * G2_ROWS, col0 = tj * 64;
+  if (t.lower && row0 + G2_ROWS - 1 < col0) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = tid & 15, ty = tid >> 4;
+  const bool aK = !t.tA, bK = t.tB != 0;
+  // a thread's elements of a slice: along K a warp takes 4 rows x 8 k (whole sectors), else rows
+  float ra[8], rb[4];
+  auto arow = [&](int q) { return aK ? 4 * ((q * 8 + warp) & 31) + (lane & 3) : tid & 127; };
+  auto ak = [&](int q) { return aK ? 8 * ((q * 8 + warp) >> 5) + (lane >> 2) : (tid >> 7) + 2 * q; };
+  auto brow = [&](int q) { return bK ? 4 * ((q * 8 + warp) & 15) + (lane & 3) : tid & 63; };
+  auto bk = [&](int q) { return bK ? 8 * ((q * 8 + warp) >> 4) + (lane >> 2) : (tid >> 6) + 4 * q; };
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int gi = row0 + arow(q), gk = k0 + ak(q);
+      ra[q] = (gi < t.M && gk < t.K) ? __ldcg(aK ? t.A + (size_t)gi * t.lda + gk : t.A + (size_t)gk * t.lda + gi) : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int gj = col0 + brow(q), gk = k0 + bk(q);
+      rb[q] = (gj < t.N && gk < t.K) ? __ldcg(bK ? t.B + (size_t)gj * t.ldb + gk : t.B + (size_t)gk * t.ldb + gj) : 0.f;
+    }
+  };
+  auto store = [&](int st) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) As[st][ak(q)][arow(q)] = ra[q];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) Bs[st][bk(q)][brow(q)] = rb[q];
+  };
+  float acc[8][4];
+#pragma unroll
+  for (int a = 0; a < 8; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
+  if (t.K > 0) {
+    load(0);
+    store(0);
+  }
+  __syncthreads();
+  int st = 0;
+  for (int k0 = 0; k0 < t.K; k0 += G2_BK) {
+    const bool more = k0 + G2_BK < t.K;
+    if (more) load(k0 + G2_BK);
+#pragma unroll 8
+    for (int k = 0; k < G2_BK; ++k) {   // (zeros beyond K)
+      const float4 a0 = *reinterpret_cast<const float4*>(&As[st][k][4 * ty]);
+      const float4 a1 = *reinterpret_cast<const float4*>(&As[st][k][64 + 4 * ty]);
+      const float2 b0 = *reinterpret_cast<const float2*>(&Bs[st][k][2 * tx]);
+      const float2 b1 = *reinterpret_cast<const float2*>(&Bs[st][k][32 + 2 * tx]);
+      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, bv[4] = {b0.x, b0.y, b1.x, b1.y};
+#pragma unroll
+      for (int a = 0; a < 8; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(av[a], bv[b], acc[a][b]);
+    }
+    if (more) store(st ^ 1);
+    __syncthreads();
+    st ^= 1;
+  }
+  const bool pairs = ((reinterpret_cast<uintptr_t>(t.C) & 7) | (t.ldc & 1)) == 0;   // two columns as one access
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {   // (all C loads of a half before its first use)
+    float c[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; b += 2) {
+        const int gi = row0 + 64 * h + 4 * ty + a, gj = col0 + 16 * b + 2 * tx;
+        const float* p = t.C + (size_t)gi * t.ldc + gj;
+        c[a][b] = c[a][b + 1] = 0.f;
+        if (t.beta == 0.f || gi >= t.M) continue;
+        if (pairs && gj + 1 < t.N) {
+          const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
+          c[a][b] = v.x;
+          c[a][b + 1] = v.y;
+        } else {
+          if (gj < t.N) c[a][b] = __ldcg(p);
+          if (gj + 1 < t.N) c[a][b + 1] = __ldcg(p + 1);
+        }
+      }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; b += 2) {
+        const int gi = row0 + 64 * h + 4 * ty + a, gj = col0 + 16 * b + 2 * tx;
+        if (gi >= t.M) continue;
+        float v0 = t.alpha * acc[4 * h + a][b], v1 = t.alpha * acc[4 * h + a][b + 1];
+        if (t.beta != 0.f) {
+          v0 = fmaf(t.beta, c[a][b], v0);
+          v1 = fmaf(t.beta, c[a][b + 1], v1);
+        }
+        float* p = t.C + (size_t)gi * t.ldc + gj;
+        if (pairs && gj + 1 < t.N) {
+          *reinterpret_cast<float2*>(p) = make_float2(v0, v1);
+        } else {
+          if (gj < t.N) p[0] = v0;
+          if (gj + 1 < t.N) p[1] = v1;
+        }
+      }
+  }
+}
+
 template <class T>
 __global__ void __launch_bounds__(GEMM_THREADS) gemm_kernel(const GemmTask<T>* __restrict__ tasks, int nTasks) {
   int lo = 0, hi = nTasks - 1;
@@ -1899,6 +2019,11 @@ int grid_for(long long n, int threads) {
 template <class T> void launch_gemm(const GemmTask<T>* d, int n, int tiles, cudaStream_t s) {
   if (n <= 0 || tiles <= 0) return;
   gemm_kernel<T><<<tiles, GEMM_THREADS, 0, s>>>(d, n);
+  RSCHOL_LAUNCH_CHECK();
+}
+void launch_gemm_rows128(const GemmTask<float>* d, int n, int tiles, cudaStream_t s) {
+  if (n <= 0 || tiles <= 0) return;
+  gemm_rows128_kernel<<<tiles, GEMM_THREADS, 0, s>>>(d, n);
   RSCHOL_LAUNCH_CHECK();
 }
 void launch_gemm_splitk_reduce(const GemmTask<double>* d, const int* ids, int nIds, const long long* elemBase,

@@ -162,6 +162,8 @@ inline int tc_tile_n(int maxN) { return maxN > 64 ? 128 : 64; }
 // ids[0..nIds) (elemBase: prefix sums of their M x N, elemBase[nIds] = elems).
 void launch_gemm_splitk_reduce(const GemmTask<float>* dTasks, const int* ids, int nIds, const long long* elemBase,
                                long long elems, cudaStream_t s);
+// The FP32 SIMT product in tiles of 128 x 64.
+void launch_gemm_rows128(const GemmTask<float>* dTasks, int nTasks, int totalTiles, cudaStream_t s);
 // The same for FP64 tasks (32 x 32 tiles; ws holds doubles).
 void launch_gemm_splitk_reduce(const GemmTask<double>* dTasks, const int* ids, int nIds, const long long* elemBase,
                                long long elems, cudaStream_t s);

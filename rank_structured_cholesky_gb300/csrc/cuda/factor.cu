@@ -57,6 +57,8 @@ void FactorEngine<float>::gemm_launch(const Step& st) {
   if (st.kind == ST_GEMM_REDUCE)
     launch_gemm_splitk_reduce(dGemm_.as<GemmTask<float>>(), dSplitIds_.as<int>() + st.off, st.count,
                               dSplitBase_.as<long long>() + st.aux, st.elems, stream);
+  else if (st.aux < 0)
+    launch_gemm_rows128(dGemm_.as<GemmTask<float>>() + st.off, st.count, st.grid, stream);
   else if (st.aux)
     launch_gemm_tc(dGemm_.as<GemmTask<float>>() + st.off, st.count, st.grid, dFlag.as<int>() + 1, stream,
                    st.aux & 0xffff, st.aux >> 16);
@@ -97,7 +99,12 @@ void FactorEngine<T>::flush_gemm(std::vector<GemmTask<T>>& batch, int) {
   if (tc && prm.schur_bf16)
     for (auto& t : batch) bf = bf || t.split != 0;
   const int kAlign = bf ? 64 : 32;   // K per pipeline stage: split-K slices start on one
-  const int rowsPerTile = tc ? 128 : simt_tile<T>;
+  // FP32 off the tensor cores: tiles of 128 x 64 where they are several waves of
+  // two blocks an SM and K is more than a slice (else the 64 x 64 ones fill the SMs better)
+  long long big = 0;
+  for (auto& t : batch) big += (long long)((t.M + 127) / 128) * ((t.N + 63) / 64);
+  const bool rows128 = std::is_same<T, float>::value && !tc && maxK > 16 && big >= 8LL * 152;
+  const int rowsPerTile = tc || rows128 ? 128 : simt_tile<T>;
   const int bn = tc ? tc_tile_n(maxN) : simt_tile<T>;   // tile width: 128 x bn on the tensor cores
   long long baseTiles = 0;
   for (auto& t : batch) baseTiles += (long long)((t.M + rowsPerTile - 1) / rowsPerTile) * ((t.N + bn - 1) / bn);
@@ -138,7 +145,8 @@ void FactorEngine<T>::flush_gemm(std::vector<GemmTask<T>>& batch, int) {
   }
   wsCur_ = std::max(wsCur_, wsCur);
   Step st{ST_GEMM, first, (int)batch.size(), tiles};
-  st.aux = tc ? bn | (bf ? 1 << 16 : 0) : 0;   // the tile width, and BF16 splits in bit 16
+  // the tile width on the tensor cores, and BF16 splits in bit 16; -1: SIMT tiles of 128 rows
+  st.aux = tc ? bn | (bf ? 1 << 16 : 0) : rows128 ? -1 : 0;
   gemm_.insert(gemm_.end(), batch.begin(), batch.end());
   steps_.push_back(st);
   if (!ids.empty()) {

@@ -1,5 +1,6 @@
 """The dense kernels at their edges: the FP64 GEMM around its 16-wide blocks and
-32-wide tiles, whole and split along K, and the Householder QR around the row
+32-wide tiles, whole and split along K, the FP32 one around its tiles of 64 and
+128 rows and slices of 16 K, with odd and even leading dimensions, and the Householder QR around the row
 counts where its panel kernel changes (512; 2048, 4096 and 8192 rows of a
 cluster's registers) and its 16-column panels.
 
@@ -24,6 +25,16 @@ def test_gemm_fp64(M, N, K, slices, tA, tB):
     out = (ctypes.c_double * 1)()
     assert rs.load_library().rschol_selftest_gemm64(M, N, K, tA, tB, slices, out) == 0
     assert out[0] <= (K + 4) * 2.0 ** -52
+
+
+@pytest.mark.parametrize("rows", [64, 128])
+@pytest.mark.parametrize("tA,tB", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (63, 65, 15), (64, 64, 16), (127, 63, 17), (128, 64, 31), (129, 130, 33),
+                                   (200, 97, 112), (257, 66, 70)])
+def test_gemm_fp32(M, N, K, tA, tB, rows):
+    out = (ctypes.c_double * 1)()
+    assert rs.load_library().rschol_selftest_gemm32(M, N, K, tA, tB, rows, out) == 0
+    assert out[0] <= (K + 4) * 2.0 ** -23
 
 
 @pytest.mark.parametrize("fp64", [0, 1])
