@@ -184,6 +184,7 @@ struct ApplyArgs {
   int nItems;
   const int* blob;
   int* sync;        // [0] error word, [1] ticket, then the counters
+  int* err;         // the error word (of the first slice of columns)
   T* w;             // permuted vector, in place
   T* t;             // S f of the interior columns
   T* wu;            // update vectors
@@ -201,7 +202,7 @@ template <class T>
 __device__ __forceinline__ void apply_producer(const ApplyArgs<T>& A, unsigned char* apsm, ApplyItem* sItem,
                                                unsigned full0, unsigned empty0) {
   const int lane = threadIdx.x & 31;
-  int* const err = A.sync;
+  int* const err = A.err;
   // Tickets are drawn in pairs (one latency for two items) as far ahead as
   // there are stages -- except in a phase of few items (ApplyItem::shallow),
   // where a CTA that holds more than a group's worth keeps items from idle

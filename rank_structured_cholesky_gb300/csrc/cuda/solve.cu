@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(NGRP * GT + 32, 3) apply_kernel(ApplyArgs<T> A
   __shared__ __align__(8) unsigned long long bars[2 * NSTAGE];
   __shared__ __align__(16) ApplyItem sItem[NSTAGE];
   const int lane = threadIdx.x & 31;
-  int* const err = A.sync;
+  int* const err = A.err;
   if (threadIdx.x == 0) {
     for (int s = 0; s < NSTAGE; ++s) {
       mbar_init(smem_u32(&bars[s]), 1);              // full: the producer's arrival and its bytes
@@ -1733,7 +1733,7 @@ void SolveEngine<T>::apply_inplace(double* w64, cudaStream_t st) {
     RSCHOL_LAUNCH_CHECK();
   }
   int* sync = dSync_.as<int>();
-  const ApplyArgs<T> args{dItems_.as<ApplyItem>(), nItems_,         dBlob_.as<int>(), sync,          w,
+  const ApplyArgs<T> args{dItems_.as<ApplyItem>(), nItems_,         dBlob_.as<int>(), sync,          sync,         w,
                           dT_.as<T>(),             dWu_.as<T>(),    dZp_.as<T>(),     dSp_.as<T>(),  dYp_.as<T>(),
                           dXp_.as<T>(),            dIp_.as<T>(),    work_};
   launch_k(apply_kernel<T>, dim3(grid_), dim3(NGRP * GT + 32), smem_, st, args);

@@ -121,6 +121,7 @@ class SolveEngine {
   // the shapes chosen for each width class so far: (class, blocks per SM, columns per pass, 0, 0, ms) rows
   std::vector<std::array<double, 6>> batch_tuning() const;
   int batch_capacity() const;
+  int batch_slices(int kp) const;   // slices of columns of a batched application
   // bumped whenever the batched apply's buffers are reallocated or its
   // shapes retuned (a graph that captured an apply must then be captured again)
   long long batch_generation() const { return batchGen_; }

@@ -17,9 +17,9 @@
 // dependent loads whatever its bytes), FP64 its 1/64 rate.  Measured, one
 // application against the earlier kernels (a triangular solve with a thread per
 // (row, column) pair, six launches per compressed level): 2D 1024^2 FP32 k = 64
-// 10.50 -> 5.99 ms, k = 8 3.62 -> 0.85 ms; 3D 40^3 FP32 k = 32 1.99 -> 0.78 ms,
-// k = 8 1.81 -> 0.39 ms; 3D 64^3 FP32 k = 16 3.23 -> 1.09 ms; 3D 44x40x47 FP64
-// k = 8 2.78 -> 1.47 ms.
+// 10.50 -> 5.89 ms, k = 8 3.62 -> 0.85 ms; 3D 40^3 FP32 k = 32 1.99 -> 0.67 ms,
+// k = 8 1.81 -> 0.40 ms; 3D 64^3 FP32 k = 16 3.23 -> 1.10 ms; 3D 44x40x47 FP64
+// k = 8 2.78 -> 1.50 ms.
 #include <algorithm>
 #include <mutex>
 #include <stdexcept>
@@ -314,38 +314,46 @@ __device__ __forceinline__ void fwd_k(const Pass<T>& p, const int* h, const int*
   for (int part = 0; part < (staged ? 1 : 2); ++part) {
     const T* M = part ? Sd : Gd;
     const int first = part ? rows : 0, cnt = staged ? rows + h[5] : part ? h[5] : rows;
-    // A wide supernode's chunk has few rows (300 columns in FP64: seven): K split over
-    // nrg / slots threads a row and vector, their sums added in order.  (With a
-    // thread for all of K one warp of four had the work, FP64 at that: 3D 44x40x47,
-    // k = 8, 1.75 -> 1.47 ms an application, k = 2 1.33 -> 0.81.  The gather of f,
-    // done over by every chunk, costs little beside: once for all chunks, in items
-    // of its own, it gained nothing.)
+    // A wide supernode's chunk has few rows (300 columns in FP64: seven): K in GT /
+    // slots slices, over the threads that would have no row -- a pass of fewer
+    // vectors has more of them, so a thread takes one slice, or two or four -- and
+    // the slices' sums added in order: the order of a sum does not depend on the
+    // width of the block.  (With a thread for all of K one warp of four had the
+    // work, FP64 at that: 3D 44x40x47, k = 8, 1.75 -> 1.50 ms an application.  The
+    // gather of f, done over by every chunk, costs little beside: once for all
+    // chunks, in items of its own, it gained nothing.)
     int slots = 1;
     while (slots < cnt) slots <<= 1;
-    if (2 * slots <= p.nrg) {
-      const int row = p.rg & (slots - 1), sl = p.rg / slots, ns = p.nrg / slots;
-      Vt acc[NR<T>];
-      int off[NR<T>];
+    if (slots <= GT / 8) {
+      const int row = p.rg & (slots - 1), sl = p.rg / slots, ns = p.nrg / slots, slices = GT / slots;
+      const int per = ((n + V - 1) / V + slices - 1) / slices * V;
+      Vt acc[4];
 #pragma unroll
-      for (int i = 0; i < NR<T>; ++i) {
-        off[i] = -1;
-        acc[i] = vzero(T(0));
-      }
-      if (row < cnt) off[0] = row * ldk;
+      for (int i = 0; i < 4; ++i) acc[i] = vzero(T(0));
       for (int j0 = 0; j0 < n; j0 += ft) {
         const int jn = min(ft, n - j0), jp = (jn + V - 1) / V * V;
-        const int per = ((jp / V + ns - 1) / ns) * V, ka = min(jp, sl * per), kb = min(jp, ka + per);
         if (j0 > 0 || part > 0) cbar();
         gather_f<T>(p, c0, j0, jn, has ? d2 : nullptr, ent2, p.rg, p.nrg, F);
         cbar();
-        rows_dot<T, true>(M, off, j0 + ka, kb - ka, F + ka * p.cgN + p.cg, p.cgN, acc);
+        if (row < cnt) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {   // slices sl, sl + ns, ... (vectors of the pass: as many)
+            if (i >= p.cgN) break;
+            const int ka = max((sl + i * ns) * per, j0), kb = min((sl + i * ns + 1) * per, j0 + jp);
+#pragma unroll 2
+            for (int k = ka; k < kb; k += V)
+              vstep(acc[i], *reinterpret_cast<const Vt*>(M + row * ldk + k), F + (k - j0) * p.cgN + p.cg, p.cgN);
+          }
+        }
       }
       cbar();
-      F[p.rg * p.cgN + p.cg] = acc[0];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i < p.cgN) F[((sl + i * ns) * slots + row) * p.cgN + p.cg] = acc[i];
       cbar();
       if (p.rg < cnt) {
         Vt v = F[row * p.cgN + p.cg], u[1] = {vzero(T(0))};
-        for (int q = 1; q < ns; ++q) vadd(v, F[(q * slots + row) * p.cgN + p.cg]);
+        for (int q = 1; q < slices; ++q) vadd(v, F[(q * slots + row) * p.cgN + p.cg]);
         const int r = first + row;
         int b[1] = {has && r < rows ? ps[r] : 0};
         const int e[1] = {has && r < rows ? ps[r + 1] : 0};
@@ -463,13 +471,17 @@ __device__ __forceinline__ void split_sum(const Pass<T>& p, int outs, typename V
 }
 
 template <class T>
-__global__ void __launch_bounds__(NGRP * GT + 32, BATCH_BLOCKS) apply_batch_kernel(ApplyArgs<T> A, int kp) {
+__global__ void __launch_bounds__(NGRP * GT + 32, BATCH_BLOCKS) apply_batch_kernel(ApplyArgs<T> A, int kp, int slices, int width,
+                                                                            int syncInts) {
   using Vt = typename Vec16<T>::type;
   constexpr int V = Vec16<T>::V, KC = 4 * V;
   extern __shared__ __align__(128) unsigned char absm[];
+  // a slice of the columns: its own tickets and counters, every slices-th block
+  const int slice = blockIdx.x % slices, colBeg = slice * width, colEnd = min(kp, colBeg + width);
+  A.sync += slice * syncInts;
   __shared__ __align__(8) unsigned long long bars[2 * NSTAGE];
   __shared__ __align__(16) ApplyItem sItem[NSTAGE];
-  int* const err = A.sync;
+  int* const err = A.err;
   if (threadIdx.x == 0) {
     for (int s = 0; s < NSTAGE; ++s) {
       mbar_init(smem_u32(&bars[s]), 1);
@@ -478,8 +490,10 @@ __global__ void __launch_bounds__(NGRP * GT + 32, BATCH_BLOCKS) apply_batch_kern
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (threadIdx.x >= NGRP * GT) {
     apply_producer<T>(A, absm, sItem, smem_u32(&bars[0]), smem_u32(&bars[NSTAGE]));
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     return;
   }
   const int grp = threadIdx.x / GT, tid = threadIdx.x % GT, warp = tid >> 5;
@@ -502,19 +516,19 @@ __global__ void __launch_bounds__(NGRP * GT + 32, BATCH_BLOCKS) apply_batch_kern
     cbar();
     const T* g0 = it.bytes0 ? data : reinterpret_cast<const T*>(it.g0);
     const T* g1 = it.bytes1 ? data + it.bytes0 / sizeof(T) : reinterpret_cast<const T*>(it.g1);
-    for (int col0 = 0; col0 < kp; col0 += KC) {
+    for (int col0 = colBeg; col0 < colEnd; col0 += KC) {
       Pass<T> p;
       p.A = &A;
       p.kp = kp;
-      const int rem = (kp - col0) / V;
+      const int rem = (colEnd - col0) / V;
       p.cgN = rem >= 3 ? 4 : rem;
       p.tid = tid;
       p.cg = tid % p.cgN;
       p.rg = tid / p.cgN;
       p.nrg = GT / p.cgN;
       p.col = col0 + p.cg * V;
-      p.act = p.col < kp;
-      if (col0 > 0) cbar();   // the buffers of the last pass
+      p.act = p.col < colEnd;
+      if (col0 > colBeg) cbar();   // the buffers of the last pass
       switch (kind) {
         case IT_FGRP: fgrp_k<T>(p, h, d, it.count, data, F); break;
         case IT_BGRP: bgrp_k<T>(p, h, d, it.count, data, F); break;
@@ -713,6 +727,7 @@ __global__ void __launch_bounds__(NGRP * GT + 32, BATCH_BLOCKS) apply_batch_kern
 template <class T>
 __global__ void __launch_bounds__(256) widen_kernel(const double* __restrict__ src, T* __restrict__ dst, long long n,
                                                     int k, int kp) {
+  pdl_enter();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n * kp; i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / kp;
     const int c = (int)(i - r * kp);
@@ -725,6 +740,7 @@ __global__ void __launch_bounds__(256) widen_kernel(const double* __restrict__ s
 template <class T>
 __global__ void __launch_bounds__(256) narrow_kernel(const T* __restrict__ src, double* __restrict__ dst, long long n,
                                                      int k, int kp, int* __restrict__ clr, int nClr) {
+  pdl_enter();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n * k; i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / k;
     const int c = (int)(i - r * k);
@@ -738,6 +754,21 @@ __global__ void __launch_bounds__(256) narrow_kernel(const T* __restrict__ src, 
 template <class T>
 int SolveEngine<T>::batch_capacity() const {
   return 64;
+}
+
+// Slices of columns that walk the items by themselves, beside each other: a pass over
+// an item is a chain of loads (FP64: of multiply-adds, 64 clocks a warp), so passes
+// one after the other leave most of the chip waiting.  Slices of a whole pass (four
+// vectors); of two or one where the items are so few that the blocks outnumber
+// them.  One application at one / two / four vectors a slice / all in turn: FP64 2D
+// 75x70 (336 items) k = 16 240 / 264 / 352 / 618 us, 110x100 (735) k = 64 579 / 433 / 417 /
+// 2382, 193x187 (2938) k = 16 775 / 618 / 600 / 972; FP32 2D 193x187 (1345) k = 64 407 /
+// 313 / 339 / 886, 3D 40x38x40 (14050) k = 64 2833 / 1601 / 1049 / 1532.
+template <class T>
+int SolveEngine<T>::batch_slices(int kp) const {
+  const long long nv = std::max(1, (kp + Vec16<T>::V - 1) / Vec16<T>::V), passes = nv * nItems_;
+  const int w = passes <= 8000 ? 1 : passes <= 24000 ? 2 : 4;
+  return (int)((nv + w - 1) / w);
 }
 
 // Buffers for blocks of kp columns; they only grow, so a changing width frees
@@ -756,8 +787,11 @@ void SolveEngine<T>::plan_batch(int kp) {
   widen(dIpB_, dIp_);
   dWB_.alloc(sizeof(T) * (size_t)std::max(1, F_.S.n) * kp);   // the working copy of W
   if (!dSyncB_.p) {
-    dSyncB_.alloc(sizeof(int) * nSync_);
-    RSCHOL_CUDA(cudaMemsetAsync(dSyncB_.p, 0, sizeof(int) * nSync_, st));
+    int slices = 1;
+    for (int c = 1; c <= batch_capacity(); ++c) slices = std::max(slices, batch_slices(c));
+    const size_t bytes = sizeof(int) * nSync_ * (size_t)slices;
+    dSyncB_.alloc(bytes);
+    RSCHOL_CUDA(cudaMemsetAsync(dSyncB_.p, 0, bytes, st));
   }
   kAllocB_ = kp;
   ++batchGen_;
@@ -849,15 +883,17 @@ void SolveEngine<T>::apply_batch_cfg(double* W64, int k, cudaStream_t st, const 
   const long long n = F_.S.n;
   T* w = dWB_.as<T>();
   const unsigned grid = (unsigned)std::min<long long>((n * kp + 255) / 256, 4096);
-  widen_kernel<T><<<grid, 256, 0, st>>>(W64, w, n, k, kp);
+  launch_k(widen_kernel<T>, dim3(grid), dim3(256), 0, st, (const double*)W64, w, n, k, kp);
   RSCHOL_LAUNCH_CHECK();
   int* sync = dSyncB_.as<int>();
-  const ApplyArgs<T> args{dItems_.as<ApplyItem>(), nItems_,         dBlob_.as<int>(), sync,           w,
+  const ApplyArgs<T> args{dItems_.as<ApplyItem>(), nItems_,         dBlob_.as<int>(), sync,           sync,          w,
                           dTB_.as<T>(),            dWuB_.as<T>(),   dZpB_.as<T>(),    dSpB_.as<T>(),  dYpB_.as<T>(),
                           dXpB_.as<T>(),           dIpB_.as<T>(),   0};
-  apply_batch_kernel<T><<<std::min(std::max(1, nItems_), sms_ * cfg.blocks), NGRP * GT + 32, smem, st>>>(args, kp);
+  const int slices = batch_slices(kp), width = ((kp / V + slices - 1) / slices) * V;
+  const int blocks = (int)std::min<long long>(std::max(1LL, (long long)nItems_ * slices), (long long)sms_ * cfg.blocks);
+  launch_k(apply_batch_kernel<T>, dim3(blocks), dim3(NGRP * GT + 32), smem, st, args, kp, slices, width, nSync_);
   RSCHOL_LAUNCH_CHECK();
-  narrow_kernel<T><<<grid, 256, 0, st>>>(w, W64, n, k, kp, sync + 1, nSync_ - 1);
+  launch_k(narrow_kernel<T>, dim3(grid), dim3(256), 0, st, (const T*)w, W64, n, k, kp, sync + 1, nSync_ * slices - 1);
   RSCHOL_LAUNCH_CHECK();
 }
 
@@ -868,7 +904,7 @@ int SolveEngine<T>::take_error_batch(cudaStream_t st) {
   RSCHOL_CUDA(cudaMemcpyAsync(&e, dSyncB_.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   RSCHOL_CUDA(cudaStreamSynchronize(st));
   if (e) {
-    RSCHOL_CUDA(cudaMemsetAsync(dSyncB_.p, 0, sizeof(int) * nSync_, st));
+    RSCHOL_CUDA(cudaMemsetAsync(dSyncB_.p, 0, dSyncB_.bytes, st));
     RSCHOL_CUDA(cudaStreamSynchronize(st));
   }
   return e;
@@ -876,6 +912,7 @@ int SolveEngine<T>::take_error_batch(cudaStream_t st) {
 
 #define RSCHOL_INST(T)                                                                               \
   template int SolveEngine<T>::batch_capacity() const;                                               \
+  template int SolveEngine<T>::batch_slices(int) const;                                              \
   template void SolveEngine<T>::plan_batch(int);                                                     \
   template const SolveEngine<T>::BatchCfg& SolveEngine<T>::config_for(int, cudaStream_t, bool);      \
   template int SolveEngine<T>::width_class(int) const;                                               \

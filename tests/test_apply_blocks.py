@@ -31,6 +31,7 @@ def test_block_is_the_direct_solve(k, precision):
     err = np.linalg.norm(x - want, axis=1) / np.linalg.norm(want, axis=1)
     assert err.max() <= tol
     assert np.array_equal(x, F.apply(b))
+    assert np.array_equal(x[:2], F.apply(b[:2]))   # a column's sums do not depend on the block's width
 
 
 @pytest.mark.parametrize("n,width", [(50, 3), (700, 12), (700, 13), (5000, 40), (90000, 20)])
