@@ -884,18 +884,18 @@ void SolveEngine<T>::plan() {
   clk.mark("layout");
   cudaStream_t st = F_.stream;
   auto up = [&](DevBuf& b, const void* src, size_t bytes) {
-    b.alloc(std::max<size_t>(bytes, 16));
+    b.alloc(bytes);
     if (bytes) RSCHOL_CUDA(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, st));
   };
   dDinv_.alloc(sizeof(T) * std::max(1LL, dinvCur));
   dT_.alloc(sizeof(T) * std::max(8LL, tCur));
-  dX_.alloc(sizeof(T) * std::max(1LL, xCur));
-  RSCHOL_CUDA(cudaMemsetAsync(dX_.p, 0, sizeof(T) * std::max(1LL, xCur), st));   // upper triangles and padding stay zero
+  dX_.alloc(sizeof(T) * xCur);   // (what a factor does not have is not allocated)
+  if (xCur > 0) RSCHOL_CUDA(cudaMemsetAsync(dX_.p, 0, sizeof(T) * xCur, st));   // upper triangles and padding stay zero
   dG_.alloc(sizeof(T) * std::max(1LL, gCur));
   dS_.alloc(sizeof(T) * std::max(1LL, sCur));
   RSCHOL_CUDA(cudaMemsetAsync(dG_.p, 0, dG_.bytes, st));   // the row padding stays zero
   RSCHOL_CUDA(cudaMemsetAsync(dS_.p, 0, dS_.bytes, st));
-  dWc_.alloc(sizeof(T) * std::max(4LL, wCur));
+  dWc_.alloc(sizeof(T) * wCur);
   for (size_t q = 0; q < dinvTasks.size(); ++q)
     dinvTasks[q].D = xTaskOff[q] >= 0 ? dX_.as<T>() + xTaskOff[q] : dDinv_.as<T>() + dinvTaskOff[q];
   for (int s = 0; s < nn; ++s) {
@@ -1519,23 +1519,23 @@ void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<l
   for (size_t q = 0; q < items.size(); ++q) items[q].shallow = count[phaseOf[q]] <= SHALLOW * NGRP * grid_;
   nSync_ = nCtr;
   auto upload = [&](DevBuf& b, const void* src, size_t bytes) {
-    b.alloc(std::max<size_t>(bytes, 16));
+    b.alloc(bytes);
     if (bytes) RSCHOL_CUDA(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, st));
   };
   nPacks_ = (int)packs.size();
   upload(dPackTiles_, packs.data(), packs.size() * sizeof(PackTile));
-  dPacked_.alloc(std::max<size_t>(16, packs.size() * (size_t)ST_DATA));
+  dPacked_.alloc(packs.size() * (size_t)ST_DATA);
   for (size_t q = 0; q < packItems.size(); ++q)
     items[packItems[q]].g0 = dPacked_.as<unsigned char>() + q * (size_t)ST_DATA;
   upload(dItems_, items.data(), items.size() * sizeof(ApplyItem));
   upload(dBlob_, blob.data(), blob.size() * sizeof(int));
   dSync_.alloc(sizeof(int) * nCtr);
   RSCHOL_CUDA(cudaMemsetAsync(dSync_.p, 0, sizeof(int) * nCtr, st));
-  dZp_.alloc(sizeof(T) * std::max(4LL, zpCur));
-  dSp_.alloc(sizeof(T) * std::max(4LL, spCur));
-  dYp_.alloc(sizeof(T) * std::max(1LL, ypCur));
-  dXp_.alloc(sizeof(T) * std::max(1LL, xpCur));
-  dIp_.alloc(sizeof(T) * std::max(1LL, ipCur));
+  dZp_.alloc(sizeof(T) * zpCur);
+  dSp_.alloc(sizeof(T) * spCur);
+  dYp_.alloc(sizeof(T) * ypCur);
+  dXp_.alloc(sizeof(T) * xpCur);
+  dIp_.alloc(sizeof(T) * ipCur);
   RSCHOL_CUDA(cudaStreamSynchronize(st));   // the host arrays go out of scope
 }
 
