@@ -1058,8 +1058,8 @@ __global__ void __launch_bounds__(256) trsm_inv_kernel(const TrsmTask<T>* __rest
 // What bounds it is the chain POTRF(p) -> TRSM(p + 1, p) -> POTRF(p + 1); as one
 // item a tile and panel (right-looking) it was 36 us a panel, 22 of them the tile's
 // factor and inverse, 5 the three hand-overs; now it is 23, and the updates read
-// and write their tiles once (Cholesky steps of a factorisation: 3D 64^3 10.3 -> 8.1
-// ms, 96^3 49.2 -> 36.8 ms, elasticity 30^3 6.3 -> 4.9 ms).
+// and write their tiles once (Cholesky steps of a factorisation: 3D 64^3 10.3 -> 7.8
+// ms, 96^3 49.2 -> 36.0 ms, elasticity 30^3 6.3 -> 4.7 ms).
 // sync[0] is the ticket, the counters follow (zeroed before every launch);
 // a wait that gives up sets flag[1].  Data written by other blocks is read
 // through L2 (ld.global.cg).
