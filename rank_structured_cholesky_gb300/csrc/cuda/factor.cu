@@ -108,7 +108,22 @@ void FactorEngine<T>::flush_gemm(std::vector<GemmTask<T>>& batch, int) {
   const int bn = tc ? tc_tile_n(maxN) : simt_tile<T>;   // tile width: 128 x bn on the tensor cores
   long long baseTiles = 0;
   for (auto& t : batch) baseTiles += (long long)((t.M + rowsPerTile - 1) / rowsPerTile) * ((t.N + bn - 1) / bn);
-  const long long want = 2LL * 152;   // two blocks per SM
+  // tensor cores, one block an SM: the number of K slices with the least waves times
+  // a wave's length -- a slice's K, a block's start and end (worth about 256 of K) and
+  // the same again for storing and adding partials.  (Against two blocks' worth of
+  // tiles an SM, K from 256: GEMM steps of 3D 64^3 5.0 -> 4.6 ms, elasticity 30^3 2.1 ->
+  // 1.8, 96^3 29.1 -> 27.9; 128 or 512 in place of 256 within 1 %.)
+  int tcSlices = 1;
+  if (tc && baseTiles > 0) {
+    double best = 1e300;
+    for (int ks = 1; ks <= 16 && (ks == 1 || maxK / ks >= 128); ++ks) {
+      const double cost = (double)((baseTiles * ks + 151) / 152) * ((maxK + ks - 1) / ks + (ks > 1 ? 512 : 256));
+      if (cost < best) {
+        best = cost;
+        tcSlices = ks;
+      }
+    }
+  }
   int tiles = 0;
   long long wsCur = 0;   // (each launch's reduction follows it: all share one workspace)
   std::vector<int> ids;
@@ -125,10 +140,11 @@ void FactorEngine<T>::flush_gemm(std::vector<GemmTask<T>>& batch, int) {
     // FP64: a tile holds its SM's FP64 unit in proportion to K, so the aim is
     // several short ones per SM, for an even last wave (slices of at least 64)
     constexpr bool f64 = std::is_same<T, double>::value;
-    const long long aim = f64 ? 8LL * 152 : want;
+    const long long aim = 8LL * 152;
     const int minK = f64 ? 128 : 256, minSlice = f64 ? 64 : 128;
-    if ((tc || f64) && !t.lower && t.K >= minK && baseTiles < aim) {
-      int ks = (int)std::min<long long>(16, std::min<long long>(t.K / minSlice, (aim + baseTiles - 1) / baseTiles));
+    if ((tc || (f64 && baseTiles < aim)) && !t.lower && t.K >= minK) {
+      int ks = f64 ? (int)std::min<long long>(16, std::min<long long>(t.K / minSlice, (aim + baseTiles - 1) / baseTiles))
+                   : std::min(tcSlices, t.K / minSlice);
       if (ks > 1) {
         const int kl = ((t.K + ks - 1) / ks + kAlign - 1) / kAlign * kAlign;
         t.kSplit = (t.K + kl - 1) / kl;
