@@ -5,6 +5,7 @@
 
 #include "solve.cuh"
 #include "solve_dev.cuh"
+#include "stage_order.h"
 
 namespace rschol {
 namespace solvedev {
@@ -89,8 +90,7 @@ __device__ __forceinline__ void vshfl_add(double2& v, int o) {
 // items in work at once): 3D 64^3 0.400 against 0.494 ms.
 
 constexpr int ST_DATA = 16384, ST_DESC = 3584, ST_BYTES = ST_DATA + ST_DESC;
-constexpr int NSTAGE = 3;
-constexpr int NGRP = 2, GT = 128, GW = GT / 32;   // consumer groups of a CTA, threads and warps of one
+constexpr int GT = 128, GW = GT / 32;   // threads and warps of a consumer group
 constexpr int IW_N = 32, IW_M = 128;     // members of a group item: n <= IW_N, m <= IW_M
 constexpr int GRP = 8;                   // most members of a group
 constexpr int GH = 10;                   // header words of a member
@@ -150,6 +150,12 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
   ok = __shfl_sync(FULL, ok, 0);
   __syncwarp();   // what lane 0 has seen complete, the others may read
   return ok != 0;
+}
+// A consumer's wait for its item k (stage_order.h); bars: the full, then the empty barriers.
+__device__ __forceinline__ bool wait_stage(int k, unsigned bars) {
+  return stage_landed(
+      k, [&](int s, unsigned parity) { return mbar_wait(bars + 8 * s, parity); },
+      [&](int s, unsigned parity) { return mbar_wait(bars + 8 * (NSTAGE + s), parity); });
 }
 // global -> shared, 16-byte aligned addresses and size, completion on bar
 __device__ __forceinline__ void bulk_copy(void* dst, const void* src, int bytes, unsigned bar) {

@@ -445,8 +445,8 @@ __global__ void __launch_bounds__(NGRP * GT + 32, 3) apply_kernel(ApplyArgs<T> A
   T* const zs = red + GT * Vec16<T>::V;                                           // GT vectors
   T* const f = zs + GT * Vec16<T>::V;                                             // the widest chunk item's columns
   for (int k = grp;; k += NGRP) {
-    const int s = k % NSTAGE, use = k / NSTAGE;
-    if (!mbar_wait(smem_u32(&bars[s]), use & 1)) {   // cannot happen while the producer runs
+    const int s = k % NSTAGE;
+    if (!wait_stage(k, smem_u32(&bars[0]))) {   // cannot happen while the producer runs
       if (tid == 0) atomicExch(err, 3);
       break;
     }

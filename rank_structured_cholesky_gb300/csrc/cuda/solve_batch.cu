@@ -499,8 +499,8 @@ __global__ void __launch_bounds__(NGRP * GT + 32, BATCH_BLOCKS) apply_batch_kern
   const int grp = threadIdx.x / GT, tid = threadIdx.x % GT, warp = tid >> 5;
   Vt* const F = reinterpret_cast<Vt*>(absm + NSTAGE * ST_BYTES + grp * FB);
   for (int k = grp;; k += NGRP) {
-    const int s = k % NSTAGE, use = k / NSTAGE;
-    if (!mbar_wait(smem_u32(&bars[s]), use & 1)) {   // cannot happen while the producer runs
+    const int s = k % NSTAGE;
+    if (!wait_stage(k, smem_u32(&bars[0]))) {   // cannot happen while the producer runs
       if (tid == 0) atomicExch(err, 3);
       break;
     }
