@@ -1506,8 +1506,10 @@ void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<l
   // and the f buffer (or a group item's buffers in their place)
   work_ = (std::max(GW * (IW_N + IW_M), 2 * GT * Vec16<T>::V + fLen_) + 3) & ~3;
   smem_ = (size_t)NSTAGE * ST_BYTES + NGRP * sizeof(T) * (size_t)work_;
-  if (smem_ > 226 * 1024) throw std::runtime_error("interior front too large for the shared-memory solve");
-  RSCHOL_CUDA(cudaFuncSetAttribute(apply_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_));
+  // the limit belongs to the kernel, not to this factor: one value for all of them
+  constexpr int maxSmem = 226 * 1024;
+  if (smem_ > maxSmem) throw std::runtime_error("interior front too large for the shared-memory solve");
+  RSCHOL_CUDA(cudaFuncSetAttribute(apply_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxSmem));
   int dev = 0, per = 0;
   RSCHOL_CUDA(cudaGetDevice(&dev));
   RSCHOL_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
