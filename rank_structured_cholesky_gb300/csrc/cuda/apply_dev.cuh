@@ -96,6 +96,9 @@ constexpr int GRP = 8;                   // most members of a group
 constexpr int GH = 10;                   // header words of a member
 constexpr int SHALLOW = 1;               // phases of up to this many items a group (in all CTAs) draw tickets singly
 constexpr int ROWS8 = 8 * GW;            // most rows of W or V in an item (eight a warp)
+// columns of f that a chunk item of the single-vector apply holds at a time: three
+// CTAs an SM then fit whatever the widest supernode is
+template <class T> constexpr int F_TILE = 4096 / (int)sizeof(T);
 
 enum ItemKind : int { IT_FGRP = 0, IT_FWD, IT_CF, IT_CU, IT_Y, IT_XT, IT_CS, IT_CX, IT_BGRP, IT_BWD, IT_CR, IT_BR, IT_END };
 

@@ -241,47 +241,61 @@ __device__ __forceinline__ void item_fwd(const ApplyArgs<T>& A, const int* h, co
   const int* ps = d + h[6];
   const int* ent = ps + rows + 1;
   const int* ent2 = d2 + n + 1;
-  for (int t0 = 0; t0 < nv * V; t0 += 2 * GT) {   // two columns and (first pass) one row a thread
-    T v[3];
-    int b[3], e[3];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int t = t0 + tid + i * GT;
-      v[i] = t < n ? __ldcg(A.w + c0 + t) : T(0);
-      b[i] = pull && t < n ? d2[t] : 0;
-      e[i] = pull && t < n ? d2[t + 1] : 0;
-    }
-    const bool in = t0 == 0 && tid < rows;
-    v[2] = T(0);
-    b[2] = pull && in ? ps[tid] : 0;
-    e[2] = pull && in ? ps[tid + 1] : 0;
-    if (pull) {
-      const int* const lists[3] = {ent2, ent2, ent};
-      pull_sums(v, lists, b, e, A.wu);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-      if (t0 + tid + i * GT < nv * V) f[t0 + tid + i * GT] = v[i];
-    if (in) ub[tid] = v[2];
-  }
-  cbar();
   const Vt* fs = reinterpret_cast<const Vt*>(f);
   const int R = rows + h[5];   // rows of G, then the chunk's rows of S
   int lt = 1;                  // threads of a row: 2^lt
   while (lt < 5 && R << (lt + 1) <= GT) ++lt;
   const int sub = tid & ((1 << lt) - 1);
-  for (int r0 = 0; r0 < R; r0 += GT >> lt) {
-    const int row = r0 + (tid >> lt);
-    T v = T(0);
-    if (row < R) {
-      const Vt* m = reinterpret_cast<const Vt*>(row < rows ? Gd : Sd) + (size_t)(row < rows ? row : row - rows) * nv;
-#pragma unroll 4
-      for (int c = sub; c < nv; c += 1 << lt) v = vdot(m[c], fs[c], v);
+  // f in tiles (a supernode of several is read in place, at most 32 rows an item: one
+  // sweep of them, its sums kept in acc); a thread's order along a row is that of one tile
+  T acc = T(0);
+  for (int j0 = 0; j0 < nv * V; j0 += F_TILE<T>) {
+    const int jn = min(F_TILE<T>, nv * V - j0);
+    if (j0 > 0) cbar();   // every thread is done with the last tile
+    for (int t0 = 0; t0 < jn; t0 += 2 * GT) {   // two columns and (first pass) one row a thread
+      T v[3];
+      int b[3], e[3];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int t = j0 + t0 + tid + i * GT;
+        const bool in = t0 + tid + i * GT < jn && t < n;
+        v[i] = in ? __ldcg(A.w + c0 + t) : T(0);
+        b[i] = pull && in ? d2[t] : 0;
+        e[i] = pull && in ? d2[t + 1] : 0;
+      }
+      const bool in = j0 == 0 && t0 == 0 && tid < rows;
+      v[2] = T(0);
+      b[2] = pull && in ? ps[tid] : 0;
+      e[2] = pull && in ? ps[tid + 1] : 0;
+      if (pull) {
+        const int* const lists[3] = {ent2, ent2, ent};
+        pull_sums(v, lists, b, e, A.wu);
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (t0 + tid + i * GT < jn) f[t0 + tid + i * GT] = v[i];
+      if (in) ub[tid] = v[2];
     }
-    for (int o = 1; o < (1 << lt); o <<= 1) v += __shfl_xor_sync(FULL, v, o);
-    if (sub == 0 && row < R) {
-      if (row < rows) A.wu[h[3] + row] = ub[row] - v;
-      else A.t[h[8] + h[4] + row - rows] = v;
+    cbar();
+    const bool last = j0 + jn >= nv * V;
+    for (int r0 = 0; r0 < R; r0 += GT >> lt) {
+      const int row = r0 + (tid >> lt);
+      T v = acc;
+      if (row < R) {
+        const Vt* m =
+            reinterpret_cast<const Vt*>(row < rows ? Gd : Sd) + (size_t)(row < rows ? row : row - rows) * nv + j0 / V;
+#pragma unroll 4
+        for (int c = sub; c < jn / V; c += 1 << lt) v = vdot(m[c], fs[c], v);
+      }
+      if (!last) {
+        acc = v;
+        continue;
+      }
+      for (int o = 1; o < (1 << lt); o <<= 1) v += __shfl_xor_sync(FULL, v, o);
+      if (sub == 0 && row < R) {
+        if (row < rows) A.wu[h[3] + row] = ub[row] - v;
+        else A.t[h[8] + h[4] + row - rows] = v;
+      }
     }
   }
   if (h[9]) {   // chunks of whole sectors: the last ones to their ends
@@ -1504,11 +1518,12 @@ void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<l
   nItems_ = (int)items.size();
   // shared memory: the stages, and per consumer group two areas of GT vectors
   // and the f buffer (or a group item's buffers in their place)
-  work_ = (std::max(GW * (IW_N + IW_M), 2 * GT * Vec16<T>::V + fLen_) + 3) & ~3;
+  work_ = (std::max(GW * (IW_N + IW_M), 2 * GT * Vec16<T>::V + std::min(fLen_, F_TILE<T>)) + 3) & ~3;
   smem_ = (size_t)NSTAGE * ST_BYTES + NGRP * sizeof(T) * (size_t)work_;
-  // the limit belongs to the kernel, not to this factor: one value for all of them
-  constexpr int maxSmem = 226 * 1024;
-  if (smem_ > maxSmem) throw std::runtime_error("interior front too large for the shared-memory solve");
+  // the limit belongs to the kernel, not to this factor: what the widest supernode needs
+  constexpr int maxWork = std::max(GW * (IW_N + IW_M), 2 * GT * Vec16<T>::V + F_TILE<T>);
+  constexpr int maxSmem = NSTAGE * ST_BYTES + NGRP * (int)sizeof(T) * maxWork;
+  static_assert(3 * (maxSmem + 1536) <= 228 * 1024, "three CTAs an SM");   // (static and reserved shared memory beside)
   RSCHOL_CUDA(cudaFuncSetAttribute(apply_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxSmem));
   int dev = 0, per = 0;
   RSCHOL_CUDA(cudaGetDevice(&dev));
