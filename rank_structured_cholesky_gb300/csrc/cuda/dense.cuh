@@ -130,6 +130,7 @@ struct ExtAddRow {
 // SM -- so a 64 x 64 x 64 product holds its SM for 64 us and leaves the others
 // idle wherever a launch has few of them: FP64 tiles are 32 wide.
 template <class T> constexpr int simt_tile = std::is_same<T, double>::value ? 32 : 64;
+template <class T> constexpr int simt_rows = std::is_same<T, double>::value ? 32 : 128;   // of the tallest tile
 template <class T> constexpr int chol_nb = std::is_same<T, double>::value ? 32 : 64;
 
 template <class T> void launch_gemm(const GemmTask<T>* dTasks, int nTasks, int totalTiles, cudaStream_t s);
@@ -162,7 +163,11 @@ inline int tc_tile_n(int maxN) { return maxN > 64 ? 128 : 64; }
 // ids[0..nIds) (elemBase: prefix sums of their M x N, elemBase[nIds] = elems).
 void launch_gemm_splitk_reduce(const GemmTask<float>* dTasks, const int* ids, int nIds, const long long* elemBase,
                                long long elems, cudaStream_t s);
-// The FP32 SIMT product in tiles of 128 x 64.
+// The FP32 SIMT product in tiles of 128 x 64: where these (tiles of them) are several
+// waves of two blocks an SM and K is more than a slice; else 64 x 64 fills the SMs better.
+template <class T> bool simt_rows128(long long tiles, int maxK) {
+  return std::is_same<T, float>::value && maxK > 16 && tiles >= 8LL * 152;
+}
 void launch_gemm_rows128(const GemmTask<float>* dTasks, int nTasks, int totalTiles, cudaStream_t s);
 // The same for FP64 tasks (32 x 32 tiles; ws holds doubles).
 void launch_gemm_splitk_reduce(const GemmTask<double>* dTasks, const int* ids, int nIds, const long long* elemBase,

@@ -99,11 +99,9 @@ void FactorEngine<T>::flush_gemm(std::vector<GemmTask<T>>& batch, int) {
   if (tc && prm.schur_bf16)
     for (auto& t : batch) bf = bf || t.split != 0;
   const int kAlign = bf ? 64 : 32;   // K per pipeline stage: split-K slices start on one
-  // FP32 off the tensor cores: tiles of 128 x 64 where they are several waves of
-  // two blocks an SM and K is more than a slice (else the 64 x 64 ones fill the SMs better)
-  long long big = 0;
+  long long big = 0;   // tiles of 128 x 64
   for (auto& t : batch) big += (long long)((t.M + 127) / 128) * ((t.N + 63) / 64);
-  const bool rows128 = std::is_same<T, float>::value && !tc && maxK > 16 && big >= 8LL * 152;
+  const bool rows128 = !tc && simt_rows128<T>(big, maxK);
   const int rowsPerTile = tc || rows128 ? 128 : simt_tile<T>;
   const int bn = tc ? tc_tile_n(maxN) : simt_tile<T>;   // tile width: 128 x bn on the tensor cores
   long long baseTiles = 0;

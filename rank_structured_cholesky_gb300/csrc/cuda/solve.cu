@@ -1565,8 +1565,12 @@ void SolveEngine<T>::plan_inverse(const std::vector<long long>& xOff) {
   // Both products run by 64-column (64-row) blocks whose K stops at the
   // triangle, so the work is n^3 / 3 per supernode.
   const Symbolic& S = F_.S;
-  const bool tc = std::is_same<T, float>::value && F_.tensor_cores();
-  const int rpt = tc ? 128 : simt_tile<T>;
+  // X of a compressed supernode by split products on the tensor cores; what takes the
+  // place of FP32 sums with the factor itself -- X, S and G of the interior supernodes,
+  // and W -- by FP32 products.  (Those in split TF32 too, 22 bits an operand: the error
+  // of an exact mixed application against 64 bits 1.3e-6 - 6.6e-6 on 3D 12^3 - 32x31x30,
+  // sigma 0; with FP32 products 2.6e-7 - 5.7e-7.)
+  const bool tcX = std::is_same<T, float>::value && F_.tensor_cores();
   const int nn = (int)S.nodes.size();
   int maxN = 0;
   for (int s = 0; s < nn; ++s)
@@ -1602,11 +1606,18 @@ void SolveEngine<T>::plan_inverse(const std::vector<long long>& xOff) {
     t.kLen = K;
     return t;
   };
-  auto flush = [&](std::vector<GemmTask<T>>& batch) {
+  auto flush = [&](std::vector<GemmTask<T>>& batch, bool tc) {
     if (batch.empty()) return;
-    int maxN = 0;
-    for (auto& t : batch) maxN = std::max(maxN, t.N);
-    const int bn = tc ? tc_tile_n(maxN) : simt_tile<T>;
+    int maxN = 0, maxK = 0;
+    long long big = 0;
+    for (auto& t : batch) {
+      maxN = std::max(maxN, t.N);
+      maxK = std::max(maxK, t.K);
+      big += (long long)((t.M + 127) / 128) * ((t.N + 63) / 64);
+    }
+    // (the SIMT tiles of 128 rows where the factor's own launches take them)
+    const bool rows128 = !tc && simt_rows128<T>(big, maxK);
+    const int bn = tc ? tc_tile_n(maxN) : simt_tile<T>, rpt = tc || rows128 ? 128 : simt_tile<T>;
     int tiles = 0;
     for (auto& t : batch) {
       t.tilesN = (t.N + bn - 1) / bn;
@@ -1614,43 +1625,46 @@ void SolveEngine<T>::plan_inverse(const std::vector<long long>& xOff) {
       t.tileBase = tiles;
       tiles += ((t.M + rpt - 1) / rpt) * t.tilesN;
     }
-    XStep xs{(long long)tasks.size(), (int)batch.size(), tiles, tc ? 1 : 0};
+    XStep xs{(long long)tasks.size(), (int)batch.size(), tiles, tc ? XS_TC : rows128 ? XS_ROWS128 : XS_SIMT};
     xs.bn = bn;
     xSteps_.push_back(xs);
     tasks.insert(tasks.end(), batch.begin(), batch.end());
     batch.clear();
   };
   for (int sz = SOLVE_RB; sz < maxN; sz *= 2) {
-    std::vector<GemmTask<T>> b1, b2;
+    std::vector<GemmTask<T>> b1[2], b2[2];   // interior, compressed
     long long t1cur = 0;
     for (int s = 0; s < nn; ++s) {
       if (xOff[s] < 0) continue;
       const int n = S.nodes[s].n, ld = nodes_[s].ld, lx = nodes_[s].ldx;
       const T* L = nodes_[s].L;
       T* X = dX_.as<T>() + xOff[s];
+      const int c = S.nodes[s].compressed;
       for (int A0 = 0; A0 + sz < n; A0 += 2 * sz) {
         const int B0 = A0 + sz, bsz = std::min(sz, n - B0);
         T* T1 = dT1_.as<T>() + t1cur;
         t1cur += (long long)bsz * sz;
         for (int a = 0; a * SOLVE_RB < sz; ++a)   // T1[:, a] = L_BA[:, a:] X_AA[a:, a]
-          b1.push_back(mk(L + (size_t)B0 * ld + A0 + a * SOLVE_RB, ld,
+          b1[c].push_back(mk(L + (size_t)B0 * ld + A0 + a * SOLVE_RB, ld,
                           X + (size_t)(A0 + a * SOLVE_RB) * lx + A0 + a * SOLVE_RB, lx, T1 + a * SOLVE_RB, sz, bsz,
                           SOLVE_RB, sz - a * SOLVE_RB, T(1)));
         for (int b = 0; b * SOLVE_RB < bsz; ++b) {   // X_BA[b, :] = -X_BB[b, :b] T1[:b, :]
           const int hb = std::min(SOLVE_RB, bsz - b * SOLVE_RB), K = std::min(bsz, (b + 1) * SOLVE_RB);
-          b2.push_back(mk(X + (size_t)(B0 + b * SOLVE_RB) * lx + B0, lx, T1, sz,
+          b2[c].push_back(mk(X + (size_t)(B0 + b * SOLVE_RB) * lx + B0, lx, T1, sz,
                           X + (size_t)(B0 + b * SOLVE_RB) * lx + A0, lx, hb, sz, K, T(-1)));
         }
       }
     }
-    flush(b1);
-    flush(b2);
+    for (auto* b : {b1, b2}) {
+      flush(b[0], false);
+      flush(b[1], tcX);
+    }
   }
   // then the products the apply reads: W = X^T U of the compressed supernodes,
   // S = X^T X and G = L21 X of the interior ones of more than 64 columns, by
   // blocks whose K starts at the triangle
   std::vector<GemmTask<T>> bw, bi;
-  const int blk = rpt;
+  constexpr int blk = simt_rows<T>;
   for (int s = 0; s < nn; ++s) {
     const SNode<T>& sn = nodes_[s];
     const int n = sn.n, lx = sn.ldx;
@@ -1674,8 +1688,8 @@ void SolveEngine<T>::plan_inverse(const std::vector<long long>& xOff) {
       }
     }
   }
-  flush(bw);
-  flush(bi);
+  flush(bw, false);
+  flush(bi, false);
   dXGemm_.alloc(std::max<size_t>(16, tasks.size() * sizeof(GemmTask<T>)));
   if (!tasks.empty())
     RSCHOL_CUDA(cudaMemcpyAsync(dXGemm_.p, tasks.data(), tasks.size() * sizeof(GemmTask<T>), cudaMemcpyHostToDevice,
@@ -1711,7 +1725,8 @@ int SolveEngine<T>::prepare(cudaStream_t st) {
   for (const XStep& x : xSteps_) {
     const GemmTask<T>* d = dXGemm_.as<GemmTask<T>>() + x.off;
     if constexpr (std::is_same<T, float>::value) {
-      if (F_.tensor_cores()) launch_gemm_tc(d, x.count, x.tiles, F_.dFlag.template as<int>() + 1, st, x.bn);
+      if (x.kind == XS_TC) launch_gemm_tc(d, x.count, x.tiles, F_.dFlag.template as<int>() + 1, st, x.bn);
+      else if (x.kind == XS_ROWS128) launch_gemm_rows128(d, x.count, x.tiles, st);
       else launch_gemm<T>(d, x.count, x.tiles, st);
     } else {
       launch_gemm<T>(d, x.count, x.tiles, st);

@@ -91,10 +91,11 @@ struct DinvTask {    // invert one lower-triangular diagonal block (h x h, h <= 
   T* D;
 };
 
+enum { XS_SIMT = 0, XS_ROWS128, XS_TC };   // SIMT in square tiles or in tiles of 128 x 64, tensor cores
 struct XStep {       // one batched GEMM launch (X = L11^{-1} doubling, W, S and G)
   long long off;
   int count, tiles;
-  int tc;            // on the tensor cores
+  int kind;
   int bn = 64;       // tensor-core tile width of the launch
 };
 
