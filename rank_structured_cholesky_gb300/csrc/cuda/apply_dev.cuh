@@ -80,8 +80,8 @@ __device__ __forceinline__ void vshfl_add(double2& v, int o) {
 // launch needs no host state and replays inside a CUDA graph.
 //
 // Bound: a chain of hand-overs (release, poll, gather, product: ~3 us each, one
-// or two a tree level and direction), then the factor's bytes.  The triangles X
-// and the products with S lie off that chain and fill its gaps.  Measured, one
+// or two a tree level and direction), then the factor's bytes.  The products with X
+// lie off that chain and fill its gaps.  Measured, one
 // application (before: a triangular solve per supernode on the chain, two
 // ticketed launches for the interior and eight launches per compressed level):
 // 3D 64^3 FP32 0.914 -> 0.376 ms (591 MB, 0.087 ms at the copy rate), 3D 96^3
@@ -195,13 +195,13 @@ struct ApplyArgs {
   int* sync;        // [0] error word, [1] ticket, then the counters
   int* err;         // the error word (of the first slice of columns)
   T* w;             // permuted vector, in place
-  T* t;             // S f of the interior columns
+  T* t;             // y = X f of the interior columns
   T* wu;            // update vectors
   T* zp;            // partials of z = W^T f
   T* sp;            // partials of s = V^T x_R
   T* yp;            // partials of X f
   T* xp;            // partials of X^T y
-  T* ip;            // partials of G^T x_R
+  T* ip;            // partials of X^T y - G^T x_R
   int work;         // elements of a group's work area in shared memory
 };
 

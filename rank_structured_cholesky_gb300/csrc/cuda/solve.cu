@@ -104,7 +104,7 @@ __device__ __forceinline__ void cols_gemv(const T* M, int r, int h, const T* v, 
 }
 
 // A group of small interior supernodes, forward: u = (children's rows) - G f
-// and t = S f; a warp a member, or several when there are fewer members.  FP32:
+// and y = X f; a warp a member, or several when there are fewer members.  FP32:
 // lanes along the rows, partial sums by shuffles.  FP64 adds run at 1/64 of the
 // FP32 rate, so there a lane forms a whole row (the odd row stride in 16-byte
 // units keeps that free of bank conflicts).
@@ -122,7 +122,7 @@ __device__ __forceinline__ void item_fgrp(const ApplyArgs<T>& A, const int* hdr0
     const int* h = hdr0 + GH * q;
     const int n = h[0], m = h[1], c0 = h[2], nv = h[7] / V;
     const Vt* G = reinterpret_cast<const Vt*>(data + h[4]);
-    const Vt* S = reinterpret_cast<const Vt*>(data + h[5]);
+    const Vt* X = reinterpret_cast<const Vt*>(data + h[5]);
     const int* ps = h[6] ? d + h[6] : nullptr;
     const int* ent = ps + n + m + 1;
     const int mp = ((m + wpn - 1) / wpn + 7) & ~7, aLo = part * mp, aHi = min(m, aLo + mp);
@@ -155,8 +155,8 @@ __device__ __forceinline__ void item_fgrp(const ApplyArgs<T>& A, const int* hdr0
       const int rows = max(0, aHi - aLo), sp = ((n + wpn - 1) / wpn + 7) & ~7, sLo = part * sp, sRows = max(0, min(n, sLo + sp) - sLo);
       const Vt* fs = reinterpret_cast<const Vt*>(f);
       const int nq = (n + V - 1) / V;
-      for (int i = lane; i < rows + sRows; i += 32) {   // rows of G, then of S
-        const Vt* row = i < rows ? G + (aLo + i) * nv : S + (sLo + i - rows) * nv;
+      for (int i = lane; i < rows + sRows; i += 32) {   // rows of G, then of X
+        const Vt* row = i < rows ? G + (aLo + i) * nv : X + (sLo + i - rows) * nv;
         T v0 = T(0), v1 = T(0);
         int c = 0;
         for (; c + 1 < nq; c += 2) {
@@ -180,7 +180,7 @@ __device__ __forceinline__ void item_fgrp(const ApplyArgs<T>& A, const int* hdr0
       }
       for (int i0 = part * rpl; i0 < n; i0 += rpl * wpn) {
         const int i = i0 + g;
-        T v = (i < n && c < nv) ? vdot(S[i * nv + c], fc, T(0)) : T(0);
+        T v = (i < n && c < nv) ? vdot(X[i * nv + c], fc, T(0)) : T(0);
         for (int o = 1; o < (1 << lg); o <<= 1) v += __shfl_xor_sync(FULL, v, o);
         if (c == 0 && i < n) t[i] = v;
       }
@@ -193,23 +193,24 @@ __device__ __forceinline__ void item_fgrp(const ApplyArgs<T>& A, const int* hdr0
   }
 }
 
-// A group, backward: x = t - G^T x_R; a warp a member.
+// A group, backward: x = X^T y - G^T x_R; a warp a member.
 template <class T>
 __device__ __forceinline__ void item_bgrp(const ApplyArgs<T>& A, const int* hdr0, const int* d, int cnt, const T* data,
                                           T* wk) {
   using Vt = typename Vec16<T>::type;
   constexpr int V = Vec16<T>::V;
   const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % GW;
-  T* xr = wk + warp * (IW_N + IW_M);
+  T* xr = wk + warp * (IW_N + IW_M);   // -x_R, then y
   for (int q = warp; q < cnt; q += GW) {
     const int* h = hdr0 + GH * q;
     const int n = h[0], m = h[1], c0 = h[2], nv = h[7] / V, nq = (n + V - 1) / V;
     const Vt* G = reinterpret_cast<const Vt*>(data + h[4]);
+    const Vt* X = reinterpret_cast<const Vt*>(data + h[5]);
     const int* rw = d + h[6];
     __syncwarp();
-    const T tl = lane < n ? __ldcg(A.t + h[8] + lane) : T(0);
+    if (lane < n) xr[m + lane] = __ldcg(A.t + h[8] + lane);
 #pragma unroll 4
-    for (int a = lane; a < m; a += 32) xr[a] = __ldcg(A.w + rw[a]);
+    for (int a = lane; a < m; a += 32) xr[a] = -__ldcg(A.w + rw[a]);
     __syncwarp();
     const int lg = nq <= 4 ? 2 : nq <= 8 ? 3 : 4;
     const int c = lane & ((1 << lg) - 1), g = lane >> lg, rpl = 32 >> lg;
@@ -217,12 +218,14 @@ __device__ __forceinline__ void item_bgrp(const ApplyArgs<T>& A, const int* hdr0
     if (c < nq) {
 #pragma unroll 4
       for (int a = g; a < m; a += rpl) vaxpy(acc, G[a * nv + c], xr[a]);
+#pragma unroll 4
+      for (int a = g; a < n; a += rpl) vaxpy(acc, X[a * nv + c], xr[m + a]);
     }
     for (int o = 1 << lg; o < 32; o <<= 1) vshfl_add(acc, o);
     __syncwarp();
     if (g == 0 && c < nq) reinterpret_cast<Vt*>(xr)[c] = acc;
     __syncwarp();
-    if (lane < n) A.w[c0 + lane] = tl - xr[lane];
+    if (lane < n) A.w[c0 + lane] = xr[lane];
   }
 }
 
@@ -230,7 +233,7 @@ __device__ __forceinline__ void item_bgrp(const ApplyArgs<T>& A, const int* hdr0
 // hdr: n, rows, c0, u offset (of the chunk's first row), s0, sRows, list, ldk, t offset, whole sectors
 template <class T>
 __device__ __forceinline__ void item_fwd(const ApplyArgs<T>& A, const int* h, const int* d, const int* d2, const T* Gd,
-                                         const T* Sd, T* f, T* ub) {
+                                         const T* Xd, T* f, T* ub) {
   using Vt = typename Vec16<T>::type;
   constexpr int V = Vec16<T>::V;
   const int tid = threadIdx.x % GT;
@@ -242,7 +245,7 @@ __device__ __forceinline__ void item_fwd(const ApplyArgs<T>& A, const int* h, co
   const int* ent = ps + rows + 1;
   const int* ent2 = d2 + n + 1;
   const Vt* fs = reinterpret_cast<const Vt*>(f);
-  const int R = rows + h[5];   // rows of G, then the chunk's rows of S
+  const int R = rows + h[5];   // rows of G, then the chunk's rows of X
   int lt = 1;                  // threads of a row: 2^lt
   while (lt < 5 && R << (lt + 1) <= GT) ++lt;
   const int sub = tid & ((1 << lt) - 1);
@@ -283,7 +286,7 @@ __device__ __forceinline__ void item_fwd(const ApplyArgs<T>& A, const int* h, co
       T v = acc;
       if (row < R) {
         const Vt* m =
-            reinterpret_cast<const Vt*>(row < rows ? Gd : Sd) + (size_t)(row < rows ? row : row - rows) * nv + j0 / V;
+            reinterpret_cast<const Vt*>(row < rows ? Gd : Xd) + (size_t)(row < rows ? row : row - rows) * nv + j0 / V;
 #pragma unroll 4
         for (int c = sub; c < jn / V; c += 1 << lt) v = vdot(m[c], fs[c], v);
       }
@@ -305,32 +308,31 @@ __device__ __forceinline__ void item_fwd(const ApplyArgs<T>& A, const int* h, co
   }
 }
 
-// One chunk of a larger interior supernode, backward: its part of G^T x_R, or
-// x = t - G^T x_R itself when it is the only one (several chunks: item BR).
-// hdr: n, rows, c0, ipOff, chunk, chunks, rows list, ldk, ip stride, t offset
+// One chunk of a larger interior supernode, backward: its part of X^T y - G^T x_R,
+// which is x when there is no other chunk (several: item BR).
+// hdr: n, rows of G, c0, ipOff, chunk, chunks, rows list, ldk, ip stride, y offset (of
+// the chunk's first row of X), rows of X
 template <class T>
-__device__ __forceinline__ void item_bwd(const ApplyArgs<T>& A, const int* h, const int* d, const T* Gd, T* xr, T* red) {
+__device__ __forceinline__ void item_bwd(const ApplyArgs<T>& A, const int* h, const int* d, const T* Gd, const T* Xd,
+                                         T* xr, T* red) {
   using Vt = typename Vec16<T>::type;
   constexpr int V = Vec16<T>::V;
   const int tid = threadIdx.x % GT, lane = tid & 31, warp = tid >> 5;
-  const int n = h[0], rows = h[1], c0 = h[2], nch = h[5], nv = h[7] / V;
-  if (rows == 0) {   // nothing above: x = t
-    for (int j = tid; j < n; j += GT) A.w[c0 + j] = __ldcg(A.t + h[9] + j);
-    return;
-  }
-  if (tid < rows) xr[tid] = __ldcg(A.w + d[h[6] + tid]);
+  const int n = h[0], rows = h[1], c0 = h[2], nch = h[5], nv = h[7] / V, R = rows + h[10];
+  if (tid < R) xr[tid] = tid < rows ? -__ldcg(A.w + d[h[6] + tid]) : __ldcg(A.t + h[9] + tid - rows);
   cbar();
   // 2^lg threads along a row (4 ... 128), the others on further rows
   int lg = 2;
   while ((1 << lg) < nv && lg < 7) ++lg;
   const int wd = 1 << lg, c = tid & (wd - 1), g = tid >> lg, ng = GT >> lg;
   const Vt* G = reinterpret_cast<const Vt*>(Gd);
+  const Vt* X = reinterpret_cast<const Vt*>(Xd) - (size_t)rows * nv;   // row a >= rows at a * nv
   Vt* rv = reinterpret_cast<Vt*>(red);
   for (int v0 = 0; v0 < nv; v0 += GT) {
     Vt acc = vzero(T(0));
     if (v0 + c < nv) {
 #pragma unroll 4
-      for (int a = g; a < rows; a += ng) vaxpy(acc, G[(size_t)a * nv + v0 + c], xr[a]);
+      for (int a = g; a < R; a += ng) vaxpy(acc, (a < rows ? G : X)[(size_t)a * nv + v0 + c], xr[a]);
     }
     for (int o = wd; o < 32; o <<= 1) vshfl_add(acc, o);
     const int parts = lg <= 5 ? GW : ng;
@@ -345,7 +347,7 @@ __device__ __forceinline__ void item_bwd(const ApplyArgs<T>& A, const int* h, co
       if (nch > 1) {
         if (j < h[8]) A.ip[h[3] + (size_t)h[4] * h[8] + j] = s;
       } else if (j < n) {
-        A.w[c0 + j] = __ldcg(A.t + h[9] + j) - s;
+        A.w[c0 + j] = s;
       }
     }
     cbar();
@@ -481,17 +483,13 @@ __global__ void __launch_bounds__(NGRP * GT + 32, 3) apply_kernel(ApplyArgs<T> A
       case IT_FGRP: item_fgrp<T>(A, h, d, it.count, data, red); break;
       case IT_BGRP: item_bgrp<T>(A, h, d, it.count, data, red); break;
       case IT_FWD: item_fwd<T>(A, h, d, d2, g0, g1, f, zs); break;
-      case IT_BWD: item_bwd<T>(A, h, d, g0, zs, red); break;
-      case IT_BR: {   // hdr: n, c0, ipOff, parts, ip stride, t offset: x = t - the parts of G^T x_R, in order
+      case IT_BWD: item_bwd<T>(A, h, d, g0, g1, zs, red); break;
+      case IT_BR: {   // hdr: n, c0, ipOff, parts, ip stride: x = the parts of X^T y - G^T x_R, added in order
         for (int k0 = 0; k0 < h[0]; k0 += GT * Vec16<T>::V) {
           const int kn = min(GT * Vec16<T>::V, h[0] - k0);
-          T t[Vec16<T>::V];
-#pragma unroll
-          for (int q = 0; q < Vec16<T>::V; ++q) t[q] = tid + q * GT < kn ? __ldcg(A.t + h[5] + k0 + tid + q * GT) : T(0);
           sum_parts<T>(A.ip + h[2], h[4], h[0], k0, h[3], zs, red);
-#pragma unroll
-          for (int q = 0; q < Vec16<T>::V; ++q)
-            if (tid + q * GT < kn) A.w[h[1] + k0 + tid + q * GT] = t[q] - zs[tid + q * GT];
+          for (int q = tid; q < kn; q += GT) A.w[h[1] + k0 + q] = zs[q];
+          cbar();
         }
         break;
       }
@@ -644,31 +642,27 @@ __global__ void __launch_bounds__(256) pack_tiles_kernel(const SNode<T>* __restr
   }
 }
 
-// [S; G] of an interior supernode of up to 64 columns from D = L11^{-1} (one
-// block): S = D^T D and G = L21 D share the product (rows) x D with the rows
-// of D^T, then of L21.  A block per 64 rows; a thread per (row, NQ of the 4 NQ
-// columns); D's zeros above the diagonal are skipped in steps of four.
-// Latency-bound: the products of all supernodes are a few GFLOP.
+// G = L21 X of an interior supernode of up to 64 columns, X = L11^{-1}.  A block per
+// 64 rows; a thread per (row, NQ of the 4 NQ columns); X's zeros above the diagonal
+// are skipped in steps of four.  Latency-bound: the products of all supernodes are a
+// few GFLOP.
 template <class T, int NQ>
 __global__ void __launch_bounds__(256) interior_ops_kernel(const SNode<T>* __restrict__ nodes,
                                                            const RowBlock* __restrict__ work) {
   constexpr int W = 4 * NQ, P = W + 1;
   extern __shared__ __align__(16) unsigned char smraw[];
-  T (*Ds)[P] = reinterpret_cast<T (*)[P]>(smraw);
+  T (*Xs)[P] = reinterpret_cast<T (*)[P]>(smraw);
   T (*Rs)[P] = reinterpret_cast<T (*)[P]>(smraw + sizeof(T) * W * P);
   const RowBlock wk = work[blockIdx.x];
   const SNode<T>& nd = nodes[wk.node];
-  const int n = nd.n, R = n + nd.m, r0 = wk.b * 64;
+  const int n = nd.n, m = nd.m, r0 = wk.b * 64;
   for (int idx = threadIdx.x; idx < W * W; idx += 256) {
     const int i = idx / W, j = idx - i * W;
-    Ds[i][j] = (i < n && j <= i) ? nd.Dinv[(size_t)i * n + j] : T(0);
+    Xs[i][j] = (i < n && j <= i) ? nd.X[(size_t)i * nd.ldx + j] : T(0);
   }
-  __syncthreads();
   for (int idx = threadIdx.x; idx < 64 * W; idx += 256) {
     const int i = idx / W, k = idx - i * W, row = r0 + i;
-    T v = T(0);
-    if (k < n && row < R) v = row < n ? Ds[k][row] : nd.L[(size_t)row * nd.ld + k];
-    Rs[i][k] = v;
+    Rs[i][k] = (k < n && row < m) ? nd.L[(size_t)(n + row) * nd.ld + k] : T(0);
   }
   __syncthreads();
   const int i = threadIdx.x >> 2, cg = threadIdx.x & 3;
@@ -681,12 +675,11 @@ __global__ void __launch_bounds__(256) interior_ops_kernel(const SNode<T>* __res
       const T l = Rs[i][4 * kb + kk];
 #pragma unroll
       for (int q = 0; q < NQ; ++q)
-        if (q <= kb) acc[q] += l * Ds[4 * kb + kk][cg + 4 * q];
+        if (q <= kb) acc[q] += l * Xs[4 * kb + kk][cg + 4 * q];
     }
   }
-  const int row = r0 + i;
-  if (row < R) {
-    T* out = row < n ? nd.Sg + (size_t)row * nd.ldk : nd.G + (size_t)(row - n) * nd.ldk;
+  if (r0 + i < m) {
+    T* out = nd.G + (size_t)(r0 + i) * nd.ldk;
 #pragma unroll
     for (int q = 0; q < NQ; ++q)
       if (cg + 4 * q < n) out[cg + 4 * q] = acc[q];
@@ -779,19 +772,16 @@ void SolveEngine<T>::plan() {
     if (cur > INT_MAX) throw std::runtime_error("solve plan: a work vector has more than 2^31 entries");
     return (int)at;
   };
-  long long dinvCur = 0, xCur = 0, gCur = 0, sCur = 0, wCur = 0;
-  std::vector<long long> xOff(nn, -1), gOff(nn, 0), sOff(nn, 0), wOff(nn, -1);
-  std::vector<long long> xTaskOff;   // per diagonal-block task: offset in the X arena, or -1
+  long long xCur = 0, xiCur = 0, gCur = 0, wCur = 0;
+  std::vector<long long> xOff(nn, 0), gOff(nn, 0), wOff(nn, -1);
   bytesPerApply_ = 0;
   std::vector<int> pos(S.n, -1);
   std::vector<DinvTask<T>> dinvTasks;
-  std::vector<long long> dinvTaskOff, dinvNodeOff(nn, 0);
+  std::vector<RowBlock> dinvOf;   // a task's supernode and block
   // X = L11^{-1} (n x ldx, upper triangle zero): the inverted 64 x 64 diagonal
   // blocks go in place
   auto plan_x = [&](int s) {
     SNode<T>& sn = nodes_[s];
-    sn.ldx = (sn.n + 3) & ~3;
-    xOff[s] = xCur;
     for (int b = 0; b * SOLVE_RB < sn.n; ++b) {
       DinvTask<T> t{};
       t.L = sn.L + (size_t)b * SOLVE_RB * sn.ld + (size_t)b * SOLVE_RB;
@@ -800,10 +790,8 @@ void SolveEngine<T>::plan() {
       t.pad = t.h;
       t.ldD = sn.ldx;
       dinvTasks.push_back(t);
-      dinvTaskOff.push_back(-1);
-      xTaskOff.push_back(xCur + (long long)b * SOLVE_RB * sn.ldx + (long long)b * SOLVE_RB);
+      dinvOf.push_back(RowBlock{s, b});
     }
-    xCur += (long long)sn.n * sn.ldx;
   };
   for (int s = 0; s < nn; ++s) {
     const Node& nd = S.nodes[s];
@@ -817,23 +805,12 @@ void SolveEngine<T>::plan() {
     if (!nd.compressed) {
       sn.L = F_.interior() + F_.frontOff[s];
       sn.r = 0;
-      if (nd.n <= SOLVE_RB) {   // D = L11^{-1} in one block: S and G follow from it
-        DinvTask<T> t{};
-        t.L = sn.L;
-        t.ld = sn.ld;
-        t.h = t.pad = t.ldD = nd.n;
-        dinvTasks.push_back(t);
-        dinvTaskOff.push_back(dinvCur);
-        xTaskOff.push_back(-1);
-        dinvNodeOff[s] = dinvCur;
-        dinvCur += (long long)nd.n * nd.n;
-      }
       // FP64: an odd row stride in 16-byte units, so that a lane a row reads
       // shared memory without bank conflicts
       sn.ldk = (nd.n + 3) & ~3;
       if (sizeof(T) == 8 && (sn.ldk = (nd.n + 1) & ~1) % 4 == 0) sn.ldk += 2;
-      if (nd.n > SOLVE_RB) plan_x(s);   // S and G follow from it
-      bytesPerApply_ += sizeof(T) * ((double)nd.n * nd.n + 2.0 * nd.m() * nd.n);
+      sn.ldx = sn.ldk;
+      bytesPerApply_ += 2.0 * sizeof(T) * ((double)nd.n + nd.m()) * nd.n;
     } else {
       sn.L = F_.compressed() + F_.frontOff[s];
       sn.r = F_.rank[s];
@@ -841,11 +818,14 @@ void SolveEngine<T>::plan() {
       sn.U = sn.r ? F_.vu() + F_.uOff[s] : nullptr;
       wOff[s] = wCur;
       wCur = (wCur + (long long)nd.n * sn.r + 3) & ~3LL;
-      plan_x(s);
+      sn.ldx = (nd.n + 3) & ~3;
+      xOff[s] = xCur;
+      xCur += (long long)nd.n * sn.ldx;
       bytesPerApply_ += 2.0 * sizeof(T) * ((double)nd.n * (nd.n + 1) / 2 + (double)sn.r * (nd.m() + nd.n));
     }
+    plan_x(s);
   }
-  // G and S of the interior supernodes, in the order of the levels (the members
+  // G and X of the interior supernodes, in the order of the levels (the members
   // of a work item are neighbours)
   for (auto& lv : F_.interiorLevels)
     for (int pass = 0; pass < 2; ++pass)
@@ -853,8 +833,8 @@ void SolveEngine<T>::plan() {
         if (group_member(s) == (pass == 0)) {
           gOff[s] = gCur;
           gCur += (long long)nodes_[s].m * nodes_[s].ldk;
-          sOff[s] = sCur;
-          sCur += (long long)nodes_[s].n * nodes_[s].ldk;
+          xOff[s] = xiCur;
+          xiCur += (long long)nodes_[s].n * nodes_[s].ldk;
         }
   // rel maps (target index of each interior child's row in the parent front)
   for (int s = 0; s < nn; ++s) {
@@ -884,15 +864,15 @@ void SolveEngine<T>::plan() {
   for (int s = 0; s < nn; ++s)
     if (S.nodes[s].compressed)
       std::stable_sort(pl[s].begin(), pl[s].end(), [](const SPull& a, const SPull& b) { return a.kind < b.kind; });
-  // S and G of the supernodes of up to 64 columns: 64-row blocks of [S; G], by
-  // column class (<= 16, <= 32, <= 64)
+  // G of the supernodes of up to 64 columns: 64-row blocks of it, by column class
+  // (<= 16, <= 32, <= 64)
   std::vector<RowBlock> opsWork;
   for (int cls = 0; cls < 3; ++cls) {
     const int lo = cls == 0 ? 0 : 8 << cls, hi = 16 << cls;
     opsClass_[cls].first = (long long)opsWork.size();
     for (int s = 0; s < nn; ++s)
       if (!S.nodes[s].compressed && S.nodes[s].n > lo && S.nodes[s].n <= hi)
-        for (int b = 0; b * 64 < S.nodes[s].n + S.nodes[s].m(); ++b) opsWork.push_back(RowBlock{s, b});
+        for (int b = 0; b * 64 < S.nodes[s].m(); ++b) opsWork.push_back(RowBlock{s, b});
     opsClass_[cls].second = (int)(opsWork.size() - opsClass_[cls].first);
   }
   clk.mark("layout");
@@ -901,30 +881,27 @@ void SolveEngine<T>::plan() {
     b.alloc(bytes);
     if (bytes) RSCHOL_CUDA(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, st));
   };
-  dDinv_.alloc(sizeof(T) * std::max(1LL, dinvCur));
   dT_.alloc(sizeof(T) * std::max(8LL, tCur));
   dX_.alloc(sizeof(T) * xCur);   // (what a factor does not have is not allocated)
   if (xCur > 0) RSCHOL_CUDA(cudaMemsetAsync(dX_.p, 0, sizeof(T) * xCur, st));   // upper triangles and padding stay zero
   dG_.alloc(sizeof(T) * std::max(1LL, gCur));
-  dS_.alloc(sizeof(T) * std::max(1LL, sCur));
+  dXi_.alloc(sizeof(T) * std::max(1LL, xiCur));
   RSCHOL_CUDA(cudaMemsetAsync(dG_.p, 0, dG_.bytes, st));   // the row padding stays zero
-  RSCHOL_CUDA(cudaMemsetAsync(dS_.p, 0, dS_.bytes, st));
+  RSCHOL_CUDA(cudaMemsetAsync(dXi_.p, 0, dXi_.bytes, st));
   dWc_.alloc(sizeof(T) * wCur);
-  for (size_t q = 0; q < dinvTasks.size(); ++q)
-    dinvTasks[q].D = xTaskOff[q] >= 0 ? dX_.as<T>() + xTaskOff[q] : dDinv_.as<T>() + dinvTaskOff[q];
   for (int s = 0; s < nn; ++s) {
-    if (xOff[s] >= 0) nodes_[s].X = dX_.as<T>() + xOff[s];
-    if (S.nodes[s].compressed) {
-      nodes_[s].W = dWc_.as<T>() + wOff[s];
-    } else {
-      nodes_[s].Dinv = dDinv_.as<T>() + dinvNodeOff[s];
-      nodes_[s].G = dG_.as<T>() + gOff[s];
-      nodes_[s].Sg = dS_.as<T>() + sOff[s];
-    }
+    SNode<T>& sn = nodes_[s];
+    sn.X = (S.nodes[s].compressed ? dX_ : dXi_).template as<T>() + xOff[s];
+    if (S.nodes[s].compressed) sn.W = dWc_.as<T>() + wOff[s];
+    else sn.G = dG_.as<T>() + gOff[s];
+  }
+  for (size_t q = 0; q < dinvTasks.size(); ++q) {
+    const SNode<T>& sn = nodes_[dinvOf[q].node];
+    dinvTasks[q].D = sn.X + (size_t)dinvOf[q].b * SOLVE_RB * (sn.ldx + 1);
   }
   nDinv_ = (int)dinvTasks.size();
   clk.mark("arenas");
-  plan_inverse(xOff);
+  plan_inverse();
   clk.mark("inverse");
   // per-row contribution lists of the compressed supernodes (in source order)
   std::vector<long long> cstart;
@@ -969,7 +946,7 @@ void SolveEngine<T>::plan() {
 }
 
 // Whether an interior supernode joins a group item: at most a warp's lanes of
-// columns and its S and G within one stage.
+// columns and its X and G within one stage.
 template <class T>
 bool SolveEngine<T>::group_member(int s) const {
   const SNode<T>& sn = nodes_[s];
@@ -1051,7 +1028,7 @@ void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<l
   // no part of one (words into a line long evicted cost its reader a fill from
   // DRAM: c2, 6 us in every reading item)
   auto part_ld = [](int n) { return (n + 7) & ~7; };
-  // chunks of the larger interior supernodes: rows of G and of S per item
+  // chunks of the larger interior supernodes: rows of G and of X per item
   struct Chunks {
     int nch, rc, per, staged, whole;
   };
@@ -1077,6 +1054,7 @@ void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<l
       c.per = ((sn.n + c.nch - 1) / c.nch + al - 1) / al * al;
       if (c.rc + c.per <= cap && c.rc <= 64) break;
     }
+    if (c.rc + c.per > GT) throw std::runtime_error("solve plan: a chunk has more rows than a group has threads");
     ipOff[s] = ipCur;
     ipCur += (long long)c.nch * part_ld(sn.n);
   }
@@ -1141,16 +1119,16 @@ void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<l
       it.count = (int)g.size();
       const SNode<T>& first = nodes_[g[0]];
       it.g0 = first.G;
-      it.g1 = first.Sg;
+      it.g1 = first.X;
       waits.clear();
-      long long gE = 0, sE = 0;
+      long long gE = 0, xE = 0;
       for (int s : g) {
         gE += (long long)nodes_[s].m * nodes_[s].ldk;
-        sE += (long long)nodes_[s].n * nodes_[s].ldk;
+        xE += (long long)nodes_[s].n * nodes_[s].ldk;
         for (int c : S.children[s]) pairs_of(waits, up[c]);
       }
       it.bytes0 = (int)(gE * E);
-      it.bytes1 = (int)(sE * E);
+      it.bytes1 = (int)(xE * E);
       begin(it, waits);
       const size_t h0 = blob.size();
       blob.resize(h0 + GH * g.size(), 0);
@@ -1163,7 +1141,7 @@ void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<l
         h[2] = sn.c0;
         h[3] = sn.uOff;
         h[4] = (int)(sn.G - first.G);
-        h[5] = (int)(gE + (sn.Sg - first.Sg));
+        h[5] = (int)(gE + (sn.X - first.X));
         h[7] = sn.ldk;
         h[8] = sn.tOff;
         if (has_pull(s)) {
@@ -1197,7 +1175,7 @@ void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<l
         it.kind = IT_FWD;
         it.sig = up[s].ctr;
         it.g0 = sn.G + (size_t)a0 * sn.ldk;
-        it.g1 = sn.Sg + (size_t)s0 * sn.ldk;
+        it.g1 = sn.X + (size_t)s0 * sn.ldk;
         if (c.staged) {
           it.bytes0 = rows * sn.ldk * E;
           it.bytes1 = sr * sn.ldk * E;
@@ -1447,18 +1425,24 @@ void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<l
       const Chunks& c = ch[s];
       waits.clear();
       wait_for(s, waits);
-      const int nch = sn.m > 0 ? (sn.m + c.rc - 1) / c.rc : 1;
+      const int nch = std::max((sn.m + c.rc - 1) / std::max(1, c.rc), (sn.n + c.per - 1) / c.per);   // not empty
       const Done parts{counter(), nch};
       for (int b = 0; b < nch; ++b) {
-        const int a0 = b * c.rc, rows = std::min(c.rc, sn.m - a0);
+        const int a0 = std::min(sn.m, b * c.rc), rows = std::min(c.rc, sn.m - a0);
+        const int s0 = std::min(sn.n, b * c.per), sr = std::min(c.per, sn.n - s0);
         ApplyItem it{};
         it.kind = IT_BWD;
         it.sig = parts.ctr;
         it.g0 = sn.G + (size_t)a0 * sn.ldk;
-        it.bytes0 = c.staged ? rows * sn.ldk * E : 0;
+        it.g1 = sn.X + (size_t)s0 * sn.ldk;
+        if (c.staged) {
+          it.bytes0 = rows * sn.ldk * E;
+          it.bytes1 = sr * sn.ldk * E;
+        }
         begin(it, waits);
-        const int list = (int)blob.size() - it.desc + 10;
-        blob.insert(blob.end(), {sn.n, rows, sn.c0, i32(ipOff[s]), b, nch, list, sn.ldk, part_ld(sn.n), sn.tOff});
+        const int list = (int)blob.size() - it.desc + 11;
+        blob.insert(blob.end(),
+                    {sn.n, rows, sn.c0, i32(ipOff[s]), b, nch, list, sn.ldk, part_ld(sn.n), sn.tOff + s0, sr});
         blob.insert(blob.end(), S.nodes[s].rows.begin() + a0, S.nodes[s].rows.begin() + a0 + rows);
         end(it);
       }
@@ -1471,13 +1455,16 @@ void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<l
       it.count = (int)g.size();
       const SNode<T>& first = nodes_[g[0]];
       it.g0 = first.G;
-      long long gE = 0;
+      it.g1 = first.X;
+      long long gE = 0, xE = 0;
       waits.clear();
       for (int s : g) {
         gE += (long long)nodes_[s].m * nodes_[s].ldk;
+        xE += (long long)nodes_[s].n * nodes_[s].ldk;
         wait_for(s, waits);
       }
       it.bytes0 = (int)(gE * E);
+      it.bytes1 = (int)(xE * E);
       begin(it, waits);
       const size_t h0 = blob.size();
       blob.resize(h0 + GH * g.size(), 0);
@@ -1488,6 +1475,7 @@ void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<l
         h[1] = sn.m;
         h[2] = sn.c0;
         h[4] = (int)(sn.G - first.G);
+        h[5] = (int)(gE + (sn.X - first.X));
         h[6] = (int)blob.size() - it.desc;
         h[7] = sn.ldk;
         h[8] = sn.tOff;
@@ -1511,7 +1499,7 @@ void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<l
       // of 400 columns held the level up for 130 - 180 us)
       const int n = nodes_[s].n, parts = solved[s].target, w = std::max(16, 1024 / parts & ~15);
       for (int c = 0; c < n; c += w)
-        push(it, waits, {std::min(w, n - c), nodes_[s].c0 + c, i32(ipOff[s] + c), parts, part_ld(n), nodes_[s].tOff + c});
+        push(it, waits, {std::min(w, n - c), nodes_[s].c0 + c, i32(ipOff[s] + c), parts, part_ld(n)});
       solved[s] = Done{it.sig, (n + w - 1) / w};
     }
   }
@@ -1557,30 +1545,27 @@ void SolveEngine<T>::plan_items(const std::vector<int>& rel, const std::vector<l
 }
 
 template <class T>
-void SolveEngine<T>::plan_inverse(const std::vector<long long>& xOff) {
-  // X = L11^{-1} of every compressed supernode, and of the interior ones of
-  // more than 64 columns, by recursive doubling: with
-  // the diagonal 64 x 64 inverses in place, for block sizes sz = 64, 128, ...
+void SolveEngine<T>::plan_inverse() {
+  // X = L11^{-1} of every supernode of more than 64 columns by recursive doubling:
+  // with the diagonal 64 x 64 inverses in place, for block sizes sz = 64, 128, ...
   // every pair (A, B) of consecutive sz-blocks gets X_BA = -X_BB (L_BA X_AA).
   // Both products run by 64-column (64-row) blocks whose K stops at the
   // triangle, so the work is n^3 / 3 per supernode.
   const Symbolic& S = F_.S;
   // X of a compressed supernode by split products on the tensor cores; what takes the
-  // place of FP32 sums with the factor itself -- X, S and G of the interior supernodes,
-  // and W -- by FP32 products.  (Those in split TF32 too, 22 bits an operand: the error
-  // of an exact mixed application against 64 bits 1.3e-6 - 6.6e-6 on 3D 12^3 - 32x31x30,
-  // sigma 0; with FP32 products 2.6e-7 - 5.7e-7.)
+  // place of FP32 sums with the factor itself -- X and G of the interior supernodes, and
+  // W -- by FP32 products.  (Those in split TF32 too, 22 bits an operand: the error of an
+  // exact mixed application against 64 bits 1.3e-6 - 6.6e-6 on 3D 12^3 - 32x31x30,
+  // sigma 0; with FP32 products 2.4e-7 - 3.9e-7, by substitution 4.3e-7 - 1.8e-6.)
   const bool tcX = std::is_same<T, float>::value && F_.tensor_cores();
   const int nn = (int)S.nodes.size();
   int maxN = 0;
-  for (int s = 0; s < nn; ++s)
-    if (xOff[s] >= 0) maxN = std::max(maxN, S.nodes[s].n);
+  for (int s = 0; s < nn; ++s) maxN = std::max(maxN, S.nodes[s].n);
   long long t1Max = 1;
   for (int sz = SOLVE_RB; sz < maxN; sz *= 2) {
     long long t1 = 0;
     for (int s = 0; s < nn; ++s) {
       const int n = S.nodes[s].n;
-      if (xOff[s] < 0) continue;
       for (int A0 = 0; A0 + sz < n; A0 += 2 * sz) t1 += (long long)std::min(sz, n - A0 - sz) * sz;
     }
     t1Max = std::max(t1Max, t1);
@@ -1635,10 +1620,9 @@ void SolveEngine<T>::plan_inverse(const std::vector<long long>& xOff) {
     std::vector<GemmTask<T>> b1[2], b2[2];   // interior, compressed
     long long t1cur = 0;
     for (int s = 0; s < nn; ++s) {
-      if (xOff[s] < 0) continue;
       const int n = S.nodes[s].n, ld = nodes_[s].ld, lx = nodes_[s].ldx;
       const T* L = nodes_[s].L;
-      T* X = dX_.as<T>() + xOff[s];
+      T* X = nodes_[s].X;
       const int c = S.nodes[s].compressed;
       for (int A0 = 0; A0 + sz < n; A0 += 2 * sz) {
         const int B0 = A0 + sz, bsz = std::min(sz, n - B0);
@@ -1660,32 +1644,26 @@ void SolveEngine<T>::plan_inverse(const std::vector<long long>& xOff) {
       flush(b[1], tcX);
     }
   }
-  // then the products the apply reads: W = X^T U of the compressed supernodes,
-  // S = X^T X and G = L21 X of the interior ones of more than 64 columns, by
-  // blocks whose K starts at the triangle
+  // then the products the apply reads: W = X^T U of the compressed supernodes and
+  // G = L21 X of the interior ones of more than 64 columns, by blocks whose K starts
+  // at the triangle
   std::vector<GemmTask<T>> bw, bi;
-  constexpr int blk = simt_rows<T>;
   for (int s = 0; s < nn; ++s) {
     const SNode<T>& sn = nodes_[s];
     const int n = sn.n, lx = sn.ldx;
     if (S.nodes[s].compressed) {
+      constexpr int blk = simt_rows<T>;
       for (int j0 = 0; sn.r > 0 && j0 < n; j0 += blk) {
         GemmTask<T> t = mk(sn.X + (size_t)j0 * lx + j0, lx, sn.U + (size_t)j0 * sn.r, sn.r,
                            const_cast<T*>(sn.W) + (size_t)j0 * sn.r, sn.r, std::min(blk, n - j0), sn.r, n - j0, T(1));
         t.tA = 1;
         bw.push_back(t);
       }
-    } else if (xOff[s] >= 0) {
-      for (int i0 = 0; i0 < n; i0 += blk) {
-        const int h = std::min(blk, n - i0);
-        GemmTask<T> t = mk(sn.X + (size_t)i0 * lx + i0, lx, sn.X + (size_t)i0 * lx, lx, sn.Sg + (size_t)i0 * sn.ldk,
-                           sn.ldk, h, n, n - i0, T(1));
-        t.tA = 1;
-        bi.push_back(t);
-        if (sn.m > 0)
-          bi.push_back(mk(sn.L + (size_t)n * sn.ld + i0, sn.ld, sn.X + (size_t)i0 * lx + i0, lx, sn.G + i0, sn.ldk,
-                          sn.m, h, n - i0, T(1)));
-      }
+    } else if (n > SOLVE_RB && sn.m > 0) {
+      constexpr int blk = simt_tile<T>;
+      for (int j0 = 0; j0 < n; j0 += blk)
+        bi.push_back(mk(sn.L + (size_t)n * sn.ld + j0, sn.ld, sn.X + (size_t)j0 * lx + j0, lx, sn.G + j0, sn.ldk,
+                        sn.m, std::min(blk, n - j0), n - j0, T(1)));
     }
   }
   flush(bw, false);
@@ -1709,7 +1687,7 @@ int SolveEngine<T>::prepare(cudaStream_t st) {
     RSCHOL_LAUNCH_CHECK();
     ++launches;
   }
-  // S and G of the interior supernodes of up to 64 columns
+  // G of the interior supernodes of up to 64 columns
   auto ops = [&](auto kernel, int cls, int nq) {
     if (opsClass_[cls].second == 0) return;
     const int smem = (int)sizeof(T) * (4 * nq + 64) * (4 * nq + 1);

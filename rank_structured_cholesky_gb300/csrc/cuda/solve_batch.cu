@@ -162,24 +162,27 @@ __device__ __forceinline__ void rows_dot(const T* M, const int (&off)[NR<T>], in
   }
 }
 
-// out(j, sum_{a < h} M[a * ld + j] X[a * xs]) for the thread's columns j < nc
+// out(j, sum_{a < h} M[a * ld + j] X[a * xs]) for the thread's columns j < nc; with an
+// M2 the rows from h0 on are its rows
 template <class T, class Out>
 __device__ __forceinline__ void cols_dot(const T* M, int ld, int h, int nc, const typename Vec16<T>::type* X, int xs,
-                                         int j0, int step, Out out) {
+                                         int j0, int step, Out out, const T* M2 = nullptr, int h0 = 0) {
   for (int jb = j0; jb < nc; jb += NR<T> * step) {
     typename Vec16<T>::type acc[NR<T>];
-    const T* m[NR<T>];
 #pragma unroll
-    for (int i = 0; i < NR<T>; ++i) {
-      acc[i] = vzero(T(0));
-      m[i] = jb + i * step < nc ? M + jb + i * step : nullptr;
-    }
+    for (int i = 0; i < NR<T>; ++i) acc[i] = vzero(T(0));
+    for (int part = 0; part < (M2 ? 2 : 1); ++part) {
+      const int aBeg = part ? h0 : 0, aEnd = M2 && !part ? h0 : h;
+      const T* m[NR<T>];
+#pragma unroll
+      for (int i = 0; i < NR<T>; ++i) m[i] = jb + i * step < nc ? (part ? M2 : M) + jb + i * step : nullptr;
 #pragma unroll 4
-    for (int a = 0; a < h; ++a) {
-      const typename Vec16<T>::type x = X[a * xs];
+      for (int a = aBeg; a < aEnd; ++a) {
+        const typename Vec16<T>::type x = X[a * xs];
 #pragma unroll
-      for (int i = 0; i < NR<T>; ++i)
-        if (m[i]) vaxpy(acc[i], x, m[i][(size_t)a * ld]);
+        for (int i = 0; i < NR<T>; ++i)
+          if (m[i]) vaxpy(acc[i], x, m[i][(size_t)(a - aBeg) * ld]);
+      }
     }
 #pragma unroll
     for (int i = 0; i < NR<T>; ++i)
@@ -204,7 +207,7 @@ __device__ __forceinline__ void fgrp_k(const Pass<T>& p, const int* h0, const in
     __syncwarp();
     gather_f<T>(p, c0, 0, n, has ? ps : nullptr, ent, rg, nrg, F);
     __syncwarp();
-    for (int r0 = 0; r0 < m + n; r0 += NR<T> * nrg) {   // rows of G, then of S
+    for (int r0 = 0; r0 < m + n; r0 += NR<T> * nrg) {   // rows of G, then of X
       Vt acc[NR<T>];
       int off[NR<T>];
 #pragma unroll
@@ -253,56 +256,60 @@ __device__ __forceinline__ void bgrp_k(const Pass<T>& p, const int* h0, const in
   for (int q = warp; q < cnt; q += GW) {
     const int* h = h0 + GH * q;
     const int n = h[0], m = h[1], c0 = h[2], ldk = h[7];
-    const T* G = data + h[4];
     const int* rw = d + h[6];
-    // the thread's columns j = rg + i nrg: 32 columns in 1, 2 or 4 sweeps of them
-    const int tile = NR<T> * nrg;   // rows of x_R a tile
+    // the thread's columns j = rg + i nrg: 32 columns in 1, 2 or 4 sweeps of them;
+    // rows a < m: -x_R with G's, then y with X's
+    const int tile = NR<T> * nrg;   // rows a tile
+    auto load = [&](int a) {
+      if (a >= m) return a < m + n ? p.ld(p.A->t, h[8] + a - m) : vzero(T(0));
+      Vt x = p.ld(p.A->w, rw[a]), v = vzero(T(0));
+      vsub(v, x);
+      return v;
+    };
     for (int jb = 0; jb < n; jb += NR<T> * nrg) {
       Vt acc[NR<T>], nx[NR<T>];
-      const T* g[NR<T>];
+      int col[NR<T>];
 #pragma unroll
       for (int i = 0; i < NR<T>; ++i) {
         acc[i] = vzero(T(0));
-        g[i] = jb + rg + i * nrg < n ? G + jb + rg + i * nrg : nullptr;
-        nx[i] = rg + i * nrg < m ? p.ld(p.A->w, rw[rg + i * nrg]) : vzero(T(0));
+        col[i] = jb + rg + i * nrg < n ? jb + rg + i * nrg : -1;
+        nx[i] = load(rg + i * nrg);
       }
-      for (int a0 = 0; a0 < m; a0 += tile) {
+      for (int a0 = 0; a0 < m + n; a0 += tile) {
         __syncwarp();
 #pragma unroll
         for (int i = 0; i < NR<T>; ++i) X[(rg + i * nrg) * p.cgN + p.cg] = nx[i];
         __syncwarp();
 #pragma unroll
-        for (int i = 0; i < NR<T>; ++i) {   // the next tile's loads under this one's products
-          const int a = a0 + tile + rg + i * nrg;
-          nx[i] = a < m ? p.ld(p.A->w, rw[a]) : vzero(T(0));
-        }
-        const int an = min(tile, m - a0);
+        for (int i = 0; i < NR<T>; ++i) nx[i] = load(a0 + tile + rg + i * nrg);   // under this tile's products
+        const int an = min(tile, m + n - a0), gn = max(0, min(an, m - a0));
 #pragma unroll 4
-        for (int a = 0; a < an; ++a) {
+        for (int a = 0; a < gn; ++a) {
           const Vt x = X[a * p.cgN + p.cg];
 #pragma unroll
           for (int i = 0; i < NR<T>; ++i)
-            if (g[i]) vaxpy(acc[i], x, g[i][(size_t)(a0 + a) * ldk]);
+            if (col[i] >= 0) vaxpy(acc[i], x, data[h[4] + (a0 + a) * ldk + col[i]]);
+        }
+#pragma unroll 4
+        for (int a = gn; a < an; ++a) {
+          const Vt x = X[a * p.cgN + p.cg];
+#pragma unroll
+          for (int i = 0; i < NR<T>; ++i)
+            if (col[i] >= 0) vaxpy(acc[i], x, data[h[5] + (a0 + a - m) * ldk + col[i]]);
         }
       }
 #pragma unroll
-      for (int i = 0; i < NR<T>; ++i) {
-        const int j = jb + rg + i * nrg;
-        if (j < n) {
-          Vt v = p.ld(p.A->t, h[8] + j);
-          vsub(v, acc[i]);
-          p.st(p.A->w, c0 + j, v);
-        }
-      }
+      for (int i = 0; i < NR<T>; ++i)
+        if (col[i] >= 0) p.st(p.A->w, c0 + col[i], acc[i]);
     }
   }
 }
 
-// One chunk: the rows of G, then of S (in a stage they follow each other; a
-// supernode too wide for one is read where it is, G's rows and S's in turn).
+// One chunk: the rows of G, then of X (in a stage they follow each other; a
+// supernode too wide for one is read where it is, G's rows and X's in turn).
 template <class T>
 __device__ __forceinline__ void fwd_k(const Pass<T>& p, const int* h, const int* d, const int* d2, const T* Gd,
-                                      const T* Sd, bool staged, typename Vec16<T>::type* F) {
+                                      const T* Xd, bool staged, typename Vec16<T>::type* F) {
   using Vt = typename Vec16<T>::type;
   constexpr int V = Vec16<T>::V;
   const int n = h[0], rows = h[1], c0 = h[2], ldk = h[7];
@@ -312,7 +319,7 @@ __device__ __forceinline__ void fwd_k(const Pass<T>& p, const int* h, const int*
   const int* ent2 = d2 + n + 1;
   const int ft = FV / p.cgN / V * V;   // rows of f a tile
   for (int part = 0; part < (staged ? 1 : 2); ++part) {
-    const T* M = part ? Sd : Gd;
+    const T* M = part ? Xd : Gd;
     const int first = part ? rows : 0, cnt = staged ? rows + h[5] : part ? h[5] : rows;
     // A wide supernode's chunk has few rows (300 columns in FP64: seven): K in GT /
     // slots slices, over the threads that would have no row -- a pass of fewer
@@ -534,28 +541,32 @@ __global__ void __launch_bounds__(NGRP * GT + 32, BATCH_BLOCKS) apply_batch_kern
         case IT_BGRP: bgrp_k<T>(p, h, d, it.count, data, F); break;
         case IT_FWD: fwd_k<T>(p, h, d, d2, it.bytes0 + it.bytes1 > 0 ? data : g0, g1, it.bytes0 + it.bytes1 > 0, F); break;
         case IT_BWD: {
-          const int n = h[0], rows = h[1];
-          if (rows == 0) {
-            for (int j = p.rg; j < n; j += p.nrg) p.st(A.w, h[2] + j, p.ld(A.t, h[9] + j));
-            break;
-          }
+          const int n = h[0], rows = h[1], R = rows + h[10];
 #pragma unroll 2
-          for (int a = p.rg; a < rows; a += p.nrg) F[a * p.cgN + p.cg] = p.ld(A.w, d[h[6] + a]);
-          cbar();
-          cols_dot<T>(g0, h[7], rows, n, F + p.cg, p.cgN, p.rg, p.nrg, [&](int j, Vt v) {
-            if (h[5] > 1) {
-              p.st(A.ip, h[3] + (long long)h[4] * h[8] + j, v);
+          for (int a = p.rg; a < R; a += p.nrg) {
+            Vt v;
+            if (a < rows) {
+              v = vzero(T(0));
+              vsub(v, p.ld(A.w, d[h[6] + a]));
             } else {
-              Vt t = p.ld(A.t, h[9] + j);
-              vsub(t, v);
-              p.st(A.w, h[2] + j, t);
+              v = p.ld(A.t, h[9] + a - rows);
             }
-          });
+            F[a * p.cgN + p.cg] = v;
+          }
+          cbar();
+          const bool staged = it.bytes0 + it.bytes1 > 0;   // (the rows of X behind those of G)
+          cols_dot<T>(
+              staged ? data : g0, h[7], R, n, F + p.cg, p.cgN, p.rg, p.nrg,
+              [&](int j, Vt v) {
+                if (h[5] > 1) p.st(A.ip, h[3] + (long long)h[4] * h[8] + j, v);
+                else p.st(A.w, h[2] + j, v);
+              },
+              staged ? nullptr : g1, rows);
           break;
         }
         case IT_BR: {
           for (int j = p.rg; j < h[0]; j += p.nrg) {
-            Vt t = p.ld(A.t, h[5] + j), x = vzero(T(0));
+            Vt x = vzero(T(0));
             for (int q0 = 0; q0 < h[3]; q0 += 16) {
               Vt v[16];
 #pragma unroll
@@ -564,8 +575,7 @@ __global__ void __launch_bounds__(NGRP * GT + 32, BATCH_BLOCKS) apply_batch_kern
 #pragma unroll
               for (int q = 0; q < 16; ++q) vadd(x, v[q]);
             }
-            vsub(t, x);
-            p.st(A.w, h[1] + j, t);
+            p.st(A.w, h[1] + j, x);
           }
           break;
         }

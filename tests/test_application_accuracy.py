@@ -61,3 +61,23 @@ def test_mixed_is_as_accurate_as_lapack_in_fp32(p, r):
     tol = 4 * _backward(A, lapack, b)
     assert _backward(A, np.array([F.apply(v) for v in b]), b) <= tol
     assert _backward(A, F.apply(b), b) <= tol
+
+
+DENSE = [(n, 0) for n in (7, 20, 33, 50, 64, 65, 100, 300, 700)]
+BORDERED = [(30, 20), (60, 50), (150, 120), (300, 250)]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("p,r", DENSE + BORDERED)
+def test_smooth_right_hand_sides(p, r, precision):
+    """b = A x of a random x: ill-conditioned blocks must not show in the residual
+    (an inverse of A's block would leave the condition number in it).  Condition
+    numbers 1e10 and, mixed, 1e4; under a border blocks of 1e6 and 1e3, which make a
+    matrix of 1e9 and 1e4.  The bound: rounding errors of sums of up to 2 p + r terms,
+    which grow as a random walk, times 4."""
+    A = _matrix(p, r, {"fp64": 1e6 if r else 1e10, "mixed": 1e3 if r else 1e4}[precision])
+    F = _factor(A, p, r, precision)
+    b = np.random.default_rng(5).standard_normal((8, A.shape[0])) @ A
+    tol = 4 * math.sqrt(A.shape[0]) * 2.0 ** (-53 if precision == "fp64" else -24)
+    assert _backward(A, np.array([F.apply(v) for v in b]), b) <= tol
+    assert _backward(A, F.apply(b), b) <= tol
