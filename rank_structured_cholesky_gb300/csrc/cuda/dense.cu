@@ -528,17 +528,9 @@ __global__ void __launch_bounds__(256) trsm_kernel(const TrsmTask<T>* __restrict
 // non-positive pivot is replaced by 1 and reported as atomicMin(flag, code).
 // 1 / p on a POTRF's critical path: the fast reciprocal (MUFU-based,
 // __fdividef, within 2 ulp) in FP32, whose factor carries larger rounding
-// errors anyway.
+// errors anyway; exact division in FP64.
 __device__ __forceinline__ float pivot_recip(float p) { return __fdividef(1.0f, p); }
-// FP64: the 20-bit estimate and two Newton steps y += y (1 - p y), four dependent
-// multiply-adds (a division is about three times as many on the chain).
-__device__ __forceinline__ double pivot_recip(double p) {
-  if (!(p > 1e-290 && p < 1e290)) return 1.0 / p;
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(p));
-  y = fma(y, fma(-p, y, 1.0), y);
-  return fma(y, fma(-p, y, 1.0), y);
-}
+__device__ __forceinline__ double pivot_recip(double p) { return 1.0 / p; }
 
 template <class T>
 __device__ void potrf_tile_reg(T* A, int ld, int n, int code, int* flag) {
@@ -728,8 +720,11 @@ __device__ void trsm_chunk_mul(T* B, int ldb, int nr, int w, T (*X)[65], T (*Li)
 }
 
 // Factor and invert one FP32 tile on the chain of the fused Cholesky: S (64 x 68
-// shared) holds the n x n lower tile, padded with a unit diagonal; on return its L,
-// and in Li (64 x 68) the inverse's lower blocks.  A column at a time (potrf_tile_reg
+// shared) holds the n x n lower tile, padded with a unit diagonal; on return its L, but
+// for the entries below the diagonal in the 16 x 16 diagonal blocks, which are still to
+// be divided by their column's diagonal (tile_entry, when the tile is stored: divided
+// here they cost the chain 2 of 18 ms a factorisation of 3D 64^3), and in Li (64 x 68)
+// the inverse's lower blocks.  A column at a time (potrf_tile_reg
 // and tile_inverse) every column costs a block barrier and a round through shared
 // memory, 22 us a tile.  Here in blocks of 16: one warp eliminates the diagonal
 // block and the identity beside it with shuffles, the rows below are multiplied by
@@ -764,13 +759,11 @@ __device__ __noinline__ void potrf_inverse_f32(float (*S)[68], float (*Li)[68], 
     }
     const float d = sqrtf(pd), rd = 1.f / d;
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const float rk = __shfl_sync(0xffffffffu, rd, k, 16);
+    for (int k = 0; k < 16; ++k)
       if (hi == 0) {
         Li[o + lj][o + k] = e[k] * rd;
-        if (k <= lj) S[o + lj][o + k] = k == lj ? d : v[k] * rk;
+        if (k <= lj) S[o + lj][o + k] = k == lj ? d : v[k];
       }
-    }
   };
   // a warp: block (R, C) of the inverse, -Li[R][R] sum_{C <= K < R} L[R][K] Li[K][C];
   // lane: column lj, rows 2 q + hi
@@ -873,6 +866,11 @@ __device__ __noinline__ void potrf_inverse_f32(float (*S)[68], float (*Li)[68], 
   if (tid == 0 && bad) atomicMin(flag, code);
 }
 
+__device__ __forceinline__ float tile_entry(const float (*S)[68], int i, int k) {
+  return (i >> 4) == (k >> 4) && k < i ? S[i][k] / S[k][k] : S[i][k];
+}
+__device__ __forceinline__ double tile_entry(const double (*S)[33], int i, int k) { return S[i][k]; }
+
 // The same for one FP64 tile (n <= 32; S, Li 32 x 33, Tm 16 x 17 shared).  A warp's
 // multiply-add holds its quarter of the FP64 unit for 64 clocks, so what counts is
 // how many each warp issues: warp w keeps rows 4 w .. 4 w + 3 (a thread: one row, every eighth
@@ -929,7 +927,7 @@ __device__ __noinline__ void potrf_inverse_f64(double (*S)[33], double (*Li)[33]
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const int k = kc + 8 * c;
-    if (8 * c <= rLast && k <= i) S[i][k] = k == i ? dia[i] : v[c] * rdia[k];
+    if (8 * c <= rLast && k <= i) S[i][k] = k == i ? dia[i] : v[c] / dia[k];
   }
   if (tid == 0 && bad) atomicMin(flag, code);
   if (!invert) return;   // (uniform; the caller's barrier follows)
@@ -1335,7 +1333,7 @@ __global__ void __launch_bounds__(256, 3) chol_fused_kernel(const CholFusedJob<T
 #pragma unroll
       for (int idx = threadIdx.x; idx < NB * NB; idx += 256) {
         const int i = idx / NB, k = idx % NB;
-        if (k <= i && i < n) F[(size_t)(r0 + i) * ld + q0 + k] = S[i][k];
+        if (k <= i && i < n) F[(size_t)(r0 + i) * ld + q0 + k] = tile_entry(S, i, k);
       }
     } else if (it.kind == CHOL_TRSM) {   // X := C Li(b)^T, the inverse tile from the workspace
 #pragma unroll
