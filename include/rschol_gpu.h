@@ -100,7 +100,10 @@ int rschol_check_structure(int n, const int* colptr, const int* rowind, const do
                            const rschol_params* params, char* msg, int msg_len);
 
 /* New values, same pattern: FactorPreconditioner::initialize with only the
- * numeric factor needed (FactorPreconditioner.cpp:115-129). */
+ * numeric factor needed (FactorPreconditioner.cpp:115-129).  The operators that an
+ * application reads (the inverses of the diagonal triangles and the products with
+ * them) are formed here too, with every factorisation; they are part of the factor's
+ * device bytes. */
 int rschol_refactor(rschol_factor* f, const double* vals);
 
 /* Same, with the new values (full CSC order) already resident on the device. */
@@ -150,22 +153,23 @@ int rschol_precond_apply_device_noalloc(rschol_factor* f, const double* d_b, dou
  * candidate launch shapes (persistent thread blocks per SM) of every width
  * class (number of right-hand sides rounded up to a power of two) up to
  * max_columns and keeps the fastest for this factor; run it while the GPU is
- * otherwise quiet.  No candidate changes any result: every shape forms each
- * column's sums in the same order.  Untuned classes use a fixed shape.  The
- * choices are listed in rschol_factor_describe ("batch_tuning": class, blocks
- * per SM, columns per pass, 0, 0, ms). */
+ * otherwise quiet.  The candidates are one and two blocks per SM; none changes
+ * any result: every shape forms each column's sums in the same order.  Untuned
+ * classes use two.  The choices are listed in rschol_factor_describe
+ * ("batch_tuning": class, blocks per SM, columns per pass, two unused fields
+ * (0), ms). */
 int rschol_factor_autotune(rschol_factor* f, int max_columns);
 
 /* Autotuner of the factor's schedule (no reference counterpart): times
  * `repeats` numeric factorisations of the factor's current values under each
  * candidate -- FP32 GEMM steps on the tensor cores (128 x 64 or 128 x 128
- * tiles) from K >= 32, 64, 96, 128 or 256, or none (64 x 64 SIMT tiles);
- * * the blocked Cholesky
- * and TRSM chains of a level as one fused launch of 64 x 64 tile items or as
- * one launch per 64-column panel -- keeps the fastest and leaves the factor
- * refactored with it (within 3 % of each other the earlier one stays, 128 first).
- * The candidates differ only in rounding.  Run it while
- * the GPU is otherwise quiet, before creating sessions on the factor.  The
+ * tiles) from K >= 32, 64, 96, 128 or 256, or none (SIMT tiles of 64 x 64, or
+ * 128 x 64 where a launch has many; FP64 is always SIMT, 32 x 32); the blocked
+ * Cholesky and TRSM chains of a level as one fused launch of tile items (64 x 64,
+ * FP64 32 x 32) or as one launch per 64-column panel -- keeps the fastest and
+ * leaves the factor refactored with it (within 3 % of each other the earlier one
+ * stays, 128 first).  The candidates differ only in rounding.  Run it while the
+ * GPU is otherwise quiet, before creating sessions on the factor.  The
  * choice is listed in rschol_factor_describe ("schedule": tc_min_k (-1: none),
  * fused, tuned_ms). */
 int rschol_factor_tune_schedule(rschol_factor* f, int repeats);

@@ -878,7 +878,7 @@ __device__ __forceinline__ double tile_entry(const double (*S)[33], int i, int k
 // multiplier is formed once; column j is published unscaled with the reciprocal of
 // its pivot, one barrier a column.  Square roots and their reciprocals by one
 // warp; the inverse's two 16 x 16 diagonal blocks by one warp, a column a lane.
-// (Cholesky steps of 3D 37x41x35 FP64 12.3 -> 12.0 ms against every
+// (Cholesky steps of 3D 37x41x35 FP64 12.3 -> 12.1 ms against every
 // thread forming all its products on every column.)
 __device__ __noinline__ void potrf_inverse_f64(double (*S)[33], double (*Li)[33], double (*Tm)[17], int n, bool invert,
                                                int code, int* flag) {
@@ -1055,9 +1055,9 @@ __global__ void __launch_bounds__(256) trsm_inv_kernel(const TrsmTask<T>* __rest
 // own: tdone[a] panels of row tile a stored, pdone[p] inverse p stored.
 // What bounds it is the chain POTRF(p) -> TRSM(p + 1, p) -> POTRF(p + 1); as one
 // item a tile and panel (right-looking) it was 36 us a panel, 22 of them the tile's
-// factor and inverse, 5 the three hand-overs; now it is 23, and the updates read
-// and write their tiles once (Cholesky steps of a factorisation: 3D 64^3 10.3 -> 7.8
-// ms, 96^3 49.2 -> 36.0 ms, elasticity 30^3 6.3 -> 4.7 ms).
+// factor and inverse, 5 the three hand-overs; now it is 22, and the updates read
+// and write their tiles once (Cholesky steps of a factorisation: 3D 64^3 10.3 -> 7.5
+// ms, 96^3 49.2 -> 35.2 ms, elasticity 30^3 6.3 -> 4.5 ms).
 // sync[0] is the ticket, the counters follow (zeroed before every launch);
 // a wait that gives up sets flag[1].  Data written by other blocks is read
 // through L2 (ld.global.cg).

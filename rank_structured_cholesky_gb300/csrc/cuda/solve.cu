@@ -726,8 +726,8 @@ __global__ void convert_kernel(const A* __restrict__ src, B* __restrict__ dst, i
   if (i < n) dst[i] = (B)src[i];
 }
 
-// Zero the interior completion counters and solved flags after their last
-// reader (the backward launch), grid-stride.
+// Zero the ticket and the items' counters after their last reader (the apply
+// kernel), grid-stride.
 __device__ __forceinline__ void clear_piece(int* c, int count) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) c[i] = 0;
 }

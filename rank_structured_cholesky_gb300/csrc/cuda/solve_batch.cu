@@ -17,9 +17,9 @@
 // dependent loads whatever its bytes), FP64 its 1/64 rate.  Measured, one
 // application against the earlier kernels (a triangular solve with a thread per
 // (row, column) pair, six launches per compressed level): 2D 1024^2 FP32 k = 64
-// 10.50 -> 5.89 ms, k = 8 3.62 -> 0.85 ms; 3D 40^3 FP32 k = 32 1.99 -> 0.67 ms,
-// k = 8 1.81 -> 0.40 ms; 3D 64^3 FP32 k = 16 3.23 -> 1.10 ms; 3D 44x40x47 FP64
-// k = 8 2.78 -> 1.50 ms.
+// 10.50 -> 6.5 ms, k = 8 3.62 -> 0.97 ms; 3D 40^3 FP32 k = 32 1.99 -> 0.70 ms,
+// k = 8 1.81 -> 0.46 ms; 3D 64^3 FP32 k = 8 2.44 -> 0.95 ms; 3D 44x40x47 FP64
+// k = 8 2.78 -> 1.60 ms.
 #include <algorithm>
 #include <mutex>
 #include <stdexcept>
@@ -771,9 +771,9 @@ int SolveEngine<T>::batch_capacity() const {
 // one after the other leave most of the chip waiting.  Slices of a whole pass (four
 // vectors); of two or one where the items are so few that the blocks outnumber
 // them.  One application at one / two / four vectors a slice / all in turn: FP64 2D
-// 75x70 (336 items) k = 16 240 / 264 / 352 / 618 us, 110x100 (735) k = 64 579 / 433 / 417 /
-// 2382, 193x187 (2938) k = 16 775 / 618 / 600 / 972; FP32 2D 193x187 (1345) k = 64 407 /
-// 313 / 339 / 886, 3D 40x38x40 (14050) k = 64 2833 / 1601 / 1049 / 1532.
+// 75x70 (343 items) k = 16 270 / 303 / 419 / 749 us, 110x100 (750) k = 64 680 / 509 / 490 /
+// 2863, 193x187 (2949) k = 16 884 / 713 / 749 / 1233; FP32 2D 193x187 (1371) k = 64 468 /
+// 354 / 381 / 1093, 3D 40x38x40 (14058) k = 64 2976 / 1678 / 1091 / 1649.
 template <class T>
 int SolveEngine<T>::batch_slices(int kp) const {
   const long long nv = std::max(1, (kp + Vec16<T>::V - 1) / Vec16<T>::V), passes = nv * nItems_;

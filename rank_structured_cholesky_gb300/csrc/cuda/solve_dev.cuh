@@ -1,6 +1,5 @@
-// Device helpers shared by the single-vector and batched solves: warp
-// reductions, bounded inter-block waits, and the ticket / completion counter
-// layout of the interior launches.
+// Device helpers shared by the single-vector and batched solves and the fused
+// Cholesky: warp reductions and bounded inter-block waits.
 #pragma once
 #include <cuda_runtime.h>
 
