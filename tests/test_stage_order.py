@@ -23,7 +23,7 @@ def test_no_item_is_taken_before_it_landed(tmp_path):
 
 
 def test_the_model_sees_a_wait_by_parity_alone(tmp_path):
-    """The driver tells: with the wait for the item before left out, it finds the order."""
+    """The model can tell: with the wait for the item before left out, it finds the order."""
     src = open(os.path.join(_build.CSRC, "cuda", "stage_order.h")).read()
     planted = src.replace("if (use > 0 && !empty(s, (use - 1) & 1)) return false;", "")
     assert planted != src
