@@ -201,9 +201,17 @@ PcgEngine::PcgEngine(int n_, const std::vector<int>& rowptr, const std::vector<i
   // 20 at two, 22 at four, 33 at eight); longer rows two, or as many as give the
   // device 1024 threads an SM (elasticity 30^3, 80 entries: 32 us at two, 35 at
   // eight, 51 at one and at sixteen, 84 at thirty-two).
+  // A row much longer than the others keeps its few threads long after the others are
+  // done: there 16, or 32 where the others are long too (60,000 rows of 15 with one of
+  // 3,000: 155 us at four, 75 at sixteen; of 50 with such a one: 198 at four, 71 at 32).
+  int longest = 0;
+  for (int i = 0; i < n; ++i) longest = std::max(longest, rowptr[i + 1] - rowptr[i]);
   tpr_ = 1;
-  if (avg > 12)
-    for (tpr_ = 2; tpr_ < 32 && (long long)n * tpr_ < 152 * 1024; tpr_ *= 2) {}
+  if (avg > 12) {
+    if (longest > 256 && longest > 8 * avg) tpr_ = avg <= 40 ? 16 : 32;
+    else
+      for (tpr_ = 2; tpr_ < 32 && (long long)n * tpr_ < 152 * 1024; tpr_ *= 2) {}
+  }
   if (const char* e = std::getenv("RSCHOL_SPMV_TPR")) {   // threads per row of the SpMV (1 ... 32)
     const int t = std::atoi(e);
     if (t == 1 || t == 2 || t == 4 || t == 8 || t == 16 || t == 32) tpr_ = t;
