@@ -83,7 +83,7 @@ struct alignas(16) ApplyItem {   // one work item of an application
   int count;                   // members of a group
   int shallow;                 // an item of a phase of few items (ticket draw)
   int desc2, desc2Bytes;       // a part of the descriptor that several items share
-  int pad;
+  int early;                   // waits that come first; the batched kernel has work between them and the others
 };
 
 template <class T>

@@ -162,27 +162,24 @@ __device__ __forceinline__ void rows_dot(const T* M, const int (&off)[NR<T>], in
   }
 }
 
-// out(j, sum_{a < h} M[a * ld + j] X[a * xs]) for the thread's columns j < nc; with an
-// M2 the rows from h0 on are its rows
+// out(j, sum_{a < h} M[a * ld + j] X[a * xs]) for the thread's columns j < nc
 template <class T, class Out>
 __device__ __forceinline__ void cols_dot(const T* M, int ld, int h, int nc, const typename Vec16<T>::type* X, int xs,
-                                         int j0, int step, Out out, const T* M2 = nullptr, int h0 = 0) {
+                                         int j0, int step, Out out) {
   for (int jb = j0; jb < nc; jb += NR<T> * step) {
     typename Vec16<T>::type acc[NR<T>];
+    const T* m[NR<T>];
 #pragma unroll
-    for (int i = 0; i < NR<T>; ++i) acc[i] = vzero(T(0));
-    for (int part = 0; part < (M2 ? 2 : 1); ++part) {
-      const int aBeg = part ? h0 : 0, aEnd = M2 && !part ? h0 : h;
-      const T* m[NR<T>];
-#pragma unroll
-      for (int i = 0; i < NR<T>; ++i) m[i] = jb + i * step < nc ? (part ? M2 : M) + jb + i * step : nullptr;
+    for (int i = 0; i < NR<T>; ++i) {
+      acc[i] = vzero(T(0));
+      m[i] = jb + i * step < nc ? M + jb + i * step : nullptr;
+    }
 #pragma unroll 4
-      for (int a = aBeg; a < aEnd; ++a) {
-        const typename Vec16<T>::type x = X[a * xs];
+    for (int a = 0; a < h; ++a) {
+      const typename Vec16<T>::type x = X[a * xs];
 #pragma unroll
-        for (int i = 0; i < NR<T>; ++i)
-          if (m[i]) vaxpy(acc[i], x, m[i][(size_t)(a - aBeg) * ld]);
-      }
+      for (int i = 0; i < NR<T>; ++i)
+        if (m[i]) vaxpy(acc[i], x, m[i][(size_t)a * ld]);
     }
 #pragma unroll
     for (int i = 0; i < NR<T>; ++i)
@@ -246,61 +243,61 @@ __device__ __forceinline__ void fgrp_k(const Pass<T>& p, const int* h0, const in
   }
 }
 
+// Backward; early: X^T y, kept in the place of x, then x = that - G^T x_R.
 template <class T>
 __device__ __forceinline__ void bgrp_k(const Pass<T>& p, const int* h0, const int* d, int cnt, const T* data,
-                                       typename Vec16<T>::type* buf) {
+                                       typename Vec16<T>::type* buf, bool early) {
   using Vt = typename Vec16<T>::type;
   const int lane = threadIdx.x & 31, warp = p.tid >> 5;
   const int rg = lane / p.cgN, nrg = 32 / p.cgN;
-  Vt* X = buf + warp * 128;   // 128 vectors: NR<T> rows a lane
+  Vt* xs = buf + warp * 128;   // 128 vectors: NR<T> rows a lane
   for (int q = warp; q < cnt; q += GW) {
     const int* h = h0 + GH * q;
-    const int n = h[0], m = h[1], c0 = h[2], ldk = h[7];
+    const int n = h[0], c0 = h[2], ldk = h[7], rows = early ? n : h[1];
+    const T* M = data + (early ? h[5] : h[4]);
     const int* rw = d + h[6];
-    // the thread's columns j = rg + i nrg: 32 columns in 1, 2 or 4 sweeps of them;
-    // rows a < m: -x_R with G's, then y with X's
-    const int tile = NR<T> * nrg;   // rows a tile
+    // the thread's columns j = rg + i nrg: 32 columns in 1, 2 or 4 sweeps of them
+    const int tile = NR<T> * nrg;   // rows of y or x_R a tile
     auto load = [&](int a) {
-      if (a >= m) return a < m + n ? p.ld(p.A->t, h[8] + a - m) : vzero(T(0));
-      Vt x = p.ld(p.A->w, rw[a]), v = vzero(T(0));
-      vsub(v, x);
-      return v;
+      return a >= rows ? vzero(T(0)) : early ? p.ld(p.A->t, h[8] + a) : p.ld(p.A->w, rw[a]);
     };
     for (int jb = 0; jb < n; jb += NR<T> * nrg) {
       Vt acc[NR<T>], nx[NR<T>];
-      int col[NR<T>];
+      const T* g[NR<T>];
 #pragma unroll
       for (int i = 0; i < NR<T>; ++i) {
         acc[i] = vzero(T(0));
-        col[i] = jb + rg + i * nrg < n ? jb + rg + i * nrg : -1;
+        g[i] = jb + rg + i * nrg < n ? M + jb + rg + i * nrg : nullptr;
         nx[i] = load(rg + i * nrg);
       }
-      for (int a0 = 0; a0 < m + n; a0 += tile) {
+      for (int a0 = 0; a0 < rows; a0 += tile) {
         __syncwarp();
 #pragma unroll
-        for (int i = 0; i < NR<T>; ++i) X[(rg + i * nrg) * p.cgN + p.cg] = nx[i];
+        for (int i = 0; i < NR<T>; ++i) xs[(rg + i * nrg) * p.cgN + p.cg] = nx[i];
         __syncwarp();
 #pragma unroll
         for (int i = 0; i < NR<T>; ++i) nx[i] = load(a0 + tile + rg + i * nrg);   // under this tile's products
-        const int an = min(tile, m + n - a0), gn = max(0, min(an, m - a0));
+        const int an = min(tile, rows - a0);
 #pragma unroll 4
-        for (int a = 0; a < gn; ++a) {
-          const Vt x = X[a * p.cgN + p.cg];
+        for (int a = 0; a < an; ++a) {
+          const Vt x = xs[a * p.cgN + p.cg];
 #pragma unroll
           for (int i = 0; i < NR<T>; ++i)
-            if (col[i] >= 0) vaxpy(acc[i], x, data[h[4] + (a0 + a) * ldk + col[i]]);
-        }
-#pragma unroll 4
-        for (int a = gn; a < an; ++a) {
-          const Vt x = X[a * p.cgN + p.cg];
-#pragma unroll
-          for (int i = 0; i < NR<T>; ++i)
-            if (col[i] >= 0) vaxpy(acc[i], x, data[h[5] + (a0 + a - m) * ldk + col[i]]);
+            if (g[i]) vaxpy(acc[i], x, g[i][(size_t)(a0 + a) * ldk]);
         }
       }
 #pragma unroll
-      for (int i = 0; i < NR<T>; ++i)
-        if (col[i] >= 0) p.st(p.A->w, c0 + col[i], acc[i]);
+      for (int i = 0; i < NR<T>; ++i) {
+        const int j = jb + rg + i * nrg;
+        if (j >= n) continue;
+        if (early) {
+          p.st(p.A->w, c0 + j, acc[i]);
+        } else {
+          Vt v = p.ld(p.A->w, c0 + j);
+          vsub(v, acc[i]);
+          p.st(p.A->w, c0 + j, v);
+        }
+      }
     }
   }
 }
@@ -519,11 +516,12 @@ __global__ void __launch_bounds__(NGRP * GT + 32, BATCH_BLOCKS) apply_batch_kern
     const int* d = it.descBytes ? reinterpret_cast<const int*>(st + ST_DATA) : A.blob + it.desc;
     const int* h = d + 2 * it.waits;
     const int* d2 = it.desc2Bytes ? reinterpret_cast<const int*>(st + ST_DATA + it.descBytes) : A.blob + it.desc2;
-    if (warp == 0) wait_list(d, it.waits, A.sync, err);
+    const int first = it.early ? it.early : it.waits;
+    if (warp == 0) wait_list(d, first, A.sync, err);
     cbar();
     const T* g0 = it.bytes0 ? data : reinterpret_cast<const T*>(it.g0);
     const T* g1 = it.bytes1 ? data + it.bytes0 / sizeof(T) : reinterpret_cast<const T*>(it.g1);
-    for (int col0 = colBeg; col0 < colEnd; col0 += KC) {
+    auto pass = [&](int col0) {
       Pass<T> p;
       p.A = &A;
       p.kp = kp;
@@ -535,33 +533,49 @@ __global__ void __launch_bounds__(NGRP * GT + 32, BATCH_BLOCKS) apply_batch_kern
       p.nrg = GT / p.cgN;
       p.col = col0 + p.cg * V;
       p.act = p.col < colEnd;
+      return p;
+    };
+    // a backward item's products with X, before the wait for its ancestors (2D 60 x 50
+    // FP64, 5 columns: 232 against 250 us; never slower)
+    if (it.early) {
+      for (int col0 = colBeg; col0 < colEnd; col0 += KC) {
+        const Pass<T> p = pass(col0);
+        if (kind == IT_BGRP) {
+          bgrp_k<T>(p, h, d, it.count, data, F, true);
+          continue;
+        }
+        if (col0 > colBeg) cbar();
+        for (int a = p.rg; a < h[10]; a += p.nrg) F[a * p.cgN + p.cg] = p.ld(A.t, h[9] + a);
+        cbar();
+        if (h[10] > 0)
+          cols_dot<T>(g1, h[7], h[10], h[0], F + p.cg, p.cgN, p.rg, p.nrg, [&](int j, Vt v) {
+            if (h[5] > 1) p.st(A.ip, h[3] + (long long)h[4] * h[8] + j, v);
+            else p.st(A.w, h[2] + j, v);
+          });
+      }
+      if (warp == 0) wait_list(d + 2 * first, it.waits - first, A.sync, err);
+      cbar();
+    }
+    for (int col0 = colBeg; col0 < colEnd; col0 += KC) {
+      const Pass<T> p = pass(col0);
       if (col0 > colBeg) cbar();   // the buffers of the last pass
       switch (kind) {
         case IT_FGRP: fgrp_k<T>(p, h, d, it.count, data, F); break;
-        case IT_BGRP: bgrp_k<T>(p, h, d, it.count, data, F); break;
+        case IT_BGRP: bgrp_k<T>(p, h, d, it.count, data, F, false); break;
         case IT_FWD: fwd_k<T>(p, h, d, d2, it.bytes0 + it.bytes1 > 0 ? data : g0, g1, it.bytes0 + it.bytes1 > 0, F); break;
-        case IT_BWD: {
-          const int n = h[0], rows = h[1], R = rows + h[10];
+        case IT_BWD: {   // less G^T x_R
+          const int rows = h[1];
+          if (rows == 0) break;
 #pragma unroll 2
-          for (int a = p.rg; a < R; a += p.nrg) {
-            Vt v;
-            if (a < rows) {
-              v = vzero(T(0));
-              vsub(v, p.ld(A.w, d[h[6] + a]));
-            } else {
-              v = p.ld(A.t, h[9] + a - rows);
-            }
-            F[a * p.cgN + p.cg] = v;
-          }
+          for (int a = p.rg; a < rows; a += p.nrg) F[a * p.cgN + p.cg] = p.ld(A.w, d[h[6] + a]);
           cbar();
-          const bool staged = it.bytes0 + it.bytes1 > 0;   // (the rows of X behind those of G)
-          cols_dot<T>(
-              staged ? data : g0, h[7], R, n, F + p.cg, p.cgN, p.rg, p.nrg,
-              [&](int j, Vt v) {
-                if (h[5] > 1) p.st(A.ip, h[3] + (long long)h[4] * h[8] + j, v);
-                else p.st(A.w, h[2] + j, v);
-              },
-              staged ? nullptr : g1, rows);
+          cols_dot<T>(g0, h[7], rows, h[0], F + p.cg, p.cgN, p.rg, p.nrg, [&](int j, Vt v) {
+            T* const to = h[5] > 1 ? A.ip : A.w;
+            const long long at = h[5] > 1 ? h[3] + (long long)h[4] * h[8] + j : h[2] + j;
+            Vt x = h[10] > 0 ? p.ld(to, at) : vzero(T(0));
+            vsub(x, v);
+            p.st(to, at, x);
+          });
           break;
         }
         case IT_BR: {
