@@ -84,9 +84,9 @@ __device__ __forceinline__ void vshfl_add(double2& v, int o) {
 // lie off that chain and fill its gaps.  Measured, one
 // application (before: a triangular solve per supernode on the chain, two
 // ticketed launches for the interior and eight launches per compressed level):
-// 3D 64^3 FP32 0.914 -> 0.394 ms (616 MB, 0.091 ms at the copy rate), 3D 96^3
-// FP32 2.23 -> 1.21 ms, 2D 193 x 187 FP64 0.632 -> 0.184 ms, 2D 40 x 37 FP64
-// 0.159 -> 0.081 ms.  Two groups of four warps against one of eight (half the
+// 3D 64^3 FP32 0.914 -> 0.397 ms (616 MB, 0.091 ms at the copy rate), 3D 96^3
+// FP32 2.23 -> 1.21 ms, 2D 193 x 187 FP64 0.632 -> 0.178 ms, 2D 40 x 37 FP64
+// 0.159 -> 0.077 ms.  Two groups of four warps against one of eight (half the
 // items in work at once): 3D 64^3 0.400 against 0.494 ms.
 
 constexpr int ST_DATA = 16384, ST_DESC = 3584, ST_BYTES = ST_DATA + ST_DESC;

@@ -20,8 +20,8 @@
 // substitutions do; S = (L11 L11^T)^{-1}, one product instead of two, leaves the
 // block's condition number in them (dense block of 100, condition 1e10, b = A x of a
 // random x, FP64: |b - A x| / |A| |x| 6.9e-9 with S, 3.2e-16 with X, 1.7e-16 by
-// substitution), and is 8 - 10 % quicker where an application is all latency (2D
-// 40 x 37 FP64 91 against 100 us, 193 x 187 171 against 189).
+// substitution), and is some 8 % quicker where an application is all latency (2D
+// 40 x 37 FP64 91 against 100 us, 193 x 187 171 against 189, in groups of eight).
 // X by inverted 64 x 64 diagonal blocks and recursive doubling X_BA = -X_BB
 // L_BA X_AA with batched GEMMs; W, and G above 64 columns, by batched GEMMs; G of
 // the small supernodes by one kernel.

@@ -17,9 +17,9 @@
 // dependent loads whatever its bytes), FP64 its 1/64 rate.  Measured, one
 // application against the earlier kernels (a triangular solve with a thread per
 // (row, column) pair, six launches per compressed level): 2D 1024^2 FP32 k = 64
-// 10.50 -> 6.5 ms, k = 8 3.62 -> 0.97 ms; 3D 40^3 FP32 k = 32 1.99 -> 0.70 ms,
-// k = 8 1.81 -> 0.46 ms; 3D 64^3 FP32 k = 8 2.44 -> 0.95 ms; 3D 44x40x47 FP64
-// k = 8 2.78 -> 1.60 ms.
+// 10.50 -> 6.5 ms, k = 8 3.62 -> 0.97 ms; 3D 40^3 FP32 k = 32 1.99 -> 0.69 ms,
+// k = 8 1.81 -> 0.46 ms; 3D 64^3 FP32 k = 8 2.44 -> 0.97 ms; 3D 44x40x47 FP64
+// k = 8 2.78 -> 1.52 ms.
 #include <algorithm>
 #include <mutex>
 #include <stdexcept>
